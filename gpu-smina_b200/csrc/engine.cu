@@ -183,7 +183,8 @@ void refresh_header(sg_engine* e, RecState& r) {
     h.pop_start = r.pop_start.as<int>();
     h.pop_atoms = r.pop_atoms.as<int>();
     h.full_start = r.full_start.as<int>();
-    h.full_atoms = r.full_atoms.as<int>();
+    h.full_list = r.full_list.as<CellAtom>();
+    h.full_charge = r.full_charge.as<double>();
     h.g = r.geom;
     for (int t = 0; t < kNumTypes; t++) {
         h.map[t] = r.map64[t].as<double>();
@@ -199,8 +200,8 @@ void refresh_header(sg_engine* e, RecState& r) {
     cuda_check(cudaStreamSynchronize(e->stream), "receptor header");
 }
 
-// build one family of cell lists (CSR) on the device
-static void build_cells(sg_engine* e, RecState& r, const std::vector<double>& lo, const std::vector<double>& hi,
+// build one family of cell lists (CSR) on the device; returns the lists' length
+static int build_cells(sg_engine* e, RecState& r, const std::vector<double>& lo, const std::vector<double>& hi,
                         DevBuf& start, DevBuf& atoms) {
     const DGeom& g = r.geom;
     const int ncells = g.cell_dim[0] * g.cell_dim[1] * g.cell_dim[2];
@@ -222,6 +223,7 @@ static void build_cells(sg_engine* e, RecState& r, const std::vector<double>& lo
                                  e->stream),
                "cell fill");
     cuda_check(cudaStreamSynchronize(e->stream), "cell fill");
+    return st[ncells];
 }
 
 // Brick of every cell along each axis.  Populate: the first grid point of
@@ -253,15 +255,23 @@ static void cell_bricks(const DGeom& g, bool first_query, std::vector<double>& l
 }
 
 // the receptor's 3 A cell lists (first-query bricks for the maps, full
-// bricks for the direct sum), built once
-void ensure_cells(sg_engine* e, RecState& r) {
-    if (r.pop_start.p) return;
+// bricks with whole atoms for the direct sum)
+static void build_receptor_cells(sg_engine* e, RecState& r) {
     std::vector<double> lo, hi;
     cell_bricks(r.geom, true, lo, hi);
     build_cells(e, r, lo, hi, r.pop_start, r.pop_atoms);
     cell_bricks(r.geom, false, lo, hi);
-    build_cells(e, r, lo, hi, r.full_start, r.full_atoms);
+    DevBuf full_atoms;
+    const int n = build_cells(e, r, lo, hi, r.full_start, full_atoms);
+    r.full_list.alloc(std::max(1, n) * sizeof(CellAtom));
+    r.full_charge.alloc(std::max(1, n) * sizeof(double));
+    cuda_check(launch_cell_pack(n, full_atoms.as<int>(), r.xyz.as<double>(), r.type.as<int>(), r.charge.as<double>(),
+                                r.full_list.as<CellAtom>(), r.full_charge.as<double>(), e->stream),
+               "cell atoms");
     refresh_header(e, r);
+}
+void ensure_cells(sg_engine* e, RecState& r) {
+    if (!r.pop_start.p) build_receptor_cells(e, r);
 }
 
 void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
@@ -334,7 +344,8 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
                                                            std::isfinite(r->coords[3 * i + 2]), "receptor: non-finite coordinate");
         RecState& s = e->rec[rid];
         s.clear_maps();
-        s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset(); s.full_atoms.reset();
+        s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset();
+        s.full_list.reset(); s.full_charge.reset();
         s.ugrid.reset();  // a new receptor starts without a user grid
         s.ug = DGeom{};
         s.gd = *gd;
@@ -346,12 +357,7 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
         s.type.upload(types.data(), sizeof(int) * std::max<size_t>(1, types.size()), e->stream);
         s.charge.upload(r->charge, sizeof(double) * std::max(1, r->num_atoms), e->stream);
         s.set = true;
-        std::vector<double> lo, hi;
-        cell_bricks(s.geom, true, lo, hi);
-        build_cells(e, s, lo, hi, s.pop_start, s.pop_atoms);
-        cell_bricks(s.geom, false, lo, hi);
-        build_cells(e, s, lo, hi, s.full_start, s.full_atoms);
-        refresh_header(e, s);
+        build_receptor_cells(e, s);
     });
 }
 
@@ -402,7 +408,8 @@ int sg_drop_receptor(sg_engine* e, int rid) {
         require(rid >= 0 && rid < SG_MAX_RECEPTORS, "receptor id out of range");
         RecState& s = e->rec[rid];
         s.clear_maps();
-        s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset(); s.full_atoms.reset();
+        s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset();
+        s.full_list.reset(); s.full_charge.reset();
         s.xyz.reset(); s.type.reset(); s.charge.reset(); s.dhdr.reset(); s.ugrid.reset();
         s.set = false;
     });
@@ -674,7 +681,7 @@ void pack_models(sg_engine* e, const sg_model_desc* models, int nmodels, PackedM
     const int* ib = out.ints.as<int>();
     const double* db = out.dbls.as<double>();
     const float* fb = out.flts.as<float>();
-    out.max_ws64 = 0;
+    out.smem64 = Smem64{};
     for (int k = 0; k < nmodels; k++) {
         DModel& h = out.host[k];
         const std::vector<size_t>& io = ioffs[k];
@@ -699,7 +706,7 @@ void pack_models(sg_engine* e, const sg_model_desc* models, int nmodels, PackedM
         int q = 0;
         h.charge = db + dd[q++]; h.local = db + dd[q++]; h.lab = db + dd[q++];
         h.forigin = db + dd[q++]; h.faxis = db + dd[q++]; h.finit = db + dd[q++];
-        out.max_ws64 = std::max(out.max_ws64, ws64_bytes(h));
+        out.smem64.add(h);
         out.max_conf = std::max(out.max_conf, h.conf_size);
         out.max_dof = std::max(out.max_dof, h.dof);
         out.max_heavy = std::max(out.max_heavy, h.nheavy);
@@ -769,6 +776,12 @@ void ensure_model_maps(sg_engine* e, RecState& r, const PackedModels& pm, const 
 
 }  // namespace sg
 
+Shape64 sg::plain_shape(sg_engine* e, const PackedModels& pm, long long items) {
+    const Shape64 sh = shape64(pm.smem64, items, e->num_sms, (size_t)e->max_smem);
+    require(sh.smem <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+    return sh;
+}
+
 // device buffer that receives results and is copied back
 template <typename T>
 struct Staged {
@@ -800,7 +813,7 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
         pack_models(e, m, 1, pm);
         if (!direct) ensure_model_maps(e, r, pm, m, 1);
         else ensure_cells(e, r);
-        require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+        const Shape64 sh = plain_shape(e, pm, nconfs);
         const DModel& h = pm.host[0];
         Staged<double> dc, de, dg, dx;
         dc.make((size_t)nconfs * h.conf_size, e->stream, confs);
@@ -823,7 +836,7 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
             e->check_device_errors();
             return;
         }
-        cuda_check(launch_eval64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
+        cuda_check(launch_eval64(pm.dmodels.as<DModel>(), sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
                                  slope, direct, de.p(), dg.p(), out_coords ? dx.p() : nullptr, e->d_err.as<int>(), e->stream),
                    "eval launch");
         de.fetch(out_e, e->stream);
@@ -880,8 +893,8 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
             e->check_device_errors();
             return;
         }
-        require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
-        cuda_check(launch_bfgs64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
+        const Shape64 sh = plain_shape(e, pm, nconfs);
+        cuda_check(launch_bfgs64(pm.dmodels.as<DModel>(), sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
                                  slope, maxiters, accurate_line, early_term, de.p(), e->d_err.as<int>(), e->stream),
                    "bfgs launch");
         dc.fetch(confs, e->stream);
@@ -900,7 +913,7 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
         PackedModels pm;
         pack_models(e, models, nmodels, pm);
         ensure_model_maps(e, r, pm, models, nmodels);
-        require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+        const Shape64 sh = plain_shape(e, pm, nchains);
         const int S = p->num_saved_mins;
         // per-chain inputs and result storage (one device allocation each)
         std::vector<double> conf0;
@@ -980,7 +993,7 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
         P.accurate_line = p->accurate_line;
         P.early_term = p->early_term;
         P.slope = p->cache_slope;
-        cuda_check(launch_mc64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(),
+        cuda_check(launch_mc64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(),
                                d_chains.as<Chain64>(), nchains, P, nhist > 0, e->d_err.as<int>(), e->stream),
                    "dock launch");
         std::vector<double> he((size_t)nchains * S), hconf(nconf_res), hxyz(nxyz_res);
@@ -1020,7 +1033,7 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
         ensure_cells(e, r);
         PackedModels pm;
         pack_models(e, models, nmodels, pm);
-        require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+        const Shape64 sh = plain_shape(e, pm, nposes);
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "refine: bad pose model");
         const int cs = pm.max_conf, hs = pm.max_heavy;
         Staged<double> dc, de, dx;
@@ -1030,7 +1043,7 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
         dx.make((size_t)nposes * hs * 3, e->stream);
         dx.zero(e->stream);  // atoms past a pose's heavy count stay 0
         dpm.make(nposes, e->stream, pose_model);
-        cuda_check(launch_refine64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(), dpm.p(), nposes,
+        cuda_check(launch_refine64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(), nposes,
                                    dc.p(), cs, cap, maxiters, nullptr, nullptr, accurate_line, early_term, de.p(), dx.p(), hs,
                                    e->d_err.as<int>(), e->stream),
                    "refine launch");
@@ -1075,7 +1088,7 @@ int sg_score(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, co
         ensure_cells(e, r);
         PackedModels pm;
         pack_models(e, models, nmodels, pm);
-        require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+        const Shape64 sh = plain_shape(e, pm, nposes);
         require(conf_stride >= pm.max_conf && (!out_coords || coord_stride >= pm.max_heavy), "score: strides too small");
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "score: bad pose model");
         Staged<double> dc, de, di, dx;
@@ -1088,7 +1101,7 @@ int sg_score(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, co
             dx.zero(e->stream);  // atoms past a pose's heavy count stay 0
         }
         dpm.make(nposes, e->stream, pose_model);
-        cuda_check(launch_score64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
+        cuda_check(launch_score64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
                                   nposes, dc.p(), conf_stride, v, slope, de.p(), di.p(), out_coords ? dx.p() : nullptr,
                                   coord_stride, e->d_err.as<int>(), e->stream),
                    "score launch");
@@ -1108,7 +1121,7 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
         ensure_cells(e, r);
         PackedModels pm;
         pack_models(e, models, nmodels, pm);
-        require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+        const Shape64 sh = plain_shape(e, pm, nposes);
         require(conf_stride >= pm.max_conf && coord_stride >= pm.max_heavy, "minimize: strides too small");
         for (int k = 0; k < nposes; k++) {
             require(pose_model[k] >= 0 && pose_model[k] < nmodels && maxiters[k] >= 0, "minimize: bad pose");
@@ -1127,7 +1140,7 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
         dpm.make(nposes, e->stream, pose_model);
         dmi.make(nposes, e->stream, maxiters);
         if (boxes) db.make((size_t)nposes * 6, e->stream, boxes);
-        cuda_check(launch_refine64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
+        cuda_check(launch_refine64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
                                    nposes, dc.p(), conf_stride, cap, 0, dmi.p(), boxes ? db.p() : nullptr,
                                    accurate_line, early_term, de.p(), dx.p(), coord_stride, e->d_err.as<int>(),
                                    e->stream),

@@ -42,7 +42,7 @@ struct RecState {
     sg_grid_dims gd{};
     DGeom geom{};
     int natoms = 0;
-    DevBuf xyz, type, charge, pop_start, pop_atoms, full_start, full_atoms;
+    DevBuf xyz, type, charge, pop_start, pop_atoms, full_start, full_list, full_charge;
     DevBuf map64[kNumTypes], cmap64[kNumTypes], map32[kNumTypes], cmap32[kNumTypes], map16[kNumTypes];
     bool built[kNumTypes] = {};
     DevBuf ugrid;  // user grid values, or empty
@@ -68,7 +68,7 @@ struct RecState {
 struct PackedModels {
     std::vector<DModel> host;  // host copies with device pointers
     DevBuf ints, dbls, flts, dmodels;
-    size_t max_ws64 = 0;
+    Smem64 smem64;  // plain-path shared memory
     int max_conf = 0, max_dof = 0, max_heavy = 0, max_atoms = 0, max_pairs = 0, max_frames = 0;
 };
 
@@ -127,17 +127,21 @@ cudaError_t launch_grid_map64(const DGeom&, int, const double*, const int*, cons
                               const DTables&, const int*, int, double**, double**, const double* ugrid,
                               const DGeom& ug, double ug_slope, cudaStream_t);
 cudaError_t launch_grid_pack(const DGeom&, const double*, float4*, uint4*, cudaStream_t);
-size_t ws64_bytes(const DModel& hm);
-cudaError_t launch_eval64(const DModel*, size_t, const DTables&, const DReceptor*, int, const double*, const double[3],
-                          double, int, double*, double*, double*, int*, cudaStream_t);
-cudaError_t launch_bfgs64(const DModel*, size_t, const DTables&, const DReceptor*, int, double*, const double[3], double,
-                          int, int, int, double*, int*, cudaStream_t);
-cudaError_t launch_mc64(const DModel*, size_t, const DTables&, const DReceptor*, const Chain64*, int,
+cudaError_t launch_cell_pack(int n, const int* atoms, const double* xyz, const int* type, const double* charge,
+                             CellAtom* list, double* list_charge, cudaStream_t s);
+// warps per item and shared memory of a plain-path launch over `items` items
+// within max_smem bytes per block
+Shape64 shape64(const Smem64& s, long long items, int num_sms, size_t max_smem);
+cudaError_t launch_eval64(const DModel*, const Shape64&, int num_sms, const DTables&, const DReceptor*, int,
+                          const double*, const double[3], double, int, double*, double*, double*, int*, cudaStream_t);
+cudaError_t launch_bfgs64(const DModel*, const Shape64&, int num_sms, const DTables&, const DReceptor*, int, double*,
+                          const double[3], double, int, int, int, double*, int*, cudaStream_t);
+cudaError_t launch_mc64(const DModel*, const Shape64&, const DTables&, const DReceptor*, const Chain64*, int,
                         const MCParams64&, bool visited, int*, cudaStream_t);
-cudaError_t launch_score64(const DModel* dms, size_t smem, const DTables& T, const DReceptor* R, const int* pose_model,
+cudaError_t launch_score64(const DModel* dms, const Shape64&, const DTables& T, const DReceptor* R, const int* pose_model,
                            int n, const double* confs, int conf_stride, const double v[3], double slope, double* e,
                            double* intra, double* coords, int coord_stride, int* err, cudaStream_t s);
-cudaError_t launch_refine64(const DModel*, size_t, const DTables&, const DReceptor*, const int*, int, double*, int,
+cudaError_t launch_refine64(const DModel*, const Shape64&, const DTables&, const DReceptor*, const int*, int, double*, int,
                             const double[3], int, const int* pose_maxiters, const double* pose_box, int, int, double*,
                             double*, int, int*, cudaStream_t);
 size_t ws32_bytes(const DModel& hm);
@@ -166,6 +170,8 @@ cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, const DTables3
 DTables32 tables32(const sg_engine* e);
 DMaps32 maps32(const sg_engine* e, const RecState& r);
 void pack_models(sg_engine* e, const sg_model_desc* models, int nmodels, PackedModels& out);
+// the plain-path launch of a batch of models; refuses a model that does not fit
+Shape64 plain_shape(sg_engine* e, const PackedModels& pm, long long items);
 struct ModelImage {
     std::vector<char> bytes;   // pools then descriptors, ready to copy to the device
     size_t dmodel_off = 0;     // byte offset of the descriptor array

@@ -397,7 +397,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
             int nposes = 0;
             for (auto& v : merged) nposes += (int)v.size();
             if (nposes > 0) {
-                require(pm.max_ws64 <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
+                const Shape64 sh = plain_shape(e, pm, nposes);
                 const int cs = pm.max_conf, hs = std::max(1, pm.max_heavy);
                 std::vector<double> confs((size_t)nposes * cs, 0.0);
                 std::vector<int> pmodel(nposes), pmaxit(nposes);
@@ -417,7 +417,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 de.alloc((size_t)nposes * sizeof(double));
                 dx.alloc((size_t)nposes * hs * 3 * sizeof(double));
                 cuda_check(cudaEventRecord(ev[2], e->stream), "event");
-                cuda_check(launch_refine64(pm.dmodels.as<DModel>(), pm.max_ws64, e->tables, r.dhdr.as<DReceptor>(),
+                cuda_check(launch_refine64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(),
                                            dpm.as<int>(), nposes, dc.as<double>(), cs, p->authentic_v, p->maxiters,
                                            dmi.as<int>(), nullptr, p->accurate_line, p->early_term, de.as<double>(),
                                            dx.as<double>(), hs, e->d_err.as<int>(), e->stream),

@@ -1,134 +1,200 @@
-// Plain (FP64) path kernels: one warp (one 32-thread block) per item.
-// Built with -fmad=false so that the arithmetic rounds exactly like the
-// CPU restatement compiled with -ffp-contract=off.
+// Plain (FP64) path kernels: one block of G warps per item (a conf, a pose or a
+// chain); the first warp runs the item and the others take parts of every
+// evaluation (dock64_eval.cuh).  Built with -fmad=false so that the arithmetic
+// rounds exactly like the CPU restatement compiled with -ffp-contract=off.
+#include <algorithm>
 #include "dock64_search.cuh"
 
 namespace sg {
 
-__device__ void init_ws64(W64& w, const DModel* m, const DTables* T, const DReceptor* R, int* err) {
-    extern __shared__ double smem64[];
-    w.s = smem64;
-    w.m = m;
-    w.T = T;
-    w.R = R;
-    w.err = err;
-    w.lane = threadIdx.x & 31;
-    w.evals = 0;
-    w.box = nullptr;
-    w.L = ws64_layout(m->natoms, m->nframes, m->npairs, m->conf_size, m->dof);
-    w.pin = reinterpret_cast<uint8_t*>(w.s + w.L.pin);
-    w.mt = reinterpret_cast<uint32_t*>(w.s + w.L.mt);
-    // model state as read: coords and frame origins (mutation reads them)
-    for (int i = w.lane; i < 3 * m->natoms; i += 32) w.s[w.L.coords + i] = m->lab[i];
-    for (int i = w.lane; i < 3 * m->nframes; i += 32) {
-        w.s[w.L.origin + i] = m->finit[i];
-        w.s[w.L.axis + i] = m->faxis[i];
-    }
-    for (int f = w.lane; f < m->nframes; f += 32) {
-        double* q = w.s + w.L.q + 4 * f;
-        q[0] = 1; q[1] = 0; q[2] = 0; q[3] = 0;
-        quat_to_mat(Quat<double>{1, 0, 0, 0}, w.s + w.L.rot + 9 * f);
-    }
-    __syncwarp();
+// copies n elements behind the workspace
+template <int G, typename T>
+__device__ __forceinline__ void stage64(int at, const T* src, int n) {
+    T* d = reinterpret_cast<T*>(smem64 + at);
+    for (int i = threadIdx.x; i < n; i += 32 * G) d[i] = src[i];
 }
 
+// The block's header, staged arrays and model state as read (coords and frame
+// origins, which mutation reads before the first evaluation).  Every thread
+// takes part.
+template <int G, bool ST>
+__device__ __forceinline__ void init64(const DModel* gm, const DTables& T, const DReceptor* R, const double* box,
+                                       int* err) {
+    Hdr64& H = hd64();
+    static_assert(sizeof(DModel) % 16 == 0, "DModel is read in 16-byte pieces");
+    for (int k = threadIdx.x; k < (int)(sizeof(DModel) / 16); k += 32 * G)
+        reinterpret_cast<int4*>(&H.m)[k] = reinterpret_cast<const int4*>(gm)[k];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        H.T = T;
+        H.box = box;
+        H.err = err;
+        H.evals = 0;
+        H.L = ws64_layout(H.m.natoms, H.m.nframes, H.m.npairs, H.m.conf_size, H.m.dof, ST, H.m.nheavy, H.m.nlevels,
+                          H.m.nlig, H.m.nblocks, H.m.ntors);
+        H.R = ST ? reinterpret_cast<const DReceptor*>(smem64 + H.L.s_receptor) : R;
+    }
+    __syncthreads();
+    const DModel& m = H.m;
+    const Ws64& L = H.L;
+    double* S = smem64;
+    if constexpr (ST) {
+        const int N = m.natoms, F = m.nframes;
+        static_assert(sizeof(DReceptor) % 8 == 0, "the receptor header is copied in 8-byte pieces");
+        stage64<G>(L.s_receptor, reinterpret_cast<const double*>(R), (int)(sizeof(DReceptor) / 8));
+        stage64<G>(L.s_type, m.type, N);
+        stage64<G>(L.s_atom_frame, m.atom_frame, N);
+        stage64<G>(L.s_csr_start, m.csr_start, m.nmov + 1);
+        stage64<G>(L.s_heavy, m.heavy, m.nheavy);
+        stage64<G>(L.s_fkind, m.fkind, F);
+        stage64<G>(L.s_fparent, m.fparent, F);
+        stage64<G>(L.s_fbegin, m.fbegin, F);
+        stage64<G>(L.s_fend, m.fend, F);
+        stage64<G>(L.s_fconf, m.fconf, F);
+        stage64<G>(L.s_fdof, m.fdof, F);
+        stage64<G>(L.s_level_start, m.level_start, m.nlevels + 1);
+        stage64<G>(L.s_level_frames, m.level_frames, F);
+        stage64<G>(L.s_child_start, m.child_start, F + 1);
+        stage64<G>(L.s_child_list, m.child_list, m.child_start[F]);
+        stage64<G>(L.s_lig_begin, m.lig_begin, m.nlig);
+        stage64<G>(L.s_lig_end, m.lig_end, m.nlig);
+        stage64<G>(L.s_lig_root, m.lig_root, m.nlig);
+        stage64<G>(L.s_lig_pair_end, m.lig_pair_end, m.nlig);
+        stage64<G>(L.s_blk_rigid, m.blk_rigid, m.nblocks);
+        stage64<G>(L.s_blk_conf, m.blk_conf, m.nblocks);
+        stage64<G>(L.s_blk_ntors, m.blk_ntors, m.nblocks);
+        stage64<G>(L.s_tor_conf, m.tor_conf, m.ntors);
+        stage64<G>(L.s_tor_dof, m.tor_dof, m.ntors);
+        stage64<G>(L.s_charge, m.charge, N);
+        stage64<G>(L.s_local, m.local, 3 * N);
+        stage64<G>(L.s_forigin, m.forigin, 3 * F);
+        stage64<G>(L.s_faxis, m.faxis, 3 * F);
+    }
+    for (int i = threadIdx.x; i < 3 * m.natoms; i += 32 * G) S[L.coords + i] = m.lab[i];
+    for (int i = threadIdx.x; i < 3 * m.nframes; i += 32 * G) {
+        S[L.origin + i] = m.finit[i];
+        S[L.axis + i] = m.faxis[i];
+    }
+    for (int f = threadIdx.x; f < m.nframes; f += 32 * G) {
+        double* q = S + L.q + 4 * f;
+        q[0] = 1; q[1] = 0; q[2] = 0; q[3] = 0;
+        quat_to_mat(Quat<double>{1, 0, 0, 0}, S + L.rot + 9 * f);
+    }
+    __syncthreads();
+}
+
+// 128 registers a thread: four resident 4-warp blocks or two 8-warp blocks per SM
+#define SG_BOUNDS64 __launch_bounds__(32 * G, G == 1 ? 16 : 16 / G)
+
 // model::eval_deriv for a batch of confs of one model
-__global__ void __launch_bounds__(32) k_eval64(const DModel* model, DTables T, const DReceptor* R, int nconfs,
-                                               const double* confs, double v0, double v1, double v2, double slope,
-                                               int direct, double* out_e, double* out_g, double* out_coords, int* err) {
-    W64 w;
-    init_ws64(w, model, &T, R, err);
-    const int k = blockIdx.x;
-    if (k >= nconfs) return;
-    const DModel& m = *model;
-    double* x = w.s + w.L.x_tmp;
-    vcopy(w, x, confs + (size_t)k * m.conf_size, m.conf_size);
-    EvalMode em{{v0, v1, v2}, slope, direct != 0};
-    double* g = w.s + w.L.g;
-    const double e = feval(w, x, g, em);
-    if (w.lane == 0) out_e[k] = e;
-    for (int i = w.lane; i < m.dof; i += 32) out_g[(size_t)k * m.dof + i] = g[i];
-    if (out_coords)
-        for (int i = w.lane; i < 3 * m.nmov; i += 32) out_coords[(size_t)k * 3 * m.nmov + i] = w.s[w.L.coords + i];
+template <int G, bool ST>
+__global__ void SG_BOUNDS64 k_eval64(const DModel* model, const __grid_constant__ DTables T, const DReceptor* R,
+                                     int nconfs, const double* confs, double v0, double v1, double v2, double slope,
+                                     int direct, double* out_e, double* out_g, double* out_coords, int* err) {
+    init64<G, ST>(model, T, R, nullptr, err);
+    if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
+    const Hdr64& H = hd64();
+    const Ws64& L = H.L;
+    const int cs = H.m.conf_size, dof = H.m.dof, nmov = H.m.nmov, lane = lane64();
+    double *x = smem64 + L.x_tmp, *g = smem64 + L.g;
+    const EvalMode em{{v0, v1, v2}, slope, direct != 0};
+    for (int k = blockIdx.x; k < nconfs; k += gridDim.x) {
+        vcopy(x, confs + (size_t)k * cs, cs);
+        const double e = feval<G, ST>(x, g, em);
+        if (lane == 0) out_e[k] = e;
+        for (int i = lane; i < dof; i += 32) out_g[(size_t)k * dof + i] = g[i];
+        if (out_coords)
+            for (int i = lane; i < 3 * nmov; i += 32) out_coords[(size_t)k * 3 * nmov + i] = smem64[L.coords + i];
+        __syncwarp();
+    }
+    release64<G>();
 }
 
 // quasi_newton on the grid maps for a batch of confs (confs updated in place)
-__global__ void __launch_bounds__(32) k_bfgs64(const DModel* model, DTables T, const DReceptor* R, int nconfs,
-                                               double* confs, double v0, double v1, double v2, double slope,
-                                               int maxiters, int accurate, int early, double* out_e, int* err) {
-    W64 w;
-    init_ws64(w, model, &T, R, err);
-    const int k = blockIdx.x;
-    if (k >= nconfs) return;
-    const DModel& m = *model;
-    double* x = w.s + w.L.x_tmp;
-    vcopy(w, x, confs + (size_t)k * m.conf_size, m.conf_size);
-    EvalMode em{{v0, v1, v2}, slope, false};
-    const double e = bfgs64(w, x, maxiters, accurate, early, em);
-    if (w.lane == 0) out_e[k] = e;
-    for (int i = w.lane; i < m.conf_size; i += 32) confs[(size_t)k * m.conf_size + i] = x[i];
+template <int G, bool ST>
+__global__ void SG_BOUNDS64 k_bfgs64(const DModel* model, const __grid_constant__ DTables T, const DReceptor* R,
+                                     int nconfs, double* confs, double v0, double v1, double v2, double slope,
+                                     int maxiters, int accurate, int early, double* out_e, int* err) {
+    init64<G, ST>(model, T, R, nullptr, err);
+    if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
+    const int cs = hd64().m.conf_size, lane = lane64();
+    double* x = smem64 + hd64().L.x_tmp;
+    const EvalMode em{{v0, v1, v2}, slope, false};
+    for (int k = blockIdx.x; k < nconfs; k += gridDim.x) {
+        vcopy(x, confs + (size_t)k * cs, cs);
+        const double e = bfgs64<G, ST>(x, maxiters, accurate, early, em);
+        if (lane == 0) out_e[k] = e;
+        for (int i = lane; i < cs; i += 32) confs[(size_t)k * cs + i] = x[i];
+        __syncwarp();
+    }
+    release64<G>();
 }
 
 // monte_carlo::operator() for one chain per block
 // VIS: chains may carry a QuickVina 2 history (a separate instantiation, so
 // smina's own search compiles exactly as without it)
-template <bool VIS>
-__global__ void __launch_bounds__(32) k_mc64(const DModel* models, DTables T, const DReceptor* R,
-                                             const Chain64* chains, int nchains, MCParams64 P, int* err) {
+template <int G, bool ST, bool VIS>
+__global__ void SG_BOUNDS64 k_mc64(const DModel* models, const __grid_constant__ DTables T, const DReceptor* R,
+                                   const Chain64* chains, int nchains, const __grid_constant__ MCParams64 P,
+                                   int* err) {
     const int c = blockIdx.x;
     if (c >= nchains) return;
     const Chain64 ch = chains[c];
-    const DModel* mp = models + ch.model;
-    W64 w;
-    init_ws64(w, mp, &T, R, err);
-    const DModel& m = *mp;
-    for (int i = w.lane; i < 625; i += 32) w.mt[i] = ch.mt[i];
-    double* tmp = w.s + w.L.x_tmp;
-    double* cand = w.s + w.L.x_cand;
-    vcopy(w, tmp, ch.conf0, m.conf_size);
-    if (w.lane == 0) *ch.out_count = 0;
+    init64<G, ST>(models + ch.model, T, R, nullptr, err);
+    if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
+    const Hdr64& H = hd64();
+    const int cs = H.m.conf_size, lane = lane64();
+    uint32_t* mt = mt64();
+    for (int i = lane; i < 625; i += 32) mt[i] = ch.mt[i];
+    double *tmp = smem64 + H.L.x_tmp, *cand = smem64 + H.L.x_cand;
+    vcopy(tmp, ch.conf0, cs);
+    if (lane == 0) *ch.out_count = 0;
     __syncwarp();
     const EvalMode hunt{{P.hunt[0], P.hunt[1], P.hunt[2]}, P.slope, false};
     const EvalMode auth{{P.auth[0], P.auth[1], P.auth[2]}, P.slope, false};
     Hist64 hist_store{};
     const Hist64* vis = nullptr;
-    if (VIS && ch.hist && m.dof <= kHistMaxN) {
-        hist_store = hist64_view(ch.hist, ch.hist_words, m.dof);
+    if (VIS && ch.hist && H.m.dof <= kHistMaxN) {
+        hist_store = hist64_view(ch.hist, ch.hist_words, H.m.dof);
         vis = &hist_store;
     }
     double tmp_e = 0, best_e = kMaxFl;
     for (unsigned step = 0; step < ch.steps; step++) {
-        vcopy(w, cand, tmp, m.conf_size);
-        mutate64(w, cand, P.amplitude);
-        const double cand_e = bfgs64(w, cand, ch.maxiters, P.accurate_line, P.early_term, hunt, vis);
-        if (step == 0 || metropolis64(w, tmp_e, cand_e, P.temperature)) {
-            vcopy(w, tmp, cand, m.conf_size);
+        vcopy(cand, tmp, cs);
+        mutate64<ST>(cand, P.amplitude);
+        const double cand_e = bfgs64<G, ST>(cand, ch.maxiters, P.accurate_line, P.early_term, hunt, vis);
+        if (step == 0 || metropolis64(tmp_e, cand_e, P.temperature)) {
+            vcopy(tmp, cand, cs);
             tmp_e = cand_e;
-            set_conf64(w, tmp);
+            set_conf64<ST>(tmp);
             const int count = *ch.out_count;
             if (tmp_e < best_e || count < P.num_saved) {
-                tmp_e = bfgs64(w, tmp, ch.maxiters, P.accurate_line, P.early_term, auth, vis);
-                set_conf64(w, tmp);
-                add_to_output64(w, ch, tmp, tmp_e, P.min_rmsd, P.num_saved);
+                tmp_e = bfgs64<G, ST>(tmp, ch.maxiters, P.accurate_line, P.early_term, auth, vis);
+                set_conf64<ST>(tmp);
+                add_to_output64<ST>(ch, tmp, tmp_e, P.min_rmsd, P.num_saved);
                 if (tmp_e < best_e) best_e = tmp_e;
             }
         }
     }
-    for (int i = w.lane; i < 625; i += 32) ch.mt[i] = w.mt[i];
-    if (w.lane == 0) *ch.evals = w.evals;
+    for (int i = lane; i < 625; i += 32) ch.mt[i] = mt[i];
+    if (lane == 0) *ch.evals = H.evals;
+    release64<G>();
 }
 
 // non_cache::within
-__device__ bool within64(W64& w, double margin) {
-    const DModel& m = *w.m;
-    const DGeom& G = w.R->g;
+template <bool ST>
+__device__ __forceinline__ bool within64(double margin) {
+    using M = MV64<ST>;
+    const Hdr64& H = hd64();
+    const DGeom& Gm = H.R->g;
+    const int* type = M::type();
     bool ok = true;
-    for (int i = w.lane; i < m.nmov; i += 32) {
-        if (is_h(m.type[i])) continue;
+    for (int i = lane64(); i < H.m.nmov; i += 32) {
+        if (is_h(type[i])) continue;
         for (int j = 0; j < 3; j++)
-            if (w.box || G.gd_n[j] > 0) {
-                const double c = w.s[w.L.coords + 3 * i + j];
-                const double lo = w.box ? w.box[j] : G.gd_begin[j], hi = w.box ? w.box[3 + j] : G.gd_end[j];
+            if (H.box || Gm.gd_n[j] > 0) {
+                const double c = smem64[H.L.coords + 3 * i + j];
+                const double lo = H.box ? H.box[j] : Gm.gd_begin[j], hi = H.box ? H.box[3 + j] : Gm.gd_end[j];
                 if (c < lo - margin || c > hi + margin) ok = false;
             }
     }
@@ -136,126 +202,168 @@ __device__ bool within64(W64& w, double margin) {
 }
 
 // refine_structure for one pose per block
-__global__ void __launch_bounds__(32) k_refine64(const DModel* models, DTables T, const DReceptor* R,
-                                                 const int* pose_model, int nposes, double* confs, int conf_stride,
-                                                 double c0, double c1, double c2, int maxiters, const int* pose_maxiters,
-                                                 const double* pose_box, int accurate, int early, double* out_e,
-                                                 double* out_coords, int coord_stride, int* err) {
+template <int G, bool ST>
+__global__ void SG_BOUNDS64 k_refine64(const DModel* models, const __grid_constant__ DTables T, const DReceptor* R,
+                                       const int* pose_model, int nposes, double* confs, int conf_stride, double c0,
+                                       double c1, double c2, int maxiters, const int* pose_maxiters,
+                                       const double* pose_box, int accurate, int early, double* out_e,
+                                       double* out_coords, int coord_stride, int* err) {
     const int k = blockIdx.x;
     if (k >= nposes) return;
-    const DModel* mp = models + pose_model[k];
-    W64 w;
-    init_ws64(w, mp, &T, R, err);
-    const DModel& m = *mp;
-    double* x = w.s + w.L.x_tmp;
-    vcopy(w, x, confs + (size_t)k * conf_stride, m.conf_size);
+    // the pose's own box, if it has one
+    init64<G, ST>(models + pose_model[k], T, R, pose_box ? pose_box + 6 * (size_t)k : nullptr, err);
+    if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
+    const Hdr64& H = hd64();
+    const int cs = H.m.conf_size, lane = lane64(), nheavy = H.m.nheavy;
+    double* x = smem64 + H.L.x_tmp;
+    vcopy(x, confs + (size_t)k * conf_stride, cs);
     if (pose_maxiters) maxiters = pose_maxiters[k];  // per-ligand iteration limit
-    if (pose_box) w.box = pose_box + 6 * (size_t)k;  // the pose's own box
     double slope = 10;
     double e = 0;
     for (int p = 0; p < 5; p++) {
         const EvalMode em{{c0, c1, c2}, slope, true};
-        e = bfgs64(w, x, maxiters, accurate, early, em);
-        set_conf64(w, x);
-        if (within64(w, 0.0001)) break;
+        e = bfgs64<G, ST>(x, maxiters, accurate, early, em);
+        set_conf64<ST>(x);
+        if (within64<ST>(0.0001)) break;
         slope *= 10;
     }
-    if (!within64(w, 0.0001)) e = kMaxFl;
-    if (w.lane == 0) out_e[k] = e;
-    for (int i = w.lane; i < m.conf_size; i += 32) confs[(size_t)k * conf_stride + i] = x[i];
-    if (out_coords)
-        for (int a = w.lane; a < m.nheavy; a += 32)
-            st3(out_coords + ((size_t)k * coord_stride + a) * 3, ld3(w.s + w.L.coords + 3 * m.heavy[a]));
+    if (!within64<ST>(0.0001)) e = kMaxFl;
+    if (lane == 0) out_e[k] = e;
+    for (int i = lane; i < cs; i += 32) confs[(size_t)k * conf_stride + i] = x[i];
+    if (out_coords) {
+        const int* heavy = MV64<ST>::heavy();
+        for (int a = lane; a < nheavy; a += 32)
+            st3(out_coords + ((size_t)k * coord_stride + a) * 3, ld3(smem64 + H.L.coords + 3 * heavy[a]));
+    }
+    release64<G>();
 }
 
 // Final rescoring (finish_docking, main.cpp:257-282): per pose, model::eval on
 // the direct receptor sum (model.cpp:938-967 with non_cache::eval) and
 // model::eval_intramolecular (model.cpp:1027-1079), both on the fast table,
 // plus the heavy-atom coordinates of the pose.
-__global__ void __launch_bounds__(32) k_score64(const DModel* models, DTables T, const DReceptor* R,
-                                                const int* pose_model, int n, const double* confs, int conf_stride,
-                                                double v0, double v1, double v2, double slope, double* out_e,
-                                                double* out_intra, double* out_coords, int coord_stride, int* err) {
+template <int G, bool ST>
+__global__ void SG_BOUNDS64 k_score64(const DModel* models, const __grid_constant__ DTables T, const DReceptor* R,
+                                      const int* pose_model, int n, const double* confs, int conf_stride, double v0,
+                                      double v1, double v2, double slope, double* out_e, double* out_intra,
+                                      double* out_coords, int coord_stride, int* err) {
     const int k = blockIdx.x;
     if (k >= n) return;
-    W64 w;
-    init_ws64(w, models + pose_model[k], &T, R, err);
-    const DModel& m = *w.m;
-    double* x = w.s + w.L.x_tmp;
-    vcopy(w, x, confs + (size_t)k * conf_stride, m.conf_size);
+    init64<G, ST>(models + pose_model[k], T, R, nullptr, err);
+    if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
+    const Hdr64& H = hd64();
+    const int lane = lane64(), nheavy = H.m.nheavy;
+    double* x = smem64 + H.L.x_tmp;
+    vcopy(x, confs + (size_t)k * conf_stride, H.m.conf_size);
     const double v[3] = {v0, v1, v2};
-    set_conf64(w, x);
-    direct_energy64(w, v[1], slope);
-    pairs_energy64(w, v);
-    __syncwarp();
-    const double e = energy64(w);
-    const double intra = intramolecular64(w, v);
-    if (w.lane == 0) {
+    set_frames64<ST>(x);
+    command64<G>(kOpScore, v, slope, 1, 0);
+    score_warp64<G, ST>(0);
+    release64<G>();
+    const double e = energy64<ST>();
+    const double intra = intramolecular64<ST>(v);
+    if (lane == 0) {
         out_e[k] = e;
         out_intra[k] = intra;
     }
-    if (out_coords)
-        for (int a = w.lane; a < m.nheavy; a += 32)
-            st3(out_coords + ((size_t)k * coord_stride + a) * 3, ld3(w.s + w.L.coords + 3 * m.heavy[a]));
+    if (out_coords) {
+        const int* heavy = MV64<ST>::heavy();
+        for (int a = lane; a < nheavy; a += 32)
+            st3(out_coords + ((size_t)k * coord_stride + a) * 3, ld3(smem64 + H.L.coords + 3 * heavy[a]));
+    }
 }
 
 // ---- host launchers -------------------------------------------------------------------------
-size_t ws64_bytes(const DModel& hm) {
-    return (size_t)ws64_layout(hm.natoms, hm.nframes, hm.npairs, hm.conf_size, hm.dof).total * sizeof(double);
+void Smem64::add(const DModel& h) {
+    auto bytes = [&](bool st) {
+        return (size_t)ws64_layout(h.natoms, h.nframes, h.npairs, h.conf_size, h.dof, st, h.nheavy, h.nlevels, h.nlig,
+                                   h.nblocks, h.ntors).total * sizeof(double);
+    };
+    plain = std::max(plain, bytes(false));
+    staged = std::max(staged, bytes(true));
 }
 
-static cudaError_t prep(const void* fn, size_t smem) {
-    if (smem > 48 * 1024) return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return cudaSuccess;
+// Warps per item: 8 while that leaves every item an SM half to itself, 4 for
+// more items (more blocks resident, and the leaders' serial parts are what then
+// fills the SM), 1 with nothing staged for models that only fit so.
+Shape64 shape64(const Smem64& s, long long items, int num_sms, size_t max_smem) {
+    const size_t xb = kXbuf64 * sizeof(double);
+    if (items <= 2LL * num_sms && s.staged + 8 * xb <= max_smem) return {8, s.staged + 8 * xb};
+    if (s.staged + 4 * xb <= max_smem) return {4, s.staged + 4 * xb};
+    return {1, s.plain};
 }
 
-cudaError_t launch_eval64(const DModel* dm, size_t smem, const DTables& T, const DReceptor* R, int n, const double* confs,
-                          const double v[3], double slope, int direct, double* e, double* g, double* coords, int* err,
-                          cudaStream_t s) {
-    cudaError_t rc = prep((const void*)k_eval64, smem);
-    if (rc != cudaSuccess) return rc;
-    k_eval64<<<n, 32, smem, s>>>(dm, T, R, n, confs, v[0], v[1], v[2], slope, direct, e, g, coords, err);
-    return cudaGetLastError();
+// Raises the kernel's dynamic shared memory limit to `smem` (never lowers it:
+// another thread's launch may be sized against the higher one).
+static cudaError_t prep64(const void* fn, size_t smem) {
+    if (smem <= 48 * 1024) return cudaSuccess;
+    cudaFuncAttributes fa{};
+    cudaError_t rc = cudaFuncGetAttributes(&fa, fn);
+    if (rc != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= smem) return rc;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-cudaError_t launch_bfgs64(const DModel* dm, size_t smem, const DTables& T, const DReceptor* R, int n, double* confs,
-                          const double v[3], double slope, int maxiters, int accurate, int early, double* e, int* err,
-                          cudaStream_t s) {
-    cudaError_t rc = prep((const void*)k_bfgs64, smem);
-    if (rc != cudaSuccess) return rc;
-    k_bfgs64<<<n, 32, smem, s>>>(dm, T, R, n, confs, v[0], v[1], v[2], slope, maxiters, accurate, early, e, err);
-    return cudaGetLastError();
+// launches kernel<G, ST> with the shape's G
+#define SG_LAUNCH64(kernel, blocks, ...)                                                        \
+    do {                                                                                        \
+        cudaError_t rc = cudaSuccess;                                                           \
+        if (sh.warps == 8) {                                                                    \
+            if ((rc = prep64((const void*)kernel(8, true), sh.smem)) != cudaSuccess) return rc; \
+            kernel(8, true)<<<blocks, 256, sh.smem, s>>>(__VA_ARGS__);                          \
+        } else if (sh.warps == 4) {                                                             \
+            if ((rc = prep64((const void*)kernel(4, true), sh.smem)) != cudaSuccess) return rc; \
+            kernel(4, true)<<<blocks, 128, sh.smem, s>>>(__VA_ARGS__);                          \
+        } else {                                                                                \
+            if ((rc = prep64((const void*)kernel(1, false), sh.smem)) != cudaSuccess) return rc;\
+            kernel(1, false)<<<blocks, 32, sh.smem, s>>>(__VA_ARGS__);                          \
+        }                                                                                       \
+        return cudaGetLastError();                                                              \
+    } while (0)
+
+// blocks that loop over the confs of one model: the model is staged once per block
+static int loop_blocks(const Shape64& sh, int n, int num_sms) { return std::min(n, num_sms * (16 / sh.warps)); }
+
+#define SG_K_EVAL(G, ST) k_eval64<G, ST>
+#define SG_K_BFGS(G, ST) k_bfgs64<G, ST>
+#define SG_K_MC(G, ST) k_mc64<G, ST, false>
+#define SG_K_MC_VIS(G, ST) k_mc64<G, ST, true>
+#define SG_K_REFINE(G, ST) k_refine64<G, ST>
+#define SG_K_SCORE(G, ST) k_score64<G, ST>
+
+cudaError_t launch_eval64(const DModel* dm, const Shape64& sh, int num_sms, const DTables& T, const DReceptor* R, int n,
+                          const double* confs, const double v[3], double slope, int direct, double* e, double* g,
+                          double* coords, int* err, cudaStream_t s) {
+    SG_LAUNCH64(SG_K_EVAL, loop_blocks(sh, n, num_sms), dm, T, R, n, confs, v[0], v[1], v[2], slope, direct, e, g, coords,
+                err);
 }
 
-cudaError_t launch_mc64(const DModel* dms, size_t smem, const DTables& T, const DReceptor* R, const Chain64* chains,
-                        int n, const MCParams64& P, bool visited, int* err, cudaStream_t s) {
-    const void* fn = visited ? (const void*)k_mc64<true> : (const void*)k_mc64<false>;
-    cudaError_t rc = prep(fn, smem);
-    if (rc != cudaSuccess) return rc;
-    if (visited) k_mc64<true><<<n, 32, smem, s>>>(dms, T, R, chains, n, P, err);
-    else k_mc64<false><<<n, 32, smem, s>>>(dms, T, R, chains, n, P, err);
-    return cudaGetLastError();
+cudaError_t launch_bfgs64(const DModel* dm, const Shape64& sh, int num_sms, const DTables& T, const DReceptor* R, int n,
+                          double* confs, const double v[3], double slope, int maxiters, int accurate, int early,
+                          double* e, int* err, cudaStream_t s) {
+    SG_LAUNCH64(SG_K_BFGS, loop_blocks(sh, n, num_sms), dm, T, R, n, confs, v[0], v[1], v[2], slope, maxiters, accurate,
+                early, e, err);
 }
 
-cudaError_t launch_refine64(const DModel* dms, size_t smem, const DTables& T, const DReceptor* R, const int* pose_model,
-                            int n, double* confs, int conf_stride, const double cap[3], int maxiters,
-                            const int* pose_maxiters, const double* pose_box, int accurate, int early, double* e,
-                            double* coords, int coord_stride, int* err, cudaStream_t s) {
-    cudaError_t rc = prep((const void*)k_refine64, smem);
-    if (rc != cudaSuccess) return rc;
-    k_refine64<<<n, 32, smem, s>>>(dms, T, R, pose_model, n, confs, conf_stride, cap[0], cap[1], cap[2], maxiters,
-                                   pose_maxiters, pose_box, accurate, early, e, coords, coord_stride, err);
-    return cudaGetLastError();
+cudaError_t launch_mc64(const DModel* dms, const Shape64& sh, const DTables& T, const DReceptor* R,
+                        const Chain64* chains, int n, const MCParams64& P, bool visited, int* err, cudaStream_t s) {
+    if (visited) SG_LAUNCH64(SG_K_MC_VIS, n, dms, T, R, chains, n, P, err);
+    SG_LAUNCH64(SG_K_MC, n, dms, T, R, chains, n, P, err);
 }
 
-cudaError_t launch_score64(const DModel* dms, size_t smem, const DTables& T, const DReceptor* R, const int* pose_model,
-                           int n, const double* confs, int conf_stride, const double v[3], double slope, double* e,
-                           double* intra, double* coords, int coord_stride, int* err, cudaStream_t s) {
-    cudaError_t rc = prep((const void*)k_score64, smem);
-    if (rc != cudaSuccess) return rc;
-    k_score64<<<n, 32, smem, s>>>(dms, T, R, pose_model, n, confs, conf_stride, v[0], v[1], v[2], slope, e, intra,
-                                  coords, coord_stride, err);
-    return cudaGetLastError();
+cudaError_t launch_refine64(const DModel* dms, const Shape64& sh, const DTables& T, const DReceptor* R,
+                            const int* pose_model, int n, double* confs, int conf_stride, const double cap[3],
+                            int maxiters, const int* pose_maxiters, const double* pose_box, int accurate, int early,
+                            double* e, double* coords, int coord_stride, int* err, cudaStream_t s) {
+    SG_LAUNCH64(SG_K_REFINE, n, dms, T, R, pose_model, n, confs, conf_stride, cap[0], cap[1], cap[2], maxiters,
+                pose_maxiters, pose_box, accurate, early, e, coords, coord_stride, err);
+}
+
+cudaError_t launch_score64(const DModel* dms, const Shape64& sh, const DTables& T, const DReceptor* R,
+                           const int* pose_model, int n, const double* confs, int conf_stride, const double v[3],
+                           double slope, double* e, double* intra, double* coords, int coord_stride, int* err,
+                           cudaStream_t s) {
+    SG_LAUNCH64(SG_K_SCORE, n, dms, T, R, pose_model, n, confs, conf_stride, v[0], v[1], v[2], slope, e, intra, coords,
+                coord_stride, err);
 }
 
 }  // namespace sg

@@ -63,6 +63,16 @@ __global__ void k_cell_lists(int natoms, const double* xyz, const int* type, DGe
     if (pass == 0 && lane == 0) count[cell] = running;
 }
 
+// a cell list's atoms whole (CellAtom) and their charges, in list order
+__global__ void k_cell_pack(int n, const int* atoms, const double* xyz, const int* type, const double* charge,
+                            CellAtom* list, double* list_charge) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int a = atoms[k];
+        list[k] = CellAtom{xyz[3 * a], xyz[3 * a + 1], xyz[3 * a + 2], type[a], 0};
+        list_charge[k] = charge[a];
+    }
+}
+
 // one thread per grid point; threads of a warp cover a compact 8x4 tile
 __global__ void __launch_bounds__(256) k_grid_map64(DGeom g, int natoms, const double* xyz, const int* rtype,
                                                     const double* rcharge, const int* cstart, const int* catoms,
@@ -152,6 +162,13 @@ cudaError_t launch_cell_lists(int natoms, const double* xyz, const int* type, co
                               cudaStream_t s) {
     const int ncells = g.cell_dim[0] * g.cell_dim[1] * g.cell_dim[2];
     k_cell_lists<<<ncells, 32, 0, s>>>(natoms, xyz, type, g, cutoff_sqr, lo, hi, count, start, atoms, pass);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_cell_pack(int n, const int* atoms, const double* xyz, const int* type, const double* charge,
+                             CellAtom* list, double* list_charge, cudaStream_t s) {
+    if (n <= 0) return cudaSuccess;
+    k_cell_pack<<<(n + 255) / 256, 256, 0, s>>>(n, atoms, xyz, type, charge, list, list_charge);
     return cudaGetLastError();
 }
 

@@ -532,15 +532,18 @@ static void launch_refines(Server& s, std::vector<std::pair<SvBatch*, SvLig*>>& 
     std::vector<DModel> dms;
     std::vector<int> pose_model, pose_maxit;
     std::vector<DReceptor*> recs;
-    size_t ws = 0;
+    Smem64 ws;
     int np = 0;
     for (auto& [b, L] : fin) {
         const DModel& h = b->img.host[L->model];
         g->cs = std::max(g->cs, h.conf_size);
         g->hs = std::max(g->hs, h.nheavy);
-        ws = std::max(ws, ws64_bytes(h));
+        ws.add(h);
     }
-    require(ws <= (size_t)e->max_smem, "serve: model too large for the plain path's shared memory");
+    // 4 warps per pose where they find room beside the search: no more shared
+    // memory than a serving block's place (else one warp, nothing staged)
+    const Shape64 sh = shape64(ws, 1ll << 40, e->num_sms, std::min((size_t)e->max_smem, s.smem_block));
+    require(sh.smem <= (size_t)e->max_smem, "serve: model too large for the plain path's shared memory");
     // refine_structure needs the pose's receptor: one launch per receptor in the group
     std::map<int, std::vector<std::pair<SvBatch*, SvLig*>>> by_rec;
     for (auto& f : fin) by_rec[f.second->req.rid].push_back(f);
@@ -594,7 +597,7 @@ static void launch_refines(Server& s, std::vector<std::pair<SvBatch*, SvLig*>>& 
         for (auto& [b, L] : members) n += (int)L->poses.size();
         if (n > 0) {
             const sg_mc_params& P = members[0].second->req.p;
-            cuda_check(launch_refine64(d_models, ws, e->tables, e->rec[rid].dhdr.as<DReceptor>(), dpm + p0, n,
+            cuda_check(launch_refine64(d_models, sh, e->tables, e->rec[rid].dhdr.as<DReceptor>(), dpm + p0, n,
                                        dc + (size_t)p0 * g->cs, g->cs, P.authentic_v, P.maxiters, dmi + p0, nullptr,
                                        P.accurate_line, P.early_term, de + p0, dx + (size_t)p0 * g->hs * 3, g->hs,
                                        s.d_err, rs),

@@ -33,6 +33,13 @@ struct DGeom {
     int cell_off[3], cell_dim[3];
 };
 
+// one receptor atom of a direct-sum cell list, whole: two 16-byte loads side by
+// side with its neighbours' instead of an index and four scattered reads
+struct __align__(16) CellAtom {
+    double x, y, z;
+    int type, pad;
+};
+
 struct DReceptor {
     int natoms;
     const double* xyz;     // [n][3]
@@ -43,7 +50,8 @@ struct DReceptor {
     const int* pop_start;   // [ncells + 1]
     const int* pop_atoms;
     const int* full_start;  // [ncells + 1]
-    const int* full_atoms;
+    const CellAtom* full_list;
+    const double* full_charge;  // charges of full_list's atoms
     DGeom g;
     const double* map[kNumTypes];        // FP64 maps or null
     const double* cmap[kNumTypes];       // FP64 charge maps or null
@@ -267,17 +275,42 @@ struct __align__(16) MCParams32 {
     double box[6];  // search box: lo xyz, hi xyz
 };
 
-// Per-warp FP64 workspace layout in shared memory (offsets in doubles)
+// Shared memory of a plain-path block (dock64_eval.cuh): the header, the
+// workspace and, when the model is staged, copies of its small arrays and of the
+// receptor header.  Offsets in doubles from the block's shared memory.
 struct Ws64 {
-    int coords, mf, eatom, origin, axis, q, rot, fF, fT, pe, pf, pin;
-    int x_tmp, x_cand, x_new, x_orig, g, g_new, g_orig, p, y, mhy, h, bcast, rmsd, mt;
-    int total;  // doubles
+    int coords, mf, eatom, origin, axis, q, rot, fF, fT, pe, pf;
+    int x_tmp, x_cand, x_new, x_orig, g, g_new, g_orig, p, y, mhy, h, mt;
+    int xbuf;  // exchange buffers of the direct sum, kXbuf64 per warp
+    // staged only
+    int cr;  // torque terms per atom
+    int s_receptor, s_type, s_atom_frame, s_csr_start, s_heavy, s_fkind, s_fparent, s_fbegin, s_fend, s_fconf, s_fdof,
+        s_level_start, s_level_frames, s_child_start, s_child_list, s_lig_begin, s_lig_end, s_lig_root, s_lig_pair_end,
+        s_blk_rigid, s_blk_conf, s_blk_ntors, s_tor_conf, s_tor_dof, s_charge, s_local, s_forigin, s_faxis;
+    int total;  // doubles; staged: without the exchange buffers, which follow
 };
+struct __align__(16) Hdr64 {
+    DModel m;
+    DTables T;
+    const DReceptor* R;
+    const double* box;  // this item's own box (lo xyz, hi xyz) for the direct sum; null: the receptor's
+    int* err;
+    unsigned long long evals;
+    // the leader's command to the block, and the energy it gets back
+    double v[3], slope, e;
+    int g_at, direct, op, pad_;
+    Ws64 L;
+};
+// 4 groups of 8 terms of 4 doubles, 4 doubles apart so that the groups' reads
+// fall in different banks
+constexpr int kXbuf64 = 4 * (8 * 4 + 4);
 
-SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof) {
-    Ws64 w;
-    int o = 0;
+SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof, bool staged, int nheavy, int nlevels,
+                       int nlig, int nblocks, int ntors) {
+    Ws64 w{};
+    int o = (int)((sizeof(Hdr64) + 15) / 16) * 2;
     auto take = [&](int n) { int r = o; o += (n + 1) & ~1; return r; };
+    auto ints = [&](int n) { return take((n + 1) / 2); };
     w.coords = take(3 * natoms);
     w.mf = take(3 * natoms);
     w.eatom = take(natoms);
@@ -289,7 +322,6 @@ SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof) {
     w.fT = take(3 * nframes);
     w.pe = take(npairs);
     w.pf = take(3 * npairs);
-    w.pin = take((npairs + 7) / 8);  // one byte per pair
     w.x_tmp = take(conf);
     w.x_cand = take(conf);
     w.x_new = take(conf);
@@ -301,12 +333,55 @@ SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof) {
     w.y = take(dof);
     w.mhy = take(dof);
     w.h = take(dof * (dof + 1) / 2);
-    w.bcast = take(16);
-    w.rmsd = take(64);
     w.mt = take(313);  // 625 uint32 words + padding
+    w.xbuf = w.mt;     // one warp's: the direct sum's kernels draw no random numbers
+    if (staged) {
+        w.cr = take(3 * natoms);
+        w.s_receptor = take((int)((sizeof(DReceptor) + 7) / 8));
+        w.s_type = ints(natoms);
+        w.s_atom_frame = ints(natoms);
+        w.s_csr_start = ints(natoms + 1);
+        w.s_heavy = ints(nheavy);
+        w.s_fkind = ints(nframes);
+        w.s_fparent = ints(nframes);
+        w.s_fbegin = ints(nframes);
+        w.s_fend = ints(nframes);
+        w.s_fconf = ints(nframes);
+        w.s_fdof = ints(nframes);
+        w.s_level_start = ints(nlevels + 1);
+        w.s_level_frames = ints(nframes);
+        w.s_child_start = ints(nframes + 1);
+        w.s_child_list = ints(nframes);
+        w.s_lig_begin = ints(nlig);
+        w.s_lig_end = ints(nlig);
+        w.s_lig_root = ints(nlig);
+        w.s_lig_pair_end = ints(nlig);
+        w.s_blk_rigid = ints(nblocks);
+        w.s_blk_conf = ints(nblocks);
+        w.s_blk_ntors = ints(nblocks);
+        w.s_tor_conf = ints(ntors);
+        w.s_tor_dof = ints(ntors);
+        w.s_charge = take(natoms);
+        w.s_local = take(3 * natoms);
+        w.s_forigin = take(3 * nframes);
+        w.s_faxis = take(3 * nframes);
+        w.xbuf = o;
+    }
     w.total = o;
     return w;
 }
+
+// the most shared memory any model of a batch takes, in bytes, with nothing
+// staged and staged (without the exchange buffers)
+struct Smem64 {
+    size_t plain = 0, staged = 0;
+    void add(const DModel& h);
+};
+// a plain-path launch: warps per item and its shared memory
+struct Shape64 {
+    int warps;
+    size_t smem;
+};
 
 // Chain bookkeeping for the plain path (global memory)
 // A chain's QuickVina 2 history (plain path, MCParams::visited) over n <=
