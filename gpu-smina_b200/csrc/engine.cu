@@ -4,31 +4,230 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
+#include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 #include "engine.h"
 
 namespace sg {
 
+// ---- the devices' pools of call temporaries ------------------------------------------------
+// Streams of different engines never wait for one another through a pool: it
+// only hands a block to another stream once the first stream's work is done.
+// When an allocation fails, what the pools keep is given back and it is tried
+// again.
+struct DevPool {
+    cudaMemPool_t pool = nullptr;
+    int users = 0;
+};
+static std::mutex g_pools_mu;
+static std::map<int, DevPool>& g_pools = *new std::map<int, DevPool>;  // (never destroyed: no CUDA call after main)
+
+static void drop_pin_rings();
+cudaMemPool_t pool_acquire(int device) {
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    DevPool& d = g_pools[device];
+    if (!d.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cuda_check(cudaMemPoolCreate(&d.pool, &props), "memory pool");
+        uint64_t keep = kPoolKept;
+        int no = 0;
+        cuda_check(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep), "memory pool");
+        cuda_check(cudaMemPoolSetAttribute(d.pool, cudaMemPoolReuseAllowInternalDependencies, &no), "memory pool");
+    }
+    d.users++;
+    return d.pool;
+}
+void pool_release(int device) {
+    std::lock_guard<std::mutex> lk(g_pools_mu);
+    DevPool& d = g_pools[device];
+    if (--d.users == 0) {
+        cudaMemPoolDestroy(d.pool);
+        d.pool = nullptr;
+    }
+    for (auto& q : g_pools)
+        if (q.second.users) return;
+    drop_pin_rings();  // the process's last engine is gone
+}
+
+static cudaError_t alloc_device(void** p, size_t n, sg_engine* pooled) {
+    if (pooled && pooled->pool) return cudaMallocFromPoolAsync(p, n, pooled->pool, pooled->stream);
+    return cudaMalloc(p, n);
+}
 void DevBuf::reset() {
-    if (p) cudaFree(p);
+    if (p) {
+        if (pool_of && pool_of->pool) cudaFreeAsync(p, pool_of->stream);
+        else cudaFree(p);
+    }
     p = nullptr;
-    bytes = 0;
+    bytes = cap = 0;
 }
 void DevBuf::alloc(size_t n) {
-    reset();
     if (n == 0) n = 16;
-    if (cudaMalloc(&p, n) != cudaSuccess) {
-        p = nullptr;
-        throw EngineError(SG_ERR_NOMEM, "device allocation of " + std::to_string(n) + " bytes failed");
+    if (p && n <= cap && cap / 2 <= n + (64 << 10)) {
+        bytes = n;
+        return;
     }
-    bytes = n;
+    reset();
+    if (alloc_device(&p, n, pool_of) != cudaSuccess) {
+        cudaGetLastError();
+        {
+            std::lock_guard<std::mutex> lk(g_pools_mu);
+            for (auto& q : g_pools)
+                if (q.second.pool) cudaMemPoolTrimTo(q.second.pool, 0);
+        }
+        if (alloc_device(&p, n, pool_of) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+            throw EngineError(SG_ERR_NOMEM, "device allocation of " + std::to_string(n) + " bytes failed");
+        }
+    }
+    bytes = cap = n;
 }
 void DevBuf::upload(const void* src, size_t n, cudaStream_t s) {
     alloc(n);
     if (n) cuda_check(cudaMemcpyAsync(p, src, n, cudaMemcpyHostToDevice, s), "upload");
+}
+
+// ---- a call's copies ----------------------------------------------------------------------
+static std::mutex g_rings_mu;
+static std::vector<std::unique_ptr<PinRing>>& g_rings = *new std::vector<std::unique_ptr<PinRing>>;  // free ones
+constexpr size_t kRingsKept = 4;  // free rings kept while the process has an engine
+static void drop_pin_rings() {
+    std::lock_guard<std::mutex> lk(g_rings_mu);
+    g_rings.clear();
+}
+
+PinRing::~PinRing() {
+    for (cudaEvent_t x : ev)
+        if (x) cudaEventDestroy(x);
+    if (p) cudaFreeHost(p);
+}
+static std::unique_ptr<PinRing> ring_get() {
+    {
+        std::lock_guard<std::mutex> lk(g_rings_mu);
+        if (!g_rings.empty()) {
+            auto r = std::move(g_rings.back());
+            g_rings.pop_back();
+            return r;
+        }
+    }
+    auto r = std::make_unique<PinRing>();
+    cuda_check(cudaHostAlloc((void**)&r->p, PinRing::kSlot * PinRing::kSlots, cudaHostAllocPortable), "pinned memory");
+    return r;
+}
+static void ring_put(std::unique_ptr<PinRing> r) {
+    for (cudaEvent_t& x : r->ev) {  // events belong to the call's device
+        if (x) cudaEventDestroy(x);
+        x = nullptr;
+    }
+    std::lock_guard<std::mutex> lk(g_rings_mu);
+    if (g_rings.size() < kRingsKept) g_rings.push_back(std::move(r));
+}
+void warm_pin_ring() {
+    {
+        std::lock_guard<std::mutex> lk(g_rings_mu);
+        if (!g_rings.empty()) return;
+    }
+    ring_put(ring_get());
+}
+static void mark(PinRing& r, int slot, cudaStream_t s) {
+    if (!r.ev[slot]) cuda_check(cudaEventCreateWithFlags(&r.ev[slot], cudaEventDisableTiming), "event");
+    cuda_check(cudaEventRecord(r.ev[slot], s), "event");
+}
+void CallIo::need_ring() {
+    if (!ring_) ring_ = ring_get();
+}
+CallIo::~CallIo() {
+    if (busy_) cudaStreamSynchronize(e_->stream);  // an error left copies in flight
+    if (ring_) ring_put(std::move(ring_));
+}
+void CallIo::in(DevBuf& dst, const void* src, size_t n) {
+    dst.alloc(n);
+    if (!n) return;
+    need_ring();
+    busy_ = true;
+    for (size_t at = 0; at < n;) {
+        if (in_used_ == PinRing::kSlot) {  // on to the other slot, once its copies are done
+            mark(*ring_, in_slot_, e_->stream);
+            in_sent_[in_slot_] = true;
+            in_slot_ ^= 1;
+            in_used_ = 0;
+            if (in_sent_[in_slot_]) cuda_check(cudaEventSynchronize(ring_->ev[in_slot_]), "copy in");
+        }
+        const size_t k = std::min(n - at, PinRing::kSlot - in_used_);
+        char* q = ring_->p + in_slot_ * PinRing::kSlot + in_used_;
+        std::memcpy(q, static_cast<const char*>(src) + at, k);
+        cuda_check(cudaMemcpyAsync(dst.as<char>() + at, q, k, cudaMemcpyHostToDevice, e_->stream), "copy in");
+        in_used_ = std::min(PinRing::kSlot, (in_used_ + k + 15) & ~(size_t)15);
+        at += k;
+    }
+}
+void CallIo::out(void* host, const void* dev, size_t n) {
+    if (host && n) outs_.push_back({host, dev, n});
+}
+// Fetches the outputs (behind the device error word, which is cleared for the
+// next call and turned into a status).
+void CallIo::finish() {
+    need_ring();
+    busy_ = true;
+    int err = kDevOk;
+    std::vector<Out> todo;
+    todo.push_back({&err, e_->d_err.p, sizeof(int)});
+    todo.insert(todo.end(), outs_.begin(), outs_.end());
+    outs_.clear();
+    std::vector<Piece> pieces[2];
+    bool sent[2] = {};
+    auto hand_over = [&](int s) {
+        if (!sent[s]) return;
+        cuda_check(cudaEventSynchronize(ring_->ev[2 + s]), "kernel");
+        for (const Piece& p : pieces[s]) std::memcpy(p.host, p.from, p.n);
+        pieces[s].clear();
+        sent[s] = false;
+    };
+    int slot = 0;
+    size_t used = 0;
+    auto flush = [&] {
+        mark(*ring_, 2 + slot, e_->stream);
+        sent[slot] = true;
+        slot ^= 1;
+        used = 0;
+    };
+    for (const Out& o : todo)
+        for (size_t at = 0; at < o.n;) {
+            if (used == PinRing::kSlot) {
+                flush();
+                hand_over(slot);
+            }
+            const size_t k = std::min(o.n - at, PinRing::kSlot - used);
+            char* q = ring_->p + (2 + slot) * PinRing::kSlot + used;
+            cuda_check(cudaMemcpyAsync(q, static_cast<const char*>(o.dev) + at, k, cudaMemcpyDeviceToHost, e_->stream),
+                       "copy out");
+            pieces[slot].push_back({static_cast<char*>(o.host) + at, q, k});
+            used = std::min(PinRing::kSlot, (used + k + 15) & ~(size_t)15);
+            at += k;
+        }
+    hand_over(slot ^ 1);
+    cuda_check(cudaStreamSynchronize(e_->stream), "kernel");  // the last slot
+    for (const Piece& p : pieces[slot]) std::memcpy(p.host, p.from, p.n);
+    busy_ = false;
+    in_used_ = 0;
+    in_sent_[0] = in_sent_[1] = false;
+    if (err != kDevOk) {
+        const int zero = 0;
+        cuda_check(cudaMemcpy(e_->d_err.p, &zero, sizeof(int), cudaMemcpyHostToDevice), "clear error word");
+        if (err == kDevOverlap) throw EngineError(SG_ERR_OVERLAP, "Ligand atom exactly overlaps receptor atom.");
+        throw EngineError(SG_ERR_ARG, "device reported an out-of-range access (error " + std::to_string(err) + ")");
+    }
 }
 
 void cuda_check(cudaError_t e, const char* what) {
@@ -66,19 +265,7 @@ using namespace sg;
 // ---- engine -----------------------------------------------------------------------------------
 sg_engine::~sg_engine() {
     if (stream) cudaStreamDestroy(stream);
-}
-
-// Reads the device error word, clears it, and turns it into a status.
-void sg_engine::check_device_errors() {
-    int h = 0;
-    cuda_check(cudaMemcpyAsync(&h, d_err.p, sizeof(int), cudaMemcpyDeviceToHost, stream), "error word");
-    cuda_check(cudaStreamSynchronize(stream), "kernel");
-    if (h != kDevOk) {
-        const int zero = 0;
-        cuda_check(cudaMemcpy(d_err.p, &zero, sizeof(int), cudaMemcpyHostToDevice), "clear error word");
-        if (h == kDevOverlap) throw EngineError(SG_ERR_OVERLAP, "Ligand atom exactly overlaps receptor atom.");
-        throw EngineError(SG_ERR_ARG, "device reported an out-of-range access (error " + std::to_string(h) + ")");
-    }
+    if (pool) pool_release(device);
 }
 
 extern "C" {
@@ -94,6 +281,8 @@ int sg_create(int device, int precision, sg_engine** out) {
     e->precision = precision;
     int rc = guarded(e.get(), [&] {
         cuda_check(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "stream");
+        e->pool = pool_acquire(device);
+        warm_pin_ring();
         e->d_err.alloc(sizeof(int));
         cuda_check(cudaMemsetAsync(e->d_err.p, 0, sizeof(int), e->stream), "memset");
         cudaDeviceProp prop;
@@ -205,7 +394,7 @@ static int build_cells(sg_engine* e, RecState& r, const std::vector<double>& lo,
                         DevBuf& start, DevBuf& atoms) {
     const DGeom& g = r.geom;
     const int ncells = g.cell_dim[0] * g.cell_dim[1] * g.cell_dim[2];
-    DevBuf dlo, dhi, dcount;
+    DevBuf dlo(e), dhi(e), dcount(e);
     dlo.upload(lo.data(), lo.size() * sizeof(double), e->stream);
     dhi.upload(hi.data(), hi.size() * sizeof(double), e->stream);
     dcount.alloc(ncells * sizeof(int));
@@ -261,7 +450,7 @@ static void build_receptor_cells(sg_engine* e, RecState& r) {
     cell_bricks(r.geom, true, lo, hi);
     build_cells(e, r, lo, hi, r.pop_start, r.pop_atoms);
     cell_bricks(r.geom, false, lo, hi);
-    DevBuf full_atoms;
+    DevBuf full_atoms(e);
     const int n = build_cells(e, r, lo, hi, r.full_start, full_atoms);
     r.full_list.alloc(std::max(1, n) * sizeof(CellAtom));
     r.full_charge.alloc(std::max(1, n) * sizeof(double));
@@ -269,9 +458,10 @@ static void build_receptor_cells(sg_engine* e, RecState& r) {
                                 r.full_list.as<CellAtom>(), r.full_charge.as<double>(), e->stream),
                "cell atoms");
     refresh_header(e, r);
+    r.cells = true;
 }
 void ensure_cells(sg_engine* e, RecState& r) {
-    if (!r.pop_start.p) build_receptor_cells(e, r);
+    if (!r.cells) build_receptor_cells(e, r);
 }
 
 void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
@@ -286,18 +476,42 @@ void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
     ensure_cells(e, r);
     const size_t npts = (size_t)r.geom.dim[0] * r.geom.dim[1] * r.geom.dim[2];
     const bool charged = e->tables.nc > 1;
+    const bool packed = e->precision != SG_PREC_FP64, half = e->precision == SG_PREC_FP32_H16;
+    // one allocation for all the new maps, each 256-byte aligned
+    const size_t ncells = (size_t)(r.geom.dim[0] - 1) * (r.geom.dim[1] - 1) * (r.geom.dim[2] - 1);
+    const size_t b64 = npts * sizeof(double), b32 = packed ? ncells * 2 * sizeof(float4) : 0,
+                 b16 = half ? ncells * sizeof(uint4) : 0;
+    auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    const size_t per_type = (up(b64) + up(b32)) * (charged ? 2 : 1) + up(b16), total = per_type * need.size();
+    std::unique_ptr<DevBuf> mem;
+    for (auto& q : r.spare)
+        if (!mem && q->bytes >= total && q->bytes / 2 <= total) mem = std::move(q);
+    r.spare.clear();
+    if (!mem) {
+        mem.reset(new DevBuf());
+        mem->alloc(total);
+    }
+    char* at = mem->as<char>();
+    auto place = [&](MapView& v, size_t n) {
+        if (!n) return;
+        v.p = at;
+        v.bytes = n;
+        at += up(n);
+    };
     std::vector<double*> maps, cmaps;
     for (int t : need) {
-        r.map64[t].alloc(npts * sizeof(double));
+        place(r.map64[t], b64);
+        place(r.map32[t], b32);
+        place(r.map16[t], b16);
         maps.push_back(r.map64[t].as<double>());
         if (charged) {
-            r.cmap64[t].alloc(npts * sizeof(double));
-            cmaps.push_back(r.cmap64[t].as<double>());
-        } else {
-            cmaps.push_back(nullptr);
+            place(r.cmap64[t], b64);
+            place(r.cmap32[t], b32);
         }
+        cmaps.push_back(r.cmap64[t].as<double>());
     }
-    DevBuf dtypes, dmaps, dcmaps;
+    r.map_mem.push_back(std::move(mem));
+    DevBuf dtypes(e), dmaps(e), dcmaps(e);
     dtypes.upload(need.data(), need.size() * sizeof(int), e->stream);
     dmaps.upload(maps.data(), maps.size() * sizeof(double*), e->stream);
     dcmaps.upload(cmaps.data(), cmaps.size() * sizeof(double*), e->stream);
@@ -306,21 +520,15 @@ void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
                                  dmaps.as<double*>(), dcmaps.as<double*>(), r.ugrid.as<double>(), r.ug, r.ug_slope,
                                  e->stream),
                "grid maps");
-    if (e->precision != SG_PREC_FP64) {
-        const size_t ncells = (size_t)(r.geom.dim[0] - 1) * (r.geom.dim[1] - 1) * (r.geom.dim[2] - 1);
+    if (packed)
         for (int t : need) {
-            r.map32[t].alloc(ncells * 2 * sizeof(float4));
-            if (e->precision == SG_PREC_FP32_H16) r.map16[t].alloc(ncells * sizeof(uint4));
             cuda_check(launch_grid_pack(r.geom, r.map64[t].as<double>(), r.map32[t].as<float4>(), r.map16[t].as<uint4>(),
                                         e->stream),
                        "pack maps");
-            if (charged) {
-                r.cmap32[t].alloc(ncells * 2 * sizeof(float4));
+            if (charged)
                 cuda_check(launch_grid_pack(r.geom, r.cmap64[t].as<double>(), r.cmap32[t].as<float4>(), nullptr, e->stream),
                            "pack charge maps");
-            }
         }
-    }
     cuda_check(cudaStreamSynchronize(e->stream), "grid maps");
     for (int t : need) r.built[t] = true;
     refresh_header(e, r);
@@ -344,8 +552,7 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
                                                            std::isfinite(r->coords[3 * i + 2]), "receptor: non-finite coordinate");
         RecState& s = e->rec[rid];
         s.clear_maps();
-        s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset();
-        s.full_list.reset(); s.full_charge.reset();
+        s.cells = false;
         s.ugrid.reset();  // a new receptor starts without a user grid
         s.ug = DGeom{};
         s.gd = *gd;
@@ -408,10 +615,11 @@ int sg_drop_receptor(sg_engine* e, int rid) {
         require(rid >= 0 && rid < SG_MAX_RECEPTORS, "receptor id out of range");
         RecState& s = e->rec[rid];
         s.clear_maps();
+        s.spare.clear();
         s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset();
         s.full_list.reset(); s.full_charge.reset();
         s.xyz.reset(); s.type.reset(); s.charge.reset(); s.dhdr.reset(); s.ugrid.reset();
-        s.set = false;
+        s.set = s.cells = false;
     });
 }
 
@@ -436,53 +644,63 @@ static bool pack_pair_chunks(const sg_model_desc& d, const std::vector<int>& pai
     const int N = d.num_atoms, P = d.num_pairs;
     out.clear();
     if (N > 255) return false;  // 8-bit atom indices (inflex atoms take part in pairs too)
+    // Chunk c's atoms as bit c of per-atom words, so that a pair meets only the
+    // chunks with room for it; its quarters' bank groups as one bit per (quarter,
+    // group), a full quarter as all of them.
     struct Chunk {
-        std::vector<char> out_used, in_used;
-        uint8_t amod[4] = {}, bmod[4] = {};  // bank groups taken per quarter (bit masks)
-        uint32_t slot[32];
+        uint32_t abank = 0, bbank = 0, slot[32];
         int fill[4] = {};
     };
     std::vector<Chunk> chunks;
+    size_t words = 0;
+    std::vector<uint64_t> first_in, second_in;  // [word][atom]
     for (int k = 0; k < P; k++) {
         const int u = d.pairs[2 * k], v = d.pairs[2 * k + 1];
         require(u >= 0 && v >= 0 && u < N && v < N && u != v, "model: pair atoms must be distinct atoms");
         require((pair_tp[k] & 0x1ff) < (int)kSlotPairMask, "model: type pair index out of range");
         const uint32_t base = ((uint32_t)(pair_tp[k] & 0x1ff) << 16) | ((pair_tp[k] >> 30) & 1 ? kSlotSwap : 0) |
                               (k >= d.num_other_pairs ? kSlotIntra : 0);
-        bool placed = false;
-        for (size_t c = 0; c < chunks.size() && !placed; c++) {
+        auto place = [&](size_t c, int o) {
+            const int a = o ? v : u, b = o ? u : v;
             Chunk& ch = chunks[c];
-            for (int o = 0; o < 2 && !placed; o++) {
-                const int a = o ? v : u, b = o ? u : v;
-                if (ch.out_used[a] || ch.in_used[b]) continue;
-                for (int q = 0; q < 4; q++) {
-                    if (ch.fill[q] == 8 || (ch.amod[q] >> (a & 7) & 1) || (ch.bmod[q] >> (b & 7) & 1)) continue;
-                    ch.out_used[a] = ch.in_used[b] = 1;
-                    ch.amod[q] |= 1 << (a & 7);
-                    ch.bmod[q] |= 1 << (b & 7);
-                    ch.slot[8 * q + ch.fill[q]++] = (o ? base ^ kSlotSwap : base) | a | (b << 8);
-                    placed = true;
-                    break;
-                }
+            const uint32_t busy = ((ch.abank >> (a & 7)) | (ch.bbank >> (b & 7))) & 0x01010101u;
+            if (busy == 0x01010101u) return false;
+            const int q = __builtin_ctz(~busy & 0x01010101u) >> 3;
+            ch.abank |= 1u << (8 * q + (a & 7));
+            ch.bbank |= 1u << (8 * q + (b & 7));
+            ch.slot[8 * q + ch.fill[q]++] = (o ? base ^ kSlotSwap : base) | a | (b << 8);
+            if (ch.fill[q] == 8) ch.abank |= 0xffu << (8 * q);
+            first_in[c / 64 * N + a] |= 1ull << (c & 63);
+            second_in[c / 64 * N + b] |= 1ull << (c & 63);
+            return true;
+        };
+        bool placed = false;
+        for (size_t w = 0; w < words && !placed; w++) {
+            const uint64_t there = chunks.size() - 64 * w >= 64 ? ~0ull : (1ull << (chunks.size() - 64 * w)) - 1;
+            const uint64_t as_is = there & ~(first_in[w * N + u] | second_in[w * N + v]),
+                           turned = there & ~(first_in[w * N + v] | second_in[w * N + u]);
+            for (uint64_t m = as_is | turned; m && !placed; m &= m - 1) {
+                const int bit = __builtin_ctzll(m);
+                placed = ((as_is >> bit) & 1 && place(64 * w + bit, 0)) || ((turned >> bit) & 1 && place(64 * w + bit, 1));
             }
         }
         if (!placed) {
             chunks.emplace_back();
-            Chunk& ch = chunks.back();
-            ch.out_used.assign(N, 0);
-            ch.in_used.assign(N, 0);
-            for (uint32_t& x : ch.slot) x = kSlotEmpty;
-            ch.out_used[u] = ch.in_used[v] = 1;
-            ch.amod[0] = 1 << (u & 7);
-            ch.bmod[0] = 1 << (v & 7);
-            ch.slot[ch.fill[0]++] = base | u | (v << 8);
+            for (uint32_t& x : chunks.back().slot) x = kSlotEmpty;
+            if (chunks.size() > 64 * words) {
+                words++;
+                first_in.resize(words * N, 0);
+                second_in.resize(words * N, 0);
+            }
+            place(chunks.size() - 1, 0);
         }
     }
+    out.reserve(32 * chunks.size());
     for (const Chunk& ch : chunks) out.insert(out.end(), ch.slot, ch.slot + 32);
     return true;
 }
 
-static void pack_one(const sg_model_desc& d, std::vector<int>& I, std::vector<double>& D, std::vector<float>& Fl,
+static void pack_one(const sg_model_desc& d, bool mixed, std::vector<int>& I, std::vector<double>& D, std::vector<float>& Fl,
                      std::vector<size_t>& ioff, std::vector<size_t>& doff, std::vector<size_t>& foff, DModel& hm) {
     const int N = d.num_atoms, M = d.num_movable, F = d.num_frames, P = d.num_pairs;
     require(N > 0 && N <= 4096 && M > 0 && M <= N, "model: atom counts out of range");
@@ -642,7 +860,7 @@ static void pack_one(const sg_model_desc& d, std::vector<int>& I, std::vector<do
     }
     {   // mixed-precision pair schedule (pack_pair_chunks)
         std::vector<uint32_t> slots;
-        const bool packable = pack_pair_chunks(d, pair_tp, slots);
+        const bool packable = mixed && pack_pair_chunks(d, pair_tp, slots);
         std::vector<int> ps(slots.begin(), slots.end());
         hm.npchunks = packable ? (int)(slots.size() / 32) : -1;
         pv(ps);
@@ -655,8 +873,10 @@ static void pack_one(const sg_model_desc& d, std::vector<int>& I, std::vector<do
         }
     };
     foff.clear();
-    pf4(d.atom_local, d.atom_charge, N); pf4(d.atom_lab, nullptr, N);
-    pf4(d.frame_origin, nullptr, F); pf4(d.frame_axis, nullptr, F); pf4(d.frame_init_origin, nullptr, F);
+    if (mixed) {
+        pf4(d.atom_local, d.atom_charge, N); pf4(d.atom_lab, nullptr, N);
+        pf4(d.frame_origin, nullptr, F); pf4(d.frame_axis, nullptr, F); pf4(d.frame_init_origin, nullptr, F);
+    }
     hm.cost = M + P + 8 * F;
     pd(d.atom_charge, N); pd(d.atom_local, 3 * (size_t)N); pd(d.atom_lab, 3 * (size_t)N);
     pd(d.frame_origin, 3 * (size_t)F); pd(d.frame_axis, 3 * (size_t)F); pd(d.frame_init_origin, 3 * (size_t)F);
@@ -667,84 +887,82 @@ static void pack_one(const sg_model_desc& d, std::vector<int>& I, std::vector<do
     require(hm.ntors + 6 * d.num_ligands == d.dof, "model: dof disagrees with the torsion count");
 }
 
-void pack_models(sg_engine* e, const sg_model_desc* models, int nmodels, PackedModels& out) {
-    require(models && nmodels > 0 && nmodels <= (1 << 20), "models: bad array");
+// The pools of a batch of models, as parts that are packed side by side on the
+// host's cores, and each descriptor's offsets into its part.
+struct PackedPart {
     std::vector<int> I;
     std::vector<double> D;
     std::vector<float> Fl;
-    std::vector<std::vector<size_t>> ioffs(nmodels), doffs(nmodels), foffs(nmodels);
-    out.host.assign(nmodels, DModel{});
-    for (int k = 0; k < nmodels; k++) pack_one(models[k], I, D, Fl, ioffs[k], doffs[k], foffs[k], out.host[k]);
-    out.ints.upload(I.data(), std::max<size_t>(1, I.size()) * sizeof(int), e->stream);
-    out.dbls.upload(D.data(), std::max<size_t>(1, D.size()) * sizeof(double), e->stream);
-    out.flts.upload(Fl.data(), std::max<size_t>(4, Fl.size()) * sizeof(float), e->stream);
-    const int* ib = out.ints.as<int>();
-    const double* db = out.dbls.as<double>();
-    const float* fb = out.flts.as<float>();
-    out.smem64 = Smem64{};
-    for (int k = 0; k < nmodels; k++) {
-        DModel& h = out.host[k];
-        const std::vector<size_t>& io = ioffs[k];
-        const std::vector<size_t>& dd = doffs[k];
-        int j = 0;
-        h.type = ib + io[j++]; h.fkind = ib + io[j++]; h.fparent = ib + io[j++]; h.fbegin = ib + io[j++];
-        h.fend = ib + io[j++]; h.fconf = ib + io[j++]; h.fdof = ib + io[j++];
-        h.atom_frame = ib + io[j++]; h.level_start = ib + io[j++]; h.level_frames = ib + io[j++];
-        h.child_start = ib + io[j++]; h.child_list = ib + io[j++]; h.pairs = ib + io[j++];
-        h.pair_group = ib + io[j++]; h.csr_start = ib + io[j++]; h.csr = ib + io[j++]; h.heavy = ib + io[j++];
-        h.lig_begin = ib + io[j++]; h.lig_end = ib + io[j++]; h.lig_root = ib + io[j++]; h.lig_pair_end = ib + io[j++];
-        h.blk_rigid = ib + io[j++]; h.blk_conf = ib + io[j++]; h.blk_dof = ib + io[j++]; h.blk_ntors = ib + io[j++];
-        h.tor_conf = ib + io[j++]; h.tor_dof = ib + io[j++]; h.tor_frame = ib + io[j++];
-        h.pair_tp = ib + io[j++];
-        h.fsub_end = ib + io[j++];
-        h.pslot = h.npchunks >= 0 ? (const uint32_t*)(ib + io[j]) : nullptr;
-        j++;
-        const std::vector<size_t>& fo = foffs[k];
-        h.local32 = (const float4*)(fb + fo[0]); h.lab32 = (const float4*)(fb + fo[1]);
-        h.forigin32 = (const float4*)(fb + fo[2]); h.faxis32 = (const float4*)(fb + fo[3]);
-        h.finit32 = (const float4*)(fb + fo[4]);
-        int q = 0;
-        h.charge = db + dd[q++]; h.local = db + dd[q++]; h.lab = db + dd[q++];
-        h.forigin = db + dd[q++]; h.faxis = db + dd[q++]; h.finit = db + dd[q++];
-        out.smem64.add(h);
-        out.max_conf = std::max(out.max_conf, h.conf_size);
-        out.max_dof = std::max(out.max_dof, h.dof);
-        out.max_heavy = std::max(out.max_heavy, h.nheavy);
-        out.max_atoms = std::max(out.max_atoms, h.natoms);
-        out.max_pairs = std::max(out.max_pairs, h.npairs);
-        out.max_frames = std::max(out.max_frames, h.nframes);
+    std::vector<std::vector<size_t>> io, dof, fo;
+    size_t i0 = 0, d0 = 0, f0 = 0;  // where the part's pools start in the batch's
+    std::exception_ptr error;
+};
+struct PackedPools {
+    std::vector<PackedPart> parts;
+    int per_part = 0;
+    size_t od = 0, of = 0, om = 0, bytes = 0;  // byte offsets of the doubles, floats and descriptors, and the end
+};
+constexpr int kPackPart = 16;    // models worth a thread (about 1 ms of packing)
+constexpr int kPackThreads = 8;
+static void pack_pools(const sg_model_desc* models, int nmodels, bool mixed, PackedPools& P, std::vector<DModel>& host) {
+    require(models && nmodels > 0 && nmodels <= (1 << 20), "models: bad array");
+    host.assign(nmodels, DModel{});
+    const int cores = std::max(1, (int)std::thread::hardware_concurrency());
+    const int nparts = std::max(1, std::min({nmodels / kPackPart, kPackThreads, cores}));
+    P.per_part = (nmodels + nparts - 1) / nparts;
+    P.parts.resize((nmodels + P.per_part - 1) / P.per_part);
+    auto work = [&](size_t q) {
+        PackedPart& part = P.parts[q];
+        const int first = (int)q * P.per_part, n = std::min(P.per_part, nmodels - first);
+        try {
+            part.io.resize(n);
+            part.dof.resize(n);
+            part.fo.resize(n);
+            for (int k = 0; k < n; k++)
+                pack_one(models[first + k], mixed, part.I, part.D, part.Fl, part.io[k], part.dof[k], part.fo[k],
+                         host[first + k]);
+            if (part.I.size() & 3) part.I.resize((part.I.size() + 3) & ~(size_t)3);  // the next part starts 16 B aligned
+        } catch (...) {
+            part.error = std::current_exception();
+        }
+    };
+    std::vector<std::thread> threads;
+    for (size_t q = 1; q < P.parts.size(); q++) {
+        try {
+            threads.emplace_back(work, q);
+        } catch (std::system_error&) {  // no more threads to be had
+            work(q);
+        }
     }
-    out.dmodels.upload(out.host.data(), out.host.size() * sizeof(DModel), e->stream);
-    cuda_check(cudaStreamSynchronize(e->stream), "model upload");
-}
-
-// Host image of the packed models for a caller that places them in device
-// memory it already owns: the int, double and float pools and then the
-// descriptors, each 16 B aligned, with every descriptor pointer aimed at
-// dev_base + its offset in the image.
-void pack_models_image(const sg_model_desc* models, int nmodels, char* dev_base, ModelImage& img) {
-    require(models && nmodels > 0 && nmodels <= (1 << 20), "models: bad array");
-    std::vector<int> I;
-    std::vector<double> D;
-    std::vector<float> Fl;
-    std::vector<std::vector<size_t>> ioffs(nmodels), doffs(nmodels), foffs(nmodels);
-    img.host.assign(nmodels, DModel{});
-    for (int k = 0; k < nmodels; k++) pack_one(models[k], I, D, Fl, ioffs[k], doffs[k], foffs[k], img.host[k]);
+    work(0);
+    for (std::thread& t : threads) t.join();
+    size_t ni = 0, nd = 0, nf = 0;
+    for (PackedPart& part : P.parts) {
+        if (part.error) std::rethrow_exception(part.error);
+        part.i0 = ni;
+        part.d0 = nd;
+        part.f0 = nf;
+        ni += part.I.size();
+        nd += part.D.size();
+        nf += part.Fl.size();
+    }
     auto r16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
-    const size_t oi = 0, od = r16(I.size() * sizeof(int)), of = od + r16(D.size() * sizeof(double));
-    img.dmodel_off = of + r16(Fl.size() * sizeof(float));
-    img.bytes.assign(img.dmodel_off + nmodels * sizeof(DModel), 0);
-    std::memcpy(img.bytes.data() + oi, I.data(), I.size() * sizeof(int));
-    std::memcpy(img.bytes.data() + od, D.data(), D.size() * sizeof(double));
-    std::memcpy(img.bytes.data() + of, Fl.data(), Fl.size() * sizeof(float));
-    const int* ib = reinterpret_cast<const int*>(dev_base + oi);
-    const double* db = reinterpret_cast<const double*>(dev_base + od);
-    const float* fb = reinterpret_cast<const float*>(dev_base + of);
-    for (int k = 0; k < nmodels; k++) {
-        DModel& h = img.host[k];
-        const std::vector<size_t>& io = ioffs[k];
-        const std::vector<size_t>& dd = doffs[k];
-        const std::vector<size_t>& fo = foffs[k];
+    P.od = r16(ni * sizeof(int));
+    P.of = P.od + r16(nd * sizeof(double));
+    P.om = P.of + r16(nf * sizeof(float));
+    P.bytes = P.om + nmodels * sizeof(DModel);
+}
+// aims every descriptor's pointers at dev_base and writes the image (pools, then
+// descriptors, each 16 B aligned)
+static void place_pools(const PackedPools& P, std::vector<DModel>& host, char* dev_base, char* image) {
+    for (size_t k = 0; k < host.size(); k++) {
+        const PackedPart& part = P.parts[k / P.per_part];
+        const size_t m = k % P.per_part;
+        const int* ib = reinterpret_cast<const int*>(dev_base) + part.i0;
+        const double* db = reinterpret_cast<const double*>(dev_base + P.od) + part.d0;
+        const float* fb = reinterpret_cast<const float*>(dev_base + P.of) + part.f0;
+        DModel& h = host[k];
+        const std::vector<size_t>&io = part.io[m], &dd = part.dof[m], &fo = part.fo[m];
         const int** ip[] = {&h.type, &h.fkind, &h.fparent, &h.fbegin, &h.fend, &h.fconf, &h.fdof, &h.atom_frame,
                             &h.level_start, &h.level_frames, &h.child_start, &h.child_list, &h.pairs, &h.pair_group,
                             &h.csr_start, &h.csr, &h.heavy, &h.lig_begin, &h.lig_end, &h.lig_root, &h.lig_pair_end,
@@ -754,23 +972,62 @@ void pack_models_image(const sg_model_desc* models, int nmodels, char* dev_base,
         for (const int** q : ip) *q = ib + io[j++];
         h.pslot = h.npchunks >= 0 ? reinterpret_cast<const uint32_t*>(ib + io[j]) : nullptr;
         const float4** fp[] = {&h.local32, &h.lab32, &h.forigin32, &h.faxis32, &h.finit32};
-        j = 0;
-        for (const float4** q : fp) *q = reinterpret_cast<const float4*>(fb + fo[j++]);
+        for (j = 0; j < fo.size(); j++) *fp[j] = reinterpret_cast<const float4*>(fb + fo[j]);
         const double** dp[] = {&h.charge, &h.local, &h.lab, &h.forigin, &h.faxis, &h.finit};
         j = 0;
         for (const double** q : dp) *q = db + dd[j++];
     }
-    std::memcpy(img.bytes.data() + img.dmodel_off, img.host.data(), nmodels * sizeof(DModel));
+    for (const PackedPart& part : P.parts) {
+        std::memcpy(image + part.i0 * sizeof(int), part.I.data(), part.I.size() * sizeof(int));
+        std::memcpy(image + P.od + part.d0 * sizeof(double), part.D.data(), part.D.size() * sizeof(double));
+        if (!part.Fl.empty())
+            std::memcpy(image + P.of + part.f0 * sizeof(float), part.Fl.data(), part.Fl.size() * sizeof(float));
+    }
+    std::memcpy(image + P.om, host.data(), host.size() * sizeof(DModel));
 }
 
-void ensure_model_maps(sg_engine* e, RecState& r, const PackedModels& pm, const sg_model_desc* models, int nmodels) {
+void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, bool mixed, PackedModels& out) {
+    PackedPools P;
+    pack_pools(models, nmodels, mixed, P, out.host);
+    out.mem.alloc(P.bytes);
+    std::unique_ptr<char[]> image(new char[P.bytes]);
+    place_pools(P, out.host, out.mem.as<char>(), image.get());
+    out.dmodels = reinterpret_cast<DModel*>(out.mem.as<char>() + P.om);
+    io.in(out.mem, image.get(), P.bytes);
+    out.smem64 = Smem64{};
+    for (const DModel& h : out.host) {
+        out.smem64.add(h);
+        out.max_conf = std::max(out.max_conf, h.conf_size);
+        out.max_dof = std::max(out.max_dof, h.dof);
+        out.max_heavy = std::max(out.max_heavy, h.nheavy);
+        out.max_atoms = std::max(out.max_atoms, h.natoms);
+        out.max_pairs = std::max(out.max_pairs, h.npairs);
+        out.max_frames = std::max(out.max_frames, h.nframes);
+    }
+}
+
+// Host image of the packed models for a caller that places them in device
+// memory it already owns, with every descriptor pointer aimed at dev_base + its
+// offset in the image.
+void pack_models_image(const sg_model_desc* models, int nmodels, char* dev_base, ModelImage& img) {
+    PackedPools P;
+    pack_pools(models, nmodels, true, P, img.host);
+    img.dmodel_off = P.om;
+    img.bytes.assign(P.bytes, 0);
+    place_pools(P, img.host, dev_base, img.bytes.data());
+}
+
+void ensure_model_maps(sg_engine* e, RecState& r, const sg_model_desc* models, int nmodels) {
+    bool seen[kNumTypes] = {};
     std::vector<int> types;
     for (int k = 0; k < nmodels; k++)
         for (int i = 0; i < models[k].num_movable; i++) {
             const int t = models[k].atom_type[i];
-            if (t < kNumTypes && !is_h(t)) types.push_back(t);
+            if (t < kNumTypes && !is_h(t) && !seen[t]) {
+                seen[t] = true;
+                types.push_back(t);
+            }
         }
-    (void)pm;
     ensure_maps(e, r, types.data(), (int)types.size());
 }
 
@@ -782,23 +1039,25 @@ Shape64 sg::plain_shape(sg_engine* e, const PackedModels& pm, long long items) {
     return sh;
 }
 
-// device buffer that receives results and is copied back
+// a call's device array: inputs come through the call's copies, results go back
+// the same way
 template <typename T>
 struct Staged {
+    CallIo& io;
+    sg_engine* e;
     sg::DevBuf d;
     size_t n = 0;
-    void make(size_t count, cudaStream_t s, const T* init = nullptr) {
+    Staged(CallIo& io_, sg_engine* e_) : io(io_), e(e_), d(e_) {}
+    void make(size_t count, const T* init = nullptr) {
         n = count;
-        d.alloc(std::max<size_t>(1, n) * sizeof(T));
-        if (init) sg::cuda_check(cudaMemcpyAsync(d.p, init, n * sizeof(T), cudaMemcpyHostToDevice, s), "stage in");
+        if (init && n) io.in(d, init, n * sizeof(T));
+        else d.alloc(std::max<size_t>(1, n) * sizeof(T));
     }
     T* p() { return d.as<T>(); }
-    void zero(cudaStream_t s) {  // for outputs with padding the kernel leaves alone
-        sg::cuda_check(cudaMemsetAsync(d.p, 0, std::max<size_t>(1, n) * sizeof(T), s), "zero output");
+    void zero() {  // for outputs with padding the kernel leaves alone
+        sg::cuda_check(cudaMemsetAsync(d.p, 0, std::max<size_t>(1, n) * sizeof(T), e->stream), "zero output");
     }
-    void fetch(T* host, cudaStream_t s) {
-        if (host && n) sg::cuda_check(cudaMemcpyAsync(host, d.p, n * sizeof(T), cudaMemcpyDeviceToHost, s), "stage out");
-    }
+    void fetch(T* host) { io.out(host, d.p, n * sizeof(T)); }
 };
 
 extern "C" {
@@ -809,17 +1068,18 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
         require(m && confs && v && out_e && out_g && nconfs > 0 && nconfs <= (1 << 24), "eval: bad arguments");
         require(e->has_tables, "no tables set");
         RecState& r = receptor_for(e, rid);
-        PackedModels pm;
-        pack_models(e, m, 1, pm);
-        if (!direct) ensure_model_maps(e, r, pm, m, 1);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, m, 1, !direct && e->precision != SG_PREC_FP64, pm);
+        if (!direct) ensure_model_maps(e, r, m, 1);
         else ensure_cells(e, r);
         const Shape64 sh = plain_shape(e, pm, nconfs);
         const DModel& h = pm.host[0];
-        Staged<double> dc, de, dg, dx;
-        dc.make((size_t)nconfs * h.conf_size, e->stream, confs);
-        de.make(nconfs, e->stream);
-        dg.make((size_t)nconfs * h.dof, e->stream);
-        if (out_coords) dx.make((size_t)nconfs * h.nmov * 3, e->stream);
+        Staged<double> dc(io, e), de(io, e), dg(io, e), dx(io, e);
+        dc.make((size_t)nconfs * h.conf_size, confs);
+        de.make(nconfs);
+        dg.make((size_t)nconfs * h.dof);
+        if (out_coords) dx.make((size_t)nconfs * h.nmov * 3);
         if (!direct && e->precision != SG_PREC_FP64) {  // the mixed-precision evaluation
             require(h.npchunks >= 0, "mixed-precision path: at most 255 atoms per model");
             const size_t ws = (ws32_bytes(h) + 15) & ~(size_t)15;
@@ -827,22 +1087,22 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
                 (size_t)stage32_bytes(h.natoms, h.nframes, h.nheavy, h.npchunks, h.nlig, h.nblocks, h.ntors);
             require(stage + (size_t)std::max(1, e->tpc / 32) * ws <= (size_t)e->max_smem,
                     "model too large for the mixed-precision path's shared memory");
-            cuda_check(launch_eval32(pm.dmodels.as<DModel>(), stage, ws, tables32(e), maps32(e, r), nconfs, dc.p(), v, slope,
+            cuda_check(launch_eval32(pm.dmodels, stage, ws, tables32(e), maps32(e, r), nconfs, dc.p(), v, slope,
                                      de.p(), dg.p(), out_coords ? dx.p() : nullptr, std::max(1, e->tpc / 32), e->stream),
                        "eval launch");
-            de.fetch(out_e, e->stream);
-            dg.fetch(out_g, e->stream);
-            if (out_coords) dx.fetch(out_coords, e->stream);
-            e->check_device_errors();
+            de.fetch(out_e);
+            dg.fetch(out_g);
+            if (out_coords) dx.fetch(out_coords);
+            io.finish();
             return;
         }
-        cuda_check(launch_eval64(pm.dmodels.as<DModel>(), sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
+        cuda_check(launch_eval64(pm.dmodels, sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
                                  slope, direct, de.p(), dg.p(), out_coords ? dx.p() : nullptr, e->d_err.as<int>(), e->stream),
                    "eval launch");
-        de.fetch(out_e, e->stream);
-        dg.fetch(out_g, e->stream);
-        if (out_coords) dx.fetch(out_coords, e->stream);
-        e->check_device_errors();
+        de.fetch(out_e);
+        dg.fetch(out_g);
+        if (out_coords) dx.fetch(out_coords);
+        io.finish();
     });
 }
 
@@ -870,13 +1130,14 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
     return guarded(e, [&] {
         require(m && confs && v && out_e && nconfs > 0 && nconfs <= (1 << 24) && maxiters >= 0, "bfgs: bad arguments");
         RecState& r = receptor_for(e, rid);
-        PackedModels pm;
-        pack_models(e, m, 1, pm);
-        ensure_model_maps(e, r, pm, m, 1);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, m, 1, e->precision != SG_PREC_FP64, pm);
+        ensure_model_maps(e, r, m, 1);
         const DModel& h = pm.host[0];
-        Staged<double> dc, de;
-        dc.make((size_t)nconfs * h.conf_size, e->stream, confs);
-        de.make(nconfs, e->stream);
+        Staged<double> dc(io, e), de(io, e);
+        dc.make((size_t)nconfs * h.conf_size, confs);
+        de.make(nconfs);
         if (e->precision != SG_PREC_FP64) {  // the batched search's mixed-precision BFGS
             require(h.npchunks >= 0, "mixed-precision path: at most 255 atoms per model");
             const size_t ws = (ws32_bytes(h) + 15) & ~(size_t)15;
@@ -884,22 +1145,22 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
                 (size_t)stage32_bytes(h.natoms, h.nframes, h.nheavy, h.npchunks, h.nlig, h.nblocks, h.ntors);
             require(stage + (size_t)std::max(1, e->tpc / 32) * ws <= (size_t)e->max_smem,
                     "model too large for the mixed-precision path's shared memory");
-            cuda_check(launch_bfgs32(pm.dmodels.as<DModel>(), stage, ws, tables32(e), maps32(e, r), nconfs, dc.p(), v,
+            cuda_check(launch_bfgs32(pm.dmodels, stage, ws, tables32(e), maps32(e, r), nconfs, dc.p(), v,
                                      slope, maxiters, accurate_line, early_term, de.p(), std::max(1, e->tpc / 32),
                                      e->stream),
                        "bfgs launch");
-            dc.fetch(confs, e->stream);
-            de.fetch(out_e, e->stream);
-            e->check_device_errors();
+            dc.fetch(confs);
+            de.fetch(out_e);
+            io.finish();
             return;
         }
         const Shape64 sh = plain_shape(e, pm, nconfs);
-        cuda_check(launch_bfgs64(pm.dmodels.as<DModel>(), sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
+        cuda_check(launch_bfgs64(pm.dmodels, sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
                                  slope, maxiters, accurate_line, early_term, de.p(), e->d_err.as<int>(), e->stream),
                    "bfgs launch");
-        dc.fetch(confs, e->stream);
-        de.fetch(out_e, e->stream);
-        e->check_device_errors();
+        dc.fetch(confs);
+        de.fetch(out_e);
+        io.finish();
     });
 }
 
@@ -910,9 +1171,10 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
         require(p->num_saved_mins >= 1 && p->num_saved_mins <= 1024 && p->maxiters >= 0 && p->temperature > 0,
                 "dock: bad search parameters");
         RecState& r = receptor_for(e, rid);
-        PackedModels pm;
-        pack_models(e, models, nmodels, pm);
-        ensure_model_maps(e, r, pm, models, nmodels);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, models, nmodels, false, pm);
+        ensure_model_maps(e, r, models, nmodels);
         const Shape64 sh = plain_shape(e, pm, nchains);
         const int S = p->num_saved_mins;
         // per-chain inputs and result storage (one device allocation each)
@@ -934,11 +1196,11 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
             nxyz_res += (size_t)S * h.nheavy * 3;
             require(out[k].e && out[k].conf && out[k].coords, "dock: null result arrays");
         }
-        Staged<double> d_conf0, d_e, d_conf, d_xyz, d_hist;
-        Staged<uint32_t> d_mt;
-        Staged<unsigned long long> d_histw;
-        Staged<int> d_order, d_count;
-        Staged<unsigned long long> d_evals;
+        Staged<double> d_conf0(io, e), d_e(io, e), d_conf(io, e), d_xyz(io, e), d_hist(io, e);
+        Staged<uint32_t> d_mt(io, e);
+        Staged<unsigned long long> d_histw(io, e);
+        Staged<int> d_order(io, e), d_count(io, e);
+        Staged<unsigned long long> d_evals(io, e);
         // QuickVina 2 histories (MCParams::visited), one block per chain whose dof fits
         std::vector<size_t> hist_off(nchains, SIZE_MAX), histw_off(nchains, SIZE_MAX);
         size_t nhist = 0, nhistw = 0;
@@ -952,18 +1214,18 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
                 nhistw += hist64_words(n);
             }
         if (nhist) {
-            d_hist.make(nhist, e->stream);
-            d_histw.make(nhistw, e->stream);
-            d_histw.zero(e->stream);  // empty histories
+            d_hist.make(nhist);
+            d_histw.make(nhistw);
+            d_histw.zero();  // empty histories
         }
-        d_conf0.make(conf0.size(), e->stream, conf0.data());
-        d_mt.make(mt.size(), e->stream, mt.data());
-        d_e.make((size_t)nchains * S, e->stream);
-        d_conf.make(nconf_res, e->stream);
-        d_xyz.make(nxyz_res, e->stream);
-        d_order.make((size_t)nchains * S, e->stream);
-        d_count.make(nchains, e->stream);
-        d_evals.make(nchains, e->stream);
+        d_conf0.make(conf0.size(), conf0.data());
+        d_mt.make(mt.size(), mt.data());
+        d_e.make((size_t)nchains * S);
+        d_conf.make(nconf_res);
+        d_xyz.make(nxyz_res);
+        d_order.make((size_t)nchains * S);
+        d_count.make(nchains);
+        d_evals.make(nchains);
         std::vector<Chain64> hc(nchains);
         for (int k = 0; k < nchains; k++) {
             hc[k].model = chains[k].model;
@@ -980,8 +1242,8 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
             hc[k].hist = hist_off[k] == SIZE_MAX ? nullptr : d_hist.p() + hist_off[k];
             hc[k].hist_words = histw_off[k] == SIZE_MAX ? nullptr : d_histw.p() + histw_off[k];
         }
-        DevBuf d_chains;
-        d_chains.upload(hc.data(), hc.size() * sizeof(Chain64), e->stream);
+        DevBuf d_chains(e);
+        io.in(d_chains, hc.data(), hc.size() * sizeof(Chain64));
         MCParams64 P;
         P.num_steps = p->num_steps;
         P.temperature = p->temperature;
@@ -993,19 +1255,19 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
         P.accurate_line = p->accurate_line;
         P.early_term = p->early_term;
         P.slope = p->cache_slope;
-        cuda_check(launch_mc64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(),
+        cuda_check(launch_mc64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(),
                                d_chains.as<Chain64>(), nchains, P, nhist > 0, e->d_err.as<int>(), e->stream),
                    "dock launch");
         std::vector<double> he((size_t)nchains * S), hconf(nconf_res), hxyz(nxyz_res);
         std::vector<int> horder((size_t)nchains * S), hcount(nchains);
         std::vector<unsigned long long> hev(nchains);
-        d_e.fetch(he.data(), e->stream);
-        d_conf.fetch(hconf.data(), e->stream);
-        d_xyz.fetch(hxyz.data(), e->stream);
-        d_order.fetch(horder.data(), e->stream);
-        d_count.fetch(hcount.data(), e->stream);
-        d_evals.fetch(hev.data(), e->stream);
-        e->check_device_errors();
+        d_e.fetch(he.data());
+        d_conf.fetch(hconf.data());
+        d_xyz.fetch(hxyz.data());
+        d_order.fetch(horder.data());
+        d_count.fetch(hcount.data());
+        d_evals.fetch(hev.data());
+        io.finish();
         for (int k = 0; k < nchains; k++) {
             const DModel& h = pm.host[chains[k].model];
             const int cnt = std::min(std::max(hcount[k], 0), S);
@@ -1031,26 +1293,27 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
         require(pose_model && confs && cap && out_e && nposes > 0 && maxiters >= 0, "refine: bad arguments");
         RecState& r = receptor_for(e, rid);
         ensure_cells(e, r);
-        PackedModels pm;
-        pack_models(e, models, nmodels, pm);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, models, nmodels, false, pm);
         const Shape64 sh = plain_shape(e, pm, nposes);
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "refine: bad pose model");
         const int cs = pm.max_conf, hs = pm.max_heavy;
-        Staged<double> dc, de, dx;
-        Staged<int> dpm;
-        dc.make((size_t)nposes * cs, e->stream, confs);
-        de.make(nposes, e->stream);
-        dx.make((size_t)nposes * hs * 3, e->stream);
-        dx.zero(e->stream);  // atoms past a pose's heavy count stay 0
-        dpm.make(nposes, e->stream, pose_model);
-        cuda_check(launch_refine64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(), nposes,
+        Staged<double> dc(io, e), de(io, e), dx(io, e);
+        Staged<int> dpm(io, e);
+        dc.make((size_t)nposes * cs, confs);
+        de.make(nposes);
+        dx.make((size_t)nposes * hs * 3);
+        dx.zero();  // atoms past a pose's heavy count stay 0
+        dpm.make(nposes, pose_model);
+        cuda_check(launch_refine64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(), nposes,
                                    dc.p(), cs, cap, maxiters, nullptr, nullptr, accurate_line, early_term, de.p(), dx.p(), hs,
                                    e->d_err.as<int>(), e->stream),
                    "refine launch");
-        dc.fetch(confs, e->stream);
-        de.fetch(out_e, e->stream);
-        if (out_coords) dx.fetch(out_coords, e->stream);
-        e->check_device_errors();
+        dc.fetch(confs);
+        de.fetch(out_e);
+        if (out_coords) dx.fetch(out_coords);
+        io.finish();
     });
 }
 
@@ -1086,29 +1349,30 @@ int sg_score(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, co
         require(e->has_tables, "no tables set");
         RecState& r = receptor_for(e, rid);
         ensure_cells(e, r);
-        PackedModels pm;
-        pack_models(e, models, nmodels, pm);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, models, nmodels, false, pm);
         const Shape64 sh = plain_shape(e, pm, nposes);
         require(conf_stride >= pm.max_conf && (!out_coords || coord_stride >= pm.max_heavy), "score: strides too small");
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "score: bad pose model");
-        Staged<double> dc, de, di, dx;
-        Staged<int> dpm;
-        dc.make((size_t)nposes * conf_stride, e->stream, confs);
-        de.make(nposes, e->stream);
-        di.make(nposes, e->stream);
+        Staged<double> dc(io, e), de(io, e), di(io, e), dx(io, e);
+        Staged<int> dpm(io, e);
+        dc.make((size_t)nposes * conf_stride, confs);
+        de.make(nposes);
+        di.make(nposes);
         if (out_coords) {
-            dx.make((size_t)nposes * coord_stride * 3, e->stream);
-            dx.zero(e->stream);  // atoms past a pose's heavy count stay 0
+            dx.make((size_t)nposes * coord_stride * 3);
+            dx.zero();  // atoms past a pose's heavy count stay 0
         }
-        dpm.make(nposes, e->stream, pose_model);
-        cuda_check(launch_score64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
+        dpm.make(nposes, pose_model);
+        cuda_check(launch_score64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
                                   nposes, dc.p(), conf_stride, v, slope, de.p(), di.p(), out_coords ? dx.p() : nullptr,
                                   coord_stride, e->d_err.as<int>(), e->stream),
                    "score launch");
-        de.fetch(out_e, e->stream);
-        di.fetch(out_intra, e->stream);
-        if (out_coords) dx.fetch(out_coords, e->stream);
-        e->check_device_errors();
+        de.fetch(out_e);
+        di.fetch(out_intra);
+        if (out_coords) dx.fetch(out_coords);
+        io.finish();
     });
 }
 
@@ -1119,8 +1383,9 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
         require(pose_model && confs && cap && maxiters && out_e && nposes > 0, "minimize: bad arguments");
         RecState& r = receptor_for(e, rid);
         ensure_cells(e, r);
-        PackedModels pm;
-        pack_models(e, models, nmodels, pm);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, models, nmodels, false, pm);
         const Shape64 sh = plain_shape(e, pm, nposes);
         require(conf_stride >= pm.max_conf && coord_stride >= pm.max_heavy, "minimize: strides too small");
         for (int k = 0; k < nposes; k++) {
@@ -1131,24 +1396,24 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
                                 boxes[6 * k + d] <= boxes[6 * k + 3 + d],
                             "minimize: a pose's box must lie inside the receptor's box");
         }
-        Staged<double> dc, de, dx, db;
-        Staged<int> dpm, dmi;
-        dc.make((size_t)nposes * conf_stride, e->stream, confs);
-        de.make(nposes, e->stream);
-        dx.make((size_t)nposes * coord_stride * 3, e->stream);
-        dx.zero(e->stream);  // atoms past a pose's heavy count stay 0
-        dpm.make(nposes, e->stream, pose_model);
-        dmi.make(nposes, e->stream, maxiters);
-        if (boxes) db.make((size_t)nposes * 6, e->stream, boxes);
-        cuda_check(launch_refine64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
+        Staged<double> dc(io, e), de(io, e), dx(io, e), db(io, e);
+        Staged<int> dpm(io, e), dmi(io, e);
+        dc.make((size_t)nposes * conf_stride, confs);
+        de.make(nposes);
+        dx.make((size_t)nposes * coord_stride * 3);
+        dx.zero();  // atoms past a pose's heavy count stay 0
+        dpm.make(nposes, pose_model);
+        dmi.make(nposes, maxiters);
+        if (boxes) db.make((size_t)nposes * 6, boxes);
+        cuda_check(launch_refine64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(), dpm.p(),
                                    nposes, dc.p(), conf_stride, cap, 0, dmi.p(), boxes ? db.p() : nullptr,
                                    accurate_line, early_term, de.p(), dx.p(), coord_stride, e->d_err.as<int>(),
                                    e->stream),
                    "minimize launch");
-        dc.fetch(confs, e->stream);
-        de.fetch(out_e, e->stream);
-        if (out_coords) dx.fetch(out_coords, e->stream);
-        e->check_device_errors();
+        dc.fetch(confs);
+        de.fetch(out_e);
+        if (out_coords) dx.fetch(out_coords);
+        io.finish();
     });
 }
 

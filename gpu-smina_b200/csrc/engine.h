@@ -1,11 +1,15 @@
 // Engine state behind the C ABI.
 #pragma once
+#include <memory>
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <cstdint>
 #include <vector>
 #include "sg_dev.cuh"
+
+struct sg_engine;
 
 namespace sg {
 
@@ -20,17 +24,77 @@ inline void require(bool ok, const std::string& msg) {
     if (!ok) throw EngineError(SG_ERR_ARG, msg);
 }
 
-// owning device allocation
+// Owning device memory.  DevBuf(engine) is a call's temporary: it comes from the
+// engine's stream-ordered pool and goes back to it on the engine's stream.
+// DevBuf() belongs to a receptor or the engine: its own allocation, kept when a
+// later one fits it without wasting half.
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     DevBuf() = default;
+    explicit DevBuf(sg_engine* e) : pool_of(e) {}
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { reset(); }
     void reset();
     void alloc(size_t n);
     void upload(const void* src, size_t n, cudaStream_t s);
+    template <typename T> T* as() const { return reinterpret_cast<T*>(p); }
+
+private:
+    sg_engine* pool_of = nullptr;
+    size_t cap = 0;
+};
+
+// Copies between the caller's memory and the device for one call, in pieces
+// through a small ring of pinned memory (PinRing): a piece is copied by the host
+// while the one before is in flight.  Inputs go at once; outputs are listed and
+// fetched by finish(), after which the caller's arrays are filled.  (Straight
+// from and to pageable memory each copy waited for the one before: 20,000
+// evaluations of a 13-dof ligand, 4.5 MB both ways, took 2.1 ms a call and take
+// 0.68 ms; 2 MB of pinned memory is enough for that, while pinning the whole
+// transfer cost a first call 6 ms.)
+struct PinRing {
+    static constexpr size_t kSlot = size_t(512) << 10;
+    static constexpr int kSlots = 4;  // two for inputs, two for outputs
+    char* p = nullptr;
+    cudaEvent_t ev[kSlots] = {};
+    ~PinRing();
+};
+class CallIo {
+public:
+    explicit CallIo(sg_engine* e) : e_(e) {}
+    CallIo(const CallIo&) = delete;
+    CallIo& operator=(const CallIo&) = delete;
+    ~CallIo();
+    void in(DevBuf& dst, const void* src, size_t n);   // allocates dst
+    void out(void* host, const void* dev, size_t n);   // dev stays as it is until finish()
+    void finish();                                     // throws the device's error, if it reported one
+
+private:
+    struct Out { void* host; const void* dev; size_t n; };
+    struct Piece { void* host; const char* from; size_t n; };
+    void need_ring();
+    sg_engine* e_;
+    std::unique_ptr<PinRing> ring_;
+    int in_slot_ = 0;
+    size_t in_used_ = 0;
+    bool in_sent_[2] = {};
+    std::vector<Out> outs_;
+    bool busy_ = false;
+};
+// a ring for the process's next call, so that the first call need not pin one
+void warm_pin_ring();
+// The device's pool of call temporaries, shared by its engines and destroyed with
+// the last of them; it keeps at most kPoolKept bytes between calls.
+constexpr size_t kPoolKept = size_t(256) << 20;
+cudaMemPool_t pool_acquire(int device);
+void pool_release(int device);
+
+// one grid map within its receptor's allocation
+struct MapView {
+    void* p = nullptr;
+    size_t bytes = 0;
     template <typename T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
@@ -43,8 +107,13 @@ struct RecState {
     DGeom geom{};
     int natoms = 0;
     DevBuf xyz, type, charge, pop_start, pop_atoms, full_start, full_list, full_charge;
-    DevBuf map64[kNumTypes], cmap64[kNumTypes], map32[kNumTypes], cmap32[kNumTypes], map16[kNumTypes];
+    // the maps of one build share an allocation; those of maps dropped for a new
+    // receptor in this place wait in `spare` for the next build, which takes one
+    // that fits and frees the others
+    std::vector<std::unique_ptr<DevBuf>> map_mem, spare;
+    MapView map64[kNumTypes], cmap64[kNumTypes], map32[kNumTypes], cmap32[kNumTypes], map16[kNumTypes];
     bool built[kNumTypes] = {};
+    bool cells = false;  // the cell lists are those of the present receptor
     DevBuf ugrid;  // user grid values, or empty
     DGeom ug{};
     double ug_slope = 1e6;
@@ -52,9 +121,11 @@ struct RecState {
     DReceptor hdr{};
     void clear_maps() {
         for (int t = 0; t < kNumTypes; t++) {
-            map64[t].reset(); cmap64[t].reset(); map32[t].reset(); cmap32[t].reset(); map16[t].reset();
+            map64[t] = cmap64[t] = map32[t] = cmap32[t] = map16[t] = MapView{};
             built[t] = false;
         }
+        for (auto& m : map_mem) spare.push_back(std::move(m));
+        map_mem.clear();
     }
     size_t map_bytes() const {
         size_t b = 0;
@@ -67,7 +138,9 @@ struct RecState {
 // a batch of models packed for the device
 struct PackedModels {
     std::vector<DModel> host;  // host copies with device pointers
-    DevBuf ints, dbls, flts, dmodels;
+    DevBuf mem;                // pools and descriptors
+    DModel* dmodels = nullptr;
+    explicit PackedModels(sg_engine* e) : mem(e) {}
     Smem64 smem64;  // plain-path shared memory
     int max_conf = 0, max_dof = 0, max_heavy = 0, max_atoms = 0, max_pairs = 0, max_frames = 0;
 };
@@ -93,8 +166,8 @@ struct sg_engine {
     sg::DTables tables{};
     sg::RecState rec[SG_MAX_RECEPTORS];
     sg::DevBuf d_err;
+    cudaMemPool_t pool = nullptr;  // temporaries of the calls
     ~sg_engine();
-    void check_device_errors();
 };
 
 namespace sg {
@@ -169,7 +242,8 @@ cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, const DTables3
 // FP32 views of the engine's tables and of a receptor's packed maps
 DTables32 tables32(const sg_engine* e);
 DMaps32 maps32(const sg_engine* e, const RecState& r);
-void pack_models(sg_engine* e, const sg_model_desc* models, int nmodels, PackedModels& out);
+// mixed: with the mixed-precision path's copies and pair schedules
+void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, bool mixed, PackedModels& out);
 // the plain-path launch of a batch of models; refuses a model that does not fit
 Shape64 plain_shape(sg_engine* e, const PackedModels& pm, long long items);
 struct ModelImage {
@@ -181,7 +255,7 @@ void pack_models_image(const sg_model_desc* models, int nmodels, char* dev_base,
 RecState& receptor_for(sg_engine* e, int rid);
 void ensure_cells(sg_engine* e, RecState& r);
 void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes);
-void ensure_model_maps(sg_engine* e, RecState& r, const PackedModels& pm, const sg_model_desc* models, int nmodels);
+void ensure_model_maps(sg_engine* e, RecState& r, const sg_model_desc* models, int nmodels);
 void refresh_header(sg_engine* e, RecState& r);
 void serve_shutdown(sg_engine* e);  // stops the engine's request loop, if one runs
 // chains per block and resident blocks per SM of a k_mc32 launch (honours

@@ -132,11 +132,12 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         require(!p->visited, "the QuickVina 2 history (visited) runs on the plain path only");
         require(e->has_tables, "no tables set");
         RecState& r = receptor_for(e, rid);
-        PackedModels pm;
-        pack_models(e, models, nmodels, pm);
-        ensure_model_maps(e, r, pm, models, nmodels);
+        CallIo io(e);
+        PackedModels pm(e);
+        pack_models(io, models, nmodels, true, pm);
+        ensure_model_maps(e, r, models, nmodels);
         check_packed(e, r, models, nmodels);
-        uint64_t h2d = pm.ints.bytes + pm.flts.bytes + pm.dbls.bytes + pm.dmodels.bytes, d2h = 0;
+        uint64_t h2d = pm.mem.bytes, d2h = 0;
         size_t ws_stride = 0, stage_stride = 0;
         for (const DModel& h : pm.host) {
             require(h.npchunks >= 0, "mixed-precision path: at most 255 atoms per model");
@@ -176,7 +177,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         }
         const int nchains = (int)hc.size();
         require(nchains <= (1 << 24), "dock_batch32: too many chains");
-        DevBuf d_e, d_conf, d_xyz, d_order, d_count, d_evals, d_hits, d_queue;
+        DevBuf d_e(e), d_conf(e), d_xyz(e), d_order(e), d_count(e), d_evals(e), d_hits(e), d_queue(e);
         d_e.alloc((size_t)nchains * S * sizeof(double));
         d_conf.alloc(std::max<size_t>(1, nconf_res) * sizeof(double));
         d_xyz.alloc(std::max<size_t>(1, nxyz_res) * sizeof(float));
@@ -244,7 +245,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         }
         const int nphases = es_n - es_first + 1;
         std::vector<size_t> res_off(nchains, 0);
-        DevBuf d_resume;
+        DevBuf d_resume(e);
         if (phased) {
             size_t nres = 0;
             for (int k = 0; k < nchains; k++) {
@@ -258,7 +259,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         std::vector<unsigned> done(nchains, 0);
         std::vector<char> stopped(njobs, 0);
         std::vector<double> hres;
-        DevBuf d_chains, d_items;
+        DevBuf d_chains(e), d_items(e);
         float mc_ms = 0;
         int first_blocks = 0;
         cudaEvent_t ev[4];
@@ -303,12 +304,12 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
             const int nitems = (int)queue.size();
             const int blocks = (int)std::min<long long>((long long)occ * e->num_sms, nitems);
             if (ph == 0) first_blocks = blocks;
-            d_chains.upload(hc.data(), hc.size() * sizeof(Chain32), e->stream);
-            d_items.upload(queue.data(), queue.size() * sizeof(Item32), e->stream);
+            io.in(d_chains, hc.data(), hc.size() * sizeof(Chain32));
+            io.in(d_items, queue.data(), queue.size() * sizeof(Item32));
             h2d += d_chains.bytes + d_items.bytes;
             cuda_check(cudaMemsetAsync(d_queue.p, 0, sizeof(unsigned), e->stream), "queue reset");
             cuda_check(cudaEventRecord(ev[0], e->stream), "event");
-            cuda_check(launch_mc32(pm.dmodels.as<DModel>(), tables32(e), maps32(e, r), nullptr, d_chains.as<Chain32>(),
+            cuda_check(launch_mc32(pm.dmodels, tables32(e), maps32(e, r), nullptr, d_chains.as<Chain32>(),
                                    d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wpb * team,
                                    stage_stride, ws_stride, team, e->stream),
                        "search launch");
@@ -356,7 +357,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         std::vector<unsigned long long> hev(nchains), hhits(2 * (size_t)nchains);
         auto fetch = [&](void* dst, const DevBuf& src, size_t bytes) {
             if (!bytes) return;
-            cuda_check(cudaMemcpyAsync(dst, src.p, bytes, cudaMemcpyDeviceToHost, e->stream), "fetch results");
+            io.out(dst, src.p, bytes);
             d2h += bytes;
         };
         fetch(he.data(), d_e, he.size() * sizeof(double));
@@ -366,7 +367,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         fetch(hcount.data(), d_count, hcount.size() * sizeof(int));
         fetch(hev.data(), d_evals, hev.size() * sizeof(unsigned long long));
         fetch(hhits.data(), d_hits, hhits.size() * sizeof(unsigned long long));
-        cuda_check(cudaStreamSynchronize(e->stream), "search");
+        io.finish();
         // merge_output_containers per ligand (chains in job order)
         std::vector<std::vector<HostPose>> merged(njobs);
         std::vector<uint64_t> job_evals(njobs, 0);
@@ -409,15 +410,15 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                         pmaxit[q] = jobs[j].maxiters > 0 ? jobs[j].maxiters : p->maxiters;
                         q++;
                     }
-                DevBuf dc, de, dx, dpm, dmi;
-                dc.upload(confs.data(), confs.size() * sizeof(double), e->stream);
-                dpm.upload(pmodel.data(), pmodel.size() * sizeof(int), e->stream);
-                dmi.upload(pmaxit.data(), pmaxit.size() * sizeof(int), e->stream);
+                DevBuf dc(e), de(e), dx(e), dpm(e), dmi(e);
+                io.in(dc, confs.data(), confs.size() * sizeof(double));
+                io.in(dpm, pmodel.data(), pmodel.size() * sizeof(int));
+                io.in(dmi, pmaxit.data(), pmaxit.size() * sizeof(int));
                 h2d += dc.bytes + dpm.bytes + dmi.bytes;
                 de.alloc((size_t)nposes * sizeof(double));
                 dx.alloc((size_t)nposes * hs * 3 * sizeof(double));
                 cuda_check(cudaEventRecord(ev[2], e->stream), "event");
-                cuda_check(launch_refine64(pm.dmodels.as<DModel>(), sh, e->tables, r.dhdr.as<DReceptor>(),
+                cuda_check(launch_refine64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(),
                                            dpm.as<int>(), nposes, dc.as<double>(), cs, p->authentic_v, p->maxiters,
                                            dmi.as<int>(), nullptr, p->accurate_line, p->early_term, de.as<double>(),
                                            dx.as<double>(), hs, e->d_err.as<int>(), e->stream),
@@ -427,7 +428,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 fetch(confs.data(), dc, confs.size() * sizeof(double));
                 fetch(re.data(), de, re.size() * sizeof(double));
                 fetch(rx.data(), dx, rx.size() * sizeof(double));
-                e->check_device_errors();
+                io.finish();
                 cuda_check(cudaEventElapsedTime(&ref_ms, ev[2], ev[3]), "event time");
                 q = 0;
                 for (int j = 0; j < njobs; j++) {
