@@ -203,11 +203,6 @@ __device__ __forceinline__ int type_pair64(int ta, int tb, bool& sw) {
     return sw ? tri_index(tb, ta) : tri_index(ta, tb);
 }
 
-__device__ __forceinline__ CellAtom load_cell_atom(const CellAtom* p) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    return CellAtom{a.x, a.y, b.x, __double2loint(b.y), 0};
-}
-
 // ---- receptor terms -------------------------------------------------------------------------
 // cache::eval_deriv: per movable atom grid energy and derivative
 template <bool ST>

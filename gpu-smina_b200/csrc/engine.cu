@@ -369,8 +369,6 @@ void refresh_header(sg_engine* e, RecState& r) {
     h.xyz = r.xyz.as<double>();
     h.type = r.type.as<int>();
     h.charge = r.charge.as<double>();
-    h.pop_start = r.pop_start.as<int>();
-    h.pop_atoms = r.pop_atoms.as<int>();
     h.full_start = r.full_start.as<int>();
     h.full_list = r.full_list.as<CellAtom>();
     h.full_charge = r.full_charge.as<double>();
@@ -387,32 +385,6 @@ void refresh_header(sg_engine* e, RecState& r) {
     if (!r.dhdr.p) r.dhdr.alloc(sizeof(DReceptor));
     cuda_check(cudaMemcpyAsync(r.dhdr.p, &h, sizeof(DReceptor), cudaMemcpyHostToDevice, e->stream), "receptor header");
     cuda_check(cudaStreamSynchronize(e->stream), "receptor header");
-}
-
-// build one family of cell lists (CSR) on the device; returns the lists' length
-static int build_cells(sg_engine* e, RecState& r, const std::vector<double>& lo, const std::vector<double>& hi,
-                        DevBuf& start, DevBuf& atoms) {
-    const DGeom& g = r.geom;
-    const int ncells = g.cell_dim[0] * g.cell_dim[1] * g.cell_dim[2];
-    DevBuf dlo(e), dhi(e), dcount(e);
-    dlo.upload(lo.data(), lo.size() * sizeof(double), e->stream);
-    dhi.upload(hi.data(), hi.size() * sizeof(double), e->stream);
-    dcount.alloc(ncells * sizeof(int));
-    cuda_check(launch_cell_lists(r.natoms, r.xyz.as<double>(), r.type.as<int>(), g, e->tables.cutoff_sqr,
-                                 dlo.as<double>(), dhi.as<double>(), dcount.as<int>(), nullptr, nullptr, 0, e->stream),
-               "cell count");
-    std::vector<int> cnt(ncells), st(ncells + 1, 0);
-    cuda_check(cudaMemcpyAsync(cnt.data(), dcount.p, ncells * sizeof(int), cudaMemcpyDeviceToHost, e->stream), "counts");
-    cuda_check(cudaStreamSynchronize(e->stream), "cell count");
-    for (int c = 0; c < ncells; c++) st[c + 1] = st[c] + cnt[c];
-    start.upload(st.data(), st.size() * sizeof(int), e->stream);
-    atoms.alloc(std::max(1, st[ncells]) * sizeof(int));
-    cuda_check(launch_cell_lists(r.natoms, r.xyz.as<double>(), r.type.as<int>(), g, e->tables.cutoff_sqr,
-                                 dlo.as<double>(), dhi.as<double>(), nullptr, start.as<int>(), atoms.as<int>(), 1,
-                                 e->stream),
-               "cell fill");
-    cuda_check(cudaStreamSynchronize(e->stream), "cell fill");
-    return st[ncells];
 }
 
 // Brick of every cell along each axis.  Populate: the first grid point of
@@ -443,20 +415,41 @@ static void cell_bricks(const DGeom& g, bool first_query, std::vector<double>& l
     }
 }
 
-// the receptor's 3 A cell lists (first-query bricks for the maps, full
-// bricks with whole atoms for the direct sum)
+// the receptor's 3 A cell lists (CSR, whole atoms): first-query bricks for the
+// maps, full bricks for the direct sum
 static void build_receptor_cells(sg_engine* e, RecState& r) {
-    std::vector<double> lo, hi;
-    cell_bricks(r.geom, true, lo, hi);
-    build_cells(e, r, lo, hi, r.pop_start, r.pop_atoms);
-    cell_bricks(r.geom, false, lo, hi);
-    DevBuf full_atoms(e);
-    const int n = build_cells(e, r, lo, hi, r.full_start, full_atoms);
-    r.full_list.alloc(std::max(1, n) * sizeof(CellAtom));
-    r.full_charge.alloc(std::max(1, n) * sizeof(double));
-    cuda_check(launch_cell_pack(n, full_atoms.as<int>(), r.xyz.as<double>(), r.type.as<int>(), r.charge.as<double>(),
-                                r.full_list.as<CellAtom>(), r.full_charge.as<double>(), e->stream),
-               "cell atoms");
+    const DGeom& g = r.geom;
+    const int ncells = g.cell_dim[0] * g.cell_dim[1] * g.cell_dim[2];
+    std::vector<double> bricks, lo, hi;
+    for (int f = 0; f < 2; f++) {
+        cell_bricks(g, f == 0, lo, hi);
+        bricks.insert(bricks.end(), lo.begin(), lo.end());
+        bricks.insert(bricks.end(), hi.begin(), hi.end());
+    }
+    DevBuf dbricks(e), dcount(e);
+    dbricks.upload(bricks.data(), bricks.size() * sizeof(double), e->stream);
+    dcount.alloc(2 * (size_t)ncells * sizeof(int));
+    auto launch = [&](const CellFamily& pop, const CellFamily& full) {
+        return launch_cell_lists(r.natoms, r.xyz.as<double>(), r.type.as<int>(), r.charge.as<double>(), g,
+                                 e->tables.cutoff_sqr, dbricks.as<double>(), dcount.as<int>(), pop, full, r.slots,
+                                 e->stream);
+    };
+    cuda_check(launch({}, {}), "cell count");
+    std::vector<int> cnt(2 * (size_t)ncells), st[2];
+    cuda_check(cudaMemcpyAsync(cnt.data(), dcount.p, cnt.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream), "counts");
+    cuda_check(cudaStreamSynchronize(e->stream), "cell count");
+    DevBuf* const bufs[2][3] = {{&r.pop_start, &r.pop_list, &r.pop_charge}, {&r.full_start, &r.full_list, &r.full_charge}};
+    CellFamily fam[2];
+    for (int f = 0; f < 2; f++) {
+        st[f].assign(ncells + 1, 0);
+        for (int c = 0; c < ncells; c++) st[f][c + 1] = st[f][c] + cnt[(size_t)f * ncells + c];
+        const size_t n = std::max(1, st[f][ncells]);
+        bufs[f][0]->upload(st[f].data(), st[f].size() * sizeof(int), e->stream);
+        bufs[f][1]->alloc(n * sizeof(CellAtom));
+        bufs[f][2]->alloc(n * sizeof(double));
+        fam[f] = {bufs[f][0]->as<int>(), bufs[f][1]->as<CellAtom>(), bufs[f][2]->as<double>()};
+    }
+    cuda_check(launch(fam[0], fam[1]), "cell fill");
     refresh_header(e, r);
     r.cells = true;
 }
@@ -511,24 +504,33 @@ void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
         cmaps.push_back(r.cmap64[t].as<double>());
     }
     r.map_mem.push_back(std::move(mem));
-    DevBuf dtypes(e), dmaps(e), dcmaps(e);
-    dtypes.upload(need.data(), need.size() * sizeof(int), e->stream);
-    dmaps.upload(maps.data(), maps.size() * sizeof(double*), e->stream);
-    dcmaps.upload(cmaps.data(), cmaps.size() * sizeof(double*), e->stream);
-    cuda_check(launch_grid_map64(r.geom, r.natoms, r.xyz.as<double>(), r.type.as<int>(), r.charge.as<double>(),
-                                 r.pop_start.as<int>(), r.pop_atoms.as<int>(), e->tables, dtypes.as<int>(), (int)need.size(),
-                                 dmaps.as<double*>(), dcmaps.as<double*>(), r.ugrid.as<double>(), r.ug, r.ug_slope,
-                                 e->stream),
-               "grid maps");
+    // one upload: map pointers, charge map pointers, maps to pack, type numbers
+    const size_t nt = need.size();
+    std::vector<GridPack> packs;
     if (packed)
         for (int t : need) {
-            cuda_check(launch_grid_pack(r.geom, r.map64[t].as<double>(), r.map32[t].as<float4>(), r.map16[t].as<uint4>(),
-                                        e->stream),
-                       "pack maps");
-            if (charged)
-                cuda_check(launch_grid_pack(r.geom, r.cmap64[t].as<double>(), r.cmap32[t].as<float4>(), nullptr, e->stream),
-                           "pack charge maps");
+            packs.push_back({r.map64[t].as<double>(), r.map32[t].as<float4>(), r.map16[t].as<uint4>()});
+            if (charged) packs.push_back({r.cmap64[t].as<double>(), r.cmap32[t].as<float4>(), nullptr});
         }
+    const size_t at_packs = 2 * nt * sizeof(double*), at_types = at_packs + packs.size() * sizeof(GridPack);
+    std::vector<char> args(at_types + nt * sizeof(int));
+    std::memcpy(args.data(), maps.data(), nt * sizeof(double*));
+    std::memcpy(args.data() + nt * sizeof(double*), cmaps.data(), nt * sizeof(double*));
+    if (!packs.empty()) std::memcpy(args.data() + at_packs, packs.data(), packs.size() * sizeof(GridPack));
+    std::memcpy(args.data() + at_types, need.data(), nt * sizeof(int));
+    DevBuf dargs(e), dtab(e);
+    dargs.upload(args.data(), args.size(), e->stream);
+    double** dmaps = dargs.as<double*>();
+    const int* dtypes = reinterpret_cast<const int*>(dargs.as<char>() + at_types);
+    dtab.alloc(std::max<size_t>(1, (size_t)r.slots.count * e->tables.n * grid_lanes((int)nt) * e->tables.nc) * sizeof(double));
+    cuda_check(launch_grid_map64(r.geom, r.pop_list.as<CellAtom>(), r.pop_charge.as<double>(), r.pop_start.as<int>(),
+                                 e->tables, dtypes, (int)nt, r.slots, dtab.as<double>(), dmaps, dmaps + nt,
+                                 r.ugrid.as<double>(), r.ug, r.ug_slope, e->num_sms, e->stream),
+               "grid maps");
+    if (packed)
+        cuda_check(launch_grid_pack(r.geom, reinterpret_cast<const GridPack*>(dargs.as<char>() + at_packs),
+                                    (int)packs.size(), e->stream),
+                   "pack maps");
     cuda_check(cudaStreamSynchronize(e->stream), "grid maps");
     for (int t : need) r.built[t] = true;
     refresh_header(e, r);
@@ -560,6 +562,12 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
         s.natoms = r->num_atoms;
         std::vector<int> types(r->type, r->type + r->num_atoms);
         for (int& t : types) if (t < 0 || t > kNumTypes) t = kNumTypes;
+        s.slots = GridSlots{};
+        for (int t = 0; t < kNumTypes; t++)
+            if (!is_h(t) && std::find(types.begin(), types.end(), t) != types.end()) {
+                s.slots.of[t] = (short)s.slots.count;
+                s.slots.type[s.slots.count++] = (short)t;
+            }
         s.xyz.upload(r->coords, sizeof(double) * 3 * std::max(1, r->num_atoms), e->stream);
         s.type.upload(types.data(), sizeof(int) * std::max<size_t>(1, types.size()), e->stream);
         s.charge.upload(r->charge, sizeof(double) * std::max(1, r->num_atoms), e->stream);
@@ -616,8 +624,8 @@ int sg_drop_receptor(sg_engine* e, int rid) {
         RecState& s = e->rec[rid];
         s.clear_maps();
         s.spare.clear();
-        s.pop_start.reset(); s.pop_atoms.reset(); s.full_start.reset();
-        s.full_list.reset(); s.full_charge.reset();
+        s.pop_start.reset(); s.pop_list.reset(); s.pop_charge.reset();
+        s.full_start.reset(); s.full_list.reset(); s.full_charge.reset();
         s.xyz.reset(); s.type.reset(); s.charge.reset(); s.dhdr.reset(); s.ugrid.reset();
         s.set = s.cells = false;
     });

@@ -106,13 +106,14 @@ struct RecState {
     sg_grid_dims gd{};
     DGeom geom{};
     int natoms = 0;
-    DevBuf xyz, type, charge, pop_start, pop_atoms, full_start, full_list, full_charge;
+    DevBuf xyz, type, charge, pop_start, pop_list, pop_charge, full_start, full_list, full_charge;
     // the maps of one build share an allocation; those of maps dropped for a new
     // receptor in this place wait in `spare` for the next build, which takes one
     // that fits and frees the others
     std::vector<std::unique_ptr<DevBuf>> map_mem, spare;
     MapView map64[kNumTypes], cmap64[kNumTypes], map32[kNumTypes], cmap32[kNumTypes], map16[kNumTypes];
     bool built[kNumTypes] = {};
+    GridSlots slots{};   // heavy atom types that occur in the receptor
     bool cells = false;  // the cell lists are those of the present receptor
     DevBuf ugrid;  // user grid values, or empty
     DGeom ug{};
@@ -194,14 +195,15 @@ int guarded(sg_engine* e, F f) {
 }
 
 // ---- launchers defined in the kernel files ---------------------------------------------------
-cudaError_t launch_cell_lists(int, const double*, const int*, const DGeom&, double, const double*, const double*, int*,
-                              const int*, int*, int, cudaStream_t);
-cudaError_t launch_grid_map64(const DGeom&, int, const double*, const int*, const double*, const int*, const int*,
-                              const DTables&, const int*, int, double**, double**, const double* ugrid,
-                              const DGeom& ug, double ug_slope, cudaStream_t);
-cudaError_t launch_grid_pack(const DGeom&, const double*, float4*, uint4*, cudaStream_t);
-cudaError_t launch_cell_pack(int n, const int* atoms, const double* xyz, const int* type, const double* charge,
-                             CellAtom* list, double* list_charge, cudaStream_t s);
+cudaError_t launch_cell_lists(int natoms, const double* xyz, const int* type, const double* charge, const DGeom& g,
+                              double cutoff_sqr, const double* bricks, int* count, const CellFamily& fam0,
+                              const CellFamily& fam1, const GridSlots& slots, cudaStream_t s);
+int grid_lanes(int ntypes);
+cudaError_t launch_grid_map64(const DGeom&, const CellAtom* list, const double* list_charge, const int* cstart,
+                              const DTables&, const int* types, int ntypes, const GridSlots&, double* tab,
+                              double** maps, double** cmaps, const double* ugrid, const DGeom& ug, double ug_slope,
+                              int num_sms, cudaStream_t);
+cudaError_t launch_grid_pack(const DGeom&, const GridPack* maps, int nmaps, cudaStream_t);
 // warps per item and shared memory of a plain-path launch over `items` items
 // within max_smem bytes per block
 Shape64 shape64(const Smem64& s, long long items, int num_sms, size_t max_smem);

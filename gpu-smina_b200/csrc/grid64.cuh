@@ -9,6 +9,11 @@
 
 namespace sg {
 
+__device__ __forceinline__ CellAtom load_cell_atom(const CellAtom* p) {
+    const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+    return CellAtom{a.x, a.y, b.x, __double2loint(b.y), __double2hiint(b.y)};
+}
+
 struct Trilin64 {
     double f000, f100, f010, f110, f001, f101, f011, f111;
     double x, y, z, penalty;

@@ -33,11 +33,30 @@ struct DGeom {
     int cell_off[3], cell_dim[3];
 };
 
-// one receptor atom of a direct-sum cell list, whole: two 16-byte loads side by
+// the receptor's atom types, numbered as they occur (map construction)
+struct GridSlots {
+    int count;
+    short type[kNumTypes];  // of each slot
+    short of[kNumTypes];    // slot of a type
+};
+// one receptor atom of a cell list, whole: two 16-byte loads side by
 // side with its neighbours' instead of an index and four scattered reads
 struct __align__(16) CellAtom {
     double x, y, z;
-    int type, pad;
+    int type, slot;  // slot: the type's number in GridSlots
+};
+
+// one family of cell lists to fill (null list: lengths only)
+struct CellFamily {
+    const int* start;  // [ncells + 1]
+    CellAtom* list;
+    double* charge;
+};
+// one map to pack: its samples and where the packed-corner copies go (or null)
+struct GridPack {
+    const double* src;
+    float4* dst32;
+    uint4* dst16;
 };
 
 struct DReceptor {
@@ -45,10 +64,7 @@ struct DReceptor {
     const double* xyz;     // [n][3]
     const int* type;
     const double* charge;
-    // cell lists for grid construction (first-query bricks) and for the
-    // direct evaluation (full 3 A bricks)
-    const int* pop_start;   // [ncells + 1]
-    const int* pop_atoms;
+    // cell lists of the direct evaluation (full 3 A bricks)
     const int* full_start;  // [ncells + 1]
     const CellAtom* full_list;
     const double* full_charge;  // charges of full_list's atoms
