@@ -1096,7 +1096,8 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
             require(stage + (size_t)std::max(1, e->tpc / 32) * ws <= (size_t)e->max_smem,
                     "model too large for the mixed-precision path's shared memory");
             cuda_check(launch_eval32(pm.dmodels, stage, ws, tables32(e), maps32(e, r), nconfs, dc.p(), v, slope,
-                                     de.p(), dg.p(), out_coords ? dx.p() : nullptr, std::max(1, e->tpc / 32), e->stream),
+                                     de.p(), dg.p(), out_coords ? dx.p() : nullptr, std::max(1, e->tpc / 32), e->num_sms,
+                                     (size_t)e->max_smem, e->stream),
                        "eval launch");
             de.fetch(out_e);
             dg.fetch(out_g);

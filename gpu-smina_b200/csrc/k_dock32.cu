@@ -13,6 +13,7 @@
 // batch composition and of the launch shape (for a given team size).
 // Reference semantics: monte_carlo.cpp:95-130; mutate.cpp:35-63;
 // bfgs.h:30-282; conf.h:98-404; coords.cpp:25-58 (add_to_output_container).
+#include <algorithm>
 #include "dock32_eval.cuh"
 
 namespace sg {
@@ -772,20 +773,43 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB) k_mc32_feed(DTa
     if (tid == 0) atomicAdd(&ctrl->exited, 1u);
 }
 
-// model::eval_deriv in FP32 for a batch of confs of one model (one team of
-// TEAM warps per conf); the model is staged like the search kernel's, the
-// warps' workspaces follow it at ws_at, ws_stride apart
+// Batches of evaluations of one model: a block of several teams stages the model
+// once and its teams take the block's share of the confs, the next one each as
+// they come free.  Bound by the latency of one evaluation; with a block per
+// conf, each staging the model for itself, 20,000 evaluations of a 32-atom ligand
+// took 186 us, now 125 us.  (BFGS keeps a block per conf: its batches are one wave
+// whose slowest conf decides, and whole blocks of 8 confs spread unevenly over
+// the SMs: 1,536 confs 3.58 -> 3.76 ms.)
+__shared__ int s_next32;  // the block's next conf
+
+// the next conf of the block's share, on every lane of a team's leader
+__device__ __forceinline__ int next_conf32(const W32& w) {
+    int k = 0;
+    if (w.lane == 0) k = atomicAdd(&s_next32, 1);
+    return __shfl_sync(kFull32, k, 0);
+}
+// block set-up: the share [lo, hi) of n confs, the descriptors and the model
+__device__ __forceinline__ int begin_confs32(const DModel* model, const DTables32& T, const DMaps32& G, int n, int ws_at,
+                                             int ws_stride) {
+    if (threadIdx.x == 0) {
+        sT32 = T;
+        sG32 = G;
+        sWs0 = ws_at;
+        sWsStride = ws_stride;
+        s_next32 = (int)((long long)n * blockIdx.x / gridDim.x);
+    }
+    stage_model(model, threadIdx.x, blockDim.x);
+    return (int)((long long)n * (blockIdx.x + 1) / gridDim.x);
+}
+
+// model::eval_deriv in FP32, one team of TEAM warps per conf
 template <int TEAM>
-__global__ void __launch_bounds__(32 * TEAM) k_eval32(const DModel* model, DTables32 T, DMaps32 G, int n,
-                                                      const double* confs, float v0, float v1, float v2, float slope,
-                                                      double* out_e, double* out_g, double* out_coords, int ws_at,
-                                                      int ws_stride) {
-    const int k = blockIdx.x;
-    if (k >= n) return;
-    if (threadIdx.x == 0) { sT32 = T; sG32 = G; sWs0 = ws_at; sWsStride = ws_stride; }
-    stage_model(model, threadIdx.x, 32 * TEAM);
+__global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
+    k_eval32(const DModel* model, DTables32 T, DMaps32 G, int n, const double* confs, float v0, float v1, float v2,
+             float slope, double* out_e, double* out_g, double* out_coords, int ws_at, int ws_stride) {
+    const int hi = begin_confs32(model, T, G, n, ws_at, ws_stride);
     if constexpr (TEAM > 1) {
-        if (threadIdx.x >= 32) {
+        if ((threadIdx.x >> 5) % TEAM != 0) {
             team_help32<TEAM>();
             return;
         }
@@ -796,18 +820,21 @@ __global__ void __launch_bounds__(32 * TEAM) k_eval32(const DModel* model, DTabl
     unsigned* C = w.counters();
     for (int i = w.lane; i < 65; i += 32) C[i] = 0;
     for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = __ldg(m.lab32 + i);  // inflex atoms stay here
-    copyd(w, w.d(L.x_tmp), confs + (size_t)k * m.conf_size, m.conf_size);
-    const float e = eval_deriv32<TEAM>(w.at(L.x_tmp), make_float3(v0, v1, v2), slope, w.at(L.g));
+    for (int k; (k = next_conf32(w)) < hi;) {
+        copyd(w, w.d(L.x_tmp), confs + (size_t)k * m.conf_size, m.conf_size);
+        const float e = eval_deriv32<TEAM>(w.at(L.x_tmp), make_float3(v0, v1, v2), slope, w.at(L.g));
+        const double* g = w.d(L.g);
+        if (w.lane == 0) out_e[k] = e;
+        for (int i = w.lane; i < m.dof; i += 32) out_g[(size_t)k * m.dof + i] = g[i];
+        if (out_coords)
+            for (int i = w.lane; i < m.nmov; i += 32) {
+                const float4 c = w.coords()[i];
+                double* o = out_coords + ((size_t)k * m.nmov + i) * 3;
+                o[0] = c.x; o[1] = c.y; o[2] = c.z;
+            }
+        __syncwarp();
+    }
     if constexpr (TEAM > 1) team_publish<TEAM>(w, make_float3(0, 0, 0), 0.f, kTeamExit);
-    const double* g = w.d(L.g);
-    if (w.lane == 0) out_e[k] = e;
-    for (int i = w.lane; i < m.dof; i += 32) out_g[(size_t)k * m.dof + i] = g[i];
-    if (out_coords)
-        for (int i = w.lane; i < m.nmov; i += 32) {
-            const float4 c = w.coords()[i];
-            double* o = out_coords + ((size_t)k * m.nmov + i) * 3;
-            o[0] = c.x; o[1] = c.y; o[2] = c.z;
-        }
 }
 
 // quasi_newton for a batch of confs of one model with the search's own
@@ -922,20 +949,48 @@ cudaError_t launch_mc32_fixed(const DModel* dms, const DTables32& T, const DMaps
     return cudaGetLastError();
 }
 
-// ws: one warp's workspace bytes (a multiple of 16); a team's block holds
-// `team` of them
+// Teams per block and blocks of an evaluation launch of n confs: the most
+// resident teams per SM, but no more teams to a block than leave every SM one
+// while there are confs for it.  ws: one warp's workspace bytes (a multiple of
+// 16); a team's block holds `team` of them each.
+struct ConfShape32 {
+    int teams, blocks;
+    size_t smem;
+};
+static cudaError_t conf_shape32(const void* fn, size_t stage, size_t ws, int team, int n, int num_sms, size_t max_smem,
+                                ConfShape32& out) {
+    out = {0, 0, 0};
+    int best = 0;
+    for (int t = SG_MC32_THREADS / 32 / team; t >= 1; t /= 2) {
+        const size_t smem = stage + (size_t)t * team * ws;
+        if (smem > max_smem || (t > 1 && (long long)t * num_sms > n)) continue;
+        int occ = 0;
+        if (prep32(fn, smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 32 * team * t, smem) != cudaSuccess) {
+            cudaGetLastError();  // this many teams do not fit; fewer may
+            continue;
+        }
+        if (occ * t > best) {
+            best = occ * t;
+            out = {t, std::min((n + t - 1) / t, occ * num_sms), smem};
+        }
+    }
+    return best > 0 ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 cudaError_t launch_eval32(const DModel* dm, size_t stage, size_t ws, const DTables32& T, const DMaps32& G, int n,
                           const double* confs, const double v[3], double slope, double* e, double* g, double* coords,
-                          int team, cudaStream_t s) {
+                          int team, int num_sms, size_t max_smem, cudaStream_t s) {
     if (!(team == 1 || team == 2 || team == 4)) return cudaErrorInvalidValue;
-    const size_t smem = stage + (size_t)team * ws;
     const void* fn = team == 4 ? (const void*)k_eval32<4> : team == 2 ? (const void*)k_eval32<2> : (const void*)k_eval32<1>;
-    cudaError_t rc = prep32(fn, smem);
+    ConfShape32 sh;
+    cudaError_t rc = conf_shape32(fn, stage, ws, team, n, num_sms, max_smem, sh);
     if (rc != cudaSuccess) return rc;
     const float v0 = (float)v[0], v1 = (float)v[1], v2 = (float)v[2], sl = (float)slope;
-    if (team == 4) k_eval32<4><<<n, 128, smem, s>>>(dm, T, G, n, confs, v0, v1, v2, sl, e, g, coords, (int)stage, (int)ws);
-    else if (team == 2) k_eval32<2><<<n, 64, smem, s>>>(dm, T, G, n, confs, v0, v1, v2, sl, e, g, coords, (int)stage, (int)ws);
-    else k_eval32<1><<<n, 32, smem, s>>>(dm, T, G, n, confs, v0, v1, v2, sl, e, g, coords, (int)stage, (int)ws);
+    const int th = 32 * team * sh.teams;
+    if (team == 4) k_eval32<4><<<sh.blocks, th, sh.smem, s>>>(dm, T, G, n, confs, v0, v1, v2, sl, e, g, coords, (int)stage, (int)ws);
+    else if (team == 2) k_eval32<2><<<sh.blocks, th, sh.smem, s>>>(dm, T, G, n, confs, v0, v1, v2, sl, e, g, coords, (int)stage, (int)ws);
+    else k_eval32<1><<<sh.blocks, th, sh.smem, s>>>(dm, T, G, n, confs, v0, v1, v2, sl, e, g, coords, (int)stage, (int)ws);
     return cudaGetLastError();
 }
 
