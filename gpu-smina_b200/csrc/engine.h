@@ -219,6 +219,9 @@ cudaError_t launch_score64(const DModel* dms, const Shape64&, const DTables& T, 
 cudaError_t launch_refine64(const DModel*, const Shape64&, const DTables&, const DReceptor*, const int*, int, double*, int,
                             const double[3], int, const int* pose_maxiters, const double* pose_box, int, int, double*,
                             double*, int, int*, cudaStream_t);
+cudaError_t launch_merge32(const DModel* dms, const MergeJob32* jobs, int njobs, const Chain32* chains, int S,
+                           double min_rmsd, int* count, int* pose_model, double* e, double* conf, int conf_stride,
+                           double* xyz, int xyz_stride, cudaStream_t s);
 size_t ws32_bytes(const DModel& hm);
 int mc32_occupancy(int team, int wpb, size_t smem);
 cudaError_t launch_mc32_feed(const DTables32& T, const FeedItem32* ring, unsigned cap, FeedCtrl32* ctrl,

@@ -1,7 +1,7 @@
 // Batched mixed-precision docking behind the C ABI (sg_dock_batch32):
 // every ligand job's chains run in one persistent search launch (k_mc32),
 // the chains of a ligand are merged like merge_output_containers with
-// min_rmsd 2, and every merged pose is refined in FP64 on the direct
+// min_rmsd 2 (k_merge32), and every merged pose is refined in FP64 on the direct
 // receptor sum (k_refine64).  Reference: gpu_docking.cpp:560-625
 // (GpuDocking::dock_batch), parallel_mc.cpp:64-98, main.cpp:165-200.
 #include <algorithm>
@@ -52,34 +52,6 @@ static void check_packed(const sg_engine* e, const RecState& r, const sg_model_d
                         (e->tables.nc == 1 || r.cmap32[t].p),
                     "mixed-precision maps missing for a ligand type");
         }
-}
-
-// add_to_output_container (coords.cpp:25-58) on the host, for the merge
-struct HostPose {
-    double e;
-    std::vector<double> conf, xyz;
-};
-static void add_pose(std::vector<HostPose>& out, HostPose&& t, double min_rmsd, int max_size) {
-    size_t ci = out.size();
-    double cr = DBL_MAX;
-    const size_t H3 = t.xyz.size();
-    for (size_t i = 0; i < out.size(); i++) {
-        double acc = 0;
-        for (size_t a = 0; a < H3; a++) {
-            const double d = t.xyz[a] - out[i].xyz[a];
-            acc += d * d;
-        }
-        const double r = H3 ? std::sqrt(acc / (double)(H3 / 3)) : 0.0;
-        if (i == 0 || r < cr) { ci = i; cr = r; }
-    }
-    if (ci < out.size() && cr < min_rmsd) {
-        if (t.e < out[ci].e) out[ci] = std::move(t);
-    } else if ((int)out.size() < max_size) {
-        out.push_back(std::move(t));
-    } else if (!out.empty() && t.e < out.back().e) {
-        out.back() = std::move(t);
-    }
-    std::stable_sort(out.begin(), out.end(), [](const HostPose& a, const HostPose& b) { return a.e < b.e; });
 }
 
 // Launch shape for chains on teams of `team` warps: chains per block (wpb)
@@ -186,6 +158,10 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         d_evals.alloc((size_t)nchains * sizeof(unsigned long long));
         d_hits.alloc((size_t)nchains * 2 * sizeof(unsigned long long));
         d_queue.alloc(sizeof(unsigned));
+        // chains of no steps never run: nothing found, nothing counted
+        cuda_check(cudaMemsetAsync(d_count.p, 0, d_count.bytes, e->stream), "counts");
+        cuda_check(cudaMemsetAsync(d_evals.p, 0, d_evals.bytes, e->stream), "counts");
+        cuda_check(cudaMemsetAsync(d_hits.p, 0, d_hits.bytes, e->stream), "counts");
         for (int k = 0; k < nchains; k++) {
             Chain32& ch = hc[k];
             ch.out_e = d_e.as<double>() + (size_t)k * S;
@@ -351,107 +327,83 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
             }
         }
         const int blocks = first_blocks;
-        std::vector<double> he((size_t)nchains * S), hconf(nconf_res);
-        std::vector<float> hxyz(nxyz_res);
-        std::vector<int> horder((size_t)nchains * S), hcount(nchains);
+        if (!d_chains.p) io.in(d_chains, hc.data(), hc.size() * sizeof(Chain32));  // no chain had steps
+        // merge_output_containers per ligand (chains in job order), then
+        // refine_structure of every merged pose, FP64 on the direct sum: both on
+        // the device, S places per ligand
+        const int cs = pm.max_conf, hs = std::max(1, pm.max_heavy);
+        const size_t nplaces = (size_t)njobs * S;
+        require(nplaces <= (size_t)1 << 30, "dock_batch32: too many results");
+        std::vector<MergeJob32> mj(njobs);
+        for (int j = 0, c = 0; j < njobs; j++) {
+            mj[j] = {jobs[j].model, c, jobs[j].num_chains};
+            c += jobs[j].num_chains;
+        }
+        DevBuf d_mj(e), d_n(e), dpm(e), de(e), dc(e), dx(e), dmi(e);
+        io.in(d_mj, mj.data(), mj.size() * sizeof(MergeJob32));
+        h2d += d_mj.bytes;
+        d_n.alloc(njobs * sizeof(int));
+        dpm.alloc(nplaces * sizeof(int));
+        de.alloc(nplaces * sizeof(double));
+        dc.alloc(nplaces * cs * sizeof(double));
+        dx.alloc(nplaces * hs * 3 * sizeof(double));
+        cuda_check(launch_merge32(pm.dmodels, d_mj.as<MergeJob32>(), njobs, d_chains.as<Chain32>(), S, 2.0, d_n.as<int>(),
+                                  dpm.as<int>(), de.as<double>(), dc.as<double>(), cs, dx.as<double>(), 3 * hs,
+                                  e->stream),
+                   "merge launch");
+        float ref_ms = 0;
+        if (refine) {
+            std::vector<int> pmaxit(nplaces);
+            for (int j = 0; j < njobs; j++)
+                std::fill_n(pmaxit.begin() + (size_t)j * S, S, jobs[j].maxiters > 0 ? jobs[j].maxiters : p->maxiters);
+            io.in(dmi, pmaxit.data(), pmaxit.size() * sizeof(int));
+            h2d += dmi.bytes;
+            const Shape64 sh = plain_shape(e, pm, nplaces);
+            cuda_check(cudaEventRecord(ev[2], e->stream), "event");
+            cuda_check(launch_refine64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(), dpm.as<int>(), (int)nplaces,
+                                       dc.as<double>(), cs, p->authentic_v, p->maxiters, dmi.as<int>(), nullptr,
+                                       p->accurate_line, p->early_term, de.as<double>(), dx.as<double>(), hs,
+                                       e->d_err.as<int>(), e->stream),
+                       "refine launch");
+            cuda_check(cudaEventRecord(ev[3], e->stream), "event");
+        }
+        std::vector<double> he(nplaces), hconf(nplaces * cs), hxyz(nplaces * hs * 3);
+        std::vector<int> hn(njobs);
         std::vector<unsigned long long> hev(nchains), hhits(2 * (size_t)nchains);
         auto fetch = [&](void* dst, const DevBuf& src, size_t bytes) {
-            if (!bytes) return;
             io.out(dst, src.p, bytes);
             d2h += bytes;
         };
-        fetch(he.data(), d_e, he.size() * sizeof(double));
-        fetch(hconf.data(), d_conf, hconf.size() * sizeof(double));
-        fetch(hxyz.data(), d_xyz, hxyz.size() * sizeof(float));
-        fetch(horder.data(), d_order, horder.size() * sizeof(int));
-        fetch(hcount.data(), d_count, hcount.size() * sizeof(int));
+        fetch(hn.data(), d_n, hn.size() * sizeof(int));
+        fetch(he.data(), de, he.size() * sizeof(double));
+        fetch(hconf.data(), dc, hconf.size() * sizeof(double));
+        fetch(hxyz.data(), dx, hxyz.size() * sizeof(double));
         fetch(hev.data(), d_evals, hev.size() * sizeof(unsigned long long));
         fetch(hhits.data(), d_hits, hhits.size() * sizeof(unsigned long long));
         io.finish();
-        // merge_output_containers per ligand (chains in job order)
-        std::vector<std::vector<HostPose>> merged(njobs);
-        std::vector<uint64_t> job_evals(njobs, 0);
+        if (refine) cuda_check(cudaEventElapsedTime(&ref_ms, ev[2], ev[3]), "event time");
         uint64_t tot_evals = 0, tot_grid = 0, tot_pair = 0;
+        std::vector<uint64_t> job_evals(njobs, 0);
         for (int k = 0; k < nchains; k++) {
-            const int j = chain_job[k];
-            const DModel& h = pm.host[hc[k].model];
-            job_evals[j] += hev[k];
+            job_evals[chain_job[k]] += hev[k];
             tot_evals += hev[k];
             tot_grid += hhits[2 * k];
             tot_pair += hhits[2 * k + 1];
-            const int cnt = std::min(std::max(hcount[k], 0), S);
-            for (int i = 0; i < cnt; i++) {
-                const int slot = horder[(size_t)k * S + i];
-                require(slot >= 0 && slot < S, "dock_batch32: corrupt result order");
-                HostPose t;
-                t.e = he[(size_t)k * S + slot];
-                const double* c = &hconf[cres_off[k] + (size_t)slot * h.conf_size];
-                t.conf.assign(c, c + h.conf_size);
-                const float* x = &hxyz[xres_off[k] + (size_t)slot * h.nheavy * 3];
-                t.xyz.assign(x, x + (size_t)h.nheavy * 3);
-                add_pose(merged[j], std::move(t), 2.0, S);
-            }
         }
-        // refine_structure of every merged pose, FP64 on the direct sum
-        float ref_ms = 0;
-        if (refine) {
-            int nposes = 0;
-            for (auto& v : merged) nposes += (int)v.size();
-            if (nposes > 0) {
-                const Shape64 sh = plain_shape(e, pm, nposes);
-                const int cs = pm.max_conf, hs = std::max(1, pm.max_heavy);
-                std::vector<double> confs((size_t)nposes * cs, 0.0);
-                std::vector<int> pmodel(nposes), pmaxit(nposes);
-                int q = 0;
-                for (int j = 0; j < njobs; j++)
-                    for (auto& t : merged[j]) {
-                        std::memcpy(&confs[(size_t)q * cs], t.conf.data(), t.conf.size() * sizeof(double));
-                        pmodel[q] = jobs[j].model;
-                        pmaxit[q] = jobs[j].maxiters > 0 ? jobs[j].maxiters : p->maxiters;
-                        q++;
-                    }
-                DevBuf dc(e), de(e), dx(e), dpm(e), dmi(e);
-                io.in(dc, confs.data(), confs.size() * sizeof(double));
-                io.in(dpm, pmodel.data(), pmodel.size() * sizeof(int));
-                io.in(dmi, pmaxit.data(), pmaxit.size() * sizeof(int));
-                h2d += dc.bytes + dpm.bytes + dmi.bytes;
-                de.alloc((size_t)nposes * sizeof(double));
-                dx.alloc((size_t)nposes * hs * 3 * sizeof(double));
-                cuda_check(cudaEventRecord(ev[2], e->stream), "event");
-                cuda_check(launch_refine64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(),
-                                           dpm.as<int>(), nposes, dc.as<double>(), cs, p->authentic_v, p->maxiters,
-                                           dmi.as<int>(), nullptr, p->accurate_line, p->early_term, de.as<double>(),
-                                           dx.as<double>(), hs, e->d_err.as<int>(), e->stream),
-                           "refine launch");
-                cuda_check(cudaEventRecord(ev[3], e->stream), "event");
-                std::vector<double> re(nposes), rx((size_t)nposes * hs * 3);
-                fetch(confs.data(), dc, confs.size() * sizeof(double));
-                fetch(re.data(), de, re.size() * sizeof(double));
-                fetch(rx.data(), dx, rx.size() * sizeof(double));
-                io.finish();
-                cuda_check(cudaEventElapsedTime(&ref_ms, ev[2], ev[3]), "event time");
-                q = 0;
-                for (int j = 0; j < njobs; j++) {
-                    const DModel& h = pm.host[jobs[j].model];
-                    for (auto& t : merged[j]) {
-                        std::memcpy(t.conf.data(), &confs[(size_t)q * cs], t.conf.size() * sizeof(double));
-                        t.e = re[q];
-                        t.xyz.assign(&rx[(size_t)q * hs * 3], &rx[(size_t)q * hs * 3] + (size_t)h.nheavy * 3);
-                        q++;
-                    }
-                    std::stable_sort(merged[j].begin(), merged[j].end(),
-                                     [](const HostPose& a, const HostPose& b) { return a.e < b.e; });
-                }
-            }
-        }
+        std::vector<int> order(S);
         for (int j = 0; j < njobs; j++) {
             const DModel& h = pm.host[jobs[j].model];
-            out[j].count = (int)merged[j].size();
+            const int n = std::min(std::max(hn[j], 0), S);
+            const double* ej = &he[(size_t)j * S];
+            std::iota(order.begin(), order.begin() + n, 0);  // best first (refinement may have changed the order)
+            std::stable_sort(order.begin(), order.begin() + n, [&](int a, int b) { return ej[a] < ej[b]; });
+            out[j].count = n;
             out[j].evals = job_evals[j];
-            for (size_t i = 0; i < merged[j].size(); i++) {
-                out[j].e[i] = merged[j][i].e;
-                std::memcpy(out[j].conf + i * h.conf_size, merged[j][i].conf.data(), h.conf_size * sizeof(double));
-                std::memcpy(out[j].coords + i * h.nheavy * 3, merged[j][i].xyz.data(), (size_t)h.nheavy * 3 * sizeof(double));
+            for (int i = 0; i < n; i++) {
+                const size_t q = (size_t)j * S + order[i];
+                out[j].e[i] = he[q];
+                std::memcpy(out[j].conf + (size_t)i * h.conf_size, &hconf[q * cs], h.conf_size * sizeof(double));
+                std::memcpy(out[j].coords + (size_t)i * h.nheavy * 3, &hxyz[q * hs * 3], (size_t)h.nheavy * 3 * sizeof(double));
             }
         }
         e->last_wpb = wpb;

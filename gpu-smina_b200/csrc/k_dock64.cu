@@ -201,6 +201,88 @@ __device__ __forceinline__ bool within64(double margin) {
     return __all_sync(kFull, ok);
 }
 
+// merge_output_containers of one ligand's chains per block (one warp):
+// add_to_output_container (coords.cpp:25-58) over the chains in order, each one's
+// poses best first.  The list holds (chain, slot) and energies; a pose's RMSD to
+// the listed ones is one lane each, its coordinates' squares added in order, as
+// the host merge did in double precision.  Bound by that serial sum; in exchange
+// the chains' containers stay on the device (41 MB for 400 ligands, whose merge took
+// a host thread 0.1 s) and the refinement follows without a host step.
+__global__ void __launch_bounds__(32) k_merge32(const DModel* models, const MergeJob32* jobs, const Chain32* chains,
+                                                int S, double min_rmsd, int* out_count, int* pose_model,
+                                                double* out_e, double* out_conf, int conf_stride, double* out_xyz,
+                                                int xyz_stride) {
+    extern __shared__ __align__(16) double smem_merge[];
+    double* le = smem_merge;                          // [S] energies, ascending
+    int* lc = reinterpret_cast<int*>(le + S);         // [S] chain
+    int* ls = lc + S;                                 // [S] slot
+    const int j = blockIdx.x, lane = threadIdx.x;
+    const MergeJob32 job = jobs[j];
+    const int H = models[job.model].nheavy, H3 = 3 * H, cs = models[job.model].conf_size;
+    int n = 0;
+    for (int c = job.first; c < job.first + job.count; c++) {
+        const Chain32& ch = chains[c];
+        const int cnt = min(max(*ch.out_count, 0), S);
+        for (int i = 0; i < cnt; i++) {
+            const int slot = min(max(ch.out_order[i], 0), S - 1);
+            const double e = ch.out_e[slot];
+            const float* x = ch.out_coords + (size_t)slot * H3;
+            double best = kMaxFl;
+            int bi = n;
+            for (int k = lane; k < n; k += 32) {
+                const float* y = chains[lc[k]].out_coords + (size_t)ls[k] * H3;
+                double acc = 0;
+#pragma unroll 6
+                for (int a = 0; a < H3; a++) {
+                    const double d = (double)x[a] - (double)y[a];
+                    acc += d * d;
+                }
+                const double r = H3 ? sqrt(acc / (double)H) : 0.0;
+                if (k == 0 || r < best) { bi = k; best = r; }
+            }
+            // pose 0's distance stands unless another's is smaller (a NaN there stays)
+            if (__shfl_sync(kFull, best != best, 0)) {
+                bi = 0;
+                best = __shfl_sync(kFull, best, 0);
+            } else {
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double ob = __shfl_xor_sync(kFull, best, o);
+                    const int oi = __shfl_xor_sync(kFull, bi, o);
+                    if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+                }
+            }
+            int at = -1;  // the place it takes
+            if (bi < n && best < min_rmsd) {
+                if (e < le[bi]) at = bi;
+            } else if (n < S) {
+                at = n++;
+            } else if (n > 0 && e < le[n - 1]) {
+                at = n - 1;
+            }
+            __syncwarp();
+            if (at >= 0 && lane == 0) {  // sorted in behind the energies not above its own
+                int k = at;
+                while (k > 0 && le[k - 1] > e) {
+                    le[k] = le[k - 1]; lc[k] = lc[k - 1]; ls[k] = ls[k - 1];
+                    k--;
+                }
+                le[k] = e; lc[k] = c; ls[k] = slot;
+            }
+            __syncwarp();
+        }
+    }
+    if (lane == 0) out_count[j] = n;
+    for (int k = 0; k < S; k++) {
+        const size_t q = (size_t)j * S + k;
+        if (lane == 0) pose_model[q] = k < n ? job.model : -1;
+        if (k >= n) continue;
+        if (lane == 0) out_e[q] = le[k];
+        const Chain32& ch = chains[lc[k]];
+        for (int i = lane; i < cs; i += 32) out_conf[q * conf_stride + i] = ch.out_conf[(size_t)ls[k] * cs + i];
+        for (int i = lane; i < H3; i += 32) out_xyz[q * xyz_stride + i] = ch.out_coords[(size_t)ls[k] * H3 + i];
+    }
+}
+
 // refine_structure for one pose per block
 template <int G, bool ST>
 __global__ void SG_BOUNDS64 k_refine64(const DModel* models, const __grid_constant__ DTables T, const DReceptor* R,
@@ -209,7 +291,7 @@ __global__ void SG_BOUNDS64 k_refine64(const DModel* models, const __grid_consta
                                        const double* pose_box, int accurate, int early, double* out_e,
                                        double* out_coords, int coord_stride, int* err) {
     const int k = blockIdx.x;
-    if (k >= nposes) return;
+    if (k >= nposes || pose_model[k] < 0) return;  // (a place of a ligand's list that holds no pose)
     // the pose's own box, if it has one
     init64<G, ST>(models + pose_model[k], T, R, pose_box ? pose_box + 6 * (size_t)k : nullptr, err);
     if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
@@ -356,6 +438,16 @@ cudaError_t launch_refine64(const DModel* dms, const Shape64& sh, const DTables&
                             double* e, double* coords, int coord_stride, int* err, cudaStream_t s) {
     SG_LAUNCH64(SG_K_REFINE, n, dms, T, R, pose_model, n, confs, conf_stride, cap[0], cap[1], cap[2], maxiters,
                 pose_maxiters, pose_box, accurate, early, e, coords, coord_stride, err);
+}
+
+// merges njobs ligands' chains into S places each (conf_stride and xyz_stride
+// doubles apart); places past a ligand's count get pose_model -1
+cudaError_t launch_merge32(const DModel* dms, const MergeJob32* jobs, int njobs, const Chain32* chains, int S,
+                           double min_rmsd, int* count, int* pose_model, double* e, double* conf, int conf_stride,
+                           double* xyz, int xyz_stride, cudaStream_t s) {
+    k_merge32<<<njobs, 32, (size_t)S * 16, s>>>(dms, jobs, chains, S, min_rmsd, count, pose_model, e, conf, conf_stride,
+                                                xyz, xyz_stride);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_score64(const DModel* dms, const Shape64& sh, const DTables& T, const DReceptor* R,

@@ -219,6 +219,11 @@ struct FeedCtrl32 {
     unsigned pad_[2];
 };
 
+// a ligand's chains [first, first + count), to be merged
+struct MergeJob32 {
+    int model, first, count;
+};
+
 // A block's unit of work: chains [first, first + count) of one model
 struct Item32 {
     int model, first, count;
