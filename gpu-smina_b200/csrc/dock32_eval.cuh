@@ -424,20 +424,15 @@ __device__ __forceinline__ void team_publish(const W32& w, float3 v, float slope
 // (G = 1: the whole of them).  X: the chain's coordinates; F: this warp's
 // force array (every movable atom's entry is written).  Returns the warp's
 // energy share (same on every lane); adds its lookups to ghits and hits.
+// the grid part, atoms k, k + G, ... of each 32 G; returns the lane's energy
 template <int G>
-__device__ __forceinline__ float eval_terms32(const W32& w, int k, const float4* X, float4* F, float3 v, float slope,
-                                              unsigned& ghits, unsigned& hits) {
+__device__ __forceinline__ float grid_terms32(const W32& w, int k, const float4* X, float4* F, float3 v, float slope,
+                                              unsigned& ghits) {
     const SModel& m = smodel();
-    SG_T0(t_grid);
     float e = 0;
-    // grid part; every movable atom gets its force reset (hydrogens: zero)
     const int nmov = m.nmov;
     const int* TYPE = sp<const int>(m.type);
     const float4* LQ = sp<const float4>(m.local32);
-    if (G > 1) {  // the atoms of other warps start at zero in this warp's array
-        for (int i = w.lane; i < nmov; i += 32) F[i] = make_float4(0, 0, 0, 0);
-        __syncwarp();
-    }
     for (int i = w.lane * G + k; i < nmov; i += 32 * G) {
         const int t = TYPE[i];
         float3 d = make_float3(0, 0, 0);
@@ -455,6 +450,21 @@ __device__ __forceinline__ float eval_terms32(const W32& w, int k, const float4*
         }
         F[i] = make_float4(d.x, d.y, d.z, 0);
     }
+    return e;
+}
+template <int G>
+__device__ __forceinline__ float eval_terms32(const W32& w, int k, const float4* X, float4* F, float3 v, float slope,
+                                              unsigned& ghits, unsigned& hits) {
+    const SModel& m = smodel();
+    SG_T0(t_grid);
+    // grid part; every movable atom gets its force reset (hydrogens: zero)
+    const int nmov = m.nmov;
+    const float4* LQ = sp<const float4>(m.local32);
+    if (G > 1) {  // the atoms of other warps start at zero in this warp's array
+        for (int i = w.lane; i < nmov; i += 32) F[i] = make_float4(0, 0, 0, 0);
+        __syncwarp();
+    }
+    float e = grid_terms32<G>(w, k, X, F, v, slope, ghits);
     __syncwarp();
     SG_T1(t_grid, 1);
     SG_T0(t_pairs);
@@ -575,6 +585,141 @@ __device__ __noinline__ void team_help32() {
     }
 }
 
+// ---- chains on several warps ------------------------------------------------------------------
+// A chain may also run on all W warps of its block with the very bits of one
+// warp, whatever W is (kWide in place of a team size).  The first warp, the
+// leader, runs the chain and the atoms' grid terms; meanwhile the helpers
+// compute the pair slots' terms into shared memory, where one warp would add
+// each to two force entries as it goes.  Then every atom's thread adds its
+// pairs in the order of the schedule, and the last warp adds each lane's energies
+// in chunk order and sums the lanes, both as one warp does.  Three block barriers
+// per evaluation; nobody waits on anything else.  For batches that leave warps
+// idle: the pairs are half of an evaluation, and their read-add-writes in shared
+// memory and table loads a serial chain on one warp.
+constexpr int kWide = 16;
+__shared__ struct {
+    float v0, v2;  // caps of the intramolecular and the other pairs
+    unsigned op;
+    float e_lane[32], e;  // the leader's grid energies per lane; the sum
+    Wide32 at;            // byte offsets in smem32
+} sWide;
+
+__device__ __forceinline__ void wide_bar() { asm volatile("bar.sync 0;" ::: "memory"); }
+
+// Pair terms of the chunks c0, c0 + stride, ...; the arithmetic of
+// eval_terms32.  Adds the lookups to hits.
+__device__ __forceinline__ void wide_pairs32(int c0, int stride, const float4* X, const float4* LQ, float v0, float v2,
+                                             unsigned& hits) {
+    const SModel& m = smodel();
+    const DTables32 T = sT32;
+    const int nch = m.npchunks, lane = threadIdx.x & 31;
+    const uint32_t* PS = sp<const uint32_t>(m.pslot);
+    float4* terms = sp<float4>(sWide.at.terms);
+    constexpr int U = 3;  // table loads in flight
+    for (int c = c0; c < nch; c += U * stride) {
+        uint32_t sl[U];
+        float3 r[U];
+        float r2[U], rem[U];
+        bool ok[U];
+        float4 tv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int cu = c + u * stride;
+            sl[u] = cu < nch ? PS[cu * 32 + lane] : kSlotEmpty;
+            r[u] = f3(X[(sl[u] >> 8) & 0xff]) - f3(X[sl[u] & 0xff]);
+            r2[u] = dot3(r[u], r[u]);
+            ok[u] = ((sl[u] >> 16) & kSlotPairMask) != kSlotPairMask && r2[u] < T.cutoff_sqr;
+        }
+        if (T.nc == 1) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const float rf = T.factor * r2[u];
+                const int i1 = ok[u] ? (int)rf : 0;
+                rem[u] = rf - (float)i1;
+                tv[u] = ok[u] ? __ldg(T.tab + (int)(((sl[u] >> 16) & 0x1ffu) * (unsigned)T.n + (unsigned)i1)) : make_float4(0, 0, 0, 0);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (c + u * stride >= nch) break;
+            float3 f = make_float3(0, 0, 0);
+            float pe = 0;
+            if (ok[u]) {
+                float dor;
+                if (T.nc == 1) {
+                    pe = tv[u].x + rem[u] * (tv[u].z - tv[u].x);
+                    dor = tv[u].y + rem[u] * (tv[u].w - tv[u].y);
+                } else {
+                    const float2 ed = table32_nc((sl[u] >> 16) & 0x1ff, (sl[u] & kSlotSwap) != 0, LQ[sl[u] & 0xff].w,
+                                                 LQ[(sl[u] >> 8) & 0xff].w, r2[u]);
+                    pe = ed.x;
+                    dor = ed.y;
+                }
+                f = dor * r[u];
+                const float vv = (sl[u] & kSlotIntra) ? v0 : v2;
+                if (pe > 0) {
+                    const float tt = (vv < 1.1920929e-07f) ? 0.f : __fdividef(vv, vv + pe);
+                    pe *= tt;
+                    f = (tt * tt) * f;
+                }
+                hits++;
+            }
+            terms[(c + u * stride) * 32 + lane] = make_float4(f.x, f.y, f.z, pe);
+        }
+    }
+}
+
+// warp k's part of the sums: its atoms' forces, and the energy on the last warp
+__device__ __forceinline__ void wide_sums32(int k, float4* F) {
+    const SModel& m = smodel();
+    const int W = blockDim.x >> 5, lane = threadIdx.x & 31;
+    const float4* terms = sp<const float4>(sWide.at.terms);
+    if (k == W - 1) {
+        float e = sWide.e_lane[lane];
+        for (int c = 0; c < m.npchunks; c++) e += terms[c * 32 + lane].w;
+        e = warp_sum(e);
+        if (lane == 0) sWide.e = e;
+    }
+    const int* start = sp<const int>(sWide.at.start);
+    const uint16_t* list = sp<const uint16_t>(sWide.at.list);
+    for (int i = threadIdx.x; i < m.nmov; i += blockDim.x) {
+        float4 t = F[i];
+        int q = start[i];
+        const int end = start[i + 1];
+        for (; q < end; q++) {
+            const unsigned s = list[q];
+            const float4 f = terms[s >> 1];
+            if (s & 1) { t.x += f.x; t.y += f.y; t.z += f.z; }
+            else { t.x -= f.x; t.y -= f.y; t.z -= f.z; }
+        }
+        F[i] = t;
+    }
+}
+
+// a helper warp of a chain on several warps, until the leader's exit
+__device__ __noinline__ void wide_help32() {
+    const SModel& m = smodel();
+    const int k = threadIdx.x >> 5, W = blockDim.x >> 5;
+    const W32 lw{sWs0, (int)(threadIdx.x & 31)};  // the leader's workspace
+    unsigned hits = 0;
+    for (;;) {
+        wide_bar();  // the leader's command and coordinates are in
+        if (sWide.op != kTeamEval) break;
+        wide_pairs32(k - 1, W - 1, lw.coords(), sp<const float4>(m.local32), sWide.v0, sWide.v2, hits);
+        wide_bar();  // terms, grid forces and energies are in
+        wide_sums32(k, lw.force());
+        wide_bar();  // forces and the energy are in
+    }
+    atomicAdd(&lw.counters()[32 + lw.lane], hits);
+    wide_bar();  // the chain's counters are complete
+}
+// leader: ends the helpers' loops; the counters then hold their lookups
+__device__ __forceinline__ void wide_release() {
+    if ((threadIdx.x & 31) == 0) sWide.op = kTeamExit;
+    wide_bar();
+    wide_bar();
+}
+
 // model::eval_deriv in FP32 on a team of G warps (called by the leader);
 // returns the energy (same on every lane), writes g (FP64)
 template <int G>
@@ -585,13 +730,32 @@ __device__ __noinline__ float eval_deriv32(int conf_at, float3 v, float slope, i
     SG_T0(t_set);
     set_conf32(conf_at);
     SG_T1(t_set, 0);
-    if constexpr (G > 1) team_publish<G>(w, v, slope, kTeamEval);
+    if constexpr (G > 1 && G < kWide) team_publish<G>(w, v, slope, kTeamEval);
     float4* X = w.coords();
     float4* Fz = w.force();
     const int nmov = m.nmov;
     unsigned ghits = 0, hits = 0;
-    float e = eval_terms32<G>(w, 0, X, Fz, v, slope, ghits, hits);
-    if constexpr (G > 1) {
+    float e;
+    if constexpr (G == kWide) {
+        if (w.lane == 0) {
+            sWide.v0 = v.x;
+            sWide.v2 = v.z;
+            sWide.op = kTeamEval;
+        }
+        wide_bar();
+        SG_T0(t_grid);
+        sWide.e_lane[w.lane] = grid_terms32<1>(w, 0, X, Fz, v, slope, ghits);
+        SG_T1(t_grid, 1);
+        SG_T0(t_pairs);
+        wide_bar();
+        wide_sums32(0, Fz);
+        wide_bar();
+        e = sWide.e;
+        SG_T1(t_pairs, 2);
+    } else {
+        e = eval_terms32<G>(w, 0, X, Fz, v, slope, ghits, hits);
+    }
+    if constexpr (G > 1 && G < kWide) {
         team_bar<G>();  // the helpers' shares are in
 #pragma unroll
         for (int k = 1; k < G; k++) {
@@ -620,7 +784,7 @@ __device__ __noinline__ float eval_deriv32(int conf_at, float3 v, float slope, i
         if (i < nmov) {
             F = f3(Fz[i]);
 #pragma unroll
-            for (int k = 1; k < G; k++) F = F + f3(sp<const float4>(w.ws + k * sWsStride + m.L.force)[i]);
+            for (int k = 1; k < (G < kWide ? G : 1); k++) F = F + f3(sp<const float4>(w.ws + k * sWsStride + m.L.force)[i]);
             Cq = cross3(f3(X[i]) - oref, F);
         }
         float3 iF = F, iC = Cq;

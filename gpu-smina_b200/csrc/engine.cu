@@ -708,9 +708,10 @@ static bool pack_pair_chunks(const sg_model_desc& d, const std::vector<int>& pai
     return true;
 }
 
-static void pack_one(const sg_model_desc& d, bool mixed, std::vector<int>& I, std::vector<double>& D, std::vector<float>& Fl,
+static void pack_one(const sg_model_desc& d, PackFor what, std::vector<int>& I, std::vector<double>& D, std::vector<float>& Fl,
                      std::vector<size_t>& ioff, std::vector<size_t>& doff, std::vector<size_t>& foff, DModel& hm) {
     const int N = d.num_atoms, M = d.num_movable, F = d.num_frames, P = d.num_pairs;
+    const bool mixed = what != kPackPlain;
     require(N > 0 && N <= 4096 && M > 0 && M <= N, "model: atom counts out of range");
     require(F > 0 && F <= 1024 && d.num_ligands >= 0 && d.num_flex >= 0 && d.num_ligands + d.num_flex > 0,
             "model: frame / ligand counts out of range");
@@ -872,6 +873,30 @@ static void pack_one(const sg_model_desc& d, bool mixed, std::vector<int>& I, st
         std::vector<int> ps(slots.begin(), slots.end());
         hm.npchunks = packable ? (int)(slots.size() / 32) : -1;
         pv(ps);
+        // the same pairs per movable atom: chunk by chunk, in a chunk the atom's
+        // pair as first atom before the one as second
+        std::vector<int> wstart, wwords;
+        if (what == kPackWide && packable && hm.npchunks <= kWideChunks) {
+            std::vector<std::vector<uint16_t>> of(M);
+            for (size_t c = 0; c < slots.size(); c += 32)
+                for (int role = 0; role < 2; role++)
+                    for (size_t k = c; k < c + 32; k++) {
+                        if (((slots[k] >> 16) & kSlotPairMask) == kSlotPairMask) continue;
+                        const int a = (slots[k] >> (8 * role)) & 0xff;
+                        if (a < M) of[a].push_back((uint16_t)(k << 1 | role));
+                    }
+            std::vector<uint16_t> wlist;
+            for (int i = 0; i < M; i++) {
+                wstart.push_back((int)wlist.size());
+                wlist.insert(wlist.end(), of[i].begin(), of[i].end());
+            }
+            wstart.push_back((int)wlist.size());
+            wwords.resize((wlist.size() + 1) / 2);
+            if (!wlist.empty()) std::memcpy(wwords.data(), wlist.data(), wlist.size() * sizeof(uint16_t));
+        }
+        hm.wstart = wstart.empty() ? nullptr : reinterpret_cast<const int*>(1);  // placed with the pools
+        pv(wstart);
+        pv(wwords);
     }
     auto pf4 = [&](const double* xyz, const double* w4, size_t n) {
         foff.push_back(Fl.size());
@@ -912,7 +937,7 @@ struct PackedPools {
 };
 constexpr int kPackPart = 16;    // models worth a thread (about 1 ms of packing)
 constexpr int kPackThreads = 8;
-static void pack_pools(const sg_model_desc* models, int nmodels, bool mixed, PackedPools& P, std::vector<DModel>& host) {
+static void pack_pools(const sg_model_desc* models, int nmodels, PackFor what, PackedPools& P, std::vector<DModel>& host) {
     require(models && nmodels > 0 && nmodels <= (1 << 20), "models: bad array");
     host.assign(nmodels, DModel{});
     const int cores = std::max(1, (int)std::thread::hardware_concurrency());
@@ -927,7 +952,7 @@ static void pack_pools(const sg_model_desc* models, int nmodels, bool mixed, Pac
             part.dof.resize(n);
             part.fo.resize(n);
             for (int k = 0; k < n; k++)
-                pack_one(models[first + k], mixed, part.I, part.D, part.Fl, part.io[k], part.dof[k], part.fo[k],
+                pack_one(models[first + k], what, part.I, part.D, part.Fl, part.io[k], part.dof[k], part.fo[k],
                          host[first + k]);
             if (part.I.size() & 3) part.I.resize((part.I.size() + 3) & ~(size_t)3);  // the next part starts 16 B aligned
         } catch (...) {
@@ -979,6 +1004,9 @@ static void place_pools(const PackedPools& P, std::vector<DModel>& host, char* d
         size_t j = 0;
         for (const int** q : ip) *q = ib + io[j++];
         h.pslot = h.npchunks >= 0 ? reinterpret_cast<const uint32_t*>(ib + io[j]) : nullptr;
+        const bool wide = h.wstart != nullptr;
+        h.wstart = wide ? ib + io[j + 1] : nullptr;
+        h.wlist = wide ? reinterpret_cast<const uint16_t*>(ib + io[j + 2]) : nullptr;
         const float4** fp[] = {&h.local32, &h.lab32, &h.forigin32, &h.faxis32, &h.finit32};
         for (j = 0; j < fo.size(); j++) *fp[j] = reinterpret_cast<const float4*>(fb + fo[j]);
         const double** dp[] = {&h.charge, &h.local, &h.lab, &h.forigin, &h.faxis, &h.finit};
@@ -994,9 +1022,9 @@ static void place_pools(const PackedPools& P, std::vector<DModel>& host, char* d
     std::memcpy(image + P.om, host.data(), host.size() * sizeof(DModel));
 }
 
-void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, bool mixed, PackedModels& out) {
+void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, PackFor what, PackedModels& out) {
     PackedPools P;
-    pack_pools(models, nmodels, mixed, P, out.host);
+    pack_pools(models, nmodels, what, P, out.host);
     out.mem.alloc(P.bytes);
     std::unique_ptr<char[]> image(new char[P.bytes]);
     place_pools(P, out.host, out.mem.as<char>(), image.get());
@@ -1019,7 +1047,7 @@ void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, bool mixe
 // offset in the image.
 void pack_models_image(const sg_model_desc* models, int nmodels, char* dev_base, ModelImage& img) {
     PackedPools P;
-    pack_pools(models, nmodels, true, P, img.host);
+    pack_pools(models, nmodels, kPackMixed, P, img.host);
     img.dmodel_off = P.om;
     img.bytes.assign(P.bytes, 0);
     place_pools(P, img.host, dev_base, img.bytes.data());
@@ -1078,7 +1106,7 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
         RecState& r = receptor_for(e, rid);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, m, 1, !direct && e->precision != SG_PREC_FP64, pm);
+        pack_models(io, m, 1, !direct && e->precision != SG_PREC_FP64 ? kPackMixed : kPackPlain, pm);
         if (!direct) ensure_model_maps(e, r, m, 1);
         else ensure_cells(e, r);
         const Shape64 sh = plain_shape(e, pm, nconfs);
@@ -1141,7 +1169,7 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
         RecState& r = receptor_for(e, rid);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, m, 1, e->precision != SG_PREC_FP64, pm);
+        pack_models(io, m, 1, e->precision != SG_PREC_FP64 ? kPackMixed : kPackPlain, pm);
         ensure_model_maps(e, r, m, 1);
         const DModel& h = pm.host[0];
         Staged<double> dc(io, e), de(io, e);
@@ -1182,7 +1210,7 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
         RecState& r = receptor_for(e, rid);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, models, nmodels, false, pm);
+        pack_models(io, models, nmodels, kPackPlain, pm);
         ensure_model_maps(e, r, models, nmodels);
         const Shape64 sh = plain_shape(e, pm, nchains);
         const int S = p->num_saved_mins;
@@ -1304,7 +1332,7 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
         ensure_cells(e, r);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, models, nmodels, false, pm);
+        pack_models(io, models, nmodels, kPackPlain, pm);
         const Shape64 sh = plain_shape(e, pm, nposes);
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "refine: bad pose model");
         const int cs = pm.max_conf, hs = pm.max_heavy;
@@ -1360,7 +1388,7 @@ int sg_score(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, co
         ensure_cells(e, r);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, models, nmodels, false, pm);
+        pack_models(io, models, nmodels, kPackPlain, pm);
         const Shape64 sh = plain_shape(e, pm, nposes);
         require(conf_stride >= pm.max_conf && (!out_coords || coord_stride >= pm.max_heavy), "score: strides too small");
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "score: bad pose model");
@@ -1394,7 +1422,7 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
         ensure_cells(e, r);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, models, nmodels, false, pm);
+        pack_models(io, models, nmodels, kPackPlain, pm);
         const Shape64 sh = plain_shape(e, pm, nposes);
         require(conf_stride >= pm.max_conf && coord_stride >= pm.max_heavy, "minimize: strides too small");
         for (int k = 0; k < nposes; k++) {

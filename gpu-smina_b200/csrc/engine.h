@@ -237,6 +237,10 @@ cudaError_t launch_mc32_fixed(const DModel*, const DTables32&, const DMaps32&, c
 cudaError_t launch_mc32(const DModel*, const DTables32&, const DMaps32&, const DMaps32* maps_tab, const Chain32*,
                         const Item32*, int nitems, const MCParams32&, unsigned*, int blocks, int wpb,
                         size_t stage_stride, size_t ws_stride, int team, cudaStream_t);
+int mc32_wide_occupancy(int warps, size_t smem);
+cudaError_t launch_mc32_wide(const DModel*, const DTables32&, const DMaps32&, const Chain32*, const Item32*, int nitems,
+                             const MCParams32&, unsigned* queue, int blocks, int warps, size_t stage_stride,
+                             size_t ws_stride, size_t smem, cudaStream_t);
 cudaError_t launch_eval32(const DModel*, size_t stage, size_t ws, const DTables32&, const DMaps32&, int, const double*,
                           const double[3], double, double*, double*, double*, int team, int num_sms, size_t max_smem,
                           cudaStream_t);
@@ -248,8 +252,10 @@ cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, const DTables3
 // FP32 views of the engine's tables and of a receptor's packed maps
 DTables32 tables32(const sg_engine* e);
 DMaps32 maps32(const sg_engine* e, const RecState& r);
-// mixed: with the mixed-precision path's copies and pair schedules
-void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, bool mixed, PackedModels& out);
+// what is packed beyond the plain path's arrays: the mixed-precision path's
+// copies and pair schedules, and the schedules seen from the atoms
+enum PackFor { kPackPlain, kPackMixed, kPackWide };
+void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, PackFor what, PackedModels& out);
 // the plain-path launch of a batch of models; refuses a model that does not fit
 Shape64 plain_shape(sg_engine* e, const PackedModels& pm, long long items);
 struct ModelImage {

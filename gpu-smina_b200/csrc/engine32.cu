@@ -1,7 +1,8 @@
 // Batched mixed-precision docking behind the C ABI (sg_dock_batch32):
-// every ligand job's chains run in one persistent search launch (k_mc32),
-// the chains of a ligand are merged like merge_output_containers with
-// min_rmsd 2 (k_merge32), and every merged pose is refined in FP64 on the direct
+// every ligand job's chains run in one persistent search launch (k_mc32, or
+// k_mc32_wide for batches that leave warps idle), the chains of a ligand are
+// merged like merge_output_containers with min_rmsd 2 (k_merge32), and every
+// merged pose is refined in FP64 on the direct
 // receptor sum (k_refine64).  Reference: gpu_docking.cpp:560-625
 // (GpuDocking::dock_batch), parallel_mc.cpp:64-98, main.cpp:165-200.
 #include <algorithm>
@@ -79,6 +80,18 @@ bool try_launch(sg_engine* e, size_t stage_stride, size_t ws_stride, int max_cha
     return best_res > 0;
 }
 
+// warps per chain of a batch on whole blocks (k_mc32_wide), or 0 when not all of
+// its chains would be resident.  One B200, 40 steps, milliseconds against one
+// warp per chain: ligands of 45 heavy atoms and 10 rotors, 8 warps 73 / 111 (8
+// chains) and 120 / 183 (296), 4 warps 140 / 190 (592); of 25 and 5, 31 / 39, 41 / 50
+// and 51 / 59; 2 warps lost, 71 / 63 (1,184).
+static int wide_warps(sg_engine* e, size_t smem, long long nchains) {
+    if (smem > (size_t)e->max_smem) return 0;
+    for (int w : {8, 4})
+        if (nchains <= (long long)mc32_wide_occupancy(w, smem) * e->num_sms) return w;
+    return 0;
+}
+
 void choose_launch(sg_engine* e, size_t stage_stride, size_t ws_stride, int max_chains, int& wpb, int& occ) {
     require(try_launch(e, stage_stride, ws_stride, max_chains, 1, 1ll << 40, wpb, occ),
             "model too large for the mixed-precision path's shared memory");
@@ -106,13 +119,16 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         RecState& r = receptor_for(e, rid);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, models, nmodels, true, pm);
+        pack_models(io, models, nmodels, kPackWide, pm);
         ensure_model_maps(e, r, models, nmodels);
         check_packed(e, r, models, nmodels);
         uint64_t h2d = pm.mem.bytes, d2h = 0;
-        size_t ws_stride = 0, stage_stride = 0;
+        size_t ws_stride = 0, stage_stride = 0, wide_bytes = 0;
+        bool wide_packed = true;
         for (const DModel& h : pm.host) {
             require(h.npchunks >= 0, "mixed-precision path: at most 255 atoms per model");
+            wide_bytes = std::max(wide_bytes, (size_t)wide32_layout(h.npchunks, h.npairs, h.nmov).total);
+            wide_packed = wide_packed && h.wstart;
             ws_stride = std::max(ws_stride, ws32_bytes(h));
             stage_stride = std::max(stage_stride, (size_t)stage32_bytes(h.natoms, h.nframes, h.nheavy, h.npchunks,
                                                                         h.nlig, h.nblocks, h.ntors));
@@ -195,6 +211,15 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 "chains per block (sg_set_chains_per_block) times warps per chain is above 8 warps per block");
         require(try_launch(e, stage_stride, ws_stride, max_chains, team, nchains, wpb, occ),
                 "model too large for the mixed-precision path's shared memory at this many threads per chain");
+        // Chains on all warps of a block each, with the same results, where the
+        // whole batch stays resident so: the most warps for which it does.
+        const int wide = team == 1 && wide_packed && !e->force_wpb
+                             ? wide_warps(e, stage_stride + ws_stride + wide_bytes, nchains) : 0;
+        const size_t wide_smem = stage_stride + ws_stride + wide_bytes;
+        if (wide) {
+            wpb = 1;
+            occ = mc32_wide_occupancy(wide, wide_smem);
+        }
         MCParams32 P{};
         for (int i = 0; i < 3; i++) {
             P.hunt[i] = (float)p->hunt_cap[i];
@@ -285,9 +310,12 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
             h2d += d_chains.bytes + d_items.bytes;
             cuda_check(cudaMemsetAsync(d_queue.p, 0, sizeof(unsigned), e->stream), "queue reset");
             cuda_check(cudaEventRecord(ev[0], e->stream), "event");
-            cuda_check(launch_mc32(pm.dmodels, tables32(e), maps32(e, r), nullptr, d_chains.as<Chain32>(),
-                                   d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wpb * team,
-                                   stage_stride, ws_stride, team, e->stream),
+            cuda_check(wide ? launch_mc32_wide(pm.dmodels, tables32(e), maps32(e, r), d_chains.as<Chain32>(),
+                                               d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wide,
+                                               stage_stride, ws_stride, wide_smem, e->stream)
+                            : launch_mc32(pm.dmodels, tables32(e), maps32(e, r), nullptr, d_chains.as<Chain32>(),
+                                          d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wpb * team,
+                                          stage_stride, ws_stride, team, e->stream),
                        "search launch");
             cuda_check(cudaEventRecord(ev[1], e->stream), "event");
             if (phased && ph + 1 < nphases) {  // the stopping rule on the best energies the chains saved

@@ -551,6 +551,7 @@ __device__ __noinline__ void run_chain32(const Chain32& ch, const MCParams32& P)
             ch.resume[cs + 2] = (double)rng.n;
         }
     }
+    if constexpr (G == kWide) wide_release();
     unsigned long long gh = C[w.lane], ph = C[32 + w.lane];
     for (int o = 16; o > 0; o >>= 1) {
         gh += __shfl_xor_sync(kFull32, gh, o);
@@ -682,6 +683,43 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB) k_mc32(const DM
         SG_T0(t_bar);
         __syncthreads();  // the staged model is in use until every warp is done
         SG_T1(t_bar, 8);
+    }
+}
+
+// The search for batches that leave warps idle: a block per chain, all its warps
+// on that chain (dock32_eval.cuh, kWide); the results are k_mc32<1>'s.
+__global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
+    k_mc32_wide(const DModel* models, DTables32 T, DMaps32 G, const Chain32* chains, const Item32* items, int nitems,
+                const __grid_constant__ MCParams32 P, unsigned* queue, int stage_stride, int ws_stride) {
+    __shared__ int s_item;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    if (tid == 0) { sT32 = T; sG32 = G; sWs0 = stage_stride; sWsStride = ws_stride; }
+    for (;;) {
+        if (tid == 0) s_item = (int)atomicAdd(queue, 1u);
+        __syncthreads();
+        const int it = s_item;
+        if (it >= nitems) break;
+        const Item32 item = items[it];
+        stage_model(models + item.model, tid, nthr);
+        const DModel& g = s_dmodel;
+        if (tid == 0) {
+            Wide32 at = wide32_layout(g.npchunks, g.npairs, g.nmov);
+            const int base = stage_stride + ws_stride;
+            at.terms += base;
+            at.list += base;
+            at.start += base;
+            sWide.at = at;
+        }
+        __syncthreads();
+        int* start = sp<int>(sWide.at.start);
+        uint16_t* list = sp<uint16_t>(sWide.at.list);
+        for (int i = tid; i <= g.nmov; i += nthr) start[i] = g.wstart[i];
+        const int n = g.wstart[g.nmov];
+        for (int i = tid; i < n; i += nthr) list[i] = g.wlist[i];
+        __syncthreads();
+        if (tid < 32) run_chain32<kWide>(chains[item.first], P);
+        else wide_help32();
+        __syncthreads();  // the staged model is in use until the chain is done
     }
 }
 
@@ -920,6 +958,25 @@ cudaError_t launch_mc32(const DModel* dms, const DTables32& T, const DMaps32& G,
     else
         k_mc32<1><<<blocks, 32 * wpb, smem, s>>>(dms, T, G, maps_tab, chains, items, nitems, P, queue,
                                                  (int)stage_stride, (int)ws_stride);
+    return cudaGetLastError();
+}
+
+// resident blocks per SM of k_mc32_wide with `warps` warps; 0 when it does not fit
+int mc32_wide_occupancy(int warps, size_t smem) {
+    int blocks = 0;
+    if (prep32((const void*)k_mc32_wide, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_mc32_wide, 32 * warps, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return blocks;
+}
+
+cudaError_t launch_mc32_wide(const DModel* dms, const DTables32& T, const DMaps32& G, const Chain32* chains,
+                             const Item32* items, int nitems, const MCParams32& P, unsigned* queue, int blocks,
+                             int warps, size_t stage_stride, size_t ws_stride, size_t smem, cudaStream_t s) {
+    k_mc32_wide<<<blocks, 32 * warps, smem, s>>>(dms, T, G, chains, items, nitems, P, queue, (int)stage_stride,
+                                                 (int)ws_stride);
     return cudaGetLastError();
 }
 

@@ -135,8 +135,14 @@ struct __align__(16) DModel {
     const uint32_t* pslot;    // [npchunks * 32]
     int cost;                 // relative cost of one evaluation (atoms + pairs + frames)
     int npchunks;
-    int pad_[2];
+    // the schedule seen from the atoms, for chains on several warps: movable atom
+    // i's pairs are wlist[wstart[i] .. wstart[i + 1]), each slot << 1 | (the atom
+    // is the second one), in the order in which one warp adds them.  Null when
+    // not packed (kWideChunks, or callers that do not use it).
+    const int* wstart;        // [nmov + 1]
+    const uint16_t* wlist;
 };
+constexpr int kWideChunks = 1024;  // the most chunks whose slots fit 15 bits
 
 constexpr uint32_t kSlotEmpty = 0x1ffu << 16;
 constexpr uint32_t kSlotPairMask = 0x1ffu;  // (slot >> 16) & mask: type pair, 0x1ff when empty
@@ -286,6 +292,21 @@ SG_HD int stage32_bytes(int natoms, int nframes, int nheavy, int npchunks, int n
     auto r = [](int b) { return (b + 15) & ~15; };
     return r((int)sizeof(SModel)) + r(16 * natoms) + 2 * r(4 * natoms) + 2 * r(16 * nframes) + 6 * r(4 * nframes) +
            r(4 * nheavy) + r(128 * npchunks) + 3 * r(4 * nlig) + 3 * r(4 * nblocks) + 2 * r(4 * ntors);
+}
+
+// Shared memory of a chain on several warps behind the workspace: a term per
+// pair slot (force, energy), the atoms' lists and their starts
+struct Wide32 {
+    int terms, list, start, total;
+};
+SG_HD Wide32 wide32_layout(int npchunks, int npairs, int nmov) {
+    auto r = [](int b) { return (b + 15) & ~15; };
+    Wide32 w;
+    w.terms = 0;
+    w.list = r(512 * npchunks);
+    w.start = w.list + r(2 * 2 * npairs);
+    w.total = w.start + r(4 * (nmov + 1));
+    return w;
 }
 
 struct __align__(16) MCParams32 {

@@ -1,0 +1,45 @@
+"""Chains on several warps each (batches that leave warps idle) against the
+search of one warp per chain, bit for bit: batches whose chains get 8 and 4 warps
+on a B200 (296 and 592 resident blocks) and some past them, a model without
+pairs, flexible residues, and charge-dependent tables."""
+import numpy as np
+import pytest
+
+import smina_b200 as sb
+import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+VINA, AD4 = "vina", "ad4_scoring"
+CASES = [
+    (VINA, [(24, 5, 11)], 1, False), (VINA, [(24, 5, 11), (50, 12, 3), (10, 0, 4)], 3, False),
+    (VINA, [(14, 3, 2)], 400, False), (VINA, [(14, 3, 2), (11, 0, 7)], 450, False), (VINA, [(12, 2, 2)], 1300, False),
+    (VINA, [(20, 4, 5)], 4, True), (AD4, [(24, 5, 11)], 5, False),
+]
+
+
+@pytest.mark.parametrize("scoring,ligs,chains,flex", CASES)
+def test_wide_chains_equal_one_warp(scoring, ligs, chains, flex):
+    gd = W.box(26.0)
+    eng = sb.Engine(0, sb.PREC_FP32)
+    eng.set_tables(W.tables(scoring))
+    if scoring == AD4:
+        eng.set_receptor(0, W.charged_receptor(1500, 3, 2), gd)
+        models = [W.charged_ligand(*lig, 1) for lig in ligs]
+    else:
+        eng.set_receptor(0, W.receptor(1500, 3), gd)
+        fx = sb.make_flex_pdbqt(3, 42, W.CENTER) if flex else None
+        models = [sb.Model(sb.make_ligand_pdbqt(*lig, W.CENTER), fx) for lig in ligs]
+    jobs = [sb.LigandJob(model=k, num_chains=chains, num_steps=6, maxiters=0, seed=9, ligand_key=k)
+            for k in range(len(models))]
+    p = models[0].search_params()
+    wide = eng.dock_batch(0, models, jobs, p, refine=False)
+    lookups = eng.batch_stats()["pair_lookups"]
+    eng.set_chains_per_block(4)  # one warp per chain
+    one = eng.dock_batch(0, models, jobs, p, refine=False)
+    assert eng.batch_stats()["pair_lookups"] == lookups
+    for a, b in zip(wide, one):
+        assert a["evals"] == b["evals"] > 0 and len(a["e"]) > 0
+        for k in ("e", "conf", "coords"):
+            assert np.array_equal(a[k], b[k]), k
+    eng.close()
