@@ -1169,7 +1169,7 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
         RecState& r = receptor_for(e, rid);
         CallIo io(e);
         PackedModels pm(e);
-        pack_models(io, m, 1, e->precision != SG_PREC_FP64 ? kPackMixed : kPackPlain, pm);
+        pack_models(io, m, 1, e->precision != SG_PREC_FP64 ? kPackWide : kPackPlain, pm);
         ensure_model_maps(e, r, m, 1);
         const DModel& h = pm.host[0];
         Staged<double> dc(io, e), de(io, e);
@@ -1182,9 +1182,10 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
                 (size_t)stage32_bytes(h.natoms, h.nframes, h.nheavy, h.npchunks, h.nlig, h.nblocks, h.ntors);
             require(stage + (size_t)std::max(1, e->tpc / 32) * ws <= (size_t)e->max_smem,
                     "model too large for the mixed-precision path's shared memory");
-            cuda_check(launch_bfgs32(pm.dmodels, stage, ws, tables32(e), maps32(e, r), nconfs, dc.p(), v,
-                                     slope, maxiters, accurate_line, early_term, de.p(), std::max(1, e->tpc / 32),
-                                     e->stream),
+            const size_t wide = h.wstart ? (size_t)wide32_layout(h.npchunks, h.npairs, h.nmov).total : 0;
+            cuda_check(launch_bfgs32(pm.dmodels, stage, ws, wide, tables32(e), maps32(e, r), nconfs, dc.p(), v, slope,
+                                     maxiters, accurate_line, early_term, de.p(), std::max(1, e->tpc / 32), e->num_sms,
+                                     (size_t)e->max_smem, e->stream),
                        "bfgs launch");
             dc.fetch(confs);
             de.fetch(out_e);

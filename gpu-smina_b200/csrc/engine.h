@@ -237,17 +237,17 @@ cudaError_t launch_mc32_fixed(const DModel*, const DTables32&, const DMaps32&, c
 cudaError_t launch_mc32(const DModel*, const DTables32&, const DMaps32&, const DMaps32* maps_tab, const Chain32*,
                         const Item32*, int nitems, const MCParams32&, unsigned*, int blocks, int wpb,
                         size_t stage_stride, size_t ws_stride, int team, cudaStream_t);
-int mc32_wide_occupancy(int warps, size_t smem);
-cudaError_t launch_mc32_wide(const DModel*, const DTables32&, const DMaps32&, const Chain32*, const Item32*, int nitems,
+int mc32_mix_occupancy(int warps, size_t smem);
+cudaError_t launch_mc32_mix(const DModel*, const DTables32&, const DMaps32&, const Chain32*, const Item32*, int nitems,
                              const MCParams32&, unsigned* queue, int blocks, int warps, size_t stage_stride,
                              size_t ws_stride, size_t smem, cudaStream_t);
 cudaError_t launch_eval32(const DModel*, size_t stage, size_t ws, const DTables32&, const DMaps32&, int, const double*,
                           const double[3], double, double*, double*, double*, int team, int num_sms, size_t max_smem,
                           cudaStream_t);
 cudaError_t gather_probe(size_t working_set, int bytes_per_lookup, int num_sms, double* gbs, cudaStream_t s);
-cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, const DTables32&, const DMaps32&, int, double*,
-                          const double v[3], double slope, int maxiters, int accurate, int early, double* e,
-                          int team, cudaStream_t);
+cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, size_t wide, const DTables32&, const DMaps32&, int,
+                          double*, const double v[3], double slope, int maxiters, int accurate, int early, double* e,
+                          int team, int num_sms, size_t max_smem, cudaStream_t);
 
 // FP32 views of the engine's tables and of a receptor's packed maps
 DTables32 tables32(const sg_engine* e);

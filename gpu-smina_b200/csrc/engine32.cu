@@ -1,10 +1,10 @@
 // Batched mixed-precision docking behind the C ABI (sg_dock_batch32):
 // every ligand job's chains run in one persistent search launch (k_mc32, or
-// k_mc32_wide for batches that leave warps idle), the chains of a ligand are
+// k_mc32_mix where some chains get a block each), the chains of a ligand are
 // merged like merge_output_containers with min_rmsd 2 (k_merge32), and every
-// merged pose is refined in FP64 on the direct
-// receptor sum (k_refine64).  Reference: gpu_docking.cpp:560-625
-// (GpuDocking::dock_batch), parallel_mc.cpp:64-98, main.cpp:165-200.
+// merged pose is refined in FP64 on the direct receptor sum (k_refine64).
+// Reference: gpu_docking.cpp:560-625 (GpuDocking::dock_batch),
+// parallel_mc.cpp:64-98, main.cpp:165-200.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -80,16 +80,86 @@ bool try_launch(sg_engine* e, size_t stage_stride, size_t ws_stride, int max_cha
     return best_res > 0;
 }
 
-// warps per chain of a batch on whole blocks (k_mc32_wide), or 0 when not all of
-// its chains would be resident.  One B200, 40 steps, milliseconds against one
-// warp per chain: ligands of 45 heavy atoms and 10 rotors, 8 warps 73 / 111 (8
-// chains) and 120 / 183 (296), 4 warps 140 / 190 (592); of 25 and 5, 31 / 39, 41 / 50
-// and 51 / 59; 2 warps lost, 71 / 63 (1,184).
-static int wide_warps(sg_engine* e, size_t smem, long long nchains) {
-    if (smem > (size_t)e->max_smem) return 0;
-    for (int w : {8, 4})
-        if (nchains <= (long long)mc32_wide_occupancy(w, smem) * e->num_sms) return w;
-    return 0;
+// ---- which chains get a block each ----------------------------------------------------------
+// One B200, 40 steps, milliseconds of search, a block of 8 or 4 warps per chain
+// against one warp per chain: ligands of 45 heavy atoms and 10 rotors 73 / 111 (8
+// chains, 8 warps), 120 / 183 (296, 8 warps), 140 / 190 (592, 4 warps); of 25 and 5
+// 31 / 39, 41 / 50 and 51 / 59 (2 warps lost, 71 / 63 at 1,184 chains).  Past that a
+// batch of mixed ligands took the 185 ms of its largest ligand's chains from 592 to
+// 2,368 chains: there the largest ones get blocks and the others a warp each: 107,
+// 126, 139 and 183 ms at 592, 1,184, 1,600 and 2,368 chains, before 177, 185, 187 and
+// 204.
+//
+// A chain's cost on one warp of a full SM, and a block's time on it as a share of
+// that, in pairs: an evaluation costs about 300 pairs' time besides its pairs, and
+// a block saves about half of the pairs' time and, having fewer neighbours, a
+// third of the rest.
+static double chain_cost(const DModel& h, unsigned steps, int maxiters) {
+    return (double)steps * std::max(1, maxiters) * (300 + h.npairs);
+}
+static double block_share(const DModel& h, int warps) {
+    return (warps == 8 ? 190 + 0.38 * h.npairs : 210 + 0.5 * h.npairs) / (300 + h.npairs);
+}
+struct PlanJob {  // chains of one ligand, `cost` each
+    int job, chains;
+    double cost;
+    const DModel* h;
+};
+struct MixPlan {
+    int warps = 0, occ = 0, wide_jobs = 0;  // 0 warps: one warp per chain throughout
+    size_t smem = 0;
+};
+// Time of a batch (jobs by falling cost, the first `wide` of them with blocks) on m
+// blocks of `warps` warps taking the longest item first: no less than the work over
+// the blocks, nor than the q + 1 shortest of the q m + 1 longest items, which share
+// a block.
+static double mix_time(const std::vector<PlanJob>& jobs, size_t wide, int warps, long long m) {
+    double load = 0, span = 0;
+    long long items = 0, next = 0;
+    size_t a = 0, b = wide;
+    while (a < wide || b < jobs.size()) {  // the two kinds merged, longest first
+        const double da = a < wide ? jobs[a].cost * block_share(*jobs[a].h, warps) : -1,
+                     db = b < jobs.size() ? jobs[b].cost : -1;
+        const double d = std::max(da, db);
+        const long long n = da >= db ? jobs[a++].chains : (jobs[b++].chains + warps - 1) / warps;
+        load += d * n;
+        items += n;
+        for (; next < items; next += m) span = std::max(span, d * (double)(next / m + 1));
+    }
+    return std::max(span, load / (double)m);
+}
+static MixPlan plan_mix(sg_engine* e, const std::vector<PlanJob>& jobs, size_t stage_stride, size_t ws_stride,
+                        size_t wide_bytes) {
+    MixPlan best;
+    double best_time = 0;
+    for (int warps : {8, 4}) {
+        const size_t smem = stage_stride + ws_stride + std::max((warps - 1) * ws_stride, wide_bytes);
+        if (smem > (size_t)e->max_smem) continue;
+        const int occ = mc32_mix_occupancy(warps, smem);
+        if (occ == 0) continue;
+        const long long m = (long long)occ * e->num_sms;
+        if (best_time == 0) {
+            // one warp per chain, faster the fewer of them share an SM (a full
+            // SM's time at 14 or more, 3/4 of it at 2 to 5); a block per chain has
+            // to gain more than the estimate's uncertainty
+            long long chains = 0;
+            for (const PlanJob& q : jobs) chains += q.chains;
+            const double full = std::min(1.0, 0.65 + 0.025 * (double)chains / e->num_sms);
+            best_time = 0.95 * full * mix_time(jobs, 0, warps, m);
+        }
+        for (size_t k = 1;; k = std::min(jobs.size(), k + (k + 1) / 2)) {
+            const double t = mix_time(jobs, k, warps, m);
+            if (t < best_time) {
+                best_time = t;
+                best.warps = warps;
+                best.occ = occ;
+                best.wide_jobs = (int)k;
+                best.smem = smem;
+            }
+            if (k == jobs.size()) break;
+        }
+    }
+    return best;
 }
 
 void choose_launch(sg_engine* e, size_t stage_stride, size_t ws_stride, int max_chains, int& wpb, int& occ) {
@@ -211,15 +281,6 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 "chains per block (sg_set_chains_per_block) times warps per chain is above 8 warps per block");
         require(try_launch(e, stage_stride, ws_stride, max_chains, team, nchains, wpb, occ),
                 "model too large for the mixed-precision path's shared memory at this many threads per chain");
-        // Chains on all warps of a block each, with the same results, where the
-        // whole batch stays resident so: the most warps for which it does.
-        const int wide = team == 1 && wide_packed && !e->force_wpb
-                             ? wide_warps(e, stage_stride + ws_stride + wide_bytes, nchains) : 0;
-        const size_t wide_smem = stage_stride + ws_stride + wide_bytes;
-        if (wide) {
-            wpb = 1;
-            occ = mc32_wide_occupancy(wide, wide_smem);
-        }
         MCParams32 P{};
         for (int i = 0; i < 3; i++) {
             P.hunt[i] = (float)p->hunt_cap[i];
@@ -262,7 +323,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         std::vector<double> hres;
         DevBuf d_chains(e), d_items(e);
         float mc_ms = 0;
-        int first_blocks = 0;
+        int first_blocks = 0, first_wpb = wpb;
         cudaEvent_t ev[4];
         for (auto& x : ev) cuda_check(cudaEventCreate(&x), "event");
         struct EvGuard {
@@ -284,17 +345,37 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 active.push_back(k);
             }
             if (active.empty()) continue;
+            // the ligands by falling cost, and which of them get a block per chain
+            std::vector<PlanJob> jobs_by_cost;
+            for (size_t a = 0; a < active.size();) {
+                const int k = active[a], j = chain_job[k];
+                int n = 0;
+                while (a + n < active.size() && chain_job[active[a + n]] == j) n++;
+                const DModel& h = pm.host[hc[k].model];
+                jobs_by_cost.push_back({j, n, chain_cost(h, hc[k].end - hc[k].begin, hc[k].maxiters), &h});
+                a += n;
+            }
+            std::stable_sort(jobs_by_cost.begin(), jobs_by_cost.end(),
+                             [](const PlanJob& a, const PlanJob& b) { return a.cost > b.cost; });
+            MixPlan mix;
+            if (team == 1 && wide_packed && !e->force_wpb) mix = plan_mix(e, jobs_by_cost, stage_stride, ws_stride, wide_bytes);
+            std::vector<char> has_block(njobs, 0);
+            std::vector<double> cost(njobs, 0);
+            for (size_t k = 0; k < jobs_by_cost.size(); k++) {
+                const PlanJob& q = jobs_by_cost[k];
+                has_block[q.job] = (int)k < mix.wide_jobs;
+                cost[q.job] = q.cost * (has_block[q.job] ? block_share(*q.h, mix.warps) : 1.0);
+            }
+            const int per_item = mix.warps ? mix.warps : wpb;
             std::vector<Item32> items;
             std::vector<double> item_cost;
             for (size_t a = 0; a < active.size();) {
                 const int k = active[a], j = chain_job[k];
+                const int most = has_block[j] ? 1 : per_item;
                 int n = 0;
-                while (a + n < active.size() && chain_job[active[a + n]] == j && n < wpb &&
-                       active[a + n] == k + n)
-                    n++;
-                items.push_back(Item32{hc[k].model, k, n, 0});
-                item_cost.push_back((double)(hc[k].end - hc[k].begin) * pm.host[hc[k].model].cost *
-                                    std::max(1, hc[k].maxiters));
+                while (a + n < active.size() && chain_job[active[a + n]] == j && n < most && active[a + n] == k + n) n++;
+                items.push_back(Item32{hc[k].model, k, n, has_block[j]});
+                item_cost.push_back(cost[j]);
                 a += n;
             }
             std::vector<int> order(items.size());
@@ -303,19 +384,23 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
             std::vector<Item32> queue(items.size());
             for (size_t k = 0; k < items.size(); k++) queue[k] = items[order[k]];
             const int nitems = (int)queue.size();
-            const int blocks = (int)std::min<long long>((long long)occ * e->num_sms, nitems);
-            if (ph == 0) first_blocks = blocks;
+            const int blocks = (int)std::min<long long>((long long)(mix.warps ? mix.occ : occ) * e->num_sms, nitems);
+            if (ph == 0) {
+                first_blocks = blocks;
+                first_wpb = !mix.warps ? wpb : mix.wide_jobs == (int)jobs_by_cost.size() ? 1 : mix.warps;
+            }
             io.in(d_chains, hc.data(), hc.size() * sizeof(Chain32));
             io.in(d_items, queue.data(), queue.size() * sizeof(Item32));
             h2d += d_chains.bytes + d_items.bytes;
             cuda_check(cudaMemsetAsync(d_queue.p, 0, sizeof(unsigned), e->stream), "queue reset");
             cuda_check(cudaEventRecord(ev[0], e->stream), "event");
-            cuda_check(wide ? launch_mc32_wide(pm.dmodels, tables32(e), maps32(e, r), d_chains.as<Chain32>(),
-                                               d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wide,
-                                               stage_stride, ws_stride, wide_smem, e->stream)
-                            : launch_mc32(pm.dmodels, tables32(e), maps32(e, r), nullptr, d_chains.as<Chain32>(),
-                                          d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wpb * team,
-                                          stage_stride, ws_stride, team, e->stream),
+            cuda_check(mix.warps
+                           ? launch_mc32_mix(pm.dmodels, tables32(e), maps32(e, r), d_chains.as<Chain32>(),
+                                             d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, mix.warps,
+                                             stage_stride, ws_stride, mix.smem, e->stream)
+                           : launch_mc32(pm.dmodels, tables32(e), maps32(e, r), nullptr, d_chains.as<Chain32>(),
+                                         d_items.as<Item32>(), nitems, P, d_queue.as<unsigned>(), blocks, wpb * team,
+                                         stage_stride, ws_stride, team, e->stream),
                        "search launch");
             cuda_check(cudaEventRecord(ev[1], e->stream), "event");
             if (phased && ph + 1 < nphases) {  // the stopping rule on the best energies the chains saved
@@ -434,7 +519,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 std::memcpy(out[j].coords + (size_t)i * h.nheavy * 3, &hxyz[q * hs * 3], (size_t)h.nheavy * 3 * sizeof(double));
             }
         }
-        e->last_wpb = wpb;
+        e->last_wpb = first_wpb;
         e->last_team = team;
         e->last_blocks = blocks;
         e->last_mc_ms = mc_ms;

@@ -686,13 +686,37 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB) k_mc32(const DM
     }
 }
 
-// The search for batches that leave warps idle: a block per chain, all its warps
-// on that chain (dock32_eval.cuh, kWide); the results are k_mc32<1>'s.
+// After stage_model: the buffers of a chain on the whole block, from byte `base`
+// of smem32, and the atoms' lists.  Every thread takes part; ends with a block
+// barrier.
+__device__ __forceinline__ void stage_wide32(int base) {
+    const DModel& g = s_dmodel;
+    if (threadIdx.x == 0) {
+        Wide32 at = wide32_layout(g.npchunks, g.npairs, g.nmov);
+        at.terms += base;
+        at.list += base;
+        at.start += base;
+        sWide.at = at;
+    }
+    __syncthreads();
+    int* start = sp<int>(sWide.at.start);
+    uint16_t* list = sp<uint16_t>(sWide.at.list);
+    for (int i = threadIdx.x; i <= g.nmov; i += blockDim.x) start[i] = g.wstart[i];
+    const int n = g.wstart[g.nmov];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = g.wlist[i];
+    __syncthreads();
+}
+
+// The search where some of a batch's chains have a block to themselves, all its
+// warps on the one chain (dock32_eval.cuh, kWide; items with rec 1), and the others
+// a warp each as in k_mc32<1>, whose results they all have: batches that leave
+// warps idle, and batches whose largest ligands would still be searching when the
+// others are done.
 __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
-    k_mc32_wide(const DModel* models, DTables32 T, DMaps32 G, const Chain32* chains, const Item32* items, int nitems,
-                const __grid_constant__ MCParams32 P, unsigned* queue, int stage_stride, int ws_stride) {
+    k_mc32_mix(const DModel* models, DTables32 T, DMaps32 G, const Chain32* chains, const Item32* items, int nitems,
+               const __grid_constant__ MCParams32 P, unsigned* queue, int stage_stride, int ws_stride) {
     __shared__ int s_item;
-    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int tid = threadIdx.x, nthr = blockDim.x, warp = tid >> 5;
     if (tid == 0) { sT32 = T; sG32 = G; sWs0 = stage_stride; sWsStride = ws_stride; }
     for (;;) {
         if (tid == 0) s_item = (int)atomicAdd(queue, 1u);
@@ -701,25 +725,14 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
         if (it >= nitems) break;
         const Item32 item = items[it];
         stage_model(models + item.model, tid, nthr);
-        const DModel& g = s_dmodel;
-        if (tid == 0) {
-            Wide32 at = wide32_layout(g.npchunks, g.npairs, g.nmov);
-            const int base = stage_stride + ws_stride;
-            at.terms += base;
-            at.list += base;
-            at.start += base;
-            sWide.at = at;
+        if (item.rec == 0) {
+            if (warp < item.count) run_chain32<1>(chains[item.first + warp], P);
+        } else {
+            stage_wide32(stage_stride + ws_stride);
+            if (warp == 0) run_chain32<kWide>(chains[item.first], P);
+            else wide_help32();
         }
-        __syncthreads();
-        int* start = sp<int>(sWide.at.start);
-        uint16_t* list = sp<uint16_t>(sWide.at.list);
-        for (int i = tid; i <= g.nmov; i += nthr) start[i] = g.wstart[i];
-        const int n = g.wstart[g.nmov];
-        for (int i = tid; i < n; i += nthr) list[i] = g.wlist[i];
-        __syncthreads();
-        if (tid < 32) run_chain32<kWide>(chains[item.first], P);
-        else wide_help32();
-        __syncthreads();  // the staged model is in use until the chain is done
+        __syncthreads();  // the staged model is in use until every chain is done
     }
 }
 
@@ -909,6 +922,36 @@ __global__ void __launch_bounds__(32 * TEAM) k_bfgs32(const DModel* model, DTabl
     if (w.lane == 0) out_e[k] = e;
 }
 
+// the same with all warps of a block on each conf and k_bfgs32<1>'s results, for
+// batches that leave warps idle
+__global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
+    k_bfgs32_wide(const DModel* model, DTables32 T, DMaps32 G, int n, double* confs, float v0, float v1, float v2,
+                  float slope, int maxiters, int accurate, int early, double* out_e, int ws_at, int ws_stride) {
+    const int k = blockIdx.x;
+    if (k >= n) return;
+    if (threadIdx.x == 0) { sT32 = T; sG32 = G; sWs0 = ws_at; sWsStride = ws_stride; }
+    stage_model(model, threadIdx.x, blockDim.x);
+    stage_wide32(ws_at + ws_stride);
+    const W32 w = here();
+    const SModel& m = smodel();
+    if (threadIdx.x < 32) {
+        unsigned* C = w.counters();
+        for (int i = w.lane; i < 65; i += 32) C[i] = 0;
+        for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = __ldg(m.lab32 + i);  // inflex atoms stay here
+        for (int f = w.lane; f < m.nframes; f += 32) w.origin()[f] = __ldg(m.finit32 + f);
+        double* c = confs + (size_t)k * m.conf_size;
+        const int x_at = w.at(m.L.x_tmp);
+        copyd(w, sp<double>(x_at), c, m.conf_size);
+        const double e = bfgs32<kWide>(x_at, maxiters, accurate, early, Mode32{make_float3(v0, v1, v2), slope});
+        wide_release();
+        const double* x = sp<double>(x_at);
+        for (int i = w.lane; i < m.conf_size; i += 32) c[i] = x[i];
+        if (w.lane == 0) out_e[k] = e;
+    } else {
+        wide_help32();
+    }
+}
+
 // ---- host launchers -----------------------------------------------------------------------
 size_t ws32_bytes(const DModel& hm) {
     return (size_t)ws32_layout(hm.natoms, hm.nframes, hm.conf_size, hm.dof).total;
@@ -961,22 +1004,22 @@ cudaError_t launch_mc32(const DModel* dms, const DTables32& T, const DMaps32& G,
     return cudaGetLastError();
 }
 
-// resident blocks per SM of k_mc32_wide with `warps` warps; 0 when it does not fit
-int mc32_wide_occupancy(int warps, size_t smem) {
+// resident blocks per SM of k_mc32_mix with `warps` warps; 0 when it does not fit
+int mc32_mix_occupancy(int warps, size_t smem) {
     int blocks = 0;
-    if (prep32((const void*)k_mc32_wide, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_mc32_wide, 32 * warps, smem) != cudaSuccess) {
+    if (prep32((const void*)k_mc32_mix, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_mc32_mix, 32 * warps, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     return blocks;
 }
 
-cudaError_t launch_mc32_wide(const DModel* dms, const DTables32& T, const DMaps32& G, const Chain32* chains,
-                             const Item32* items, int nitems, const MCParams32& P, unsigned* queue, int blocks,
-                             int warps, size_t stage_stride, size_t ws_stride, size_t smem, cudaStream_t s) {
-    k_mc32_wide<<<blocks, 32 * warps, smem, s>>>(dms, T, G, chains, items, nitems, P, queue, (int)stage_stride,
-                                                 (int)ws_stride);
+cudaError_t launch_mc32_mix(const DModel* dms, const DTables32& T, const DMaps32& G, const Chain32* chains,
+                            const Item32* items, int nitems, const MCParams32& P, unsigned* queue, int blocks,
+                            int warps, size_t stage_stride, size_t ws_stride, size_t smem, cudaStream_t s) {
+    k_mc32_mix<<<blocks, 32 * warps, smem, s>>>(dms, T, G, chains, items, nitems, P, queue, (int)stage_stride,
+                                                (int)ws_stride);
     return cudaGetLastError();
 }
 
@@ -1051,9 +1094,26 @@ cudaError_t launch_eval32(const DModel* dm, size_t stage, size_t ws, const DTabl
     return cudaGetLastError();
 }
 
-cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, const DTables32& T, const DMaps32& G, int n,
-                          double* confs, const double v[3], double slope, int maxiters, int accurate, int early,
-                          double* e, int team, cudaStream_t s) {
+// wide: the buffers' bytes of a conf on a whole block, or 0: not packed for it.
+// Used while all confs are resident so, 8 warps each, else 4 (as for the search's
+// chains).
+cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide, const DTables32& T, const DMaps32& G,
+                          int n, double* confs, const double v[3], double slope, int maxiters, int accurate, int early,
+                          double* e, int team, int num_sms, size_t max_smem, cudaStream_t s) {
+    if (team == 1 && wide)
+        for (int warps : {8, 4}) {
+            const size_t smem = stage + ws + wide;
+            int occ = 0;
+            if (smem > max_smem || prep32((const void*)k_bfgs32_wide, smem) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bfgs32_wide, 32 * warps, smem) != cudaSuccess) {
+                cudaGetLastError();
+                break;
+            }
+            if (n > (long long)occ * num_sms) continue;
+            k_bfgs32_wide<<<n, 32 * warps, smem, s>>>(dm, T, G, n, confs, (float)v[0], (float)v[1], (float)v[2],
+                                                      (float)slope, maxiters, accurate, early, e, (int)stage, (int)ws);
+            return cudaGetLastError();
+        }
     if (!(team == 1 || team == 2 || team == 4)) return cudaErrorInvalidValue;
     const size_t smem = stage + (size_t)team * ws;
     const void* fn = team == 4 ? (const void*)k_bfgs32<4> : team == 2 ? (const void*)k_bfgs32<2> : (const void*)k_bfgs32<1>;

@@ -233,7 +233,8 @@ struct MergeJob32 {
 // A block's unit of work: chains [first, first + count) of one model
 struct Item32 {
     int model, first, count;
-    int rec;  // receptor slot in the launch's map table (0 when the launch has one receptor)
+    int rec;  // receptor slot in the launch's map table (0 when the launch has one receptor); k_mc32_mix:
+              // 1 for a chain that has its block to itself
 };
 
 // per-warp workspace (bytes, 16 B aligned)
