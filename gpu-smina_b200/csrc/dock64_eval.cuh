@@ -24,10 +24,13 @@
 //  - energy: the last warp adds the ordered energy sums while the others add
 //    forces and the first warp walks the tree back.
 // Measured on one B200 against one warp per item with everything read from
-// global memory and lane 0 adding the sums: refinement of 1,890 poses of 210
-// ligands 303 -> 55 ms, of 9 poses of one ligand 7.9 -> 1.5 ms; rescoring of 2,000
-// poses 0.54 -> 0.20 ms; 8 chains of 40 steps 88 -> 62 ms; 1,500 charge-dependent
-// evaluations 126 -> 84 us.  Bits unchanged.
+// global memory and lane 0 adding the sums, with calls: refinement of 1,890 poses
+// of 210 ligands 270 -> 29 ms, of 9 poses of one ligand 7.3 -> 1.2 ms; 8 chains of 40
+// steps 87 -> 59 ms; kernels alone: rescoring of 2,000 poses 0.54 -> 0.20 ms, 1,500
+// charge-dependent evaluations 126 -> 84 us.  Bits unchanged.  What is left of an
+// evaluation is the leader's instructions, about 3,400 of them at 7 to 8 cycles each
+// (frames, tree derivative, BFGS); four lanes per frame and one per frame and
+// component took more instructions and were slower.
 // The first warp, the leader, runs the chain (BFGS, line searches, mutation)
 // and calls the others in for each evaluation: two numbers of warps (4 and 8)
 // by the number of items, plus one warp with nothing staged for models whose
@@ -94,13 +97,14 @@ __device__ __noinline__ void set_frames64(const double* conf) {
     const int *fkind = M::fkind(), *fconf = M::fconf(), *fparent = M::fparent(), *ls = M::level_start(),
               *lf = M::level_frames();
     const double *forigin = M::forigin(), *faxis = M::faxis();
-    for (int f = lane; f < F; f += 32)
+    for (int t = lane; t < 2 * F; t += 32) {  // a lane each for the cosine and the sine
+        const int f = t >> 1;
         if (fkind[f] != SG_FRAME_RIGID) {
             double angle = conf[fconf[f]];
             normalize_angle(angle);
-            S[L.q + 4 * f] = fd_cos(angle / 2);
-            S[L.q + 4 * f + 1] = fd_sin(angle / 2);
+            S[L.q + 4 * f + (t & 1)] = (t & 1) ? fd_sin(angle / 2) : fd_cos(angle / 2);
         }
+    }
     __syncwarp();
     for (int lv = 0; lv < nlevels; lv++) {
         for (int idx = ls[lv] + lane; idx < ls[lv + 1]; idx += 32) {
@@ -271,10 +275,86 @@ __device__ __forceinline__ Clamped64 clamp64(const DReceptor& R, const double* b
     return c;
 }
 
+// a list entry's lookup under way: its separation and, where one table value is
+// one load, the values
+template <int NC>
+struct Term64 {
+    bool in;
+    V3<double> r;
+    double rem, r2;
+    double2 a, b;
+    int type;
+};
+// atom `at` of type t against list entry x (there: the lane has one)
+template <int NC, bool ENERGY_ONLY>
+__device__ __forceinline__ Term64<NC> look_up64(const DTables& T, bool there, CellAtom x, V3<double> at, int t) {
+    Term64<NC> q{false, {0, 0, 0}, 0, 0, {0, 0}, {0, 0}, 0};
+    if (there) {
+        q.r = V3<double>{at.x - x.x, at.y - x.y, at.z - x.z};
+        q.r2 = norm2(q.r);
+        q.type = x.type;
+        q.in = q.r2 < T.cutoff_sqr;
+        if (NC == 1 && q.in) {
+            bool sw;
+            const size_t row = (size_t)type_pair64(t, q.type, sw) * T.n;
+            const double rf = T.factor * q.r2;
+            const size_t i1 = (size_t)rf;
+            q.rem = rf - (double)i1;
+            if (ENERGY_ONLY) {
+                q.a.x = __ldg(T.fast + row + i1);
+            } else {
+                const double2* s = reinterpret_cast<const double2*>(T.smooth) + row + i1;
+                q.a = __ldg(s);
+                q.b = __ldg(s + 1);
+            }
+        }
+    }
+    return q;
+}
+// The group's terms within the cutoff, squeezed into its exchange buffer X and
+// added to its lanes' sums in list order.  charge: of this lane's entry.
+template <int NC, bool ENERGY_ONLY>
+__device__ __forceinline__ double add_up64(const DTables& T, Term64<NC> q, int t, double qi, const double* charge,
+                                           double* X, int* err, double acc) {
+    const int lane = lane64(), gl = lane & 7;
+    const unsigned gm = (__ballot_sync(kFull, q.in) >> (lane & 24)) & 0xffu;
+    const int cnt = __popc(gm);
+    if (q.in) {
+        double* x = X + 4 * __popc(gm & ((1u << gl) - 1));
+        double pe, dor = 0;
+        if (!ENERGY_ONLY && q.r2 < kEps) atomicExch(err, kDevOverlap);
+        if (NC == 1) {
+            pe = q.a.x;
+            if (!ENERGY_ONLY) {
+                pe = q.a.x + q.rem * (q.b.x - q.a.x);
+                dor = q.a.y + q.rem * (q.b.y - q.a.y);
+            }
+        } else {
+            bool sw;
+            const int pr = type_pair64(t, q.type, sw);
+            if (ENERGY_ONLY) pe = table_fast64(T, pr, sw, qi, *charge, q.r2);
+            else table_deriv64(T, pr, sw, qi, *charge, q.r2, pe, dor);
+        }
+        if (ENERGY_ONLY) {
+            x[0] = pe;
+        } else {
+            const V3<double> f = dor * q.r;
+            reinterpret_cast<double2*>(x)[0] = make_double2(pe, f.x);
+            reinterpret_cast<double2*>(x)[1] = make_double2(f.y, f.z);
+        }
+    }
+    __syncwarp();
+    if (gl < (ENERGY_ONLY ? 1 : 4))
+        for (int j = 0; j < cnt; j++) acc += X[4 * j + gl];
+    __syncwarp();
+    return acc;
+}
+
 // non_cache::eval_deriv (ENERGY_ONLY: non_cache::eval on the fast table, into
 // eatom only): direct sum over the 3 A cell list of the clamped atom, 8 lanes
-// per atom and 16 list entries a round
-template <int G, bool ST, bool ENERGY_ONLY>
+// per atom and 16 list entries a round; a round's table values are on their way
+// while the round before is added up
+template <int G, bool ST, bool ENERGY_ONLY, int NC>
 __device__ __forceinline__ void direct_atoms64(int k, double v, double slope) {
     using M = MV64<ST>;
     const Hdr64& H = hd64();
@@ -288,7 +368,6 @@ __device__ __forceinline__ void direct_atoms64(int k, double v, double slope) {
     const int* heavy = M::heavy();
     const double* charge = M::charge();
     const int nmov = H.m.nmov, nheavy = H.m.nheavy;
-    const double cutoff_sqr = T.cutoff_sqr;
     const CellAtom* list = R.full_list;
     for (int i = 32 * k + lane; i < nmov; i += 32 * G)
         if (type[i] >= kNumTypes || is_h(type[i])) {
@@ -303,62 +382,25 @@ __device__ __forceinline__ void direct_atoms64(int k, double v, double slope) {
         const Clamped64 c = clamp64(R, ENERGY_ONLY ? nullptr : H.box, S + L.coords + 3 * i, act);
         const double qi = charge[i];
         double acc = 0;  // lane gl < 4 of a group: energy, x, y, z
-        CellAtom nx[2];
-#pragma unroll
-        for (int u = 0; u < 2; u++)
-            if (c.kb + gl + 8 * u < c.ke) nx[u] = load_cell_atom(list + c.kb + gl + 8 * u);
-        for (int k0 = c.kb; __any_sync(kFull, k0 < c.ke); k0 += 16) {
-            bool in[2];
-            double pe[2], r2[2];
-            V3<double> f[2];
-            int tj[2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int kk = k0 + gl + 8 * u;
-                in[u] = false;
-                if (kk < c.ke) {
-                    f[u] = V3<double>{c.adj[0] - nx[u].x, c.adj[1] - nx[u].y, c.adj[2] - nx[u].z};
-                    r2[u] = norm2(f[u]);
-                    tj[u] = nx[u].type;
-                    in[u] = r2[u] < cutoff_sqr;
-                }
-                if (kk + 16 < c.ke) nx[u] = load_cell_atom(list + kk + 16);
-            }
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-                if (in[u]) {
-                    const double qj = T.nc > 1 ? R.full_charge[k0 + gl + 8 * u] : 0.0;
-                    bool sw;
-                    const int pr = type_pair64(t, tj[u], sw);
-                    if (ENERGY_ONLY) {
-                        pe[u] = table_fast64(T, pr, sw, qi, qj, r2[u]);
-                    } else {
-                        if (r2[u] < kEps) atomicExch(H.err, kDevOverlap);
-                        double dor;
-                        table_deriv64(T, pr, sw, qi, qj, r2[u], pe[u], dor);
-                        f[u] = dor * f[u];
-                    }
-                }
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const unsigned mask = __ballot_sync(kFull, in[u]);
-                if (!mask) continue;
-                const unsigned gm = (mask >> (8 * grp)) & 0xffu;
-                const int cnt = __popc(gm);
-                if (in[u]) {
-                    double* x = X + 4 * __popc(gm & ((1u << gl) - 1));
-                    if (ENERGY_ONLY) {
-                        x[0] = pe[u];
-                    } else {
-                        reinterpret_cast<double2*>(x)[0] = make_double2(pe[u], f[u].x);
-                        reinterpret_cast<double2*>(x)[1] = make_double2(f[u].y, f[u].z);
-                    }
-                }
-                __syncwarp();
-                if (gl < (ENERGY_ONLY ? 1 : 4))
-                    for (int j = 0; j < cnt; j++) acc += X[4 * j + gl];
-                __syncwarp();
-            }
+        CellAtom n0{0, 0, 0, 0, 0}, n1 = n0;
+        Term64<NC> q0, q1;
+        int kk = c.kb + gl;
+        const V3<double> at{c.adj[0], c.adj[1], c.adj[2]};
+        const int ke = c.ke;
+        const double* list_charge = R.full_charge;
+        if (kk < ke) n0 = load_cell_atom(list + kk);
+        if (kk + 8 < ke) n1 = load_cell_atom(list + kk + 8);
+        q0 = look_up64<NC, ENERGY_ONLY>(T, kk < ke, n0, at, t);
+        q1 = look_up64<NC, ENERGY_ONLY>(T, kk + 8 < ke, n1, at, t);
+        if (kk + 16 < ke) n0 = load_cell_atom(list + kk + 16);
+        if (kk + 24 < ke) n1 = load_cell_atom(list + kk + 24);
+        for (; __any_sync(kFull, kk - gl < ke); kk += 16) {
+            acc = add_up64<NC, ENERGY_ONLY>(T, q0, t, qi, list_charge + kk, X, H.err, acc);
+            q0 = look_up64<NC, ENERGY_ONLY>(T, kk + 16 < ke, n0, at, t);
+            if (kk + 32 < ke) n0 = load_cell_atom(list + kk + 32);
+            acc = add_up64<NC, ENERGY_ONLY>(T, q1, t, qi, list_charge + kk + 8, X, H.err, acc);
+            q1 = look_up64<NC, ENERGY_ONLY>(T, kk + 24 < ke, n1, at, t);
+            if (kk + 40 < ke) n1 = load_cell_atom(list + kk + 40);
         }
         double this_e = __shfl_sync(kFull, acc, 8 * grp);
         V3<double> deriv{__shfl_sync(kFull, acc, 8 * grp + 1), __shfl_sync(kFull, acc, 8 * grp + 2),
@@ -436,6 +478,9 @@ __device__ __forceinline__ void gather_forces64(int t0, int nt) {
     double* S = smem64;
     const int* csr_start = M::csr_start();
     const int* csr = H.m.csr;
+    const uint16_t* csr16 = reinterpret_cast<const uint16_t*>(smem64 + L.s_csr);
+    const bool staged = ST && L.s_csr != 0;
+    auto entry = [&](int q) { return staged ? (int)csr16[q] : __ldg(csr + q); };
     const int n3 = 3 * H.m.nmov;
     for (int t = t0; t < n3; t += nt) {
         const int i = t / 3, c = t - 3 * i;
@@ -447,14 +492,14 @@ __device__ __forceinline__ void gather_forces64(int t0, int nt) {
             int w[4];
             double x[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) w[u] = __ldg(csr + q + u);
+            for (int u = 0; u < 4; u++) w[u] = entry(q + u);
 #pragma unroll
             for (int u = 0; u < 4; u++) x[u] = pf[3 * (w[u] >> 1)];
 #pragma unroll
             for (int u = 0; u < 4; u++) f += (w[u] & 1) ? x[u] : -x[u];
         }
         for (; q < e; q++) {
-            const int w = __ldg(csr + q);
+            const int w = entry(q);
             const double x = pf[3 * (w >> 1)];
             f += (w & 1) ? x : -x;
         }
@@ -649,7 +694,8 @@ __device__ __noinline__ void eval_warp64(int k) {
     set_atoms64<ST>(threadIdx.x, 32 * G);
     bar64<G>();
     if (H.direct) {
-        direct_atoms64<G, ST, false>(k, H.v[1], H.slope);
+        if (H.T.nc == 1) direct_atoms64<G, ST, false, 1>(k, H.v[1], H.slope);
+        else direct_atoms64<G, ST, false, 4>(k, H.v[1], H.slope);
         pairs64<ST, false>(threadIdx.x, 32 * G, H.v[2], H.v[0]);
     } else {
         // the first warps take the atoms; the pairs start on the others
@@ -677,7 +723,8 @@ __device__ __noinline__ void score_warp64(int k) {
     Hdr64& H = hd64();
     set_atoms64<ST>(threadIdx.x, 32 * G);
     bar64<G>();
-    direct_atoms64<G, ST, true>(k, H.v[1], H.slope);
+    if (H.T.nc == 1) direct_atoms64<G, ST, true, 1>(k, H.v[1], H.slope);
+    else direct_atoms64<G, ST, true, 4>(k, H.v[1], H.slope);
     pairs64<ST, true>(threadIdx.x, 32 * G, H.v[2], H.v[0]);
     bar64<G>();
 }

@@ -42,6 +42,9 @@ __device__ __forceinline__ void init64(const DModel* gm, const DTables& T, const
         const int N = m.natoms, F = m.nframes;
         static_assert(sizeof(DReceptor) % 8 == 0, "the receptor header is copied in 8-byte pieces");
         stage64<G>(L.s_receptor, reinterpret_cast<const double*>(R), (int)(sizeof(DReceptor) / 8));
+        uint16_t* csr = reinterpret_cast<uint16_t*>(smem64 + L.s_csr);
+        if (L.s_csr)
+            for (int i = threadIdx.x; i < m.csr_start[m.nmov]; i += 32 * G) csr[i] = (uint16_t)m.csr[i];
         stage64<G>(L.s_type, m.type, N);
         stage64<G>(L.s_atom_frame, m.atom_frame, N);
         stage64<G>(L.s_csr_start, m.csr_start, m.nmov + 1);

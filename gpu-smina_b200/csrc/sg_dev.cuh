@@ -327,7 +327,7 @@ struct Ws64 {
     int xbuf;  // exchange buffers of the direct sum, kXbuf64 per warp
     // staged only
     int cr;  // torque terms per atom
-    int s_receptor, s_type, s_atom_frame, s_csr_start, s_heavy, s_fkind, s_fparent, s_fbegin, s_fend, s_fconf, s_fdof,
+    int s_receptor, s_csr, s_type, s_atom_frame, s_csr_start, s_heavy, s_fkind, s_fparent, s_fbegin, s_fend, s_fconf, s_fdof,
         s_level_start, s_level_frames, s_child_start, s_child_list, s_lig_begin, s_lig_end, s_lig_root, s_lig_pair_end,
         s_blk_rigid, s_blk_conf, s_blk_ntors, s_tor_conf, s_tor_dof, s_charge, s_local, s_forigin, s_faxis;
     int total;  // doubles; staged: without the exchange buffers, which follow
@@ -347,6 +347,9 @@ struct __align__(16) Hdr64 {
 // 4 groups of 8 terms of 4 doubles, 4 doubles apart so that the groups' reads
 // fall in different banks
 constexpr int kXbuf64 = 4 * (8 * 4 + 4);
+// models of more pairs leave their pair lists in global memory, so that they
+// still fit an SM staged (entries are 16 bits: pair << 1 | side)
+constexpr int kCsr16Pairs = 4096;
 
 SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof, bool staged, int nheavy, int nlevels,
                        int nlig, int nblocks, int ntors) {
@@ -381,6 +384,7 @@ SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof, b
     if (staged) {
         w.cr = take(3 * natoms);
         w.s_receptor = take((int)((sizeof(DReceptor) + 7) / 8));
+        if (npairs <= kCsr16Pairs) w.s_csr = take((2 * npairs + 3) / 4);  // 0: left in global memory
         w.s_type = ints(natoms);
         w.s_atom_frame = ints(natoms);
         w.s_csr_start = ints(natoms + 1);
