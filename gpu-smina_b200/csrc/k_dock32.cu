@@ -36,10 +36,12 @@ __device__ __forceinline__ void warp_sum3_d(double& a, double& b, double& c) {
 }
 __device__ __forceinline__ double dotd(const W32& w, const double* a, const double* b, int n) {
     double t = 0;
+    SG_ROLLED
     for (int i = w.lane; i < n; i += 32) t += a[i] * b[i];
     return warp_sum_d(t);
 }
 __device__ __forceinline__ void copyd(const W32& w, double* d, const double* s, int n) {
+    SG_ROLLED
     for (int i = w.lane; i < n; i += 32) d[i] = s[i];
     __syncwarp();
 }
@@ -81,6 +83,7 @@ __device__ __forceinline__ void increment32(const W32& w, double* x, const doubl
     const int* fdof = sp<const int>(m.fdof);
     const int* tor_conf = sp<const int>(m.tor_conf);
     const int* tor_dof = sp<const int>(m.tor_dof);
+    SG_ROLLED
     for (int l = w.lane; l < m.nlig; l += 32) {
         const int f = lig_root[l];
         double* c = x + fconf[f];
@@ -88,6 +91,7 @@ __device__ __forceinline__ void increment32(const W32& w, double* x, const doubl
         c[0] += alpha * d[0]; c[1] += alpha * d[1]; c[2] += alpha * d[2];
         q_increment32(c + 3, alpha * d[3], alpha * d[4], alpha * d[5]);
     }
+    SG_ROLLED
     for (int k = w.lane; k < m.ntors; k += 32) {
         double& t = x[tor_conf[k]];
         t = wrap_pi(t + wrap_pi(alpha * p[tor_dof[k]]));
@@ -103,6 +107,7 @@ __device__ double conf_value32(const double* x, int i) {
     const int* fdof = sp<const int>(m.fdof);
     const int* tor_conf = sp<const int>(m.tor_conf);
     const int* tor_dof = sp<const int>(m.tor_dof);
+    SG_ROLLED
     for (int l = 0; l < m.nlig; l++) {
         const int f = lig_root[l];
         const int d0 = fdof[f];
@@ -114,6 +119,7 @@ __device__ double conf_value32(const double* x, int i) {
             return j == 0 ? a.x : j == 1 ? a.y : a.z;
         }
     }
+    SG_ROLLED
     for (int k = 0; k < m.ntors; k++)
         if (tor_dof[k] == i) return x[tor_conf[k]];
     return 0;
@@ -170,12 +176,14 @@ __device__ __noinline__ double2 line_accurate32(W32 w, int x_at, double pg, doub
     const double slope = pg;
     auto give_up = [&]() {
         copyd(w, x_new, x, m.conf_size);
+        SG_ROLLED
         for (int i = w.lane; i < n; i += 32) g_new[i] = 0;
         __syncwarp();
         return make_double2(0.0, f1);
     };
     if (slope >= 0) return give_up();
     double test = 0;
+    SG_ROLLED
     for (int i = w.lane; i < n; i += 32) test = fmax(test, fabs(p[i]) / fmax(fabs(conf_value32(x, i)), 1.0));
     for (int o = 16; o > 0; o >>= 1) test = fmax(test, __shfl_xor_sync(kFull32, test, o));
     alamin = kEps / test;
@@ -227,6 +235,7 @@ __device__ __noinline__ double bfgs32(int x_at, int maxiters, int accurate, int 
     double* h = w.d(L.h);
     double *g = sp<double>(g_at), *g_new = sp<double>(gn_at), *g_orig = w.d(L.g_orig), *p = sp<double>(p_at);
     double *y = w.d(L.y), *x_new = sp<double>(xn_at), *x_orig = w.d(L.x_orig), *mhy = w.d(L.mhy);
+    SG_ROLLED
     for (int i = w.lane; i < n; i += 32)
         for (int j = 0; j < n; j++) h[j * n + i] = (i == j) ? 1.0 : 0.0;
     __syncwarp();
@@ -237,6 +246,7 @@ __device__ __noinline__ double bfgs32(int x_at, int maxiters, int accurate, int 
     for (int step = 0; step < maxiters; step++) {
         SG_T0(t_alg);
         double pg = 0;  // p . g, for the line search
+        SG_ROLLED
         for (int i = w.lane; i < n; i += 32) {
             double sum = 0;
             SG_ROLLED
@@ -259,6 +269,7 @@ __device__ __noinline__ double bfgs32(int x_at, int maxiters, int accurate, int 
         SG_T0(t_alg2);
         // y = g_new - g, g = g_new, and the three dot products the update needs
         double gg = 0, yy = 0, yp = 0;
+        SG_ROLLED
         for (int i = w.lane; i < n; i += 32) {
             const double gi = g_new[i], yi = gi - g[i];
             y[i] = yi;
@@ -276,12 +287,14 @@ __device__ __noinline__ double bfgs32(int x_at, int maxiters, int accurate, int 
         if (!(gg >= 1e-4)) break;
         if (step == 0 && fabs(yy) > kEps) {
             const double dg = alpha * yp / yy;
+            SG_ROLLED
             for (int i = w.lane; i < n; i += 32) h[i * n + i] = dg;
             __syncwarp();
         }
         // bfgs_update
         if (alpha * yp >= kEps) {
             double yhy = 0;
+            SG_ROLLED
             for (int i = w.lane; i < n; i += 32) {
                 double sum = 0;
                 SG_ROLLED
@@ -293,6 +306,7 @@ __device__ __noinline__ double bfgs32(int x_at, int maxiters, int accurate, int 
             __syncwarp();
             const double r = 1 / (alpha * yp);
             const double c1 = alpha * r, c2 = alpha * alpha * (r * r * yhy + r);
+            SG_ROLLED
             for (int i = w.lane; i < n; i += 32) {
                 const double mi = mhy[i], pi = p[i];
                 SG_ROLLED
@@ -334,6 +348,7 @@ __device__ __forceinline__ double gyration32(const W32& w, int l) {
     float acc = 0;
     int cnt = 0;
     const int end = sp<const int>(m.lig_end)[l];
+    SG_ROLLED
     for (int i = sp<const int>(m.lig_begin)[l] + w.lane; i < end; i += 32)
         if (!is_h(type[i])) {
             const float3 d = f3(w.coords()[i]) - o;
@@ -351,10 +366,12 @@ __device__ __forceinline__ void mutate32(const W32& w, Philox& rng, double* x, d
     const int* blk_ntors = sp<const int>(m.blk_ntors);
     const int* blk_conf = sp<const int>(m.blk_conf);
     int num = 0;
+    SG_ROLLED
     for (int b = 0; b < m.nblocks; b++) num += (blk_rigid[b] ? 2 : 0) + blk_ntors[b];
     if (num == 0) return;
     int which = ph_int(rng, num);
     int lig = 0;
+    SG_ROLLED
     for (int b = 0; b < m.nblocks; b++) {
         double* c = x + blk_conf[b];
         if (blk_rigid[b]) {
@@ -397,6 +414,7 @@ __device__ __forceinline__ void randomize32(const W32& w, Philox& rng, double* x
     const int* blk_rigid = sp<const int>(m.blk_rigid);
     const int* blk_ntors = sp<const int>(m.blk_ntors);
     const int* blk_conf = sp<const int>(m.blk_conf);
+    SG_ROLLED
     for (int b = 0; b < m.nblocks; b++) {
         double* c = x + blk_conf[b];
         if (blk_rigid[b]) {
@@ -411,6 +429,7 @@ __device__ __forceinline__ void randomize32(const W32& w, Philox& rng, double* x
             c += 7;
         }
         const int nt = blk_ntors[b];
+        SG_ROLLED
         for (int t = 0; t < nt; t++) {
             const double a = ph_range(rng, -kPi, kPi);
             if (w.lane == 0) c[t] = a;
@@ -430,9 +449,11 @@ __device__ __forceinline__ int add_output32(const W32& w, const Chain32& ch, con
     // RMSD to every saved pose: lanes over atoms, one pose at a time
     float best = 3.4e38f;
     int bj = count;
+    SG_ROLLED
     for (int j = 0; j < count; j++) {
         const float* oc = ch.out_coords + (size_t)ch.out_order[j] * H * 3;
         float acc = 0;
+        SG_ROLLED
         for (int a = w.lane; a < H; a += 32) {
             const float3 c = f3(X[heavy[a]]);
             const float dx = c.x - oc[3 * a], dy = c.y - oc[3 * a + 1], dz = c.z - oc[3 * a + 2];
@@ -454,7 +475,9 @@ __device__ __forceinline__ int add_output32(const W32& w, const Chain32& ch, con
     }
     __syncwarp();
     if (target >= 0) {
+        SG_ROLLED
         for (int i = w.lane; i < cs; i += 32) ch.out_conf[(size_t)target * cs + i] = x[i];
+        SG_ROLLED
         for (int a = w.lane; a < H; a += 32) {
             const float3 c = f3(X[heavy[a]]);
             float* o = ch.out_coords + ((size_t)target * H + a) * 3;
@@ -465,6 +488,7 @@ __device__ __forceinline__ int add_output32(const W32& w, const Chain32& ch, con
     __syncwarp();
     if (w.lane == 0) {
         *ch.out_count = count;
+        SG_ROLLED
         for (int i = 1; i < count; i++) {  // stable insertion sort by energy
             const int key = ch.out_order[i];
             const double ek = ch.out_e[key];
@@ -487,6 +511,7 @@ __device__ __noinline__ void run_chain32(const Chain32& ch, const MCParams32& P)
     const SModel& m = smodel();
     const Ws32& L = m.L;
     unsigned* C = w.counters();
+    SG_ROLLED
     for (int i = w.lane; i < 65; i += 32) C[i] = 0;
     const int cs = m.conf_size;
     // model state as read (mutation may read it before the first set)
@@ -500,8 +525,11 @@ __device__ __noinline__ void run_chain32(const Chain32& ch, const MCParams32& P)
     int count = 0;
     const float4* saved_xyz = ch.resume ? reinterpret_cast<const float4*>(ch.resume + resume32_coords_at(cs)) : nullptr;
     if (resumed) {  // a later phase: the state the previous one saved
+        SG_ROLLED
         for (int i = w.lane; i < cs; i += 32) tmp[i] = ch.resume[i];
+        SG_ROLLED
         for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = saved_xyz[i];
+        SG_ROLLED
         for (int f = w.lane; f < m.nframes; f += 32) w.origin()[f] = saved_xyz[m.natoms + f];
         tmp_e = ch.resume[cs];
         best_e = ch.resume[cs + 1];
@@ -511,7 +539,9 @@ __device__ __noinline__ void run_chain32(const Chain32& ch, const MCParams32& P)
     } else {
         // (L2-only loads: a serving grid may read a ligand placed where an
         // earlier one was, and this SM's L1 may still hold the earlier one's lines)
+        SG_ROLLED
         for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = __ldcg(m.lab32 + i);
+        SG_ROLLED
         for (int f = w.lane; f < m.nframes; f += 32) w.origin()[f] = __ldcg(m.finit32 + f);
         __syncwarp();
         randomize32(w, rng, tmp, ch.box ? ch.box : P.box);
@@ -542,8 +572,11 @@ __device__ __noinline__ void run_chain32(const Chain32& ch, const MCParams32& P)
     __syncwarp();
     if (ch.resume) {  // the state a later phase resumes from (and the best energy, for the stopping rule)
         float4* sx = reinterpret_cast<float4*>(ch.resume + resume32_coords_at(cs));
+        SG_ROLLED
         for (int i = w.lane; i < cs; i += 32) ch.resume[i] = tmp[i];
+        SG_ROLLED
         for (int i = w.lane; i < m.natoms; i += 32) sx[i] = w.coords()[i];
+        SG_ROLLED
         for (int f = w.lane; f < m.nframes; f += 32) sx[m.natoms + f] = w.origin()[f];
         if (w.lane == 0) {
             ch.resume[cs] = tmp_e;
@@ -585,6 +618,7 @@ __device__ __forceinline__ int stage_arr(const T* src, int n, int& o, int tid, i
     const int at = o;
     T* d = sp<T>(at);
     o += (n * (int)sizeof(T) + 15) & ~15;
+    SG_ROLLED
     for (int i = tid; i < n; i += nthr) d[i] = __ldcg(src + i);
     return at;
 }
@@ -593,6 +627,7 @@ __shared__ __align__(16) DModel s_dmodel;  // the staged model's descriptor (its
 
 __device__ void stage_model(const DModel* gm, int tid, int nthr) {
     static_assert(sizeof(DModel) % 16 == 0, "DModel is read in 16-byte pieces");
+    SG_ROLLED
     for (int k = tid; k < (int)(sizeof(DModel) / 16); k += nthr)
         reinterpret_cast<int4*>(&s_dmodel)[k] = __ldcg(reinterpret_cast<const int4*>(gm) + k);
     __syncthreads();
@@ -701,8 +736,10 @@ __device__ __forceinline__ void stage_wide32(int base) {
     __syncthreads();
     int* start = sp<int>(sWide.at.start);
     uint16_t* list = sp<uint16_t>(sWide.at.list);
+    SG_ROLLED
     for (int i = threadIdx.x; i <= g.nmov; i += blockDim.x) start[i] = g.wstart[i];
     const int n = g.wstart[g.nmov];
+    SG_ROLLED
     for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = g.wlist[i];
     __syncthreads();
 }
@@ -869,15 +906,19 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
     const SModel& m = smodel();
     const Ws32& L = m.L;
     unsigned* C = w.counters();
+    SG_ROLLED
     for (int i = w.lane; i < 65; i += 32) C[i] = 0;
+    SG_ROLLED
     for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = __ldg(m.lab32 + i);  // inflex atoms stay here
     for (int k; (k = next_conf32(w)) < hi;) {
         copyd(w, w.d(L.x_tmp), confs + (size_t)k * m.conf_size, m.conf_size);
         const float e = eval_deriv32<TEAM>(w.at(L.x_tmp), make_float3(v0, v1, v2), slope, w.at(L.g));
         const double* g = w.d(L.g);
         if (w.lane == 0) out_e[k] = e;
+        SG_ROLLED
         for (int i = w.lane; i < m.dof; i += 32) out_g[(size_t)k * m.dof + i] = g[i];
         if (out_coords)
+            SG_ROLLED
             for (int i = w.lane; i < m.nmov; i += 32) {
                 const float4 c = w.coords()[i];
                 double* o = out_coords + ((size_t)k * m.nmov + i) * 3;
@@ -910,14 +951,18 @@ __global__ void __launch_bounds__(32 * TEAM) k_bfgs32(const DModel* model, DTabl
     const SModel& m = smodel();
     const Ws32& L = m.L;
     unsigned* C = w.counters();
+    SG_ROLLED
     for (int i = w.lane; i < 65; i += 32) C[i] = 0;
+    SG_ROLLED
     for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = __ldg(m.lab32 + i);  // inflex atoms stay here
+    SG_ROLLED
     for (int f = w.lane; f < m.nframes; f += 32) w.origin()[f] = __ldg(m.finit32 + f);
     double* c = confs + (size_t)k * m.conf_size;
     copyd(w, w.d(L.x_tmp), c, m.conf_size);
     const double e = bfgs32<TEAM>(w.at(L.x_tmp), maxiters, accurate, early, Mode32{make_float3(v0, v1, v2), slope});
     if constexpr (TEAM > 1) team_publish<TEAM>(w, make_float3(0, 0, 0), 0.f, kTeamExit);
     const double* x = w.d(L.x_tmp);
+    SG_ROLLED
     for (int i = w.lane; i < m.conf_size; i += 32) c[i] = x[i];
     if (w.lane == 0) out_e[k] = e;
 }
@@ -936,8 +981,11 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
     const SModel& m = smodel();
     if (threadIdx.x < 32) {
         unsigned* C = w.counters();
+        SG_ROLLED
         for (int i = w.lane; i < 65; i += 32) C[i] = 0;
+        SG_ROLLED
         for (int i = w.lane; i < m.natoms; i += 32) w.coords()[i] = __ldg(m.lab32 + i);  // inflex atoms stay here
+        SG_ROLLED
         for (int f = w.lane; f < m.nframes; f += 32) w.origin()[f] = __ldg(m.finit32 + f);
         double* c = confs + (size_t)k * m.conf_size;
         const int x_at = w.at(m.L.x_tmp);
@@ -945,6 +993,7 @@ __global__ void __launch_bounds__(SG_MC32_THREADS, SG_MC32_MINB)
         const double e = bfgs32<kWide>(x_at, maxiters, accurate, early, Mode32{make_float3(v0, v1, v2), slope});
         wide_release();
         const double* x = sp<double>(x_at);
+        SG_ROLLED
         for (int i = w.lane; i < m.conf_size; i += 32) c[i] = x[i];
         if (w.lane == 0) out_e[k] = e;
     } else {
