@@ -1183,7 +1183,7 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
             require(stage + (size_t)std::max(1, e->tpc / 32) * ws <= (size_t)e->max_smem,
                     "model too large for the mixed-precision path's shared memory");
             const size_t wide = h.wstart ? (size_t)wide32_layout(h.npchunks, h.npairs, h.nmov).total : 0;
-            cuda_check(launch_bfgs32(pm.dmodels, stage, ws, wide, tables32(e), maps32(e, r), nconfs, dc.p(), v, slope,
+            cuda_check(launch_bfgs32(pm.dmodels, stage, ws, wide, h.npairs, tables32(e), maps32(e, r), nconfs, dc.p(), v, slope,
                                      maxiters, accurate_line, early_term, de.p(), std::max(1, e->tpc / 32), e->num_sms,
                                      (size_t)e->max_smem, e->stream),
                        "bfgs launch");

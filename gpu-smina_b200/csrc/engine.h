@@ -245,8 +245,8 @@ cudaError_t launch_eval32(const DModel*, size_t stage, size_t ws, const DTables3
                           const double[3], double, double*, double*, double*, int team, int num_sms, size_t max_smem,
                           cudaStream_t);
 cudaError_t gather_probe(size_t working_set, int bytes_per_lookup, int num_sms, double* gbs, cudaStream_t s);
-cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, size_t wide, const DTables32&, const DMaps32&, int,
-                          double*, const double v[3], double slope, int maxiters, int accurate, int early, double* e,
+cudaError_t launch_bfgs32(const DModel*, size_t stage, size_t ws, size_t wide, int npairs, const DTables32&,
+                          const DMaps32&, int, double*, const double v[3], double slope, int maxiters, int accurate, int early, double* e,
                           int team, int num_sms, size_t max_smem, cudaStream_t);
 
 // FP32 views of the engine's tables and of a receptor's packed maps

@@ -1144,11 +1144,18 @@ cudaError_t launch_eval32(const DModel* dm, size_t stage, size_t ws, const DTabl
 }
 
 // wide: the buffers' bytes of a conf on a whole block, or 0: not packed for it.
-// Used while all confs are resident so, 8 warps each, else 4 (as for the search's
-// chains).
-cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide, const DTables32& T, const DMaps32& G,
-                          int n, double* confs, const double v[3], double slope, int maxiters, int accurate, int early,
-                          double* e, int team, int num_sms, size_t max_smem, cudaStream_t s) {
+// With 8 warps per block while all confs are resident so.  With 4 beyond that,
+// up to 1 + pairs / 200 resident batches: the more of an evaluation its pairs
+// are, the longer blocks that take confs one after the other win against one
+// warp per conf, whose slowest conf decides.  One B200, milliseconds of 4 warps
+// against one: 50 heavy atoms and 12 rotors (1,000 pairs; 592 resident) 2.2 / 3.9 at
+// 592 confs, 3.3 / 4.4 at 1,536, 5.4 / 5.5 at 3,500, 7.9 / 7.5 at 6,000; 24 and 5 (150)
+// 0.85 / 1.15 at 592, 1.15 / 1.19 at 1,200, 1.55 / 1.44 at 2,000; 12 and 2 (25) 0.55 / 0.58
+// at 592, 0.71 / 0.62 at 800.
+cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide, int npairs, const DTables32& T,
+                          const DMaps32& G, int n, double* confs, const double v[3], double slope, int maxiters,
+                          int accurate, int early, double* e, int team, int num_sms, size_t max_smem,
+                          cudaStream_t s) {
     if (team == 1 && wide)
         for (int warps : {8, 4}) {
             const size_t smem = stage + ws + wide;
@@ -1158,7 +1165,8 @@ cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide
                 cudaGetLastError();
                 break;
             }
-            if (n > (long long)occ * num_sms) continue;
+            const double most = (double)occ * num_sms * (warps == 8 ? 1.0 : 1.0 + npairs / 200.0);
+            if (n > most) continue;
             k_bfgs32_wide<<<n, 32 * warps, smem, s>>>(dm, T, G, n, confs, (float)v[0], (float)v[1], (float)v[2],
                                                       (float)slope, maxiters, accurate, early, e, (int)stage, (int)ws);
             return cudaGetLastError();
