@@ -1069,8 +1069,8 @@ void ensure_model_maps(sg_engine* e, RecState& r, const sg_model_desc* models, i
 
 }  // namespace sg
 
-Shape64 sg::plain_shape(sg_engine* e, const PackedModels& pm, long long items) {
-    const Shape64 sh = shape64(pm.smem64, items, e->num_sms, (size_t)e->max_smem);
+Shape64 sg::plain_shape(sg_engine* e, const PackedModels& pm, long long items, bool refine) {
+    const Shape64 sh = shape64(pm.smem64, items, refine, e->num_sms, (size_t)e->max_smem);
     require(sh.smem <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
     return sh;
 }
@@ -1334,7 +1334,7 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
-        const Shape64 sh = plain_shape(e, pm, nposes);
+        const Shape64 sh = plain_shape(e, pm, nposes, true);
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "refine: bad pose model");
         const int cs = pm.max_conf, hs = pm.max_heavy;
         Staged<double> dc(io, e), de(io, e), dx(io, e);
@@ -1424,7 +1424,7 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
-        const Shape64 sh = plain_shape(e, pm, nposes);
+        const Shape64 sh = plain_shape(e, pm, nposes, true);
         require(conf_stride >= pm.max_conf && coord_stride >= pm.max_heavy, "minimize: strides too small");
         for (int k = 0; k < nposes; k++) {
             require(pose_model[k] >= 0 && pose_model[k] < nmodels && maxiters[k] >= 0, "minimize: bad pose");

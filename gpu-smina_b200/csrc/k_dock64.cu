@@ -368,12 +368,14 @@ void Smem64::add(const DModel& h) {
     staged = std::max(staged, bytes(true));
 }
 
-// Warps per item: 8 while that leaves every item an SM half to itself, 4 for
-// more items (more blocks resident, and the leaders' serial parts are what then
-// fills the SM), 1 with nothing staged for models that only fit so.
-Shape64 shape64(const Smem64& s, long long items, int num_sms, size_t max_smem) {
+// Warps per item: 8 for refinements, whose direct sums keep them busy (one B200, 8
+// warps against 4: 9 poses 1.19 / 1.59 ms, 297 7.1 / 9.6, 1,890 30.8 / 38.4), and for few
+// items; 4 for more chains or evaluations on the maps than two per SM (10 steps of
+// 700 chains 60.5 / 53.6 ms, of 296 31.2 / 31.8); 1 with nothing staged for models that
+// only fit so.
+Shape64 shape64(const Smem64& s, long long items, bool refine, int num_sms, size_t max_smem) {
     const size_t xb = kXbuf64 * sizeof(double);
-    if (items <= 2LL * num_sms && s.staged + 8 * xb <= max_smem) return {8, s.staged + 8 * xb};
+    if ((refine || items <= 2LL * num_sms) && s.staged + 8 * xb <= max_smem) return {8, s.staged + 8 * xb};
     if (s.staged + 4 * xb <= max_smem) return {4, s.staged + 4 * xb};
     return {1, s.plain};
 }
