@@ -1078,11 +1078,11 @@ def main():
             "e2e": {"value": e2e, "unit": UNIT,
                     "h2d_bytes_per_step": int(sum(r[2]["h2d_bytes"] for r in recs) / len(recs)),
                     "d2h_bytes_per_step": int(sum(r[2]["d2h_bytes"] for r in recs) / len(recs))},
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": 3 * args.steps,  # search, merge, refinement
             "clocks": {k: clocks[k] for k in ("sm_mhz", "sm_max_mhz", "reasons")},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
-                         "kernel": "k_mc32"},
+                         "kernel": "k_mc32, k_mc32_mix"},
             "roofline_l2": roof_l2,
             "cpu_baseline": cpu,
             "accuracy": accuracy,
