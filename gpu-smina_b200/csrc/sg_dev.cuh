@@ -1,6 +1,7 @@
 // Device-resident data of the engine: pair tables, receptor + grid maps,
 // packed docking models, and the launch parameters of the kernels.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include <cuda_fp16.h>
@@ -325,7 +326,7 @@ struct Ws64 {
     int coords, mf, eatom, origin, axis, q, rot, fF, fT, pe, pf;
     int x_tmp, x_cand, x_new, x_orig, g, g_new, g_orig, p, y, mhy, h, mt;
     int xbuf;  // exchange buffers of the direct sum, kXbuf64 per warp
-    // staged only
+    // staged only, from here
     int cr;  // torque terms per atom
     int s_receptor, s_csr, s_type, s_atom_frame, s_csr_start, s_heavy, s_fkind, s_fparent, s_fbegin, s_fend, s_fconf, s_fdof,
         s_level_start, s_level_frames, s_child_start, s_child_list, s_lig_begin, s_lig_end, s_lig_root, s_lig_pair_end,
@@ -354,7 +355,10 @@ constexpr int kCsr16Pairs = 4096;
 SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof, bool staged, int nheavy, int nlevels,
                        int nlig, int nblocks, int ntors) {
     Ws64 w{};
-    int o = (int)((sizeof(Hdr64) + 15) / 16) * 2;
+    // (nothing staged: the header ends with the offsets that such a block reads,
+    // so that its workspace takes no more than the models of its kind ever did)
+    const size_t header = staged ? sizeof(Hdr64) : offsetof(Hdr64, L) + offsetof(Ws64, cr);
+    int o = (int)((header + 15) / 16) * 2;
     auto take = [&](int n) { int r = o; o += (n + 1) & ~1; return r; };
     auto ints = [&](int n) { return take((n + 1) / 2); };
     w.coords = take(3 * natoms);
