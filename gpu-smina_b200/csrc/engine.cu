@@ -20,8 +20,8 @@ namespace sg {
 // ---- the devices' pools of call temporaries ------------------------------------------------
 // Streams of different engines never wait for one another through a pool: it
 // only hands a block to another stream once the first stream's work is done.
-// When an allocation fails, what the pools keep is given back and it is tried
-// again.
+// When an allocation fails, what the pools and the dropped maps (below) keep is
+// given back and it is tried again.
 struct DevPool {
     cudaMemPool_t pool = nullptr;
     int users = 0;
@@ -59,6 +59,68 @@ void pool_release(int device) {
     drop_pin_rings();  // the process's last engine is gone
 }
 
+// ---- dropped maps ------------------------------------------------------------------------
+// A receptor's maps that new tables, a user grid or another receptor in its place
+// make void: their allocations wait here for the next map build in that place,
+// which takes one that fits and frees the others (18 maps of a 22 A box with a new
+// user grid 22 ms of cudaFree and cudaMalloc otherwise, 0.7 ms so).  At most
+// kDroppedKept bytes per device, the oldest freed first; a direct sum in that
+// place frees them too, and an allocation that fails frees all on its device.
+struct DroppedMaps {
+    RecState* of;
+    int device;
+    std::unique_ptr<DevBuf> mem;
+};
+constexpr size_t kDroppedKept = size_t(2) << 30;
+static std::mutex g_dropped_mu;
+static std::vector<DroppedMaps>& g_dropped = *new std::vector<DroppedMaps>;  // oldest first
+
+// frees those that `which` picks
+template <typename F>
+static void free_dropped(F which) {
+    std::lock_guard<std::mutex> lk(g_dropped_mu);
+    g_dropped.erase(std::remove_if(g_dropped.begin(), g_dropped.end(), which), g_dropped.end());
+}
+static void free_dropped_of(RecState& r) {
+    free_dropped([&](const DroppedMaps& d) { return d.of == &r; });
+}
+RecState::~RecState() { free_dropped_of(*this); }
+// forgets r's maps, their memory kept for its next ones
+static void drop_maps(sg_engine* e, RecState& r) {
+    size_t kept = 0;
+    {
+        std::lock_guard<std::mutex> lk(g_dropped_mu);
+        g_dropped.reserve(g_dropped.size() + r.map_mem.size());
+        for (auto& m : r.map_mem) g_dropped.push_back({&r, e->device, std::move(m)});
+        for (const DroppedMaps& d : g_dropped) kept += d.device == e->device ? d.mem->bytes : 0;
+    }
+    r.clear_maps();
+    free_dropped([&](const DroppedMaps& d) {
+        if (d.device != e->device || kept <= kDroppedKept) return false;
+        kept -= d.mem->bytes;
+        return true;
+    });
+}
+// memory for n bytes of r's maps
+static std::unique_ptr<DevBuf> map_memory(RecState& r, size_t n) {
+    std::unique_ptr<DevBuf> mem;
+    {
+        std::lock_guard<std::mutex> lk(g_dropped_mu);
+        for (auto d = g_dropped.begin(); d != g_dropped.end() && !mem; ++d)
+            if (d->of == &r && d->mem->bytes >= n && d->mem->bytes / 2 <= n) {
+                mem = std::move(d->mem);
+                g_dropped.erase(d);
+                break;
+            }
+    }
+    free_dropped_of(r);
+    if (!mem) {
+        mem.reset(new DevBuf());
+        mem->alloc(n);
+    }
+    return mem;
+}
+
 static cudaError_t alloc_device(void** p, size_t n, sg_engine* pooled) {
     if (pooled && pooled->pool) return cudaMallocFromPoolAsync(p, n, pooled->pool, pooled->stream);
     return cudaMalloc(p, n);
@@ -80,6 +142,9 @@ void DevBuf::alloc(size_t n) {
     reset();
     if (alloc_device(&p, n, pool_of) != cudaSuccess) {
         cudaGetLastError();
+        int device = 0;
+        cudaGetDevice(&device);
+        free_dropped([&](const DroppedMaps& d) { return d.device == device; });
         {
             std::lock_guard<std::mutex> lk(g_pools_mu);
             for (auto& q : g_pools)
@@ -347,7 +412,7 @@ int sg_set_tables(sg_engine* e, const sg_tables_desc* t) {
         e->tables.smooth = (const double*)e->tab_smooth.p;
         e->tables.fast = (const double*)e->tab_fast.p;
         e->has_tables = true;
-        for (auto& r : e->rec) r.clear_maps();  // maps depend on the tables
+        for (auto& r : e->rec) drop_maps(e, r);  // maps depend on the tables
         cuda_check(cudaStreamSynchronize(e->stream), "tables");
     });
 }
@@ -456,6 +521,12 @@ static void build_receptor_cells(sg_engine* e, RecState& r) {
 void ensure_cells(sg_engine* e, RecState& r) {
     if (!r.cells) build_receptor_cells(e, r);
 }
+RecState& direct_receptor(sg_engine* e, int rid) {
+    RecState& r = receptor_for(e, rid);
+    ensure_cells(e, r);
+    free_dropped_of(r);
+    return r;
+}
 
 void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
     require(e->has_tables, "no tables set");
@@ -476,14 +547,7 @@ void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
                  b16 = half ? ncells * sizeof(uint4) : 0;
     auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
     const size_t per_type = (up(b64) + up(b32)) * (charged ? 2 : 1) + up(b16), total = per_type * need.size();
-    std::unique_ptr<DevBuf> mem;
-    for (auto& q : r.spare)
-        if (!mem && q->bytes >= total && q->bytes / 2 <= total) mem = std::move(q);
-    r.spare.clear();
-    if (!mem) {
-        mem.reset(new DevBuf());
-        mem->alloc(total);
-    }
+    std::unique_ptr<DevBuf> mem = map_memory(r, total);
     char* at = mem->as<char>();
     auto place = [&](MapView& v, size_t n) {
         if (!n) return;
@@ -553,7 +617,7 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
         for (int i = 0; i < r->num_atoms; i++) require(std::isfinite(r->coords[3 * i]) && std::isfinite(r->coords[3 * i + 1]) &&
                                                            std::isfinite(r->coords[3 * i + 2]), "receptor: non-finite coordinate");
         RecState& s = e->rec[rid];
-        s.clear_maps();
+        drop_maps(e, s);
         s.cells = false;
         s.ugrid.reset();  // a new receptor starts without a user grid
         s.ug = DGeom{};
@@ -613,7 +677,7 @@ int sg_set_user_grid(sg_engine* e, int rid, const sg_grid_dims* gd, const double
             r.ugrid.reset();
             r.ug = DGeom{};
         }
-        r.clear_maps();
+        drop_maps(e, r);
         refresh_header(e, r);
     });
 }
@@ -623,7 +687,7 @@ int sg_drop_receptor(sg_engine* e, int rid) {
         require(rid >= 0 && rid < SG_MAX_RECEPTORS, "receptor id out of range");
         RecState& s = e->rec[rid];
         s.clear_maps();
-        s.spare.clear();
+        free_dropped_of(s);
         s.pop_start.reset(); s.pop_list.reset(); s.pop_charge.reset();
         s.full_start.reset(); s.full_list.reset(); s.full_charge.reset();
         s.xyz.reset(); s.type.reset(); s.charge.reset(); s.dhdr.reset(); s.ugrid.reset();
@@ -1103,12 +1167,11 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
     return guarded(e, [&] {
         require(m && confs && v && out_e && out_g && nconfs > 0 && nconfs <= (1 << 24), "eval: bad arguments");
         require(e->has_tables, "no tables set");
-        RecState& r = receptor_for(e, rid);
+        RecState& r = direct ? direct_receptor(e, rid) : receptor_for(e, rid);
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, m, 1, !direct && e->precision != SG_PREC_FP64 ? kPackMixed : kPackPlain, pm);
         if (!direct) ensure_model_maps(e, r, m, 1);
-        else ensure_cells(e, r);
         const Shape64 sh = plain_shape(e, pm, nconfs);
         const DModel& h = pm.host[0];
         Staged<double> dc(io, e), de(io, e), dg(io, e), dx(io, e);
@@ -1329,8 +1392,7 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
               double* out_coords) {
     return guarded(e, [&] {
         require(pose_model && confs && cap && out_e && nposes > 0 && maxiters >= 0, "refine: bad arguments");
-        RecState& r = receptor_for(e, rid);
-        ensure_cells(e, r);
+        RecState& r = direct_receptor(e, rid);
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
@@ -1385,8 +1447,7 @@ int sg_score(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, co
         require(pose_model && confs && v && out_e && out_intra && nposes > 0 && nposes <= (1 << 24),
                 "score: bad arguments");
         require(e->has_tables, "no tables set");
-        RecState& r = receptor_for(e, rid);
-        ensure_cells(e, r);
+        RecState& r = direct_receptor(e, rid);
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
@@ -1419,8 +1480,7 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
                 int accurate_line, int early_term, double* out_e, double* out_coords, int coord_stride) {
     return guarded(e, [&] {
         require(pose_model && confs && cap && maxiters && out_e && nposes > 0, "minimize: bad arguments");
-        RecState& r = receptor_for(e, rid);
-        ensure_cells(e, r);
+        RecState& r = direct_receptor(e, rid);
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);

@@ -107,10 +107,9 @@ struct RecState {
     DGeom geom{};
     int natoms = 0;
     DevBuf xyz, type, charge, pop_start, pop_list, pop_charge, full_start, full_list, full_charge;
-    // the maps of one build share an allocation; those of maps dropped for a new
-    // receptor in this place wait in `spare` for the next build, which takes one
-    // that fits and frees the others
-    std::vector<std::unique_ptr<DevBuf>> map_mem, spare;
+    // the maps of one build share an allocation (void maps' allocations wait for the
+    // next build in this place: drop_maps)
+    std::vector<std::unique_ptr<DevBuf>> map_mem;
     MapView map64[kNumTypes], cmap64[kNumTypes], map32[kNumTypes], cmap32[kNumTypes], map16[kNumTypes];
     bool built[kNumTypes] = {};
     GridSlots slots{};   // heavy atom types that occur in the receptor
@@ -125,9 +124,12 @@ struct RecState {
             map64[t] = cmap64[t] = map32[t] = cmap32[t] = map16[t] = MapView{};
             built[t] = false;
         }
-        for (auto& m : map_mem) spare.push_back(std::move(m));
         map_mem.clear();
     }
+    RecState() = default;
+    RecState(const RecState&) = delete;
+    RecState& operator=(const RecState&) = delete;
+    ~RecState();
     size_t map_bytes() const {
         size_t b = 0;
         for (int t = 0; t < kNumTypes; t++)
@@ -265,6 +267,7 @@ struct ModelImage {
 };
 void pack_models_image(const sg_model_desc* models, int nmodels, char* dev_base, ModelImage& img);
 RecState& receptor_for(sg_engine* e, int rid);
+RecState& direct_receptor(sg_engine* e, int rid);  // for the direct sum: cell lists in place, no dropped maps kept
 void ensure_cells(sg_engine* e, RecState& r);
 void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes);
 void ensure_model_maps(sg_engine* e, RecState& r, const sg_model_desc* models, int nmodels);

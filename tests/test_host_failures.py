@@ -1,0 +1,104 @@
+"""The engine's host side when something runs out or overlaps, on a CUDA runtime
+of host memory (tests/cpp/fake_cudart.cpp, loaded in front of the real one):
+device and host allocations that fail, memory kept between calls, and calls on
+several threads.  Kernels do not run here; what is checked is which calls
+succeed, what stays allocated and that nothing ends the process.  Each case is a
+process of its own."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+HEAD = """
+import ctypes as C, sys, threading
+sys.path[:0] = [{root!r} + "/gpu-smina_b200", {root!r} + "/tests"]
+fake = C.CDLL({lib!r})
+fake.fake_live.restype = C.c_size_t
+fake.fake_limit.argtypes = [C.c_size_t]
+import numpy as np
+import smina_b200 as sb, workloads as W
+T, R, gd, m = W.tables(), W.receptor(), W.box(), W.ligand()
+HEAVY = [t for t in range(2, 27)]
+def engine(precision=sb.PREC_FP32, tables=T, receptor=True):
+    e = sb.Engine(0, precision)
+    e.set_tables(tables)
+    if receptor: e.set_receptor(0, R, gd)
+    return e
+def status(f, *a, **k):
+    try:
+        f(*a, **k)
+        return sb.SG_OK
+    except sb.SminaError as x:
+        return x.code
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    lib = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-shared", "-fPIC", "-I/usr/local/cuda/include",
+                        os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), "-pthread", "-o", lib],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+    def go(body):
+        r = subprocess.run([sys.executable, "-c", HEAD.format(root=ROOT, lib=lib) + body], capture_output=True, text=True,
+                           timeout=300, env=dict(os.environ, LD_PRELOAD=lib))
+        assert r.returncode == 0, r.stdout + r.stderr
+    return go
+
+
+def test_dropped_maps_are_bounded(run):
+    """Void maps wait for the next build in their place: freed by a direct sum
+    there, by a drop and with the engine, and never more than 2 GiB."""
+    run("""
+e = engine()
+x = W.random_confs(m, gd, 1, 1)
+bare = fake.fake_live()
+near = lambda: abs(fake.fake_live() - bare) < 2 << 20
+def built():
+    e.build_grids(0, HEAVY)
+    assert fake.fake_live() > bare + (50 << 20)
+grid = W.box(6.0)
+void = (lambda: e.set_receptor(0, R, gd), lambda: e.set_tables(T),
+        lambda: e.set_user_grid(0, grid, np.zeros(sb.grid_points(grid))))
+direct = (lambda: e.minimize(0, [m], [0], x), lambda: e.refine(0, [m], [0], x), lambda: e.score(0, [m], [0], x),
+          lambda: e.eval_direct(0, m, x))
+for change in void:
+    for use in direct:
+        built(); change(); use(); assert near()
+    built(); size = fake.fake_live(); change(); built(); assert abs(fake.fake_live() - size) < 2 << 20
+sb.load().sg_drop_receptor(e._h, 0)
+assert fake.fake_live() < bare
+fake.fake_limit(64 << 30)
+for k in range(16): e.set_receptor(k, R, W.box(36.0))
+bare = fake.fake_live()
+for k in range(16): e.build_grids(k, HEAVY)
+assert fake.fake_live() > bare + (8 << 30)
+e.set_tables(T)
+assert bare < fake.fake_live() <= bare + (2 << 30)
+e.close()
+assert fake.fake_live() == 0
+""")
+
+
+def test_dropped_maps_give_way_to_allocations(run):
+    """An allocation that needs the memory of dropped maps gets it: the same
+    engine's, another slot's and another engine's."""
+    run("""
+a, b = engine(), engine()
+a.set_receptor(1, R, gd)
+before = fake.fake_live()
+a.build_grids(0, HEAVY)
+maps = fake.fake_live() - before
+for user, rid in ((a, 1), (b, 0)):
+    a.set_receptor(0, R, gd)  # drops slot 0's maps
+    fake.fake_limit(fake.fake_live() + maps // 4)
+    assert status(user.build_grids, rid, HEAVY) == sb.SG_OK
+    fake.fake_limit(8 << 30)
+    user.set_tables(T)
+    a.build_grids(0, HEAVY)
+""")
