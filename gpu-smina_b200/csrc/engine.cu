@@ -387,6 +387,9 @@ int sg_set_tables(sg_engine* e, const sg_tables_desc* t) {
         require(t->num_components == 1 || t->num_components == 4, "tables: num_components must be 1 or 4");
         require(t->factor > 0 && t->cutoff_sqr > 0, "tables: factor and cutoff must be positive");
         require(t->n >= (int)(size_t)(t->factor * t->cutoff_sqr) + 3 && t->n < (1 << 24), "tables: n too small");
+        // (without tables from here on, should one of the uploads fail)
+        e->has_tables = false;
+        for (auto& r : e->rec) drop_maps(e, r);  // maps depend on the tables
         const size_t np = kNumTypePairs;
         e->tab_smooth.upload(t->smooth, np * t->n * t->num_components * 2 * sizeof(double), e->stream);
         e->tab_fast.upload(t->fast, np * t->n * t->num_components * sizeof(double), e->stream);
@@ -411,9 +414,8 @@ int sg_set_tables(sg_engine* e, const sg_tables_desc* t) {
         e->tables.cutoff_sqr = t->cutoff_sqr;
         e->tables.smooth = (const double*)e->tab_smooth.p;
         e->tables.fast = (const double*)e->tab_fast.p;
-        e->has_tables = true;
-        for (auto& r : e->rec) drop_maps(e, r);  // maps depend on the tables
         cuda_check(cudaStreamSynchronize(e->stream), "tables");
+        e->has_tables = true;
     });
 }
 
@@ -425,6 +427,7 @@ namespace sg {
 RecState& receptor_for(sg_engine* e, int rid) {
     require(rid >= 0 && rid < SG_MAX_RECEPTORS, "receptor id out of range");
     require(e->rec[rid].set, "receptor " + std::to_string(rid) + " has not been set");
+    require(e->has_tables, "no tables set");
     return e->rec[rid];
 }
 
@@ -617,8 +620,8 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
         for (int i = 0; i < r->num_atoms; i++) require(std::isfinite(r->coords[3 * i]) && std::isfinite(r->coords[3 * i + 1]) &&
                                                            std::isfinite(r->coords[3 * i + 2]), "receptor: non-finite coordinate");
         RecState& s = e->rec[rid];
+        s.set = s.cells = false;  // (no receptor in this place, should a step fail)
         drop_maps(e, s);
-        s.cells = false;
         s.ugrid.reset();  // a new receptor starts without a user grid
         s.ug = DGeom{};
         s.gd = *gd;
@@ -635,8 +638,8 @@ int sg_set_receptor(sg_engine* e, int rid, const sg_receptor_desc* r, const sg_g
         s.xyz.upload(r->coords, sizeof(double) * 3 * std::max(1, r->num_atoms), e->stream);
         s.type.upload(types.data(), sizeof(int) * std::max<size_t>(1, types.size()), e->stream);
         s.charge.upload(r->charge, sizeof(double) * std::max(1, r->num_atoms), e->stream);
-        s.set = true;
         build_receptor_cells(e, s);
+        s.set = true;
     });
 }
 
@@ -662,6 +665,12 @@ int sg_get_grid(sg_engine* e, int rid, int type, double* data, double* chargedat
 int sg_set_user_grid(sg_engine* e, int rid, const sg_grid_dims* gd, const double* data, double cache_slope) {
     return guarded(e, [&] {
         RecState& r = receptor_for(e, rid);
+        auto without = [&] {
+            r.ugrid.reset();
+            r.ug = DGeom{};
+            drop_maps(e, r);
+            refresh_header(e, r);
+        };
         if (gd && data) {
             for (int i = 0; i < 3; i++) {
                 require(gd->n[i] >= 1 && gd->n[i] <= 4096, "user grid: n must be in [1, 4096]");
@@ -670,15 +679,19 @@ int sg_set_user_grid(sg_engine* e, int rid, const sg_grid_dims* gd, const double
             require(std::isfinite(cache_slope), "user grid: non-finite slope");
             const size_t n = (size_t)(gd->n[0] + 1) * (gd->n[1] + 1) * (gd->n[2] + 1);
             for (size_t k = 0; k < n; k++) require(std::isfinite(data[k]), "user grid: non-finite value");
-            r.ugrid.upload(data, n * sizeof(double), e->stream);
+            try {
+                r.ugrid.upload(data, n * sizeof(double), e->stream);
+            } catch (...) {  // the old grid's memory is gone
+                without();
+                throw;
+            }
             r.ug = make_geom(*gd);
             r.ug_slope = cache_slope;
+            drop_maps(e, r);
+            refresh_header(e, r);
         } else {
-            r.ugrid.reset();
-            r.ug = DGeom{};
+            without();
         }
-        drop_maps(e, r);
-        refresh_header(e, r);
     });
 }
 

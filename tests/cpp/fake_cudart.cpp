@@ -13,6 +13,7 @@
 #include <map>
 #include <mutex>
 #include <new>
+#include <set>
 #include <string>
 #include <thread>
 
@@ -23,6 +24,7 @@ struct State {
     std::map<const void*, int> max_dynamic;  // per kernel
     std::map<std::string, int> launches;
     std::map<void*, std::pair<size_t, bool>> blocks;  // device memory: bytes, of a pool
+    std::set<void*> freed;  // blocks of at most 1 MB given back (their addresses are not used again)
 };
 State& st() {
     static State* s = new State;
@@ -52,7 +54,8 @@ cudaError_t give(void* p) {
     st().blocks.erase(p);
     live -= b.first;
     if (b.second) kept += b.first;
-    std::free(p);
+    if (b.first <= (1 << 20)) st().freed.insert(p);
+    else std::free(p);
     return cudaSuccess;
 }
 }  // namespace
@@ -72,6 +75,17 @@ void operator delete(void* p, size_t) noexcept { std::free(p); }
 extern "C" {
 void fake_limit(size_t n) { limit = n; }
 size_t fake_live() { return live; }
+int fake_dangling() {  // pointers to freed blocks in live ones of at most 4 KB
+    std::lock_guard<std::mutex> lk(mu);
+    int n = 0;
+    for (auto& b : st().blocks)
+        for (size_t k = 0; b.second.first <= 4096 && k + 8 <= b.second.first; k += 8) {
+            void* q;
+            std::memcpy(&q, static_cast<char*>(b.first) + k, 8);
+            n += (int)st().freed.count(q);
+        }
+    return n;
+}
 int fake_host_allocs() { return host_allocs; }
 void fake_sync_ms(int ms) { sync_ms = ms; }
 void fake_attr_ms(int ms) { attr_ms = ms; }

@@ -102,3 +102,44 @@ for user, rid in ((a, 1), (b, 0)):
     user.set_tables(T)
     a.build_grids(0, HEAVY)
 """)
+
+
+def test_a_failed_change_leaves_nothing_half_set(run):
+    """After an allocation failed in sg_set_receptor or sg_set_tables, calls that
+    would use the receptor or the tables are refused; after one in
+    sg_set_user_grid the receptor has no grid.  Nothing runs on freed memory."""
+    run("""
+x = W.random_confs(m, gd, 2, 1)
+big = W.receptor(9000)
+e = engine()
+uses = (lambda: e.bfgs(0, m, x), lambda: e.eval(0, m, x), lambda: e.minimize(0, [m], [0, 0], x),
+        lambda: e.score(0, [m], [0, 0], x), lambda: e.build_grids(0, [2]))
+def refused():
+    n = fake.fake_launches(b"")
+    assert all(status(f) == sb.SG_ERR_ARG for f in uses) and fake.fake_launches(b"") == n
+def after_failures(change, check, least):
+    failed, room = 0, 0
+    while True:
+        fake.fake_limit(fake.fake_live() + room)
+        rc = status(change)
+        fake.fake_limit(8 << 30)
+        if rc == sb.SG_OK: break
+        assert rc == sb.SG_ERR_NOMEM
+        check()
+        failed += 1
+        room += 256 << 10
+    assert failed >= least, failed
+    assert all(status(f) == sb.SG_OK for f in uses), [status(f) for f in uses]
+after_failures(lambda: e.set_receptor(0, big, W.box(30.0)), refused, 2)
+def bare():  # the receptor without maps, so that none give way
+    e.set_receptor(0, R, gd)
+    uses[2]()
+bare()
+after_failures(lambda: e.set_tables(W.tables("ad4_scoring")), refused, 2)
+small, larger = W.box(6.0), W.box(12.0)
+bare()
+e.set_user_grid(0, small, np.zeros(sb.grid_points(small)))
+def no_grid(): assert fake.fake_dangling() == 0
+no_grid()
+after_failures(lambda: e.set_user_grid(0, larger, np.zeros(sb.grid_points(larger))), no_grid, 1)
+""")
