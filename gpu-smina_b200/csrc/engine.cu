@@ -570,7 +570,16 @@ void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
         }
         cmaps.push_back(r.cmap64[t].as<double>());
     }
-    r.map_mem.push_back(std::move(mem));
+    // their memory goes back with its maps when a later step fails
+    struct Undo {
+        RecState& r;
+        const std::vector<int>& need;
+        bool done = false;
+        ~Undo() {
+            if (done) return;
+            for (int t : need) r.map64[t] = r.cmap64[t] = r.map32[t] = r.cmap32[t] = r.map16[t] = MapView{};
+        }
+    } undo{r, need};
     // one upload: map pointers, charge map pointers, maps to pack, type numbers
     const size_t nt = need.size();
     std::vector<GridPack> packs;
@@ -599,6 +608,8 @@ void ensure_maps(sg_engine* e, RecState& r, const int* types, int ntypes) {
                                     (int)packs.size(), e->stream),
                    "pack maps");
     cuda_check(cudaStreamSynchronize(e->stream), "grid maps");
+    r.map_mem.push_back(std::move(mem));
+    undo.done = true;
     for (int t : need) r.built[t] = true;
     refresh_header(e, r);
 }

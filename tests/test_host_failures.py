@@ -143,3 +143,22 @@ def no_grid(): assert fake.fake_dangling() == 0
 no_grid()
 after_failures(lambda: e.set_user_grid(0, larger, np.zeros(sb.grid_points(larger))), no_grid, 1)
 """)
+
+
+def test_a_failed_map_build_keeps_no_memory(run):
+    """Memory taken for maps whose build then fails is given back."""
+    run("""
+e = engine()
+bare = fake.fake_live()
+e.build_grids(0, HEAVY)
+maps = fake.fake_live() - bare
+e.set_receptor(0, R, gd)
+e.minimize(0, [m], [0], W.random_confs(m, gd, 1, 1))  # without maps again
+bare = fake.fake_live()
+fake.fake_limit(bare + maps + (64 << 10))  # room for the maps, not for the table that they are built from
+for k in range(3):
+    assert status(e.build_grids, 0, HEAVY) == sb.SG_ERR_NOMEM
+    assert fake.fake_live() - bare < 1 << 20, k
+fake.fake_limit(8 << 30)
+assert status(e.build_grids, 0, HEAVY) == sb.SG_OK
+""")
