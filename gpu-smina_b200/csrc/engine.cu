@@ -10,7 +10,6 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 #include "engine.h"
@@ -196,7 +195,10 @@ static void ring_put(std::unique_ptr<PinRing> r) {
         x = nullptr;
     }
     std::lock_guard<std::mutex> lk(g_rings_mu);
-    if (g_rings.size() < kRingsKept) g_rings.push_back(std::move(r));
+    try {
+        if (g_rings.size() < kRingsKept) g_rings.push_back(std::move(r));
+    } catch (std::bad_alloc&) {  // not kept then (callers are destructors)
+    }
 }
 void warm_pin_ring() {
     {
@@ -1048,10 +1050,11 @@ static void pack_pools(const sg_model_desc* models, int nmodels, PackFor what, P
         }
     };
     std::vector<std::thread> threads;
+    threads.reserve(P.parts.size());  // (nothing may throw past a thread that has not been joined)
     for (size_t q = 1; q < P.parts.size(); q++) {
         try {
             threads.emplace_back(work, q);
-        } catch (std::system_error&) {  // no more threads to be had
+        } catch (...) {  // no thread or no memory for one
             work(q);
         }
     }

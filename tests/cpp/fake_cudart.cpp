@@ -34,11 +34,17 @@ size_t limit = size_t(8) << 30, live = 0, kept = 0;  // live: allocated; kept: f
 std::atomic<int> host_allocs{0}, sync_ms{0}, attr_ms{0};
 thread_local long new_countdown = 0;
 thread_local bool new_fired = false;
+struct Held {  // the runtime's own state: locked, and its allocations not counted
+    std::lock_guard<std::mutex> lock{mu};
+    long countdown = new_countdown;
+    Held() { new_countdown = 0; }
+    ~Held() { new_countdown = countdown; }
+};
 void nap(int ms) {
     if (ms) std::this_thread::sleep_for(std::chrono::milliseconds(ms));
 }
 cudaError_t take(void** p, size_t n, bool pooled) {
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     const size_t reused = pooled ? std::min(n, kept) : 0;
     if (live + kept - reused + n > limit) return cudaErrorMemoryAllocation;
     *p = std::calloc(1, n ? n : 1);
@@ -49,7 +55,7 @@ cudaError_t take(void** p, size_t n, bool pooled) {
 }
 cudaError_t give(void* p) {
     if (!p) return cudaSuccess;
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     const auto b = st().blocks[p];
     st().blocks.erase(p);
     live -= b.first;
@@ -76,7 +82,7 @@ extern "C" {
 void fake_limit(size_t n) { limit = n; }
 size_t fake_live() { return live; }
 int fake_dangling() {  // pointers to freed blocks in live ones of at most 4 KB
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     int n = 0;
     for (auto& b : st().blocks)
         for (size_t k = 0; b.second.first <= 4096 && k + 8 <= b.second.first; k += 8) {
@@ -92,14 +98,14 @@ void fake_attr_ms(int ms) { attr_ms = ms; }
 void fake_fail_new(long nth) { new_countdown = nth; new_fired = false; }
 int fake_new_fired() { new_countdown = 0; return new_fired; }
 int fake_launches(const char* part) {  // launches of kernels whose (mangled) name holds `part`
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     int n = 0;
     for (auto& k : st().launches)
         if (k.first.find(part) != std::string::npos) n += k.second;
     return n;
 }
 int fake_max_dynamic(const char* part) {  // the largest dynamic shared memory such a kernel is set to
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     int n = 0;
     for (auto& k : st().kernels)
         if (k.second.find(part) != std::string::npos && st().max_dynamic.count(k.first))
@@ -111,7 +117,7 @@ void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}
 void __cudaUnregisterFatBinary(void**) {}
 void __cudaRegisterFunction(void**, const char* host, char*, const char* name, int, uint3*, uint3*, dim3*, dim3*, int*) {
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     st().kernels[host] = name;
 }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
@@ -123,7 +129,7 @@ cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void*) {
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t, cudaStream_t) {
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     st().launches[st().kernels[f]]++;
     return cudaSuccess;
 }
@@ -131,14 +137,14 @@ cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* f) {
     *a = cudaFuncAttributes{};
     a->sharedSizeBytes = 2048;
     {
-        std::lock_guard<std::mutex> lk(mu);
+        Held held;
         a->maxDynamicSharedSizeBytes = st().max_dynamic.count(f) ? st().max_dynamic[f] : 48 * 1024;
     }
     nap(attr_ms);
     return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v) {
-    std::lock_guard<std::mutex> lk(mu);
+    Held held;
     st().max_dynamic[f] = v;
     return cudaSuccess;
 }
@@ -173,9 +179,9 @@ cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStrea
 cudaError_t cudaFree(void* p) { return give(p); }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return give(p); }
 cudaError_t cudaMemPoolCreate(cudaMemPool_t* p, const cudaMemPoolProps*) { *p = (cudaMemPool_t)1; return cudaSuccess; }
-cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { std::lock_guard<std::mutex> lk(mu); kept = 0; return cudaSuccess; }
+cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { Held held; kept = 0; return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
-cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { std::lock_guard<std::mutex> lk(mu); kept = 0; return cudaSuccess; }
+cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { Held held; kept = 0; return cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = limit - live - kept; *t = limit; return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { host_allocs++; *p = std::malloc(n); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }

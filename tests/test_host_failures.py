@@ -162,3 +162,38 @@ for k in range(3):
 fake.fake_limit(8 << 30)
 assert status(e.build_grids, 0, HEAVY) == sb.SG_OK
 """)
+
+
+@pytest.mark.parametrize("call", ["score", "minimize", "dock", "dock_batch", "eval", "bfgs", "set_receptor", "build_grids"])
+def test_host_allocation_failures_are_statuses(run, call):
+    """The nth host allocation of a call fails, for every n: the call returns
+    SG_ERR_NOMEM (or does without), the process goes on and the next call works."""
+    run(f"call = {call!r}" + """
+e = engine(sb.PREC_FP64 if call == "dock" else sb.PREC_FP32)
+few = 64 if call == "score" else 3  # 64 models are packed on several threads
+ms = [W.ligand(10 + k % 7, k % 3, k) for k in range(few)]
+x = [W.random_confs(q, gd, 1, 1)[0] for q in ms]
+cs = max(q.conf_size for q in ms)
+confs = np.array([np.pad(c, (0, cs - len(c))) for c in x])
+pm, p = list(range(few)), ms[0].search_params()
+c0, mt = ms[0].seed_chains(5, 2, gd)
+f = {"score": lambda: e.score(0, ms, pm, confs), "minimize": lambda: e.minimize(0, ms, pm, confs),
+     "dock": lambda: e.dock(0, ms[:1], [0, 0], c0, mt, p, steps=1),
+     "dock_batch": lambda: e.dock_batch(0, ms, [sb.LigandJob(model=k, num_chains=2, num_steps=2, maxiters=0, seed=1,
+                                                             ligand_key=k) for k in pm], p),
+     "eval": lambda: e.eval(0, ms[0], x[:1]), "bfgs": lambda: e.bfgs(0, ms[0], x[:1]),
+     "set_receptor": lambda: e.set_receptor(0, R, gd),
+     "build_grids": lambda: (e.set_receptor(0, R, gd), e.build_grids(0, HEAVY))}[call]
+assert status(f) == sb.SG_OK
+n, failed = 0, 0
+while True:
+    n += 1
+    fake.fake_fail_new(n)
+    rc = status(f)
+    if not fake.fake_new_fired(): break
+    assert rc in (sb.SG_OK, sb.SG_ERR_NOMEM), rc
+    failed += rc == sb.SG_ERR_NOMEM
+    if call in ("set_receptor", "build_grids"): e.set_receptor(0, R, gd)
+    if n % 16 == 0: assert status(f) == sb.SG_OK
+assert failed > 10 and status(f) == sb.SG_OK
+""")
