@@ -197,3 +197,24 @@ while True:
     if n % 16 == 0: assert status(f) == sb.SG_OK
 assert failed > 10 and status(f) == sb.SG_OK
 """)
+
+
+def test_engines_on_threads_pin_memory_once(run):
+    """Calls on eight engines at once pin one ring of memory each and keep it."""
+    run("""
+es = [engine() for _ in range(8)]
+x = W.random_confs(m, gd, 4, 1)
+for e in es: e.eval(0, m, x)
+def at_once():
+    fake.fake_sync_ms(40)  # every call lasts until all have begun
+    ts = [threading.Thread(target=e.eval, args=(0, m, x)) for e in es]
+    for t in ts: t.start()
+    for t in ts: t.join()
+    fake.fake_sync_ms(0)
+before = fake.fake_host_allocs()
+at_once()
+first = fake.fake_host_allocs()
+assert first - before <= 8
+for k in range(3): at_once()
+assert fake.fake_host_allocs() == first
+""")
