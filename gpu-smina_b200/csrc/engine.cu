@@ -304,6 +304,15 @@ void CallIo::finish() {
     }
 }
 
+cudaError_t raise_dynamic_smem(const void* kernel, size_t smem) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes fa{};
+    cudaError_t rc = cudaFuncGetAttributes(&fa, kernel);
+    if (rc != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= smem) return rc;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
 void cuda_check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) {
         // a failed call that does not poison the context still stays the

@@ -1006,16 +1006,6 @@ size_t ws32_bytes(const DModel& hm) {
     return (size_t)ws32_layout(hm.natoms, hm.nframes, hm.conf_size, hm.dof).total;
 }
 
-// Raises the kernel's dynamic shared memory limit to `smem` (never lowers it,
-// so launches sized against an earlier, larger limit stay valid).
-static cudaError_t prep32(const void* fn, size_t smem) {
-    cudaFuncAttributes fa{};
-    cudaError_t rc = cudaFuncGetAttributes(&fa, fn);
-    if (rc != cudaSuccess) return rc;
-    if ((size_t)fa.maxDynamicSharedSizeBytes >= smem) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
 static const void* k_mc32_for(int team) {
     return team == 4 ? (const void*)k_mc32<4> : team == 2 ? (const void*)k_mc32<2> : (const void*)k_mc32<1>;
 }
@@ -1026,7 +1016,7 @@ static const void* k_mc32_for(int team) {
 int mc32_occupancy(int team, int wpb, size_t smem) {
     int blocks = 0;
     const void* fn = k_mc32_for(team);
-    if (prep32(fn, smem) != cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, 32 * wpb, smem) !=
+    if (raise_dynamic_smem(fn, smem) != cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, fn, 32 * wpb, smem) !=
                                                cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -1039,7 +1029,7 @@ cudaError_t launch_mc32(const DModel* dms, const DTables32& T, const DMaps32& G,
                         int blocks, int wpb, size_t stage_stride, size_t ws_stride, int team, cudaStream_t s) {
     if (!(team == 1 || team == 2 || team == 4) || wpb % team) return cudaErrorInvalidValue;
     const size_t smem = stage_stride + (size_t)wpb * ws_stride;
-    cudaError_t rc = prep32(k_mc32_for(team), smem);
+    cudaError_t rc = raise_dynamic_smem(k_mc32_for(team), smem);
     if (rc != cudaSuccess) return rc;
     if (team == 4)
         k_mc32<4><<<blocks, 32 * wpb, smem, s>>>(dms, T, G, maps_tab, chains, items, nitems, P, queue,
@@ -1056,7 +1046,7 @@ cudaError_t launch_mc32(const DModel* dms, const DTables32& T, const DMaps32& G,
 // resident blocks per SM of k_mc32_mix with `warps` warps; 0 when it does not fit
 int mc32_mix_occupancy(int warps, size_t smem) {
     int blocks = 0;
-    if (prep32((const void*)k_mc32_mix, smem) != cudaSuccess ||
+    if (raise_dynamic_smem((const void*)k_mc32_mix, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_mc32_mix, 32 * warps, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -1076,7 +1066,7 @@ cudaError_t launch_mc32_mix(const DModel* dms, const DTables32& T, const DMaps32
 // launches (serving's many concurrent ones, the no-allocation entry point's)
 // set no function attribute while other launches of the kernel run.  The
 // first use also loads the kernel's module.
-cudaError_t mc32_reserve_smem(size_t smem) { return prep32((const void*)k_mc32<1>, smem); }
+cudaError_t mc32_reserve_smem(size_t smem) { return raise_dynamic_smem((const void*)k_mc32<1>, smem); }
 
 // the largest dynamic shared memory a k_mc32 block can take: the device's
 // opt-in limit less the kernel's static shared memory
@@ -1114,7 +1104,7 @@ static cudaError_t conf_shape32(const void* fn, size_t stage, size_t ws, int tea
         const size_t smem = stage + (size_t)t * team * ws;
         if (smem > max_smem || (t > 1 && (long long)t * num_sms > n)) continue;
         int occ = 0;
-        if (prep32(fn, smem) != cudaSuccess ||
+        if (raise_dynamic_smem(fn, smem) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, 32 * team * t, smem) != cudaSuccess) {
             cudaGetLastError();  // this many teams do not fit; fewer may
             continue;
@@ -1160,7 +1150,7 @@ cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide
         for (int warps : {8, 4}) {
             const size_t smem = stage + ws + wide;
             int occ = 0;
-            if (smem > max_smem || prep32((const void*)k_bfgs32_wide, smem) != cudaSuccess ||
+            if (smem > max_smem || raise_dynamic_smem((const void*)k_bfgs32_wide, smem) != cudaSuccess ||
                 cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bfgs32_wide, 32 * warps, smem) != cudaSuccess) {
                 cudaGetLastError();
                 break;
@@ -1174,7 +1164,7 @@ cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide
     if (!(team == 1 || team == 2 || team == 4)) return cudaErrorInvalidValue;
     const size_t smem = stage + (size_t)team * ws;
     const void* fn = team == 4 ? (const void*)k_bfgs32<4> : team == 2 ? (const void*)k_bfgs32<2> : (const void*)k_bfgs32<1>;
-    cudaError_t rc = prep32(fn, smem);
+    cudaError_t rc = raise_dynamic_smem(fn, smem);
     if (rc != cudaSuccess) return rc;
     const float v0 = (float)v[0], v1 = (float)v[1], v2 = (float)v[2], sl = (float)slope;
     if (team == 4)
@@ -1195,7 +1185,7 @@ cudaError_t launch_mc32_feed(const DTables32& T, const FeedItem32* ring, unsigne
 }
 
 // raises k_mc32_feed's dynamic shared-memory limit ahead of its launches
-cudaError_t mc32_feed_reserve_smem(size_t smem) { return prep32((const void*)k_mc32_feed, smem); }
+cudaError_t mc32_feed_reserve_smem(size_t smem) { return raise_dynamic_smem((const void*)k_mc32_feed, smem); }
 
 // the largest dynamic shared memory a k_mc32_feed block can take within
 // `optin` bytes: less the kernel's static shared memory

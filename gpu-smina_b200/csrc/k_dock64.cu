@@ -380,14 +380,8 @@ Shape64 shape64(const Smem64& s, long long items, bool refine, int num_sms, size
     return {1, s.plain};
 }
 
-// Raises the kernel's dynamic shared memory limit to `smem` (never lowers it:
-// another thread's launch may be sized against the higher one).
 static cudaError_t prep64(const void* fn, size_t smem) {
-    if (smem <= 48 * 1024) return cudaSuccess;
-    cudaFuncAttributes fa{};
-    cudaError_t rc = cudaFuncGetAttributes(&fa, fn);
-    if (rc != cudaSuccess || (size_t)fa.maxDynamicSharedSizeBytes >= smem) return rc;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return smem <= 48 * 1024 ? cudaSuccess : raise_dynamic_smem(fn, smem);
 }
 
 // launches kernel<G, ST> with the shape's G

@@ -428,6 +428,9 @@ struct Smem64 {
     size_t plain = 0, staged = 0;
     void add(const DModel& h);
 };
+// Raises a kernel's limit of dynamic shared memory to `smem` and never lowers it,
+// whatever other threads do: their launches may be sized against a higher one.
+cudaError_t raise_dynamic_smem(const void* kernel, size_t smem);
 // a plain-path launch: warps per item and its shared memory
 struct Shape64 {
     int warps;

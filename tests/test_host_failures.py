@@ -218,3 +218,24 @@ assert first - before <= 8
 for k in range(3): at_once()
 assert fake.fake_host_allocs() == first
 """)
+
+
+def test_threads_do_not_lower_a_kernels_shared_memory(run):
+    """Two engines launch the same kernel at once, the one that needs less
+    shared memory a little later: the limit ends at the larger need."""
+    run("""
+es = [engine(sb.PREC_FP64), engine(sb.PREC_FP64)]
+ms = [W.ligand(80, 20, 7), W.ligand(60, 12, 3)]  # both above the 48 KB that need no limit
+for kernel, f in ((b"k_score64", lambda e, q: e.score(0, [q], [0], W.random_confs(q, gd, 1, 1))),
+                  (b"k_refine64", lambda e, q: e.minimize(0, [q], [0], W.random_confs(q, gd, 1, 1)))):
+    fake.fake_attr_ms(200)
+    ts = [threading.Thread(target=f, args=a) for a in zip(es, ms)]
+    ts[0].start()
+    threading.Event().wait(0.1)
+    ts[1].start()
+    for t in ts: t.join()
+    fake.fake_attr_ms(0)
+    both = fake.fake_max_dynamic(kernel)
+    f(es[0], ms[0])  # raises it again, had it been lowered
+    assert both == fake.fake_max_dynamic(kernel) > 49152
+""")
