@@ -204,85 +204,148 @@ __device__ __forceinline__ bool within64(double margin) {
     return __all_sync(kFull, ok);
 }
 
-// merge_output_containers of one ligand's chains per block (one warp):
-// add_to_output_container (coords.cpp:25-58) over the chains in order, each one's
-// poses best first.  The list holds (chain, slot) and energies; a pose's RMSD to
-// the listed ones is one lane each, its coordinates' squares added in order, as
-// the host merge did in double precision.  Bound by that serial sum; in exchange
-// the chains' containers stay on the device (41 MB for 400 ligands, whose merge took
-// a host thread 0.1 s) and the refinement follows without a host step.
-__global__ void __launch_bounds__(32) k_merge32(const DModel* models, const MergeJob32* jobs, const Chain32* chains,
-                                                int S, double min_rmsd, int* out_count, int* pose_model,
-                                                double* out_e, double* out_conf, int conf_stride, double* out_xyz,
-                                                int xyz_stride) {
+// merge_output_containers of one ligand's chains per block: add_to_output_container
+// (coords.cpp:25-58) over the chains in order, each one's poses best first.  The
+// list holds the energies (ascending), the poses' places and their columns of D.
+// Poses are taken in groups of `group`: all distances of a group's poses to the
+// list and to one another at once, one thread each (a pose's squares added in
+// order, as the host merge does in double precision), then the first warp takes
+// the poses one by one with what D holds.  Bound by the latency of both.  For
+// 1,000 chains of one 24-atom ligand (9 poses kept, search 36 ms) a call took 48 ms on
+// one B200, for 512 chains of a 10-atom one with up to 1,000 poses kept 161 ms; with one
+// warp that measured each pose when its turn came, and one lane that moved the
+// list, 63 and 500 ms.
+__host__ __device__ constexpr size_t merge32_bytes(int S, int group) {
+    return (size_t)S * (sizeof(double) + sizeof(int2) + sizeof(int)) +
+           (size_t)group * (sizeof(double) + sizeof(int2) + (S + group) * sizeof(double)) + 16;
+}
+constexpr int kMergeThreads = 256;
+__global__ void __launch_bounds__(kMergeThreads) k_merge32(const DModel* models, const MergeJob32* jobs,
+                                                           const Chain32* chains, int S, int group, double min_rmsd,
+                                                           int* out_count, int* pose_model, double* out_e,
+                                                           double* out_conf, int conf_stride, double* out_xyz,
+                                                           int xyz_stride) {
     extern __shared__ __align__(16) double smem_merge[];
-    double* le = smem_merge;                          // [S] energies, ascending
-    int* lc = reinterpret_cast<int*>(le + S);         // [S] chain
-    int* ls = lc + S;                                 // [S] slot
-    const int j = blockIdx.x, lane = threadIdx.x;
+    double* le = smem_merge;               // [S] the list: energies,
+    double* D = le + S;                    // [group][S + group] distances
+    double* ge = D + (size_t)group * (S + group);  // [group] the group: energies,
+    int2* at_list = reinterpret_cast<int2*>(ge + group);  // [S] chain and slot,
+    int2* at_group = at_list + S;                         // [group] chain and slot
+    int* col = reinterpret_cast<int*>(at_group + group);  // [S] column of D
+    __shared__ int s_taken;
+    const int j = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const MergeJob32 job = jobs[j];
     const int H = models[job.model].nheavy, H3 = 3 * H, cs = models[job.model].conf_size;
-    int n = 0;
-    for (int c = job.first; c < job.first + job.count; c++) {
-        const Chain32& ch = chains[c];
-        const int cnt = min(max(*ch.out_count, 0), S);
-        for (int i = 0; i < cnt; i++) {
-            const int slot = min(max(ch.out_order[i], 0), S - 1);
-            const double e = ch.out_e[slot];
-            const float* x = ch.out_coords + (size_t)slot * H3;
-            double best = kMaxFl;
-            int bi = n;
-            for (int k = lane; k < n; k += 32) {
-                const float* y = chains[lc[k]].out_coords + (size_t)ls[k] * H3;
-                double acc = 0;
-#pragma unroll 6
-                for (int a = 0; a < H3; a++) {
-                    const double d = (double)x[a] - (double)y[a];
-                    acc += d * d;
+    auto coords = [&](int2 q) { return chains[q.x].out_coords + (size_t)q.y * H3; };
+    int n = 0, c = job.first, i = 0;  // the list's length (all threads); the next pose's chain and rank (first warp)
+    for (;;) {
+        if (tid < 32) {  // the next group
+            int taken = 0;
+            while (taken < group && c < job.first + job.count) {
+                const Chain32& ch = chains[c];
+                const int cnt = min(max(*ch.out_count, 0), S), k = min(min(cnt - i, group - taken), 32);
+                if (lane < k) {
+                    const int slot = min(max(ch.out_order[i + lane], 0), S - 1);
+                    at_group[taken + lane] = make_int2(c, slot);
+                    ge[taken + lane] = ch.out_e[slot];
                 }
-                const double r = H3 ? sqrt(acc / (double)H) : 0.0;
-                if (k == 0 || r < best) { bi = k; best = r; }
+                taken += k;
+                i += k;
+                if (i >= cnt) { c++; i = 0; }
             }
-            // pose 0's distance stands unless another's is smaller (a NaN there stays)
-            if (__shfl_sync(kFull, best != best, 0)) {
-                bi = 0;
-                best = __shfl_sync(kFull, best, 0);
-            } else {
-                for (int o = 16; o > 0; o >>= 1) {
-                    const double ob = __shfl_xor_sync(kFull, best, o);
-                    const int oi = __shfl_xor_sync(kFull, bi, o);
-                    if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-                }
-            }
-            int at = -1;  // the place it takes
-            if (bi < n && best < min_rmsd) {
-                if (e < le[bi]) at = bi;
-            } else if (n < S) {
-                at = n++;
-            } else if (n > 0 && e < le[n - 1]) {
-                at = n - 1;
-            }
-            __syncwarp();
-            if (at >= 0 && lane == 0) {  // sorted in behind the energies not above its own
-                int k = at;
-                while (k > 0 && le[k - 1] > e) {
-                    le[k] = le[k - 1]; lc[k] = lc[k - 1]; ls[k] = ls[k - 1];
-                    k--;
-                }
-                le[k] = e; lc[k] = c; ls[k] = slot;
-            }
-            __syncwarp();
+            if (lane == 0) s_taken = taken;
         }
+        __syncthreads();
+        const int g = s_taken;
+        if (g == 0) break;
+        for (int t = tid; t < g * (n + g); t += kMergeThreads) {
+            const int p = t / (n + g), q = t - p * (n + g);
+            if (q >= n + p) continue;
+            const float *x = coords(at_group[p]), *y = coords(q < n ? at_list[q] : at_group[q - n]);
+            double acc = 0;
+#pragma unroll 6
+            for (int a = 0; a < H3; a++) {
+                const double d = (double)x[a] - (double)y[a];
+                acc += d * d;
+            }
+            D[p * (S + group) + q] = H3 ? sqrt(acc / (double)H) : 0.0;
+        }
+        for (int k = tid; k < n; k += kMergeThreads) col[k] = k;
+        __syncthreads();
+        if (tid < 32) {
+            const int n0 = n;
+            for (int p = 0; p < g; p++) {
+                const double* d = D + p * (S + group);
+                const double e = ge[p];
+                double best = kMaxFl;
+                int bi = n;
+                for (int k = lane; k < n; k += 32) {
+                    const double r = d[col[k]];
+                    if (k == 0 || r < best) { bi = k; best = r; }
+                }
+                // pose 0's distance stands unless another's is smaller (a NaN there stays)
+                if (__shfl_sync(kFull, best != best, 0)) {
+                    bi = 0;
+                    best = __shfl_sync(kFull, best, 0);
+                } else {
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const double ob = __shfl_xor_sync(kFull, best, o);
+                        const int oi = __shfl_xor_sync(kFull, bi, o);
+                        if (ob < best || (ob == best && oi < bi)) { best = ob; bi = oi; }
+                    }
+                }
+                int at = -1;  // the place it takes
+                if (bi < n && best < min_rmsd) {
+                    if (e < le[bi]) at = bi;
+                } else if (n < S) {
+                    at = n++;
+                } else if (n > 0 && e < le[n - 1]) {
+                    at = n - 1;
+                }
+                __syncwarp();
+                if (at < 0) continue;
+                // sorted in behind the last energy before `at` that is not above its own
+                int k = 0;
+                for (int b = at - 1; b >= 0; b -= 32) {
+                    const unsigned keep = __ballot_sync(kFull, b - lane >= 0 && !(le[b - lane] > e));
+                    if (keep) {
+                        k = b - __ffs(keep) + 2;
+                        break;
+                    }
+                }
+                for (int b = at - 1; b >= k; b -= 32) {  // those in between move up by one, the last ones first
+                    const int f = b - lane;
+                    double ef = 0;
+                    int2 af{};
+                    int cf = 0;
+                    if (f >= k) { ef = le[f]; af = at_list[f]; cf = col[f]; }
+                    __syncwarp();
+                    if (f >= k) { le[f + 1] = ef; at_list[f + 1] = af; col[f + 1] = cf; }
+                    __syncwarp();
+                }
+                if (lane == 0) {
+                    le[k] = e;
+                    at_list[k] = at_group[p];
+                    col[k] = n0 + p;
+                }
+                __syncwarp();
+            }
+            if (lane == 0) s_taken = n;
+        }
+        __syncthreads();
+        n = s_taken;
+        __syncthreads();
     }
-    if (lane == 0) out_count[j] = n;
-    for (int k = 0; k < S; k++) {
+    if (tid == 0) out_count[j] = n;
+    for (int k = tid >> 5; k < S; k += kMergeThreads / 32) {
         const size_t q = (size_t)j * S + k;
         if (lane == 0) pose_model[q] = k < n ? job.model : -1;
         if (k >= n) continue;
         if (lane == 0) out_e[q] = le[k];
-        const Chain32& ch = chains[lc[k]];
-        for (int i = lane; i < cs; i += 32) out_conf[q * conf_stride + i] = ch.out_conf[(size_t)ls[k] * cs + i];
-        for (int i = lane; i < H3; i += 32) out_xyz[q * xyz_stride + i] = ch.out_coords[(size_t)ls[k] * H3 + i];
+        const double* conf = chains[at_list[k].x].out_conf + (size_t)at_list[k].y * cs;
+        const float* x = coords(at_list[k]);
+        for (int a = lane; a < cs; a += 32) out_conf[q * conf_stride + a] = conf[a];
+        for (int a = lane; a < H3; a += 32) out_xyz[q * xyz_stride + a] = x[a];
     }
 }
 
@@ -444,8 +507,15 @@ cudaError_t launch_refine64(const DModel* dms, const Shape64& sh, const DTables&
 cudaError_t launch_merge32(const DModel* dms, const MergeJob32* jobs, int njobs, const Chain32* chains, int S,
                            double min_rmsd, int* count, int* pose_model, double* e, double* conf, int conf_stride,
                            double* xyz, int xyz_stride, cudaStream_t s) {
-    k_merge32<<<njobs, 32, (size_t)S * 16, s>>>(dms, jobs, chains, S, min_rmsd, count, pose_model, e, conf, conf_stride,
-                                                xyz, xyz_stride);
+    // groups as large as 48 KB allow (32 up to 120 places or so), else of 8 poses
+    const int group = merge32_bytes(S, 32) <= 48 * 1024 ? 32 : 8;
+    const size_t smem = merge32_bytes(S, group);
+    if (smem > 48 * 1024 - 64) {
+        const cudaError_t rc = raise_dynamic_smem((const void*)k_merge32, smem);
+        if (rc != cudaSuccess) return rc;
+    }
+    k_merge32<<<njobs, kMergeThreads, smem, s>>>(dms, jobs, chains, S, group, min_rmsd, count, pose_model, e, conf,
+                                                 conf_stride, xyz, xyz_stride);
     return cudaGetLastError();
 }
 
