@@ -66,27 +66,32 @@ __device__ V3<double> rand_in_sphere() {
 
 // ---- ordered scalar products ----------------------------------------------------------
 // sum over lanes 0 .. cnt - 1 of t, in lane order, onto s (same on every lane)
+template <bool ST>
 __device__ __forceinline__ double add_in_order64(double s, double t, int cnt) {
     int j = 0;
-    for (; j + 4 <= cnt; j += 4) {
+    for (; ST && j + 4 <= cnt; j += 4) {
         double x[4];
 #pragma unroll
         for (int u = 0; u < 4; u++) x[u] = __shfl_sync(kFull, t, j + u);
 #pragma unroll
         for (int u = 0; u < 4; u++) s += x[u];
     }
+#pragma unroll 1
     for (; j < cnt; j++) s += __shfl_sync(kFull, t, j);
     return s;
 }
+template <bool ST>
 __device__ __forceinline__ double sprod64(const double* a, const double* b, int n) {
     double s = 0;
+#pragma unroll 1
     for (int i0 = 0; i0 < n; i0 += 32) {
         const int i = i0 + lane64();
-        s = add_in_order64(s, i < n ? a[i] * b[i] : 0.0, min(32, n - i0));
+        s = add_in_order64<ST>(s, i < n ? a[i] * b[i] : 0.0, min(32, n - i0));
     }
     return s;
 }
 __device__ __forceinline__ void vcopy(double* d, const double* s, int n) {
+#pragma unroll 1
     for (int i = lane64(); i < n; i += 32) d[i] = s[i];
     __syncwarp();
 }
@@ -100,6 +105,7 @@ __device__ __noinline__ void conf_increment64(double* x, const double* p, double
               *tor_dof = M::tor_dof();
     const int nlig = H.m.nlig, ntors = H.m.ntors;
     // the last lanes take the ligands' rigid parts, so that a torsion lane never does both
+#pragma unroll 1
     for (int l = 31 - lane64(); l < nlig; l += 32) {
         const int f = lig_root[l];
         double* c = x + fconf[f];
@@ -110,6 +116,7 @@ __device__ __noinline__ void conf_increment64(double* x, const double* p, double
         q_increment(q, alpha * V3<double>{d[3], d[4], d[5]});
         c[3] = q.a; c[4] = q.b; c[5] = q.c; c[6] = q.d;
     }
+#pragma unroll 1
     for (int k = lane64(); k < ntors; k += 32) {
         double& t = x[tor_conf[k]];
         t += normalized_angle(alpha * p[tor_dof[k]]);
@@ -158,7 +165,7 @@ __device__ __forceinline__ double fast_line_search64(const double* x, const doub
                                                      double* x_new, double* g_new, double& f1, const EvalMode& em) {
     const int n = hd64().m.dof, cs = hd64().m.conf_size;
     double alpha = 1;
-    const double pg = sprod64(p, g, n);
+    const double pg = sprod64<ST>(p, g, n);
     for (unsigned trial = 0; trial < 10; trial++) {
         vcopy(x_new, x, cs);
         conf_increment64<ST>(x_new, p, alpha);
@@ -175,7 +182,7 @@ __device__ __noinline__ double accurate_line_search64(const double* x, const dou
     const int n = hd64().m.dof, cs = hd64().m.conf_size;
     double a, alpha, alpha2 = 0, alamin, b, disc, f2 = 0, rhs1, rhs2, tmplam = 0;
     const double ALF = 1.0e-4, FIRST = 1.0;
-    const double slope = sprod64(g, p, n);
+    const double slope = sprod64<ST>(g, p, n);
     if (slope >= 0) {
         vcopy(x_new, x, cs);
         for (int i = lane64(); i < n; i += 32) g_new[i] = 0;
@@ -228,11 +235,13 @@ __device__ __noinline__ double accurate_line_search64(const double* x, const dou
 // ---- BFGS on the triangular inverse Hessian -------------------------------------------
 // Lane i sums row i: entries (j, i) of column i up to the diagonal, then along
 // the row (one more than the column's length further each time).
+template <bool ST>
 __device__ __forceinline__ void minus_mat_vec64(const double* h, const double* in, double* out, int n) {
+#pragma unroll 1
     for (int i = lane64(); i < n; i += 32) {
         double sum = 0;
         int at = i * (i + 1) / 2;
-#pragma unroll 4
+#pragma unroll(ST ? 4 : 1)
         for (int j = 0; j < n; j++) {
             sum += h[at] * in[j];
             at += j < i ? 1 : j + 1;
@@ -242,22 +251,25 @@ __device__ __forceinline__ void minus_mat_vec64(const double* h, const double* i
     __syncwarp();
 }
 
+template <bool ST>
 __device__ __forceinline__ void bfgs_update64(double* h, const double* p, const double* y, double yp, double alpha,
                                               int n) {
     if (alpha * yp < kEps) return;
     double* mhy = smem64 + hd64().L.mhy;
-    minus_mat_vec64(h, y, mhy, n);
-    const double yhy = -sprod64(y, mhy, n);
+    minus_mat_vec64<ST>(h, y, mhy, n);
+    const double yhy = -sprod64<ST>(y, mhy, n);
     const double r = 1 / (alpha * yp);
     const double c1 = alpha * r, c2 = +alpha * alpha * (r * r * yhy + r);
     if (n <= 32) {  // lane i owns p[i] and mhy[i]
         const int i = lane64();
         const double pi = i < n ? p[i] : 0.0, mi = i < n ? mhy[i] : 0.0, c2p = c2 * pi;
-#pragma unroll 2
+#pragma unroll(ST ? 2 : 1)
         for (int j = 0; j < n; j++)
             if (i <= j) h[i + j * (j + 1) / 2] += c1 * (mi * p[j] + mhy[j] * pi) + c2p * p[j];
     } else {
+#pragma unroll 1
         for (int j = 0; j < n; j++)
+#pragma unroll 1
             for (int i = lane64(); i <= j; i += 32)
                 h[i + j * (j + 1) / 2] += c1 * (mhy[i] * p[j] + mhy[j] * p[i]) + c2 * p[i] * p[j];
     }
@@ -390,8 +402,10 @@ __device__ __noinline__ double bfgs64(double* x, int maxiters, int accurate, int
     double *g = S + L.g, *g_new = S + L.g_new, *g_orig = S + L.g_orig, *p = S + L.p, *y = S + L.y;
     double *x_new = S + L.x_new, *x_orig = S + L.x_orig;
     const int lane = lane64();
+#pragma unroll 1
     for (int t = lane; t < n * (n + 1) / 2; t += 32) h[t] = 0;
     __syncwarp();
+#pragma unroll 1
     for (int i = lane; i < n; i += 32) h[i + i * (i + 1) / 2] = 1;
     __syncwarp();
     double f0 = feval<G, ST>(x, g, em);
@@ -403,11 +417,12 @@ __device__ __noinline__ double bfgs64(double* x, int maxiters, int accurate, int
     vcopy(g_orig, g, n);
     vcopy(x_orig, x, cs);
     for (int step = 0; step < maxiters; step++) {
-        minus_mat_vec64(h, g, p, n);
+        minus_mat_vec64<ST>(h, g, p, n);
         double f1 = 0;
         const double alpha = accurate ? accurate_line_search64<G, ST>(x, g, f0, p, x_new, g_new, f1, em)
                                       : fast_line_search64<G, ST>(x, g, f0, p, x_new, g_new, f1, em);
         if (alpha == 0) break;
+#pragma unroll 1
         for (int i = lane; i < n; i += 32) { double t = g_new[i]; t -= g[i]; y[i] = t; }
         __syncwarp();
         const double prevf0 = f0;
@@ -415,18 +430,19 @@ __device__ __noinline__ double bfgs64(double* x, int maxiters, int accurate, int
         vcopy(x, x_new, cs);
         if (early && fabs(prevf0 - f0) < 1e-5) break;
         vcopy(g, g_new, n);
-        const double gn = sprod64(g, g, n);
+        const double gn = sprod64<ST>(g, g, n);
         if (!(gn >= 1e-4)) break;
-        const double yp = sprod64(y, p, n);
+        const double yp = sprod64<ST>(y, p, n);
         if (step == 0) {
-            const double yy = sprod64(y, y, n);
+            const double yy = sprod64<ST>(y, y, n);
             if (fabs(yy) > kEps) {
                 const double d = alpha * yp / yy;
+#pragma unroll 1
                 for (int i = lane; i < n; i += 32) h[i + i * (i + 1) / 2] = d;
                 __syncwarp();
             }
         }
-        bfgs_update64(h, p, y, yp, alpha, n);
+        bfgs_update64<ST>(h, p, y, yp, alpha, n);
         if (vis) hist64_add<ST>(*vis, x, f0, g);
     }
     if (!(f0 <= f_orig)) {
@@ -452,7 +468,7 @@ __device__ __forceinline__ double gyration64(int l) {
         const int i = i0 + lane64();
         const bool heavy = i < e && !is_h(type[i]);
         counter += __popc(__ballot_sync(kFull, heavy));
-        acc = add_in_order64(acc, heavy ? dist2(ld3(S + L.coords + 3 * i), o) : 0.0, min(32, e - i0));
+        acc = add_in_order64<ST>(acc, heavy ? dist2(ld3(S + L.coords + 3 * i), o) : 0.0, min(32, e - i0));
     }
     return counter > 0 ? sqrt(acc / counter) : 0;
 }

@@ -1176,8 +1176,8 @@ void ensure_model_maps(sg_engine* e, RecState& r, const sg_model_desc* models, i
 
 }  // namespace sg
 
-Shape64 sg::plain_shape(sg_engine* e, const PackedModels& pm, long long items, bool refine) {
-    const Shape64 sh = shape64(pm.smem64, items, refine, e->num_sms, (size_t)e->max_smem);
+Shape64 sg::plain_shape(sg_engine* e, const PackedModels& pm, long long items, Work64 work) {
+    const Shape64 sh = shape64(pm.smem64, items, work, e->num_sms, (size_t)e->max_smem);
     require(sh.smem <= (size_t)e->max_smem, "model too large for the plain path's shared memory");
     return sh;
 }
@@ -1215,7 +1215,7 @@ static int eval_common(sg_engine* e, int rid, const sg_model_desc* m, int nconfs
         PackedModels pm(e);
         pack_models(io, m, 1, !direct && e->precision != SG_PREC_FP64 ? kPackMixed : kPackPlain, pm);
         if (!direct) ensure_model_maps(e, r, m, 1);
-        const Shape64 sh = plain_shape(e, pm, nconfs);
+        const Shape64 sh = plain_shape(e, pm, nconfs, Work64::eval);
         const DModel& h = pm.host[0];
         Staged<double> dc(io, e), de(io, e), dg(io, e), dx(io, e);
         dc.make((size_t)nconfs * h.conf_size, confs);
@@ -1298,8 +1298,8 @@ int sg_bfgs(sg_engine* e, int rid, const sg_model_desc* m, int nconfs, double* c
             io.finish();
             return;
         }
-        const Shape64 sh = plain_shape(e, pm, nconfs);
-        cuda_check(launch_bfgs64(pm.dmodels, sh, e->num_sms, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
+        const Shape64 sh = plain_shape(e, pm, nconfs, Work64::bfgs);
+        cuda_check(launch_bfgs64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(), nconfs, dc.p(), v,
                                  slope, maxiters, accurate_line, early_term, de.p(), e->d_err.as<int>(), e->stream),
                    "bfgs launch");
         dc.fetch(confs);
@@ -1319,7 +1319,7 @@ int sg_dock(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, con
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
         ensure_model_maps(e, r, models, nmodels);
-        const Shape64 sh = plain_shape(e, pm, nchains);
+        const Shape64 sh = plain_shape(e, pm, nchains, Work64::chain);
         const int S = p->num_saved_mins;
         // per-chain inputs and result storage (one device allocation each)
         std::vector<double> conf0;
@@ -1439,7 +1439,7 @@ int sg_refine(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, c
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
-        const Shape64 sh = plain_shape(e, pm, nposes, true);
+        const Shape64 sh = plain_shape(e, pm, nposes, Work64::refine);
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "refine: bad pose model");
         const int cs = pm.max_conf, hs = pm.max_heavy;
         Staged<double> dc(io, e), de(io, e), dx(io, e);
@@ -1494,7 +1494,7 @@ int sg_score(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, co
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
-        const Shape64 sh = plain_shape(e, pm, nposes);
+        const Shape64 sh = plain_shape(e, pm, nposes, Work64::eval);
         require(conf_stride >= pm.max_conf && (!out_coords || coord_stride >= pm.max_heavy), "score: strides too small");
         for (int k = 0; k < nposes; k++) require(pose_model[k] >= 0 && pose_model[k] < nmodels, "score: bad pose model");
         Staged<double> dc(io, e), de(io, e), di(io, e), dx(io, e);
@@ -1527,7 +1527,7 @@ int sg_minimize(sg_engine* e, int rid, const sg_model_desc* models, int nmodels,
         CallIo io(e);
         PackedModels pm(e);
         pack_models(io, models, nmodels, kPackPlain, pm);
-        const Shape64 sh = plain_shape(e, pm, nposes, true);
+        const Shape64 sh = plain_shape(e, pm, nposes, Work64::refine);
         require(conf_stride >= pm.max_conf && coord_stride >= pm.max_heavy, "minimize: strides too small");
         for (int k = 0; k < nposes; k++) {
             require(pose_model[k] >= 0 && pose_model[k] < nmodels && maxiters[k] >= 0, "minimize: bad pose");

@@ -208,10 +208,10 @@ cudaError_t launch_grid_map64(const DGeom&, const CellAtom* list, const double* 
 cudaError_t launch_grid_pack(const DGeom&, const GridPack* maps, int nmaps, cudaStream_t);
 // warps per item and shared memory of a plain-path launch over `items` items
 // within max_smem bytes per block
-Shape64 shape64(const Smem64& s, long long items, bool refine, int num_sms, size_t max_smem);
+Shape64 shape64(const Smem64& s, long long items, Work64 work, int num_sms, size_t max_smem);
 cudaError_t launch_eval64(const DModel*, const Shape64&, int num_sms, const DTables&, const DReceptor*, int,
                           const double*, const double[3], double, int, double*, double*, double*, int*, cudaStream_t);
-cudaError_t launch_bfgs64(const DModel*, const Shape64&, int num_sms, const DTables&, const DReceptor*, int, double*,
+cudaError_t launch_bfgs64(const DModel*, const Shape64&, const DTables&, const DReceptor*, int, double*,
                           const double[3], double, int, int, int, double*, int*, cudaStream_t);
 cudaError_t launch_mc64(const DModel*, const Shape64&, const DTables&, const DReceptor*, const Chain64*, int,
                         const MCParams64&, bool visited, int*, cudaStream_t);
@@ -259,7 +259,7 @@ DMaps32 maps32(const sg_engine* e, const RecState& r);
 enum PackFor { kPackPlain, kPackMixed, kPackWide };
 void pack_models(CallIo& io, const sg_model_desc* models, int nmodels, PackFor what, PackedModels& out);
 // the plain-path launch of a batch of models; refuses a model that does not fit
-Shape64 plain_shape(sg_engine* e, const PackedModels& pm, long long items, bool refine = false);
+Shape64 plain_shape(sg_engine* e, const PackedModels& pm, long long items, Work64 work);
 struct ModelImage {
     std::vector<char> bytes;   // pools then descriptors, ready to copy to the device
     size_t dmodel_off = 0;     // byte offset of the descriptor array

@@ -481,7 +481,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
                 std::fill_n(pmaxit.begin() + (size_t)j * S, S, jobs[j].maxiters > 0 ? jobs[j].maxiters : p->maxiters);
             io.in(dmi, pmaxit.data(), pmaxit.size() * sizeof(int));
             h2d += dmi.bytes;
-            const Shape64 sh = plain_shape(e, pm, nplaces, true);
+            const Shape64 sh = plain_shape(e, pm, nplaces, Work64::refine);
             cuda_check(cudaEventRecord(ev[2], e->stream), "event");
             cuda_check(launch_refine64(pm.dmodels, sh, e->tables, r.dhdr.as<DReceptor>(), dpm.as<int>(), (int)nplaces,
                                        dc.as<double>(), cs, p->authentic_v, p->maxiters, dmi.as<int>(), nullptr,

@@ -113,23 +113,24 @@ __global__ void SG_BOUNDS64 k_eval64(const DModel* model, const __grid_constant_
     release64<G>();
 }
 
-// quasi_newton on the grid maps for a batch of confs (confs updated in place)
+// quasi_newton on the grid maps, a conf per block (confs updated in place).  Confs
+// take very different numbers of evaluations: blocks that each looped over a fixed
+// share of them took 20 to 50 % longer past one resident batch.
 template <int G, bool ST>
 __global__ void SG_BOUNDS64 k_bfgs64(const DModel* model, const __grid_constant__ DTables T, const DReceptor* R,
                                      int nconfs, double* confs, double v0, double v1, double v2, double slope,
                                      int maxiters, int accurate, int early, double* out_e, int* err) {
+    const int k = blockIdx.x;
+    if (k >= nconfs) return;
     init64<G, ST>(model, T, R, nullptr, err);
     if (threadIdx.x >= 32) return help64<G, ST>(threadIdx.x >> 5);
     const int cs = hd64().m.conf_size, lane = lane64();
     double* x = smem64 + hd64().L.x_tmp;
     const EvalMode em{{v0, v1, v2}, slope, false};
-    for (int k = blockIdx.x; k < nconfs; k += gridDim.x) {
-        vcopy(x, confs + (size_t)k * cs, cs);
-        const double e = bfgs64<G, ST>(x, maxiters, accurate, early, em);
-        if (lane == 0) out_e[k] = e;
-        for (int i = lane; i < cs; i += 32) confs[(size_t)k * cs + i] = x[i];
-        __syncwarp();
-    }
+    vcopy(x, confs + (size_t)k * cs, cs);
+    const double e = bfgs64<G, ST>(x, maxiters, accurate, early, em);
+    if (lane == 0) out_e[k] = e;
+    for (int i = lane; i < cs; i += 32) confs[(size_t)k * cs + i] = x[i];
     release64<G>();
 }
 
@@ -427,6 +428,7 @@ void Smem64::add(const DModel& h) {
         return (size_t)ws64_layout(h.natoms, h.nframes, h.npairs, h.conf_size, h.dof, st, h.nheavy, h.nlevels, h.nlig,
                                    h.nblocks, h.ntors).total * sizeof(double);
     };
+    pairs = std::max(pairs, h.npairs);
     plain = std::max(plain, bytes(false));
     staged = std::max(staged, bytes(true));
 }
@@ -435,11 +437,17 @@ void Smem64::add(const DModel& h) {
 // warps against 4: 9 poses 1.19 / 1.59 ms, 297 7.1 / 9.6, 1,890 30.8 / 38.4), and for few
 // items; 4 for more chains or evaluations on the maps than two per SM (10 steps of
 // 700 chains 60.5 / 53.6 ms, of 296 31.2 / 31.8); 1 with nothing staged for models that
-// only fit so.
-Shape64 shape64(const Smem64& s, long long items, bool refine, int num_sms, size_t max_smem) {
+// only fit so, and for many local optimisations of models with few pairs, where
+// the leaders' serial work fills the device: milliseconds of 4 warps against 1
+// without pairs 0.66 / 0.66 at 592 confs, 1.03 / 0.73 at 1,184, 11.7 / 4.4 at 20,000; 174
+// pairs 3.1 / 3.7 at 1,184, 5.2 / 4.1 at 2,400, 9.5 / 7.2 at 5,000; 316 pairs 8.1 / 8.5 at
+// 2,400, 15.1 / 14.0 at 5,000; 482 pairs 17.6 / 19.5 at 5,000.
+Shape64 shape64(const Smem64& s, long long items, Work64 work, int num_sms, size_t max_smem) {
     const size_t xb = kXbuf64 * sizeof(double);
-    if ((refine || items <= 2LL * num_sms) && s.staged + 8 * xb <= max_smem) return {8, s.staged + 8 * xb};
-    if (s.staged + 4 * xb <= max_smem) return {4, s.staged + 4 * xb};
+    const bool one = work == Work64::bfgs && s.pairs <= 350 && items > (long long)num_sms * (4 + s.pairs / 30);
+    if (!one && (work == Work64::refine || items <= 2LL * num_sms) && s.staged + 8 * xb <= max_smem)
+        return {8, s.staged + 8 * xb};
+    if (!one && s.staged + 4 * xb <= max_smem) return {4, s.staged + 4 * xb};
     return {1, s.plain};
 }
 
@@ -481,10 +489,10 @@ cudaError_t launch_eval64(const DModel* dm, const Shape64& sh, int num_sms, cons
                 err);
 }
 
-cudaError_t launch_bfgs64(const DModel* dm, const Shape64& sh, int num_sms, const DTables& T, const DReceptor* R, int n,
+cudaError_t launch_bfgs64(const DModel* dm, const Shape64& sh, const DTables& T, const DReceptor* R, int n,
                           double* confs, const double v[3], double slope, int maxiters, int accurate, int early,
                           double* e, int* err, cudaStream_t s) {
-    SG_LAUNCH64(SG_K_BFGS, loop_blocks(sh, n, num_sms), dm, T, R, n, confs, v[0], v[1], v[2], slope, maxiters, accurate,
+    SG_LAUNCH64(SG_K_BFGS, n, dm, T, R, n, confs, v[0], v[1], v[2], slope, maxiters, accurate,
                 early, e, err);
 }
 

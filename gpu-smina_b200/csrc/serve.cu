@@ -542,7 +542,7 @@ static void launch_refines(Server& s, std::vector<std::pair<SvBatch*, SvLig*>>& 
     }
     // 4 warps per pose where they find room beside the search: no more shared
     // memory than a serving block's place (else one warp, nothing staged)
-    const Shape64 sh = shape64(ws, 1ll << 40, false, e->num_sms, std::min((size_t)e->max_smem, s.smem_block));
+    const Shape64 sh = shape64(ws, 1ll << 40, Work64::eval, e->num_sms, std::min((size_t)e->max_smem, s.smem_block));
     require(sh.smem <= (size_t)e->max_smem, "serve: model too large for the plain path's shared memory");
     // refine_structure needs the pose's receptor: one launch per receptor in the group
     std::map<int, std::vector<std::pair<SvBatch*, SvLig*>>> by_rec;

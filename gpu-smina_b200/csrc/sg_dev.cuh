@@ -423,14 +423,18 @@ SG_HD Ws64 ws64_layout(int natoms, int nframes, int npairs, int conf, int dof, b
 }
 
 // the most shared memory any model of a batch takes, in bytes, with nothing
-// staged and staged (without the exchange buffers)
+// staged and staged (without the exchange buffers), and the most pairs
 struct Smem64 {
     size_t plain = 0, staged = 0;
+    int pairs = 0;
     void add(const DModel& h);
 };
 // Raises a kernel's limit of dynamic shared memory to `smem` and never lowers it,
 // whatever other threads do: their launches may be sized against a higher one.
 cudaError_t raise_dynamic_smem(const void* kernel, size_t smem);
+// what the items of a plain-path launch do: evaluations (or rescoring), local
+// optimisations on the maps, search chains, refinements on the direct sum
+enum class Work64 { eval, bfgs, chain, refine };
 // a plain-path launch: warps per item and its shared memory
 struct Shape64 {
     int warps;

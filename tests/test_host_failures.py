@@ -239,3 +239,22 @@ for kernel, f in ((b"k_score64", lambda e, q: e.score(0, [q], [0], W.random_conf
     f(es[0], ms[0])  # raises it again, had it been lowered
     assert both == fake.fake_max_dynamic(kernel) > 49152
 """)
+
+
+def test_launch_shapes_of_local_optimisations(run):
+    """Warps per conf of the plain path's local optimisation, by the number of
+    confs and of the model's pairs: one warp for many confs of small models."""
+    run("""
+e = engine(sb.PREC_FP64)
+def warps(lig, n):
+    q = W.ligand(*lig)
+    x = np.repeat(W.random_confs(q, gd, 1, 1), n, 0)
+    before = [fake.fake_launches(b"k_bfgs64ILi%dE" % w) for w in (1, 4, 8)]
+    e.bfgs(0, q, x)
+    return [w for w, k in zip((1, 4, 8), before) if fake.fake_launches(b"k_bfgs64ILi%dE" % w) != k]
+SMALL, MIDDLE, LARGE = (10, 0, 4), (24, 5, 11), (36, 8, 5)
+for lig, n, w in ((SMALL, 1, 8), (SMALL, 296, 8), (SMALL, 297, 4), (SMALL, 592, 4), (SMALL, 593, 1), (SMALL, 20000, 1),
+                  (MIDDLE, 296, 8), (MIDDLE, 1184, 4), (MIDDLE, 2400, 1), (MIDDLE, 20000, 1), (LARGE, 296, 8),
+                  (LARGE, 297, 4), (LARGE, 20000, 4), ((116, 30, 5), 2, 1)):
+    assert warps(lig, n) == [w], (lig, n, w, warps(lig, n))
+""")

@@ -54,3 +54,20 @@ def test_every_kernel_at_every_shape(lig, n):
     same(b1.e, b0.e, "chain energies")
     same(b1.coords, b0.coords, "chain poses")
     eng.close()
+
+
+@pytest.mark.parametrize("lig,n", [((10, 0, 4), 593), ((24, 5, 11), 2000)])
+def test_many_small_optimisations_equal_few(lig, n):
+    """Past a few confs per SM small models get one warp per conf: the same bits
+    as in calls of 4 and 8 warps per conf."""
+    eng = sb.Engine(0, sb.PREC_FP64)
+    eng.set_tables(W.tables())
+    eng.set_receptor(0, W.receptor(1500, 3), W.box(26.0))
+    m = W.ligand(*lig)
+    confs = W.random_confs(m, W.box(26.0), n, 5)
+    c1, e1 = eng.bfgs(0, m, confs)
+    for size in (500, 250):  # 4 warps, 8 warps
+        parts = [eng.bfgs(0, m, confs[k:k + size]) for k in range(0, n, size)]
+        same(c1, np.concatenate([c for c, _ in parts]), "confs")
+        same(e1, np.concatenate([e for _, e in parts]), "energies")
+    eng.close()
