@@ -434,8 +434,10 @@ void Smem64::add(const DModel& h) {
 }
 
 // Warps per item: 8 for refinements, whose direct sums keep them busy (one B200, 8
-// warps against 4: 9 poses 1.19 / 1.59 ms, 297 7.1 / 9.6, 1,890 30.8 / 38.4), and for few
-// items; 4 for more chains or evaluations on the maps than two per SM (10 steps of
+// warps against 4: 9 poses of a 24-atom ligand 1.04 / 1.39 ms, 296 2.2 / 3.0; 1,890 of a
+// 50-atom one 52 / 67), but for many of models with hardly any pairs (without pairs
+// 1.97 / 1.50 at 592 poses, 20.3 / 13.9 at 10,000; 61 pairs 3.3 / 2.7 at 1,200; 105 pairs 5.7 / 7.0),
+// and for few items; 4 for more chains or evaluations on the maps than two per SM (10 steps of
 // 700 chains 60.5 / 53.6 ms, of 296 31.2 / 31.8); 1 with nothing staged for models that
 // only fit so, and for many local optimisations of models with few pairs, where
 // the leaders' serial work fills the device: milliseconds of 4 warps against 1
@@ -445,7 +447,8 @@ void Smem64::add(const DModel& h) {
 Shape64 shape64(const Smem64& s, long long items, Work64 work, int num_sms, size_t max_smem) {
     const size_t xb = kXbuf64 * sizeof(double);
     const bool one = work == Work64::bfgs && s.pairs <= 350 && items > (long long)num_sms * (4 + s.pairs / 30);
-    if (!one && (work == Work64::refine || items <= 2LL * num_sms) && s.staged + 8 * xb <= max_smem)
+    const bool eight = items <= 2LL * num_sms || (work == Work64::refine && s.pairs > 80);
+    if (!one && eight && s.staged + 8 * xb <= max_smem)
         return {8, s.staged + 8 * xb};
     if (!one && s.staged + 4 * xb <= max_smem) return {4, s.staged + 4 * xb};
     return {1, s.plain};

@@ -258,3 +258,21 @@ for lig, n, w in ((SMALL, 1, 8), (SMALL, 296, 8), (SMALL, 297, 4), (SMALL, 592, 
                   (LARGE, 297, 4), (LARGE, 20000, 4), ((116, 30, 5), 2, 1)):
     assert warps(lig, n) == [w], (lig, n, w, warps(lig, n))
 """)
+
+
+def test_launch_shapes_of_refinements(run):
+    """Warps per pose of the refinements: 8, but 4 for many poses of models with
+    hardly any pairs."""
+    run("""
+e = engine(sb.PREC_FP64)
+def warps(lig, n, call):
+    q = W.ligand(*lig)
+    x = np.repeat(W.random_confs(q, gd, 1, 1), n, 0)
+    before = [fake.fake_launches(b"k_refine64ILi%dE" % w) for w in (1, 4, 8)]
+    getattr(e, call)(0, [q], [0] * n, x)
+    return [w for w, k in zip((1, 4, 8), before) if fake.fake_launches(b"k_refine64ILi%dE" % w) != k]
+for call in ("refine", "minimize"):
+    for lig, n, w in (((10, 0, 4), 296, 8), ((10, 0, 4), 297, 4), ((16, 2, 6), 5000, 4), ((24, 5, 11), 5000, 8),
+                      ((50, 12, 3), 5000, 8), ((116, 30, 5), 2, 1)):
+        assert warps(lig, n, call) == [w], (lig, n, w, warps(lig, n, call))
+""")
