@@ -1133,34 +1133,44 @@ cudaError_t launch_eval32(const DModel* dm, size_t stage, size_t ws, const DTabl
     return cudaGetLastError();
 }
 
-// wide: the buffers' bytes of a conf on a whole block, or 0: not packed for it.
-// With 8 warps per block while all confs are resident so.  With 4 beyond that,
-// up to 1 + pairs / 200 resident batches: the more of an evaluation its pairs
-// are, the longer blocks that take confs one after the other win against one
-// warp per conf, whose slowest conf decides.  One B200, milliseconds of 4 warps
-// against one: 50 heavy atoms and 12 rotors (1,000 pairs; 592 resident) 2.2 / 3.9 at
-// 592 confs, 3.3 / 4.4 at 1,536, 5.4 / 5.5 at 3,500, 7.9 / 7.5 at 6,000; 24 and 5 (150)
-// 0.85 / 1.15 at 592, 1.15 / 1.19 at 1,200, 1.55 / 1.44 at 2,000; 12 and 2 (25) 0.55 / 0.58
-// at 592, 0.71 / 0.62 at 800.
+// Warps per block of k_bfgs32_wide for n confs, or 0: one warp per conf.  8 while
+// all confs are resident so.  Beyond that 4, up to 1 + pairs / 200 resident batches:
+// the more of an evaluation its pairs are, the longer blocks that take confs one
+// after the other win against one warp per conf, whose slowest conf decides; but 2.2
+// at most, as past that it depends on the confs which one wins.  One B200, 4 warps
+// against one, milliseconds: 985 pairs (592 resident) 2.6 / 4.2 at 592 confs, 4.2 / 4.5 at
+// 1,000, 4.8 / 4.7 at 1,250, 5.7 / 4.8 at 1,536 in a box that the ligand fills (and 3.1 / 4.1 in
+// a larger one, where most confs are done early); 482 pairs 1.4 / 2.3, 2.2 / 2.4, 2.5 / 2.5 and
+// 2.8 / 2.6; 174 pairs 0.9 / 1.3, 1.2 / 1.3, 1.4 / 1.3; 61 pairs 0.63 / 0.77, 0.83 / 0.79.
+// Where shared memory keeps 4-warp blocks to the same number, 8 warps win further
+// (2,705 pairs, 296 resident: 8 warps against one 7.9 / 11.8 at 592, 15.5 / 19.3 at 1,536, 36.9 /
+// 40.4 at 4,000, 54.2 / 57.2 at 6,000).
+static int wide_warps32(size_t smem, int n, int npairs, int num_sms, size_t max_smem) {
+    const void* fn = (const void*)k_bfgs32_wide;
+    int occ8 = 0, occ4 = 0;
+    if (smem > max_smem || raise_dynamic_smem(fn, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ8, fn, 256, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ4, fn, 128, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    if ((double)n <= (double)num_sms * occ8 * (occ4 == occ8 ? 20 : 1)) return 8;
+    return (double)n <= (double)num_sms * occ4 * std::min(2.2, 1.0 + npairs / 200.0) ? 4 : 0;
+}
+
+// wide: the buffers' bytes of a conf on a whole block, or 0: not packed for it
 cudaError_t launch_bfgs32(const DModel* dm, size_t stage, size_t ws, size_t wide, int npairs, const DTables32& T,
                           const DMaps32& G, int n, double* confs, const double v[3], double slope, int maxiters,
                           int accurate, int early, double* e, int team, int num_sms, size_t max_smem,
                           cudaStream_t s) {
-    if (team == 1 && wide)
-        for (int warps : {8, 4}) {
-            const size_t smem = stage + ws + wide;
-            int occ = 0;
-            if (smem > max_smem || raise_dynamic_smem((const void*)k_bfgs32_wide, smem) != cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bfgs32_wide, 32 * warps, smem) != cudaSuccess) {
-                cudaGetLastError();
-                break;
-            }
-            const double most = (double)occ * num_sms * (warps == 8 ? 1.0 : 1.0 + npairs / 200.0);
-            if (n > most) continue;
+    if (team == 1 && wide) {
+        const size_t smem = stage + ws + wide;
+        if (const int warps = wide_warps32(smem, n, npairs, num_sms, max_smem)) {
             k_bfgs32_wide<<<n, 32 * warps, smem, s>>>(dm, T, G, n, confs, (float)v[0], (float)v[1], (float)v[2],
                                                       (float)slope, maxiters, accurate, early, e, (int)stage, (int)ws);
             return cudaGetLastError();
         }
+    }
     if (!(team == 1 || team == 2 || team == 4)) return cudaErrorInvalidValue;
     const size_t smem = stage + (size_t)team * ws;
     const void* fn = team == 4 ? (const void*)k_bfgs32<4> : team == 2 ? (const void*)k_bfgs32<2> : (const void*)k_bfgs32<1>;

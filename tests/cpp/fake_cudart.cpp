@@ -22,7 +22,7 @@ std::mutex mu;
 struct State {
     std::map<const void*, std::string> kernels;
     std::map<const void*, int> max_dynamic;  // per kernel
-    std::map<std::string, int> launches;
+    std::map<std::string, int> launches, threads;  // threads: of the last launch's blocks
     std::map<void*, std::pair<size_t, bool>> blocks;  // device memory: bytes, of a pool
     std::set<void*> freed;  // blocks of at most 1 MB given back (their addresses are not used again)
 };
@@ -104,6 +104,12 @@ int fake_launches(const char* part) {  // launches of kernels whose (mangled) na
         if (k.first.find(part) != std::string::npos) n += k.second;
     return n;
 }
+int fake_threads(const char* part) {  // threads per block of such a kernel's last launch
+    Held held;
+    for (auto& k : st().threads)
+        if (k.first.find(part) != std::string::npos) return k.second;
+    return 0;
+}
 int fake_max_dynamic(const char* part) {  // the largest dynamic shared memory such a kernel is set to
     Held held;
     int n = 0;
@@ -121,16 +127,23 @@ void __cudaRegisterFunction(void**, const char* host, char*, const char* name, i
     st().kernels[host] = name;
 }
 void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
-unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, cudaStream_t) { return 0; }
-cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void*) {
-    *g = dim3(1);
-    *b = dim3(1);
+static thread_local dim3 call_grid, call_block;
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t, cudaStream_t) {
+    call_grid = g;
+    call_block = b;
+    return 0;
+}
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* s, void* stream) {
+    *g = call_grid;
+    *b = call_block;
     *s = 0;
+    *static_cast<cudaStream_t*>(stream) = nullptr;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t, cudaStream_t) {
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3 block, void**, size_t, cudaStream_t) {
     Held held;
     st().launches[st().kernels[f]]++;
+    st().threads[st().kernels[f]] = (int)(block.x * block.y * block.z);
     return cudaSuccess;
 }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* f) {

@@ -276,3 +276,24 @@ for call in ("refine", "minimize"):
                       ((50, 12, 3), 5000, 8), ((116, 30, 5), 2, 1)):
         assert warps(lig, n, call) == [w], (lig, n, w, warps(lig, n, call))
 """)
+
+
+def test_launch_shapes_of_mixed_precision_optimisations(run):
+    """Warps per conf of the FP32 local optimisation (with the occupancies of
+    128 registers a thread): 8 while all confs are resident, 4 up to 2.2 resident
+    batches and fewer the fewer pairs there are, then one; 8 further where shared
+    memory leaves no more room for 4."""
+    run("""
+e = engine()
+def warps(lig, n):
+    q = W.ligand(*lig)
+    x = np.repeat(W.random_confs(q, gd, 1, 1), n, 0)
+    before = fake.fake_launches(b"k_bfgs32_wide")
+    e.bfgs(0, q, x)
+    return fake.fake_threads(b"k_bfgs32_wide") // 32 if fake.fake_launches(b"k_bfgs32_wide") != before else 1
+NONE, FEW, MANY, LARGE = (10, 0, 4), (16, 2, 6), (50, 12, 3), (80, 20, 7)  # 0, 61, 985 and 2,705 pairs
+for lig, n, w in ((NONE, 1, 8), (NONE, 296, 8), (NONE, 592, 4), (NONE, 593, 1), (FEW, 297, 4), (FEW, 772, 4),
+                  (FEW, 773, 1), (MANY, 296, 8), (MANY, 297, 4), (MANY, 1302, 4), (MANY, 1303, 1), (LARGE, 297, 8),
+                  (LARGE, 5920, 8), (LARGE, 5921, 1)):
+    assert warps(lig, n) == w, (lig, n, w, warps(lig, n))
+""")

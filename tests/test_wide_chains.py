@@ -43,3 +43,27 @@ def test_wide_chains_equal_one_warp(scoring, ligs, chains, flex):
         for k in ("e", "conf", "coords"):
             assert np.array_equal(a[k], b[k]), k
     eng.close()
+
+
+@pytest.mark.parametrize("scoring,lig,flex,prec", [
+    (VINA, (10, 0, 4), False, sb.PREC_FP32), (VINA, (24, 5, 11), False, sb.PREC_FP32),
+    (VINA, (50, 12, 3), False, sb.PREC_FP32_H16), (VINA, (20, 4, 5), True, sb.PREC_FP32),
+    (AD4, (24, 5, 11), False, sb.PREC_FP32)])
+def test_wide_optimisations_equal_one_warp(scoring, lig, flex, prec):
+    """sg_bfgs: a conf's bits do not depend on the number of confs of the call,
+    which decides between 8 warps, 4 and one per conf (test_host_failures.py)."""
+    gd = W.box(26.0)
+    eng = sb.Engine(0, prec)
+    eng.set_tables(W.tables(scoring))
+    eng.set_receptor(0, W.charged_receptor(1500, 3, 2) if scoring == AD4 else W.receptor(1500, 3), gd)
+    fx = sb.make_flex_pdbqt(3, 42, W.CENTER) if flex else None
+    m = W.charged_ligand(*lig, 1) if scoring == AD4 else sb.Model(sb.make_ligand_pdbqt(*lig, W.CENTER), fx)
+    confs = W.random_confs(m, gd, 1400, 5)
+    one = eng.bfgs(0, m, confs)
+    assert np.isfinite(one[1]).all() and (one[0] != confs).any()
+    for size in (592, 250, 1):
+        last = 8 if size == 1 else len(confs)
+        parts = [eng.bfgs(0, m, confs[k:min(k + size, last)]) for k in range(0, last, size)]
+        assert np.array_equal(np.concatenate([c for c, _ in parts]), one[0][:last]), size
+        assert np.array_equal(np.concatenate([e for _, e in parts]), one[1][:last]), size
+    eng.close()
