@@ -162,6 +162,7 @@ struct sg_engine {
     int force_wpb = 0, last_wpb = 0, last_blocks = 0;
     int tpc = 32;        // threads per chain of the batched search: 32, 64, 128, or 0 (by the batch's size)
     int last_team = 1;   // warps per chain of the last batched search
+    int last_block_warps = 0, last_block_ligands = 0;  // ... and its chains with a block each
     bool es_on = false;   // early stop of the batched search (--fast; sg_set_early_stop)
     sg_early_stop es{};
     double last_mc_ms = 0, last_refine_ms = 0;

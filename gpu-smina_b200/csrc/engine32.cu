@@ -333,7 +333,7 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         std::vector<double> hres;
         DevBuf d_chains(e), d_items(e);
         float mc_ms = 0;
-        int first_blocks = 0, first_wpb = wpb;
+        int first_blocks = 0, first_wpb = wpb, first_warps = 0, first_wide = 0;
         cudaEvent_t ev[4];
         for (auto& x : ev) cuda_check(cudaEventCreate(&x), "event");
         struct EvGuard {
@@ -395,8 +395,10 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
             for (size_t k = 0; k < items.size(); k++) queue[k] = items[order[k]];
             const int nitems = (int)queue.size();
             const int blocks = (int)std::min<long long>((long long)(mix.warps ? mix.occ : occ) * e->num_sms, nitems);
-            if (ph == 0) {
+            if (first_blocks == 0) {
                 first_blocks = blocks;
+                first_warps = mix.warps;
+                first_wide = mix.wide_jobs;
                 first_wpb = !mix.warps ? wpb : mix.wide_jobs == (int)jobs_by_cost.size() ? 1 : mix.warps;
             }
             io.in(d_chains, hc.data(), hc.size() * sizeof(Chain32));
@@ -532,6 +534,8 @@ int sg_dock_batch32(sg_engine* e, int rid, const sg_model_desc* models, int nmod
         e->last_wpb = first_wpb;
         e->last_team = team;
         e->last_blocks = blocks;
+        e->last_block_warps = first_warps;
+        e->last_block_ligands = first_wide;
         e->last_mc_ms = mc_ms;
         e->last_refine_ms = ref_ms;
         e->last_evals = tot_evals;
@@ -548,6 +552,13 @@ int sg_batch_stats(const sg_engine* e, double* mc_ms, double* refine_ms, int* ch
     if (refine_ms) *refine_ms = e->last_refine_ms;
     if (chains_per_block) *chains_per_block = e->last_wpb;
     if (blocks) *blocks = e->last_blocks;
+    return SG_OK;
+}
+
+int sg_batch_blocks(const sg_engine* e, int* warps, int* ligands) {
+    if (!e) return SG_ERR_ARG;
+    if (warps) *warps = e->last_block_warps;
+    if (ligands) *ligands = e->last_block_ligands;
     return SG_OK;
 }
 

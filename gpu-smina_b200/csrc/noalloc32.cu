@@ -161,8 +161,8 @@ int sg_dock_batch32_noalloc(sg_engine* e, int rid, const sg_model_desc* models, 
             nxyz_res += (size_t)J.num_chains * S * h.nheavy * 3;
         }
         require(nchains <= (size_t(1) << 24), "dock_batch32_noalloc: at most 2^24 chains per call");
-        // launch shape as sg_dock_batch32 picks it (a shape set by
-        // sg_set_chains_per_block or sg_autotune32 included)
+        // the launch shape set by sg_set_chains_per_block or sg_autotune32, or the
+        // one with the most resident chains per SM
         int wpb = 1, occ = 1;
         choose_launch(e, stage_stride, ws_stride, max_chains, wpb, occ);
         size_t nitems_sz = 0;

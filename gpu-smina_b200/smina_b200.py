@@ -170,6 +170,7 @@ def _declare(L):
         "sg_dock_batch32_noalloc": [vp, C.c_int, C.POINTER(ModelDesc), C.c_int, C.POINTER(LigandJob), C.c_int,
                                     C.POINTER(MCParams), C.POINTER(LigandResult)],
         "sg_batch_stats": [vp, _dp, _dp, _ip, _ip],
+        "sg_batch_blocks": [vp, _ip, _ip],
         "sg_batch_counters": [vp] + [C.POINTER(C.c_uint64)] * 5,
         "sg_set_chains_per_block": [vp, C.c_int],
         "sg_set_threads_per_chain": [vp, C.c_int],
@@ -647,13 +648,14 @@ class Engine:
     def batch_stats(self):
         """Timing and counters of the last dock_batch call."""
         mc, rf = C.c_double(), C.c_double()
-        wpb, blocks = C.c_int(), C.c_int()
+        wpb, blocks, warps, ligands = C.c_int(), C.c_int(), C.c_int(), C.c_int()
         self._check(load().sg_batch_stats(self._h, C.byref(mc), C.byref(rf), C.byref(wpb), C.byref(blocks)))
+        self._check(load().sg_batch_blocks(self._h, C.byref(warps), C.byref(ligands)))
         ctr = [C.c_uint64() for _ in range(5)]
         self._check(load().sg_batch_counters(self._h, *[C.byref(c) for c in ctr]))
         return {"mc_ms": mc.value, "refine_ms": rf.value, "chains_per_block": wpb.value, "blocks": blocks.value,
-                "evals": ctr[0].value, "grid_lookups": ctr[1].value, "pair_lookups": ctr[2].value,
-                "h2d_bytes": ctr[3].value, "d2h_bytes": ctr[4].value}
+                "block_warps": warps.value, "block_ligands": ligands.value,
+                "evals": ctr[0].value, "grid_lookups": ctr[1].value, "pair_lookups": ctr[2].value, "h2d_bytes": ctr[3].value, "d2h_bytes": ctr[4].value}
 
     # ---- serving (continuous batching) ----------------------------------------
     def probe_gather(self, working_set_bytes, bytes_per_lookup):

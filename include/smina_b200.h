@@ -349,8 +349,9 @@ int sg_dock_batch32(sg_engine* e, int receptor_id, const sg_model_desc* models, 
  *     memory per device, held until the process exits.  Engine creation
  *     also loads the search kernel and raises its shared-memory limit, so a
  *     call loads no module and sets no kernel attribute;
- *   - the launch shape is the one sg_dock_batch32 would pick, including a
- *     shape set by sg_set_chains_per_block or sg_autotune32;
+ *   - the launch shape is the one set by sg_set_chains_per_block or
+ *     sg_autotune32, or else the one with the most resident chains per SM;
+ *     no chain gets a block to itself as in sg_dock_batch32;
  *   - every call reuses the same array, so calls that overlap on one GPU
  *     (two engines, or two host threads) corrupt each other: keep them
  *     apart.
@@ -392,6 +393,12 @@ int sg_set_early_stop(sg_engine* e, const sg_early_stop* es);
 /* Timing and launch shape of the last sg_dock_batch32 call. */
 int sg_batch_stats(const sg_engine* e, double* mc_ms, double* refine_ms,
                    int* chains_per_block, int* blocks);
+/* Ligands of the last sg_dock_batch32 call whose chains had a thread block
+ * each in its (first) search launch, and the warps of such a block: 8 or 4, 0
+ * when there were none.  sg_batch_stats' chains_per_block is 1 when all had
+ * one; beside others it is the most chains that a block of one-warp chains
+ * then holds. */
+int sg_batch_blocks(const sg_engine* e, int* warps, int* ligands);
 
 /* Work counters of the last sg_dock_batch32 call: eval_deriv calls, grid
  * map lookups (one packed cell each), in-cutoff pair table lookups, and
@@ -400,9 +407,13 @@ int sg_batch_counters(const sg_engine* e, uint64_t* evals, uint64_t* grid_lookup
                       uint64_t* pair_lookups, uint64_t* h2d_bytes, uint64_t* d2h_bytes);
 
 /* Chains per block of the search kernel: 1, 2, 4 or 8 (at most 8 warps
- * per block, so 2 with 128 threads per chain), or 0 to pick the shape with
- * the most resident chains per SM (the default; a batch of at most one
- * chain per SM then runs one chain per block).  The chains of one block
+ * per block, so 2 with 128 threads per chain), or 0 (the default) to pick the
+ * shape per call: for a batch that is resident at once the one that loads the
+ * fullest SM least, else the one with the most resident chains per SM; and at
+ * 32 threads per chain, in batches that leave warps idle, chains that have a
+ * whole block of 8 or 4 warps each (all of the batch, or its largest ligands
+ * beside the others), with the results of one warp.  A shape set here is used
+ * as it is: one warp (or team) per chain throughout.  The chains of one block
  * share one copy of their ligand's model. */
 int sg_set_chains_per_block(sg_engine* e, int n);
 
@@ -419,8 +430,11 @@ int sg_set_chains_per_block(sg_engine* e, int n);
  * loop (sg_serve_*) reads the setting at each upload; with 0 it picks, per
  * upload, the most at which the work items already on the device and the
  * new batch's all have a block (each result reports its value).  FP64
- * engines ignore it: the plain path runs one warp per chain.
- * sg_threads_per_chain reports the setting and the last batch's value. */
+ * engines ignore it: the plain path picks 8, 4 or 1 warps per item by the
+ * batch, with the same results.
+ * sg_threads_per_chain reports the setting and the last batch's value; chains
+ * that had a whole block (sg_batch_blocks) count as 32 there, whose results
+ * they have. */
 int sg_set_threads_per_chain(sg_engine* e, int threads);
 int sg_threads_per_chain(const sg_engine* e, int* configured, int* last_batch);
 

@@ -190,8 +190,8 @@ public:
               s.threads_per_chain == 128))
             throw std::runtime_error("threads_per_chain: 0 (automatic), 32, 64 or 128");
         if (s.fp64 && s.threads_per_chain > 32)
-            throw std::runtime_error("threads_per_chain above 32 needs the FP32 search (the FP64 path runs one warp "
-                                     "per chain, bit for bit as the CPU search)");
+            throw std::runtime_error("threads_per_chain above 32 needs the FP32 search (the FP64 path picks its "
+                                     "warps per chain itself, bit for bit as the CPU search)");
         if (s.skip_visited && !s.fp64)
             throw std::runtime_error("skip_visited needs the double precision search (fp64)");
         for (size_t i = 0; i < s.devices.size(); i++) {

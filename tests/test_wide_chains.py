@@ -1,7 +1,8 @@
 """Chains on several warps each (batches that leave warps idle) against the
 search of one warp per chain, bit for bit: batches whose chains get 8 and 4 warps
 on a B200 (296 and 592 resident blocks) and some past them, a model without
-pairs, flexible residues, and charge-dependent tables."""
+pairs, flexible residues, and charge-dependent tables; and local optimisations
+on several warps against one."""
 import numpy as np
 import pytest
 
@@ -66,4 +67,43 @@ def test_wide_optimisations_equal_one_warp(scoring, lig, flex, prec):
         parts = [eng.bfgs(0, m, confs[k:min(k + size, last)]) for k in range(0, last, size)]
         assert np.array_equal(np.concatenate([c for c, _ in parts]), one[0][:last]), size
         assert np.array_equal(np.concatenate([e for _, e in parts]), one[1][:last]), size
+    eng.close()
+
+
+# ligands with their chains -> warps of the blocks, ligands that get them, and chains
+# per block (148 SMs; two resident 8-warp or four 4-warp blocks on each)
+SMALL, MIDDLE, LARGE = (12, 2, 2), (24, 5, 11), (50, 12, 3)
+PLANS = [([(MIDDLE, 8)], (8, 1, 1)), ([(MIDDLE, 500)], (4, 1, 1)), ([(SMALL, 1300)], (0, 0, 1)),
+         ([(LARGE, 20), (MIDDLE, 100), (SMALL, 900)], (8, 1, 8)),
+         ([(LARGE, 300), (MIDDLE, 300), (SMALL, 600)], (4, 1, 4))]
+
+
+@pytest.mark.parametrize("early", [False, True])
+@pytest.mark.parametrize("ligs,plan", PLANS)
+def test_each_plan_equals_one_warp(ligs, plan, early):
+    """Blocks for all chains, for none and for the largest ligand beside the
+    others' warps, in one search and in phases that resume (early stop, which
+    here stops no ligand): the plan, and the bits of one warp per chain."""
+    eng = sb.Engine(0, sb.PREC_FP32)
+    eng.set_tables(W.tables())
+    eng.set_receptor(0, W.receptor(1500, 3), W.box(26.0))
+    models = [W.ligand(*lig) for lig, _ in ligs]
+    jobs = [sb.LigandJob(model=k, num_chains=n, num_steps=6, maxiters=0, seed=9, ligand_key=k)
+            for k, (_, n) in enumerate(ligs)]
+    p = models[0].search_params()
+    if early:
+        eng.set_early_stop(checkpoints=3, first=1, fraction=1.0, eps=0.0)
+    runs = []
+    for shape in (0, 8):
+        eng.set_chains_per_block(shape)
+        r = eng.dock_batch(0, models, jobs, p, refine=False)
+        runs.append((r, eng.batch_stats()))
+    (wide, sw), (one, so) = runs
+    assert (sw["block_warps"], sw["block_ligands"], sw["chains_per_block"]) == plan
+    assert (so["block_warps"], so["block_ligands"], so["chains_per_block"]) == (0, 0, 8)
+    assert sw["pair_lookups"] == so["pair_lookups"] > 0 and sw["grid_lookups"] == so["grid_lookups"] > 0
+    for a, b in zip(wide, one):
+        assert a["evals"] == b["evals"] > 0 and len(a["e"]) > 0
+        for k in ("e", "conf", "coords"):
+            assert np.array_equal(a[k], b[k]), k
     eng.close()
