@@ -633,21 +633,30 @@ int sg_autotune32(sg_engine* e, int rid, const sg_model_desc* models, int nmodel
     for (int j = 0; j < njobs; j++)
         res[j] = {0, &se[(size_t)j * S], &sc[(size_t)j * S * max_conf], &sx[(size_t)j * S * max_heavy * 3], 0};
     double best = -1;
-    int best_c = 0;
-    for (int i = 0; i < 4; i++) {
-        if (evals_per_s) evals_per_s[i] = 0;
-        e->force_wpb = cands[i];
+    int best_c = 0, kept = keep;
+    for (int i = 0; i < 5; i++) {  // the shapes, then what sg_dock_batch32 picks by itself
+        const bool automatic = i == 4;
+        if (!automatic && evals_per_s) evals_per_s[i] = 0;
+        e->force_wpb = automatic ? 0 : cands[i];
         const int rc = sg_dock_batch32(e, rid, models, nmodels, sample.data(), njobs, p, 0, res.data());
         if (rc != SG_OK && rc != SG_ERR_ARG) {  // a device error ends the search; the shape stays as it was
             e->force_wpb = keep;
             return rc;
         }
-        if (rc != SG_OK || e->last_wpb != cands[i] || e->last_mc_ms <= 0) continue;  // shape not possible here
+        const int c = e->last_wpb;
+        if (rc != SG_OK || (!automatic && c != cands[i]) || e->last_mc_ms <= 0) continue;  // shape not possible here
         const double v = (double)e->last_evals / (e->last_mc_ms * 1e-3);
-        if (evals_per_s) evals_per_s[i] = v;
-        if (v > best) { best = v; best_c = cands[i]; }
+        if (v > best) {
+            best = v;
+            best_c = c;
+            kept = automatic ? 0 : c;
+            if (evals_per_s) evals_per_s[std::find(cands, cands + 4, c) - cands] = v;
+        } else if (automatic && c == best_c && e->last_block_ligands == 0) {
+            kept = 0;  // the same launch as the fastest shape's
+        }
+        if (!automatic && evals_per_s) evals_per_s[i] = v;
     }
-    e->force_wpb = best_c ? best_c : keep;
+    e->force_wpb = kept;
     if (chosen) *chosen = best_c;
     if (!best_c) {
         e->err = "autotune: no launch shape ran (" + e->err + ")";

@@ -726,8 +726,9 @@ class Engine:
             self._check(load().sg_set_early_stop(self._h, C.cast(C.byref(es), C.c_void_p)))
 
     def autotune(self, rid, models, jobs, params: MCParams, step_fraction=0.01):
-        """Times the search at 8, 4, 2 and 1 chains per block on ``jobs`` with
-        scaled step counts and keeps the fastest shape (sg_autotune32).
+        """Times the search at 8, 4, 2 and 1 chains per block and at the automatic
+        launch shape on ``jobs`` with scaled step counts and keeps the fastest
+        (sg_autotune32).
         Returns (chosen, {shape: eval_deriv calls per second})."""
         descs = (ModelDesc * len(models))(*[m.desc for m in models])
         J = (LigandJob * len(jobs))(*jobs)

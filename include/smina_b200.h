@@ -440,11 +440,14 @@ int sg_threads_per_chain(const sg_engine* e, int* configured, int* last_batch);
 
 /* Launch-shape autotuner for the search kernel: runs the given jobs with
  * their step counts scaled by step_fraction (0 < f <= 1, at least one step
- * each; no refinement) once per shape of 8, 4, 2 and 1 chains per block,
- * times each search launch with CUDA events and keeps the fastest shape
- * (as sg_set_chains_per_block would).  evals_per_s[4] (may be null) gets
+ * each; no refinement) once per shape of 8, 4, 2 and 1 chains per block and
+ * once as sg_dock_batch32 launches them by itself, times each search launch
+ * with CUDA events and keeps the fastest (as sg_set_chains_per_block would,
+ * with 0 for the automatic launch).  evals_per_s[4] (may be null) gets
  * each shape's eval_deriv calls per second, 0 for a shape that cannot run;
- * *chosen the shape kept.  Results of later calls do not depend on the
+ * *chosen the chains per block of what is kept.  When that is the automatic
+ * launch, both are those that sg_batch_stats gives for it (1 when every chain
+ * has a whole block).  Results of later calls do not depend on the
  * shape.  The reference picks its launch shape (threads per chain) from the
  * occupancy calculator alone: Residency / mc_residency,
  * src/gpu/gpu_kernels.h:70-88. */

@@ -107,3 +107,23 @@ def test_each_plan_equals_one_warp(ligs, plan, early):
         for k in ("e", "conf", "coords"):
             assert np.array_equal(a[k], b[k]), k
     eng.close()
+
+
+def test_autotune_keeps_the_automatic_launch_where_it_is_fastest():
+    """A lone ligand's chains are fastest on a block each (50 heavy atoms: about
+    half the time of one warp per chain), which is what sg_dock_batch32 does by
+    itself: tuning must not turn that off."""
+    eng = sb.Engine(0, sb.PREC_FP32)
+    eng.set_tables(W.tables())
+    eng.set_receptor(0, W.receptor(1500, 3), W.box(26.0))
+    m = W.ligand(*LARGE)
+    jobs = [sb.LigandJob(model=0, num_chains=8, num_steps=40, maxiters=0, seed=9, ligand_key=1)]
+    p = m.search_params()
+    chosen, rates = eng.autotune(0, [m], jobs, p, step_fraction=0.5)
+    assert chosen == 1 and rates[1] == max(rates.values())
+    tuned = eng.dock_batch(0, [m], jobs, p, refine=False)
+    assert eng.batch_stats()["block_warps"] == 8
+    eng.set_chains_per_block(1)
+    one = eng.dock_batch(0, [m], jobs, p, refine=False)
+    assert eng.batch_stats()["block_warps"] == 0 and np.array_equal(tuned[0]["conf"], one[0]["conf"])
+    eng.close()
