@@ -981,7 +981,7 @@ static void pack_one(const sg_model_desc& d, PackFor what, std::vector<int>& I, 
         pv(ps);
         // the same pairs per movable atom: chunk by chunk, in a chunk the atom's
         // pair as first atom before the one as second
-        std::vector<int> wstart, wwords;
+        hm.wstart = nullptr;
         if (what == kPackWide && packable && hm.npchunks <= kWideChunks) {
             std::vector<std::vector<uint16_t>> of(M);
             for (size_t c = 0; c < slots.size(); c += 32)
@@ -992,17 +992,17 @@ static void pack_one(const sg_model_desc& d, PackFor what, std::vector<int>& I, 
                         if (a < M) of[a].push_back((uint16_t)(k << 1 | role));
                     }
             std::vector<uint16_t> wlist;
+            std::vector<int> wide;
             for (int i = 0; i < M; i++) {
-                wstart.push_back((int)wlist.size());
+                wide.push_back((int)wlist.size());
                 wlist.insert(wlist.end(), of[i].begin(), of[i].end());
             }
-            wstart.push_back((int)wlist.size());
-            wwords.resize((wlist.size() + 1) / 2);
-            if (!wlist.empty()) std::memcpy(wwords.data(), wlist.data(), wlist.size() * sizeof(uint16_t));
+            wide.push_back((int)wlist.size());
+            wide.resize(M + 1 + (wlist.size() + 1) / 2);
+            if (!wlist.empty()) std::memcpy(&wide[M + 1], wlist.data(), wlist.size() * sizeof(uint16_t));
+            hm.wstart = reinterpret_cast<const int*>(1);  // placed with the pools
+            pv(wide);
         }
-        hm.wstart = wstart.empty() ? nullptr : reinterpret_cast<const int*>(1);  // placed with the pools
-        pv(wstart);
-        pv(wwords);
     }
     auto pf4 = [&](const double* xyz, const double* w4, size_t n) {
         foff.push_back(Fl.size());
@@ -1111,9 +1111,7 @@ static void place_pools(const PackedPools& P, std::vector<DModel>& host, char* d
         size_t j = 0;
         for (const int** q : ip) *q = ib + io[j++];
         h.pslot = h.npchunks >= 0 ? reinterpret_cast<const uint32_t*>(ib + io[j]) : nullptr;
-        const bool wide = h.wstart != nullptr;
-        h.wstart = wide ? ib + io[j + 1] : nullptr;
-        h.wlist = wide ? reinterpret_cast<const uint16_t*>(ib + io[j + 2]) : nullptr;
+        if (h.wstart) h.wstart = ib + io[j + 1];
         const float4** fp[] = {&h.local32, &h.lab32, &h.forigin32, &h.faxis32, &h.finit32};
         for (j = 0; j < fo.size(); j++) *fp[j] = reinterpret_cast<const float4*>(fb + fo[j]);
         const double** dp[] = {&h.charge, &h.local, &h.lab, &h.forigin, &h.faxis, &h.finit};

@@ -739,8 +739,9 @@ __device__ __forceinline__ void stage_wide32(int base) {
     SG_ROLLED
     for (int i = threadIdx.x; i <= g.nmov; i += blockDim.x) start[i] = g.wstart[i];
     const int n = g.wstart[g.nmov];
+    const uint16_t* wlist = reinterpret_cast<const uint16_t*>(g.wstart + g.nmov + 1);
     SG_ROLLED
-    for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = g.wlist[i];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) list[i] = wlist[i];
     __syncthreads();
 }
 

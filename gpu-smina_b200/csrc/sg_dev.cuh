@@ -136,12 +136,12 @@ struct __align__(16) DModel {
     const uint32_t* pslot;    // [npchunks * 32]
     int cost;                 // relative cost of one evaluation (atoms + pairs + frames)
     int npchunks;
-    // the schedule seen from the atoms, for chains on several warps: movable atom
-    // i's pairs are wlist[wstart[i] .. wstart[i + 1]), each slot << 1 | (the atom
-    // is the second one), in the order in which one warp adds them.  Null when
-    // not packed (kWideChunks, or callers that do not use it).
-    const int* wstart;        // [nmov + 1]
-    const uint16_t* wlist;
+    // the schedule seen from the atoms, for chains on several warps: where each
+    // movable atom's list starts and the last one ends, then the lists as 16-bit
+    // words, each slot << 1 | (the atom is the second one), in the order in which one
+    // warp adds the pairs.  Null when not packed (kWideChunks, or callers that
+    // do not use it).
+    const int* wstart;        // [nmov + 1], then uint16_t[wstart[nmov]]
 };
 constexpr int kWideChunks = 1024;  // the most chunks whose slots fit 15 bits
 

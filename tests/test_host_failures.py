@@ -297,3 +297,25 @@ for lig, n, w in ((NONE, 1, 8), (NONE, 296, 8), (NONE, 592, 4), (NONE, 593, 1), 
                   (LARGE, 5920, 8), (LARGE, 5921, 1)):
     assert warps(lig, n) == w, (lig, n, w, warps(lig, n))
 """)
+
+
+def test_batches_at_the_fixed_scratch_arrays_limit(run):
+    """The largest batches that sg_dock_batch32_noalloc has taken still fit its
+    8 MiB (3,757 ligands of 10 atoms, 209 of 24 with 8 chains of 9 places), the
+    next larger ones do not."""
+    run("""
+e = engine()
+def fits(lig, models, chains, places):
+    q = W.ligand(*lig)
+    e.build_grids(0, sorted({t for t in q.types() if 1 < t < 27}))
+    p = q.search_params()
+    p.num_saved_mins = places
+    jobs = [sb.LigandJob(model=k, num_chains=chains, num_steps=1, maxiters=0, seed=1, ligand_key=k) for k in range(models)]
+    try:
+        e.dock_batch_noalloc(0, [q] * models, jobs, p)
+    except sb.SminaError as x:  # (no kernel has written the results)
+        return "corrupt" in str(x)
+    return True
+for lig, models, chains, places in (((10, 0, 4), 3757, 1, 1), ((24, 5, 11), 209, 8, 9), ((50, 12, 3), 219, 1, 1)):
+    assert fits(lig, models, chains, places) and not fits(lig, models + 1, chains, places), lig
+""")
