@@ -359,7 +359,8 @@ int sg_create(int device, int precision, sg_engine** out) {
     if (precision < SG_PREC_FP64 || precision > SG_PREC_FP32_H16) return SG_ERR_ARG;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) return SG_ERR_CUDA;
-    std::unique_ptr<sg_engine> e(new sg_engine());
+    std::unique_ptr<sg_engine> e(new (std::nothrow) sg_engine());
+    if (!e) return SG_ERR_NOMEM;
     e->device = device;
     e->precision = precision;
     int rc = guarded(e.get(), [&] {

@@ -616,53 +616,51 @@ int sg_set_chains_per_block(sg_engine* e, int n) {
 int sg_autotune32(sg_engine* e, int rid, const sg_model_desc* models, int nmodels, const sg_ligand_job* jobs, int njobs,
                   const sg_mc_params* p, double step_fraction, double* evals_per_s, int* chosen) {
     if (!e || !jobs || !p || njobs <= 0 || !(step_fraction > 0 && step_fraction <= 1)) return SG_ERR_ARG;
-    const int cands[4] = {8, 4, 2, 1};
-    const int keep = e->force_wpb;
-    // the sample: every job with its step count scaled (at least one step)
-    std::vector<sg_ligand_job> sample(jobs, jobs + njobs);
-    for (auto& j : sample) j.num_steps = std::max(1, (int)(j.num_steps * step_fraction));
-    const int S = p->num_saved_mins;
-    int max_conf = 1, max_heavy = 1;
-    for (int k = 0; k < nmodels && models; k++) {
-        max_conf = std::max(max_conf, models[k].conf_size);
-        max_heavy = std::max(max_heavy, models[k].num_movable);  // bounds the heavy atoms
-    }
-    std::vector<double> se((size_t)njobs * std::max(S, 1)), sc((size_t)njobs * std::max(S, 1) * max_conf),
-        sx((size_t)njobs * std::max(S, 1) * max_heavy * 3);
-    std::vector<sg_ligand_result> res(njobs);
-    for (int j = 0; j < njobs; j++)
-        res[j] = {0, &se[(size_t)j * S], &sc[(size_t)j * S * max_conf], &sx[(size_t)j * S * max_heavy * 3], 0};
-    double best = -1;
-    int best_c = 0, kept = keep;
-    for (int i = 0; i < 5; i++) {  // the shapes, then what sg_dock_batch32 picks by itself
-        const bool automatic = i == 4;
-        if (!automatic && evals_per_s) evals_per_s[i] = 0;
-        e->force_wpb = automatic ? 0 : cands[i];
-        const int rc = sg_dock_batch32(e, rid, models, nmodels, sample.data(), njobs, p, 0, res.data());
-        if (rc != SG_OK && rc != SG_ERR_ARG) {  // a device error ends the search; the shape stays as it was
-            e->force_wpb = keep;
-            return rc;
+    return guarded(e, [&] {
+        const int cands[4] = {8, 4, 2, 1};
+        const int keep = e->force_wpb;
+        // the sample: every job with its step count scaled (at least one step)
+        std::vector<sg_ligand_job> sample(jobs, jobs + njobs);
+        for (auto& j : sample) j.num_steps = std::max(1, (int)(j.num_steps * step_fraction));
+        const int S = p->num_saved_mins;
+        int max_conf = 1, max_heavy = 1;
+        for (int k = 0; k < nmodels && models; k++) {
+            max_conf = std::max(max_conf, models[k].conf_size);
+            max_heavy = std::max(max_heavy, models[k].num_movable);  // bounds the heavy atoms
         }
-        const int c = e->last_wpb;
-        if (rc != SG_OK || (!automatic && c != cands[i]) || e->last_mc_ms <= 0) continue;  // shape not possible here
-        const double v = (double)e->last_evals / (e->last_mc_ms * 1e-3);
-        if (v > best) {
-            best = v;
-            best_c = c;
-            kept = automatic ? 0 : c;
-            if (evals_per_s) evals_per_s[std::find(cands, cands + 4, c) - cands] = v;
-        } else if (automatic && c == best_c && e->last_block_ligands == 0) {
-            kept = 0;  // the same launch as the fastest shape's
+        std::vector<double> se((size_t)njobs * std::max(S, 1)), sc((size_t)njobs * std::max(S, 1) * max_conf),
+            sx((size_t)njobs * std::max(S, 1) * max_heavy * 3);
+        std::vector<sg_ligand_result> res(njobs);
+        for (int j = 0; j < njobs; j++)
+            res[j] = {0, &se[(size_t)j * S], &sc[(size_t)j * S * max_conf], &sx[(size_t)j * S * max_heavy * 3], 0};
+        double best = -1;
+        int best_c = 0, kept = keep;
+        for (int i = 0; i < 5; i++) {  // the shapes, then what sg_dock_batch32 picks by itself
+            const bool automatic = i == 4;
+            if (!automatic && evals_per_s) evals_per_s[i] = 0;
+            e->force_wpb = automatic ? 0 : cands[i];
+            const int rc = sg_dock_batch32(e, rid, models, nmodels, sample.data(), njobs, p, 0, res.data());
+            if (rc != SG_OK && rc != SG_ERR_ARG) {  // a device error ends the search; the shape stays as it was
+                e->force_wpb = keep;
+                throw EngineError(rc, std::string(e->err));
+            }
+            const int c = e->last_wpb;
+            if (rc != SG_OK || (!automatic && c != cands[i]) || e->last_mc_ms <= 0) continue;  // shape not possible here
+            const double v = (double)e->last_evals / (e->last_mc_ms * 1e-3);
+            if (v > best) {
+                best = v;
+                best_c = c;
+                kept = automatic ? 0 : c;
+                if (evals_per_s) evals_per_s[std::find(cands, cands + 4, c) - cands] = v;
+            } else if (automatic && c == best_c && e->last_block_ligands == 0) {
+                kept = 0;  // the same launch as the fastest shape's
+            }
+            if (!automatic && evals_per_s) evals_per_s[i] = v;
         }
-        if (!automatic && evals_per_s) evals_per_s[i] = v;
-    }
-    e->force_wpb = kept;
-    if (chosen) *chosen = best_c;
-    if (!best_c) {
-        e->err = "autotune: no launch shape ran (" + e->err + ")";
-        return SG_ERR_ARG;
-    }
-    return SG_OK;
+        e->force_wpb = kept;
+        if (chosen) *chosen = best_c;
+        require(best_c, "autotune: no launch shape ran (" + e->err + ")");
+    });
 }
 
 }  // extern "C"

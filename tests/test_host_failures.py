@@ -164,7 +164,8 @@ assert status(e.build_grids, 0, HEAVY) == sb.SG_OK
 """)
 
 
-@pytest.mark.parametrize("call", ["score", "minimize", "dock", "dock_batch", "eval", "bfgs", "set_receptor", "build_grids"])
+@pytest.mark.parametrize("call", ["score", "minimize", "dock", "dock_batch", "eval", "bfgs", "set_receptor", "build_grids",
+                                  "create", "autotune"])
 def test_host_allocation_failures_are_statuses(run, call):
     """The nth host allocation of a call fails, for every n: the call returns
     SG_ERR_NOMEM (or does without), the process goes on and the next call works."""
@@ -182,7 +183,9 @@ f = {"score": lambda: e.score(0, ms, pm, confs), "minimize": lambda: e.minimize(
      "dock_batch": lambda: e.dock_batch(0, ms, [sb.LigandJob(model=k, num_chains=2, num_steps=2, maxiters=0, seed=1,
                                                              ligand_key=k) for k in pm], p),
      "eval": lambda: e.eval(0, ms[0], x[:1]), "bfgs": lambda: e.bfgs(0, ms[0], x[:1]),
-     "set_receptor": lambda: e.set_receptor(0, R, gd),
+     "set_receptor": lambda: e.set_receptor(0, R, gd), "create": lambda: sb.Engine(0, sb.PREC_FP32).close(),
+     "autotune": lambda: e.autotune(0, ms, [sb.LigandJob(model=0, num_chains=2, num_steps=2, maxiters=0, seed=1,
+                                                         ligand_key=0)], p, 1.0),
      "build_grids": lambda: (e.set_receptor(0, R, gd), e.build_grids(0, HEAVY))}[call]
 assert status(f) == sb.SG_OK
 n, failed = 0, 0
@@ -195,7 +198,7 @@ while True:
     failed += rc == sb.SG_ERR_NOMEM
     if call in ("set_receptor", "build_grids"): e.set_receptor(0, R, gd)
     if n % 16 == 0: assert status(f) == sb.SG_OK
-assert failed > 10 and status(f) == sb.SG_OK
+assert failed > (1 if call == "create" else 10) and status(f) == sb.SG_OK
 """)
 
 
