@@ -25,12 +25,13 @@
 //    forces and the first warp walks the tree back.
 // Measured on one B200 against one warp per item with everything read from
 // global memory and lane 0 adding the sums, with calls: refinement of 1,890 poses
-// of 210 ligands 270 -> 29 ms, of 9 poses of one ligand 7.3 -> 1.2 ms; 8 chains of 40
-// steps 87 -> 59 ms; kernels alone: rescoring of 2,000 poses 0.54 -> 0.20 ms, 1,500
-// charge-dependent evaluations 126 -> 84 us.  Bits unchanged.  What is left of an
+// of 210 ligands 197 -> 21 ms, of 9 poses of one ligand 6.3 -> 1.1 ms; 8 chains of 40
+// steps 78 -> 62 ms; kernels alone: rescoring of 2,000 poses 0.54 -> 0.18 ms, 1,500
+// charge-dependent evaluations 126 -> 77 us.  Bits unchanged.  What is left of an
 // evaluation is the leader's instructions, about 3,400 of them at 7 to 8 cycles each
-// (frames, tree derivative, BFGS); four lanes per frame and one per frame and
-// component took more instructions and were slower.
+// (frames, tree derivative, BFGS); four lanes per frame (6,500 -> 9,100 cycles an
+// evaluation) and one per frame and component (5,900 -> 7,400) took more
+// instructions.
 // The first warp, the leader, runs the chain (BFGS, line searches, mutation)
 // and calls the others in for each evaluation: two numbers of warps (4 and 8)
 // by the number of items, plus one warp with nothing staged for models whose

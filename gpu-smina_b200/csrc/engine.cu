@@ -66,7 +66,7 @@ void pool_release(int device) {
 // A receptor's maps that new tables, a user grid or another receptor in its place
 // make void: their allocations wait here for the next map build in that place,
 // which takes one that fits and frees the others (18 maps of a 22 A box with a new
-// user grid 22 ms of cudaFree and cudaMalloc otherwise, 0.7 ms so).  At most
+// user grid 22 ms of cudaFree and cudaMalloc otherwise, 0.7 to 1.2 ms so).  At most
 // kDroppedKept bytes per device, the oldest freed first; a direct sum in that
 // place frees them too, and an allocation that fails frees all on its device.
 struct DroppedMaps {
