@@ -211,11 +211,13 @@ __device__ __forceinline__ bool within64(double margin) {
 // Poses are taken in groups of `group`: all distances of a group's poses to the
 // list and to one another at once, one thread each (a pose's squares added in
 // order, as the host merge does in double precision), then the first warp takes
-// the poses one by one with what D holds.  Bound by the latency of both.  For
-// 1,000 chains of one 24-atom ligand (9 poses kept, search 36 ms) a call took 48 ms on
-// one B200, for 512 chains of a 10-atom one with up to 1,000 poses kept 161 ms; with one
-// warp that measured each pose when its turn came, and one lane that moved the
-// list, 63 and 500 ms.
+// the poses one by one with what D holds.  Once the list is full, poses no better
+// than its last one are left out of the groups: they would change nothing.  Bound
+// by latency.  For 1,000 chains of one 24-atom ligand (9 poses kept, search 36 ms) a
+// call took 37 ms on one B200, for 512 chains of a 10-atom one with up to 1,000 poses
+// kept (search 8 ms) 95 ms; without leaving poses out 48 and 161, and with one warp that
+// measured each pose when its turn came, and one lane that moved the list, 63 and
+// 500 ms.
 __host__ __device__ constexpr size_t merge32_bytes(int S, int group) {
     return (size_t)S * (sizeof(double) + sizeof(int2) + sizeof(int)) +
            (size_t)group * (sizeof(double) + sizeof(int2) + (S + group) * sizeof(double)) + 16;
@@ -238,21 +240,53 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge32(const DModel* models,
     const MergeJob32 job = jobs[j];
     const int H = models[job.model].nheavy, H3 = 3 * H, cs = models[job.model].conf_size;
     auto coords = [&](int2 q) { return chains[q.x].out_coords + (size_t)q.y * H3; };
-    int n = 0, c = job.first, i = 0;  // the list's length (all threads); the next pose's chain and rank (first warp)
+    int n = 0;  // the list's length
+    // the first warp's place among the chains: of chains [base, base + 32) those in
+    // `todo` are left, the first of them from its pose i on
+    const int end = job.first + job.count;
+    int base = job.first - 32, i = 0;
+    unsigned todo = 0;
+    bool nan = false;  // the list holds a NaN, or has
     for (;;) {
         if (tid < 32) {  // the next group
+            // a pose that is no better than the last one of a full list changes nothing
+            const bool full = n == S && !nan;
+            const double worst = full ? le[S - 1] : 0;
             int taken = 0;
-            while (taken < group && c < job.first + job.count) {
+            while (taken < group) {
+                if (!todo) {  // a chain per lane: has it any pose to offer?
+                    base += 32;
+                    if (base >= end) break;
+                    bool some = false;
+                    if (base + lane < end) {
+                        const Chain32& ch = chains[base + lane];
+                        const int cnt = min(max(*ch.out_count, 0), S);
+                        some = cnt > 0 && !full;
+                        if (full)
+                            for (int k = 0; k < cnt && !some; k++)
+                                some = !(ch.out_e[min(max(ch.out_order[k], 0), S - 1)] >= worst);
+                    }
+                    todo = __ballot_sync(kFull, some);
+                    continue;
+                }
+                const int c = base + __ffs(todo) - 1;
                 const Chain32& ch = chains[c];
                 const int cnt = min(max(*ch.out_count, 0), S), k = min(min(cnt - i, group - taken), 32);
+                int slot = 0;
+                double e = 0;
                 if (lane < k) {
-                    const int slot = min(max(ch.out_order[i + lane], 0), S - 1);
-                    at_group[taken + lane] = make_int2(c, slot);
-                    ge[taken + lane] = ch.out_e[slot];
+                    slot = min(max(ch.out_order[i + lane], 0), S - 1);
+                    e = ch.out_e[slot];
                 }
-                taken += k;
+                const unsigned mask = __ballot_sync(kFull, lane < k && !(full && e >= worst));
+                if (mask >> lane & 1) {
+                    const int at = taken + __popc(mask & ((1u << lane) - 1));
+                    at_group[at] = make_int2(c, slot);
+                    ge[at] = e;
+                }
+                taken += __popc(mask);
                 i += k;
-                if (i >= cnt) { c++; i = 0; }
+                if (i >= cnt) { todo &= todo - 1; i = 0; }
             }
             if (lane == 0) s_taken = taken;
         }
@@ -305,6 +339,7 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge32(const DModel* models,
                 }
                 __syncwarp();
                 if (at < 0) continue;
+                nan |= e != e;
                 // sorted in behind the last energy before `at` that is not above its own
                 int k = 0;
                 for (int b = at - 1; b >= 0; b -= 32) {

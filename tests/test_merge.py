@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("lig,chains,places,steps", [
     ((10, 0, 4), 1, 1, 20), ((24, 5, 11), 33, 1, 10), ((24, 5, 11), 200, 9, 20), ((12, 2, 2), 100, 33, 60),
-    ((10, 0, 4), 40, 130, 120), ((10, 0, 4), 25, 200, 300), ((10, 0, 4), 20, 1024, 400)])
+    ((12, 2, 2), 1500, 9, 8), ((10, 0, 4), 40, 130, 120), ((10, 0, 4), 25, 200, 300), ((10, 0, 4), 20, 1024, 400)])
 def test_merge_equals_the_hosts(lig, chains, places, steps):
     eng = sb.Engine(0, sb.PREC_FP32)
     eng.set_tables(W.tables())
