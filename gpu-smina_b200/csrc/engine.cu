@@ -177,7 +177,8 @@ static void drop_pin_rings() {
 PinRing::~PinRing() {
     for (cudaEvent_t x : ev)
         if (x) cudaEventDestroy(x);
-    if (p) cudaFreeHost(p);
+    if (pinned) cudaFreeHost(p);
+    else delete[] p;
 }
 static std::unique_ptr<PinRing> ring_get() {
     {
@@ -189,7 +190,13 @@ static std::unique_ptr<PinRing> ring_get() {
         }
     }
     auto r = std::make_unique<PinRing>();
-    cuda_check(cudaHostAlloc((void**)&r->p, PinRing::kSlot * PinRing::kSlots, cudaHostAllocPortable), "pinned memory");
+    constexpr size_t n = PinRing::kSlot * PinRing::kSlots;
+    r->pinned = cudaHostAlloc((void**)&r->p, n, cudaHostAllocPortable) == cudaSuccess;
+    if (!r->pinned) {
+        cudaGetLastError();
+        r->p = nullptr;
+        r->p = new char[n];
+    }
     return r;
 }
 // As many free rings are kept as the process has engines (a call at a time on
@@ -203,7 +210,7 @@ static void ring_put(std::unique_ptr<PinRing> r) {
     }
     std::lock_guard<std::mutex> lk(g_rings_mu);
     try {
-        if (g_rings.size() < g_engines) g_rings.push_back(std::move(r));
+        if (r->pinned && g_rings.size() < g_engines) g_rings.push_back(std::move(r));
     } catch (std::bad_alloc&) {  // not kept then (callers are destructors)
     }
 }

@@ -58,6 +58,7 @@ struct PinRing {
     static constexpr size_t kSlot = size_t(512) << 10;
     static constexpr int kSlots = 4;  // two for inputs, two for outputs
     char* p = nullptr;
+    bool pinned = false;  // else, where none could be had, pageable: copies through it then wait
     cudaEvent_t ev[kSlots] = {};
     ~PinRing();
 };

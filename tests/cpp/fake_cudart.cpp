@@ -31,7 +31,7 @@ State& st() {
     return *s;
 }
 size_t limit = size_t(8) << 30, live = 0, kept = 0;  // live: allocated; kept: freed but held by the pools
-std::atomic<int> host_allocs{0}, sync_ms{0}, attr_ms{0};
+std::atomic<int> host_allocs{0}, no_pinned{0}, sync_ms{0}, attr_ms{0};
 thread_local long new_countdown = 0;
 thread_local bool new_fired = false;
 struct Held {  // the runtime's own state: locked, and its allocations not counted
@@ -93,6 +93,7 @@ int fake_dangling() {  // pointers to freed blocks in live ones of at most 4 KB
     return n;
 }
 int fake_host_allocs() { return host_allocs; }
+void fake_no_pinned(int none) { no_pinned = none; }
 void fake_sync_ms(int ms) { sync_ms = ms; }
 void fake_attr_ms(int ms) { attr_ms = ms; }
 void fake_fail_new(long nth) { new_countdown = nth; new_fired = false; }
@@ -196,7 +197,13 @@ cudaError_t cudaMemPoolDestroy(cudaMemPool_t) { Held held; kept = 0; return cuda
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { Held held; kept = 0; return cudaSuccess; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = limit - live - kept; *t = limit; return cudaSuccess; }
-cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { host_allocs++; *p = std::malloc(n); return cudaSuccess; }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+    *p = nullptr;
+    if (no_pinned) return cudaErrorMemoryAllocation;
+    host_allocs++;
+    *p = std::malloc(n);
+    return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { *d = h; return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }

@@ -319,3 +319,17 @@ def fits(lig, models, chains, places):
 for lig, models, chains, places in (((10, 0, 4), 3757, 1, 1), ((24, 5, 11), 209, 8, 9), ((50, 12, 3), 219, 1, 1)):
     assert fits(lig, models, chains, places) and not fits(lig, models + 1, chains, places), lig
 """)
+
+
+def test_calls_do_without_pinned_memory(run):
+    """Where no memory can be pinned, engines are created and calls copy all the same."""
+    run("""
+fake.fake_no_pinned(1)
+e = engine()
+x = W.random_confs(m, gd, 30000, 1)
+assert status(e.eval, 0, m, x) == sb.SG_OK and fake.fake_host_allocs() == 0
+c, _ = e.bfgs(0, m, x)  # (no kernel changes them: out and back)
+assert np.array_equal(c, x)
+fake.fake_no_pinned(0)
+assert status(e.eval, 0, m, x) == sb.SG_OK and fake.fake_host_allocs() == 1
+""")
